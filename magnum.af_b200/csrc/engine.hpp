@@ -185,6 +185,8 @@ class Demag {
     template <typename R> cplx_t<R>* S1();
     template <typename R> cplx_t<R>* S2();
     void build_tensor(cudaStream_t st);
+    void transform_octant(const double* oct, int comp, int Lx, int Ly, int Lz, double* quad, double scale, DevBuf* work,
+                          cudaStream_t st);
 
     MeshDims md_;
     bool pbc_ = false;
@@ -244,9 +246,10 @@ void eval_terms(const std::vector<Term*>& terms, const MeshDims& md, const R* m,
 void stage_m32(const double* m64, float* m32, int64_t n, cudaStream_t st);
 void widen_m(const float* m32, double* m64, int64_t n, cudaStream_t st);  // FP32 -> FP64, exact
 
-// Newell tensor on the padded grid, one component [Pz][Py][Px] (newell.cu);
-// symmetric = true gives the parity-exact tensor the spectral pipeline uses.
-void newell_component(double* out, int comp, const MeshDims& md, int Px, int Py, int Pz, bool symmetric,
-                      cudaStream_t st);
+// Newell tensor on the padded grid, one component [Pz][Py][Px], as the reference
+// assembles it, and its entries at the offsets 0 <= j < (o0, o1, o2), [o2][o1][o0]
+// (newell.cu).
+void newell_component(double* out, int comp, const MeshDims& md, int Px, int Py, int Pz, cudaStream_t st);
+void newell_octant(double* out, int comp, const MeshDims& md, int o0, int o1, int o2, cudaStream_t st);
 
 }  // namespace mafb

@@ -257,15 +257,91 @@ void stage_m32(const double* m64, float* m32, int64_t n, cudaStream_t st) {
     MAF_LAUNCH_CHECK();
 }
 
-// Extract the real part of the spectral tensor on the stored quadrant.
-__global__ void k_reduce_tensor(const double2* __restrict__ spec, double* __restrict__ dst, int nxh, int pitch, int Py,
-                                int Kz, int Ky) {
-    const int64_t total = (int64_t)Kz * Ky * nxh;
+// ---------------------------------------------------------------------------
+// Parity of the tensor.  Component comp (0..5: xx, xy, xz, yy, yz, zz) is odd
+// along the axes its letters name once (xy: x and y) and even along the others.
+// On a periodic grid of even length L an odd function vanishes at j = 0 and at
+// j = L/2 (the plane there never reaches the truncated output of the zero-padded
+// convolution), so the entries at 0 <= j <= L/2 determine the component, its
+// transform is real (odd axes come in pairs) and has the same parity.
+// ---------------------------------------------------------------------------
+__host__ __device__ __forceinline__ bool tensor_odd(int comp, int axis) {
+    return axis == 0 ? (comp == 1 || comp == 2) : axis == 1 ? (comp == 1 || comp == 4) : (comp == 2 || comp == 4);
+}
+
+// Entry at the wrapped index i of an axis of length L: the stored offset j, the
+// sign, and whether it is zero by parity (odd).
+__device__ __forceinline__ int wrap_offset(int i, int L, bool odd, bool& neg, bool& zero) {
+    const int j = 2 * i <= L ? i : L - i;
+    if (odd) {
+        neg = neg != (2 * i > L);
+        zero = zero || j == 0 || 2 * i == L;
+    }
+    return j;
+}
+
+// rows [nz][ny][L] of real values from the octant [nz][ny][o0]: the x axis
+// completed by parity; rows on the zero planes of the other axes are zero
+__global__ void k_tensor_rows(const double* __restrict__ oct, double* __restrict__ out, int comp, int o0, int ny,
+                              int nz, int Ly, int Lz, int L) {
+    const int64_t total = (int64_t)L * ny * nz;
+    const bool ox = tensor_odd(comp, 0), oy = tensor_odd(comp, 1), oz = tensor_odd(comp, 2);
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int x = (int)(i % L);
+        const int64_t r = i / L;
+        const int y = (int)(r % ny), z = (int)(r / ny);
+        bool neg = false, zero = (oy && (y == 0 || 2 * y == Ly)) || (oz && (z == 0 || 2 * z == Lz));
+        const int j = wrap_offset(x, L, ox, neg, zero);
+        const double v = zero || j >= o0 ? 0.0 : oct[r * o0 + j];
+        out[i] = neg ? -v : v;
+    }
+}
+
+// spectrum rows completed along one axis by parity: out [A][L][B][pitch] from the
+// rows a sa + j sj + b of in, j <= L/2 (y: A = z planes, B = 1; z: A = 1, B = ky rows)
+__global__ void k_tensor_wrap(const double2* __restrict__ in, double2* __restrict__ out, int64_t A, int L, int64_t B,
+                              int64_t sa, int64_t sj, int odd, int pitch, int nxh) {
+    const int64_t total = A * L * B * nxh;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int x = (int)(i % nxh);
+        int64_t r = i / nxh;
+        const int64_t o = r * pitch + x;
+        const int64_t b = r % B;
+        r /= B;
+        const int l = (int)(r % L);
+        const int64_t a = r / L;
+        bool neg = false, zero = false;
+        const int j = wrap_offset(l, L, odd != 0, neg, zero);
+        double2 v = make_double2(0.0, 0.0);
+        if (!zero) v = in[(a * sa + j * sj + b) * pitch + x];
+        out[o] = neg ? make_double2(-v.x, -v.y) : v;
+    }
+}
+
+// scaled real part of the spectrum on the stored quadrant
+__global__ void k_tensor_real(const double2* __restrict__ spec, double* __restrict__ dst, int64_t rows, int nxh,
+                              int pitch, double scale, int Ky, int spec_ky) {
+    const int64_t total = rows * nxh;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int kx = (int)(i % nxh);
-        const int ky = (int)((i / nxh) % Ky);
-        const int kz = (int)(i / ((int64_t)nxh * Ky));
-        dst[i] = spec[((int64_t)kz * Py + ky) * pitch + kx].x;
+        const int64_t r = i / nxh;
+        dst[i] = scale * spec[((r / Ky) * spec_ky + r % Ky) * pitch + kx].x;
+    }
+}
+
+// the parity-exact tensor on the padded grid [Pz][Py][Px] from its octant
+__global__ void k_tensor_full(const double* __restrict__ oct, double* __restrict__ out, int comp, int o0, int o1,
+                              int Px, int Py, int Pz) {
+    const int64_t total = (int64_t)Px * Py * Pz;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+        const int x = (int)(i % Px);
+        const int64_t r = i / Px;
+        bool neg = false, zero = false;
+        const int jx = wrap_offset(x, Px, tensor_odd(comp, 0), neg, zero);
+        const int jy = wrap_offset((int)(r % Py), Py, tensor_odd(comp, 1), neg, zero);
+        const int jz = wrap_offset((int)(r / Py), Pz, tensor_odd(comp, 2), neg, zero);
+        const double v = zero ? 0.0 : oct[((int64_t)jz * o1 + jy) * o0 + jx];
+        out[i] = neg ? -v : v;
     }
 }
 
@@ -362,34 +438,59 @@ Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, boo
     }
 }
 
+// Real spectrum (times scale) on the quadrant [Lz/2+1][Ly/2+1][Lx/2+1] (Lz = 1: one
+// plane) of the periodic function of lengths (Lx, Ly, Lz) that a tensor component's
+// octant `oct` [z][y][x] (the same quadrant of offsets) completes by parity.  Each
+// axis is completed just before its transform, so the x transforms run on a quarter
+// of the rows, the y transforms on half of the planes and the z transforms on half of
+// the rows.  work: two buffers kept between calls.
+void Demag::transform_octant(const double* oct, int comp, int Lx, int Ly, int Lz, double* quad, double scale,
+                             DevBuf* work, cudaStream_t st) {
+    const int nxh = Lx / 2 + 1, Ky = Ly / 2 + 1, Kz = Lz == 1 ? 1 : Lz / 2 + 1;
+    const int pitch = (nxh + 3) / 4 * 4;
+    const size_t csz = sizeof(double2);
+    // A: the completed real rows, then the completed y columns; B: the x spectra, then the completed z columns
+    work[0].ensure(std::max(sizeof(double) * (size_t)Lx * Ky * Kz, csz * (size_t)Kz * Ly * pitch));
+    work[1].ensure(csz * (size_t)std::max<int64_t>((int64_t)Ky * Kz, Lz > 1 ? (int64_t)Lz * Ky : 0) * pitch);
+    auto grid = [](int64_t n) { return (unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16); };
+    double* rows = work[0].as<double>();
+    double2* ycol = work[0].as<double2>();
+    double2* xs = work[1].as<double2>();
+    k_tensor_rows<<<grid((int64_t)Lx * Ky * Kz), 256, 0, st>>>(oct, rows, comp, nxh, Ky, Kz, Ly, Lz, Lx);
+    MAF_LAUNCH_CHECK();
+    launch_xfwd<double>(rows, Lx, (int64_t)Ky * Kz, (int64_t)Ky * Kz, nullptr, 1.0, xs, pitch, Lx, tw_, st);
+    k_tensor_wrap<<<grid((int64_t)Kz * Ly * nxh), 256, 0, st>>>(xs, ycol, Kz, Ly, 1, Ky, 1, tensor_odd(comp, 1),
+                                                                pitch, nxh);
+    MAF_LAUNCH_CHECK();
+    launch_cols<double, -1>(ycol, ycol, Ly, Ly, Ly, nxh, pitch, pitch, (int64_t)Ly * pitch, (int64_t)Ly * pitch, Kz,
+                            tw_, tune, st);
+    if (Lz > 1) {
+        double2* zcol = work[1].as<double2>();
+        k_tensor_wrap<<<grid((int64_t)Lz * Ky * nxh), 256, 0, st>>>(ycol, zcol, 1, Lz, Ky, 0, Ly,
+                                                                    tensor_odd(comp, 2), pitch, nxh);
+        MAF_LAUNCH_CHECK();
+        launch_cols<double, -1>(zcol, zcol, Lz, Lz, Lz, nxh, (int64_t)Ky * pitch, (int64_t)Ky * pitch, pitch, pitch,
+                                Ky, tw_, tune, st);
+        k_tensor_real<<<grid((int64_t)Kz * Ky * nxh), 256, 0, st>>>(zcol, quad, (int64_t)Kz * Ky, nxh, pitch, scale,
+                                                                    Ky, Ky);
+    } else {
+        k_tensor_real<<<grid((int64_t)Ky * nxh), 256, 0, st>>>(ycol, quad, Ky, nxh, pitch, scale, Ky, Ly);
+    }
+    MAF_LAUNCH_CHECK();
+}
+
 void Demag::build_tensor(cudaStream_t st) {
-    const int Px_ = Px(), Py_ = Py(), Pz_ = Pz();
-    const int64_t nreal = (int64_t)Px_ * Py_ * Pz_;
-    const int Ky = md_.ny + 1;
-    const int Kz = md_.nz == 1 ? 1 : md_.nz + 1;
-    const int64_t cstride = (int64_t)Kz * Ky * nxh();
+    const int Kx = md_.nx + 1, Ky = md_.ny + 1, Kz = md_.nz == 1 ? 1 : md_.nz + 1;
+    const int64_t cstride = (int64_t)Kz * Ky * Kx;
     Nred64_.alloc(sizeof(double) * cstride * ncomp());
-    DevBuf real(sizeof(double) * nreal);
-    DevBuf spec(sizeof(double2) * (int64_t)Pz_ * Py_ * pitch_);
+    DevBuf oct(sizeof(double) * cstride), work[2];
     const int comps6[6] = {0, 1, 2, 3, 4, 5};
     const int comps4[4] = {0, 1, 3, 5};
     const int* comps = md_.nz == 1 ? comps4 : comps6;
     for (int ci = 0; ci < ncomp(); ++ci) {
-        newell_component(real.as<double>(), comps[ci], md_, Px_, Py_, Pz_, true, st);
-        // 3-D R2C of the real tensor component
-        launch_xfwd<double>(real.as<double>(), Px_, (int64_t)Py_ * Pz_, (int64_t)Py_ * Pz_, nullptr, 1.0,
-                            spec.as<double2>(), pitch_, Px_, tw_, st);
-        launch_cols<double, -1>(spec.as<double2>(), spec.as<double2>(), Py_, Py_, Py_, nxh(), pitch_, pitch_,
-                                (int64_t)Py_ * pitch_, (int64_t)Py_ * pitch_, Pz_, tw_, tune, st);
-        if (Pz_ > 1)
-            launch_cols<double, -1>(spec.as<double2>(), spec.as<double2>(), Pz_, Pz_, Pz_, nxh(),
-                                    (int64_t)Py_ * pitch_, (int64_t)Py_ * pitch_, pitch_, pitch_, Py_, tw_, tune,
-                                    st);
-        const int64_t total = cstride;
-        const int64_t blocks = std::min<int64_t>(ceil_div(total, 256), (int64_t)sm_count() * 16);
-        k_reduce_tensor<<<(unsigned)blocks, 256, 0, st>>>(spec.as<double2>(), Nred64_.as<double>() + ci * cstride,
-                                                           nxh(), pitch_, Py_, Kz, Ky);
-        MAF_LAUNCH_CHECK();
+        newell_octant(oct.as<double>(), comps[ci], md_, Kx, Ky, Kz, st);
+        transform_octant(oct.as<double>(), comps[ci], Px(), Py(), Pz(), Nred64_.as<double>() + ci * cstride, 1.0, work,
+                         st);
     }
     MAF_CUDA(cudaStreamSynchronize(st));
 }
@@ -401,9 +502,18 @@ void Demag::download_tensor(double* host, cudaStream_t st) const {
 
 void Demag::download_real_tensor(double* host, bool symmetric, cudaStream_t st) {
     const int64_t nreal = (int64_t)Px() * Py() * Pz();
-    DevBuf real(sizeof(double) * nreal);
+    const int Kx = md_.nx + 1, Ky = md_.ny + 1, Kz = md_.nz == 1 ? 1 : md_.nz + 1;
+    DevBuf real(sizeof(double) * nreal), oct;
+    if (symmetric) oct.alloc(sizeof(double) * Kx * Ky * Kz);
     for (int c = 0; c < 6; ++c) {
-        newell_component(real.as<double>(), c, md_, Px(), Py(), Pz(), symmetric, st);
+        if (symmetric) {
+            newell_octant(oct.as<double>(), c, md_, Kx, Ky, Kz, st);
+            k_tensor_full<<<(unsigned)std::min<int64_t>(ceil_div(nreal, 256), (int64_t)sm_count() * 16), 256, 0, st>>>(
+                oct.as<double>(), real.as<double>(), c, Kx, Ky, Px(), Py(), Pz());
+            MAF_LAUNCH_CHECK();
+        } else {
+            newell_component(real.as<double>(), c, md_, Px(), Py(), Pz(), st);
+        }
         MAF_CUDA(cudaMemcpyAsync(host + c * nreal, real.p, sizeof(double) * nreal, cudaMemcpyDeviceToHost, st));
     }
     MAF_CUDA(cudaStreamSynchronize(st));

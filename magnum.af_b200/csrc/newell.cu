@@ -9,6 +9,8 @@
 // reference's host build.  Only the elementary functions differ (CUDA's
 // asinh/atan instead of the host libm), which perturbs far-field entries at
 // the level of their own cancellation noise.
+#include <algorithm>
+
 #include "engine.hpp"
 
 namespace mafb {
@@ -73,19 +75,9 @@ __device__ __forceinline__ double newell_comp(int comp, int j0, int j1, int j2, 
     }
 }
 
-// sym == 0: the reference's setup_N value at every padded index.
-// sym == 1: the parity-exact tensor that the spectral pipeline transforms: the
-//   value at (|j0|,|j1|,|j2|) times the component's parity sign (xy odd in x,y;
-//   xz odd in x,z; yz odd in y,z), and zero for an odd component where it
-//   vanishes in exact arithmetic (j = 0 along an odd axis) and on its Nyquist
-//   plane j = -P/2, which never reaches the truncated output.  The field on the
-//   mesh is the reference's up to the rounding noise of its 27-point sums; the
-//   exact symmetry makes the spectral tensor real with exact even/odd symmetry
-//   in ky and kz (and Nxz = Nyz = 0 for a single layer).
-__global__ void k_newell(double* __restrict__ out, int comp, int Px, int Py, int Pz, double dx, double dy, double dz,
-                         int sym) {
+// The reference's setup_N value at every padded index.
+__global__ void k_newell(double* __restrict__ out, int comp, int Px, int Py, int Pz, double dx, double dy, double dz) {
     const int64_t total = (int64_t)Px * Py * Pz;
-    const bool ox = comp == 1 || comp == 2, oy = comp == 1 || comp == 4, oz = comp == 2 || comp == 4;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
          idx += (int64_t)gridDim.x * blockDim.x) {
         const int i0 = (int)(idx % Px);
@@ -94,31 +86,38 @@ __global__ void k_newell(double* __restrict__ out, int comp, int Px, int Py, int
         const int j0 = (i0 + Px / 2) % Px - Px / 2;
         const int j1 = (i1 + Py / 2) % Py - Py / 2;
         const int j2 = (i2 + Pz / 2) % Pz - Pz / 2;
-        double v;
-        if (!sym) {
-            v = newell_comp(comp, j0, j1, j2, dx, dy, dz);
-        } else {
-            // an odd function vanishes at j = 0 and, on the periodic grid, at j = -P/2
-            const bool zero = (ox && (j0 == 0 || i0 == Px / 2)) || (oy && (j1 == 0 || i1 == Py / 2)) ||
-                              (oz && (j2 == 0 || i2 == Pz / 2));
-            if (zero) {
-                v = 0.0;
-            } else {
-                v = newell_comp(comp, abs(j0), abs(j1), abs(j2), dx, dy, dz);
-                const bool neg = (ox && j0 < 0) ^ (oy && j1 < 0) ^ (oz && j2 < 0);
-                if (neg) v = -v;
-            }
-        }
-        out[idx] = v;
+        out[idx] = newell_comp(comp, j0, j1, j2, dx, dy, dz);
     }
 }
 
-void newell_component(double* out, int comp, const MeshDims& md, int Px, int Py, int Pz, bool symmetric,
-                      cudaStream_t st) {
-    const int64_t total = (int64_t)Px * Py * Pz;
-    const int threads = 128;
-    const int64_t blocks = std::min<int64_t>(ceil_div(total, threads), (int64_t)sm_count() * 64);
-    k_newell<<<(unsigned)blocks, threads, 0, st>>>(out, comp, Px, Py, Pz, md.dx, md.dy, md.dz, symmetric ? 1 : 0);
+// The component at the offsets 0 <= j < (o0, o1, o2) only, one thread per entry.
+// The parity-exact tensor that the spectral pipeline transforms is even or odd
+// along each axis, so these entries carry all of it (fields.cu, tensor_odd)
+// and the 27 evaluations of f or g per entry (FP64 asinh and atan: the kernel is
+// bound on the FP64 pipe) are made for an eighth of the padded grid.
+__global__ void k_newell_octant(double* __restrict__ out, int comp, int o0, int o1, int o2, double dx, double dy,
+                                double dz) {
+    const int64_t total = (int64_t)o0 * o1 * o2;
+    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
+         idx += (int64_t)gridDim.x * blockDim.x) {
+        const int j0 = (int)(idx % o0);
+        const int j1 = (int)((idx / o0) % o1);
+        const int j2 = (int)(idx / ((int64_t)o0 * o1));
+        out[idx] = newell_comp(comp, j0, j1, j2, dx, dy, dz);
+    }
+}
+
+static unsigned newell_blocks(int64_t total) {
+    return (unsigned)std::min<int64_t>(ceil_div(total, 128), (int64_t)sm_count() * 64);
+}
+
+void newell_component(double* out, int comp, const MeshDims& md, int Px, int Py, int Pz, cudaStream_t st) {
+    k_newell<<<newell_blocks((int64_t)Px * Py * Pz), 128, 0, st>>>(out, comp, Px, Py, Pz, md.dx, md.dy, md.dz);
+    MAF_LAUNCH_CHECK();
+}
+
+void newell_octant(double* out, int comp, const MeshDims& md, int o0, int o1, int o2, cudaStream_t st) {
+    k_newell_octant<<<newell_blocks((int64_t)o0 * o1 * o2), 128, 0, st>>>(out, comp, o0, o1, o2, md.dx, md.dy, md.dz);
     MAF_LAUNCH_CHECK();
 }
 
