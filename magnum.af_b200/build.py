@@ -39,7 +39,7 @@ SOURCES = {
     "umma.o": ("umma.cu", []),
     "nn.o": ("nn.cu", []),
 }
-for _part in (1, 2, 3):
+for _part in (1, 2, 3, 4, 5):
     for _real in (4, 8):
         SOURCES["fields_ct_%d_%d.o" % (_part, _real)] = (
             "fields_ct.cu", ["-DMAF_CT_PART=%d" % _part, "-DMAF_CT_REAL=%d" % _real])

@@ -592,7 +592,8 @@ struct maf_lbfgs_s {
     double tolerance = 1e-6;
     size_t maxIter = 230;
     DevBuf sV[5], yV[5], q, s, y, grad, grad_old, x_old, wa, red;
-    DevBuf coef;           // device scalars: alpha[5] of the two-loop recursion, its current dot product, 3 more
+    DevBuf coef;           // device scalars: alpha[5], the recursion's dot product, (energy, slope), six reductions,
+                           // and the reductions' block counter
     double rho[5] = {};    // 1 / (s . y) of each stored pair
     unsigned long long fevals = 0, iterations = 0;
     double last_gradnorm = 0;
@@ -606,32 +607,51 @@ struct LbfgsCtx {
     int64_t n3, N;
     cudaStream_t stream;
     double* red() const { return h->red.as<double>(); }
+    unsigned* counter() const;
     double dot(const DevBuf& a, const DevBuf& b) const {
         return dot_host(a.as<double>(), b.as<double>(), n3, red(), stream);
     }
     double maxabs(const double* a) const { return maxabs_host(a, n3, red(), stream); }
 };
 
+// device scalars of maf_lbfgs_s::coef
+constexpr int kLbDot = 5, kLbEnergy = 6, kLbSix = 8, kLbCounter = 14, kLbScalars = 16;
+
+unsigned* LbfgsCtx::counter() const { return reinterpret_cast<unsigned*>(h->coef.as<double>() + kLbCounter); }
+
 // EnergyAndGradient of the state's current m and the directional derivative g . s,
-// read back with one synchronisation (the energy scaled as eval_terms scales it)
-void lbfgs_egrad_dg(const LbfgsCtx& c, DevBuf& g, const DevBuf& s, double& f, double& dg) {
+// left on the device as (energy density, slope) behind the recursion's last dot product
+void lbfgs_egrad_launch(const LbfgsCtx& c, DevBuf& g, const DevBuf& s) {
     std::vector<Term*> terms;
     for (auto& t : c.h->terms) terms.push_back(t.get());
-    double* two = c.h->coef.as<double>() + 6;
+    int ne = 0;
     EpilogueArgs ep;
     ep.kind = EPI_EGRAD;
     ep.out = g.p;
     ep.llg.m64 = c.st->s.m64.as<double>();
-    ep.energy_dev = two;
+    ep.npartials = &ne;
     eval_on_state(c.st, terms, ep, nullptr);
-    c.h->fevals++;
-    dot_dev(g.as<double>(), s.as<double>(), c.n3, c.red(), two + 1, c.stream);
-    double v[2];
-    MAF_CUDA(cudaMemcpyAsync(v, two, sizeof(v), cudaMemcpyDeviceToHost, c.stream));
+    double* coef = c.h->coef.as<double>();
+    lb_slope(g.as<double>(), s.as<double>(), c.n3, c.st->scratch.as<double>(), ne, c.red(), c.counter(),
+             coef + kLbEnergy, c.stream);
+}
+
+// Reads (dot product, energy, slope) back with one synchronisation; the energy
+// scaled as eval_terms scales it
+void lbfgs_read_egrad(const LbfgsCtx& c, double& dot, double& f, double& dg) {
+    double v[3];
+    MAF_CUDA(cudaMemcpyAsync(v, c.h->coef.as<double>() + kLbDot, sizeof(v), cudaMemcpyDeviceToHost, c.stream));
     MAF_CUDA(cudaStreamSynchronize(c.stream));
     const MeshDims& md = c.st->s.md;
-    f = v[0] * md.dx * md.dy * md.dz;
-    dg = v[1];
+    dot = v[0];
+    f = v[1] * md.dx * md.dy * md.dz;
+    dg = v[2];
+}
+
+// m = normalize(x_old + stp s)
+void lbfgs_move(const LbfgsCtx& c, const DevBuf& x_old, double stp, const DevBuf& s) {
+    normalize_combine(c.st->s.m64.as<double>(), x_old.as<double>(), stp, s.as<double>(), c.N, c.stream);
+    c.st->m32_valid = false;
 }
 
 // EnergyAndGradient (lbfgs_minimizer.cpp:38-42) of the state's current m
@@ -745,9 +765,10 @@ void cstep(double& stx, double& fx, double& dx, double& sty, double& fy, double&
 }
 
 // cvsrch (lbfgs_minimizer.cpp:213-360): wa = x_old, s = search direction (device)
-// (dginit_known: g . s when the caller has it already, else NaN)
+// (dginit_known: g . s at x_old when the caller has it already, else NaN; first: energy
+// and slope at the first trial step `stp` when the caller has evaluated it, else null)
 void cvsrch(const LbfgsCtx& c, const DevBuf& wa, double& f, DevBuf& g, double& stp, const DevBuf& s, double tolf,
-            double dginit_known) {
+            double dginit_known, const double* first) {
     int infoc = 1;
     const double xtol = 1e-15, ftol = 1.0e-4, gtol = 0.9, eps = tolf;
     const double stpmin = 1e-15, stpmax = 1e15, xtrapf = 4;
@@ -760,7 +781,6 @@ void cvsrch(const LbfgsCtx& c, const DevBuf& wa, double& f, DevBuf& g, double& s
     double width = stpmax - stpmin, width1 = 2 * width;
     double stx = 0.0, fx = finit, dgx = dginit, sty = 0.0, fy = finit, dgy = dginit;
     double stmin = 0, stmax = 0;
-    StateD& S = c.st->s;
     while (true) {
         if (brackt) {
             stmin = std::min(stx, sty);
@@ -774,10 +794,18 @@ void cvsrch(const LbfgsCtx& c, const DevBuf& wa, double& f, DevBuf& g, double& s
         if ((brackt && ((stp <= stmin) || (stp >= stmax))) || (nfev >= maxfev - 1) || (infoc == 0) ||
             (brackt && (stmax - stmin <= xtol * stmax)))
             stp = stx;
-        normalize_combine(S.m64.as<double>(), wa.as<double>(), stp, s.as<double>(), S.md.N(), c.stream);
-        c.st->m32_valid = false;
         double dg;
-        lbfgs_egrad_dg(c, g, s, f, dg);
+        if (first) {
+            f = first[0];
+            dg = first[1];
+            first = nullptr;
+        } else {
+            double dot;
+            lbfgs_move(c, wa, stp, s);
+            lbfgs_egrad_launch(c, g, s);
+            lbfgs_read_egrad(c, dot, f, dg);
+        }
+        c.h->fevals++;
         nfev++;
         const double ftest1 = finit + stp * dgtest;
         const double ftest2 = finit + eps * std::fabs(finit);
@@ -822,15 +850,10 @@ double lbfgs_minimize(maf_lbfgs_s* h, maf_state_s* st) {
         h->sV[i].ensure(sizeof(double) * n3);
         h->yV[i].ensure(sizeof(double) * n3);
     }
-    h->red.ensure(sizeof(double) * (red_blocks() + 8));
-    h->coef.ensure(sizeof(double) * 10);
-    double* alpha_d = h->coef.as<double>();  // alpha[0..4]
-    double* dot_d = alpha_d + 5;             // the dot product of the current recursion step
-    double* trio_d = alpha_d + 6;            // up to three reductions read back with one synchronisation
-    auto read_back = [&](int k, double* out) {
-        MAF_CUDA(cudaMemcpyAsync(out, trio_d, sizeof(double) * k, cudaMemcpyDeviceToHost, S.stream));
-        MAF_CUDA(cudaStreamSynchronize(S.stream));
-    };
+    h->red.ensure(sizeof(double) * (6 * red_blocks() + 8));
+    h->coef.ensure(sizeof(double) * kLbScalars);
+    MAF_CUDA(cudaMemsetAsync(h->coef.p, 0, sizeof(double) * kLbScalars, S.stream));
+    double* coef = h->coef.as<double>();
     LbfgsCtx c{h, st, n3, S.md.N(), S.stream};
     const double eps = 2.22e-16, eps2 = std::sqrt(eps), epsr = std::pow(eps, 0.9);
     const double tolf2 = std::sqrt(h->tolerance), tolf3 = std::pow(h->tolerance, 0.3333333333333333333333333);
@@ -845,49 +868,76 @@ double lbfgs_minimize(maf_lbfgs_s* h, maf_state_s* st) {
     int order[5] = {0, 1, 2, 3, 4};  // logical slot -> buffer (std::rotate of the reference)
     do {
         const double f_old = f;
-        MAF_CUDA(cudaMemcpyAsync(h->x_old.p, S.m64.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
-        MAF_CUDA(cudaMemcpyAsync(h->grad_old.p, h->grad.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
-        MAF_CUDA(cudaMemcpyAsync(h->q.p, h->grad.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
         const int k = (int)std::min(m, iter);
         // the two-loop recursion stays on the device: alpha_i = rho_i (s_i . q) and
         // beta = rho_i (y_i . q) are formed by the kernels that use them, with the
         // reference's operations in its order (rho_i = 1 / (s_i . y_i) is kept from when
-        // the pair was stored: the same value as recomputing it); no host synchronisation
-        for (int i = k - 1; i >= 0; --i) {
-            const DevBuf& sv = h->sV[order[i]];
-            const DevBuf& yv = h->yV[order[i]];
-            dot_dev(sv.as<double>(), h->q.as<double>(), n3, c.red(), dot_d, S.stream);
-            axpby_rho(h->q.as<double>(), yv.as<double>(), dot_d, h->rho[order[i]], nullptr, alpha_d + i, n3,
-                      S.stream);
+        // the pair was stored: the same value as recomputing it).  Step 0 copies x and the
+        // gradient; steps 1 .. k are the first loop and k+1 .. 2k the second; each forms the
+        // dot product of the next, the last one grad . q and the search direction s = -q.
+        for (int step = 0; step <= 2 * k; ++step) {
+            LbRecur a;
+            a.q_in = step == 0 ? h->grad.as<double>() : h->q.as<double>();
+            a.q = h->q.as<double>();
+            a.d = coef + kLbDot;
+            if (step == 0) {
+                a.x = S.m64.as<double>();
+                a.x_copy = h->x_old.as<double>();
+                a.g_copy = h->grad_old.as<double>();
+            } else if (step <= k) {
+                const int i = k - step;
+                a.u = h->yV[order[i]].as<double>();
+                a.rho = h->rho[order[i]];
+                a.alpha_out = coef + i;
+            } else {
+                const int i = step - k - 1;
+                a.u = h->sV[order[i]].as<double>();
+                a.rho = h->rho[order[i]];
+                a.alpha_in = coef + i;
+            }
+            if (step == k) {
+                a.scaled = 1;
+                a.scale = H0k;
+            }
+            if (step == 2 * k) {
+                a.w = h->grad.as<double>();
+                a.dir = h->s.as<double>();
+            } else if (step < k) {
+                a.w = h->sV[order[k - 1 - step]].as<double>();
+            } else {
+                a.w = h->yV[order[step - k]].as<double>();
+            }
+            lb_recur(a, n3, c.red(), c.counter(), S.stream);
         }
-        axpby(h->q.as<double>(), H0k, h->q.as<double>(), 0.0, nullptr, n3, S.stream);
-        for (int i = 0; i < k; ++i) {
-            const DevBuf& sv = h->sV[order[i]];
-            const DevBuf& yv = h->yV[order[i]];
-            dot_dev(yv.as<double>(), h->q.as<double>(), n3, c.red(), dot_d, S.stream);
-            axpby_rho(h->q.as<double>(), sv.as<double>(), dot_d, h->rho[order[i]], alpha_d + i, nullptr, n3,
-                      S.stream);
+        // the line search's first trial is always the full step: it is evaluated before
+        // grad . q is known to the host, and undone in the rare case of no descent
+        double rate = 1.0, dotq, first[2];
+        lbfgs_move(c, h->x_old, rate, h->s);
+        lbfgs_egrad_launch(c, h->grad, h->s);
+        lbfgs_read_egrad(c, dotq, first[0], first[1]);
+        const double phiPrime0 = -dotq;
+        if (phiPrime0 < 0) {
+            // with s = -q exactly (a negation), grad . s = -(grad . q) = phiPrime0 to the bit
+            cvsrch(c, h->x_old, f, h->grad, rate, h->s, h->tolerance, phiPrime0, first);
+        } else {
+            MAF_CUDA(cudaMemcpyAsync(S.m64.p, h->x_old.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
+            MAF_CUDA(cudaMemcpyAsync(h->grad.p, h->grad_old.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
+            st->m32_valid = false;
+            if (phiPrime0 > 0) {
+                axpby(h->s.as<double>(), -1.0, h->grad.as<double>(), 0.0, nullptr, n3, S.stream);
+                iter = 0;
+            }
+            cvsrch(c, h->x_old, f, h->grad, rate, h->s, h->tolerance,
+                   phiPrime0 == 0 ? phiPrime0 : std::numeric_limits<double>::quiet_NaN(), nullptr);
         }
-        const double phiPrime0 = -c.dot(h->grad, h->q);
-        if (phiPrime0 > 0) {
-            MAF_CUDA(cudaMemcpyAsync(h->q.p, h->grad.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
-            iter = 0;
-        }
-        // search direction -q (held in s until the step is known)
-        axpby(h->s.as<double>(), -1.0, h->q.as<double>(), 0.0, nullptr, n3, S.stream);
-        double rate = 1.0;
-        // with s = -q exactly (a negation), grad . s = -(grad . q) = phiPrime0 to the bit
-        cvsrch(c, h->x_old, f, h->grad, rate, h->s, h->tolerance,
-               phiPrime0 > 0 ? std::numeric_limits<double>::quiet_NaN() : phiPrime0);
         const double f1 = 1 + std::fabs(f);
-        // max|grad|, and ahead of the convergence test the step s = m - x_old with
-        // max|s| and max|m| (unused if the gradient test ends the run): one synchronisation
-        axpby(h->s.as<double>(), 1.0, S.m64.as<double>(), -1.0, h->x_old.as<double>(), n3, S.stream);
-        double mx[3];
-        reduce_dev(h->grad.as<double>(), nullptr, n3, 1, c.red(), trio_d, S.stream);
-        reduce_dev(h->s.as<double>(), nullptr, n3, 1, c.red(), trio_d + 1, S.stream);
-        reduce_dev(S.m64.as<double>(), nullptr, n3, 1, c.red(), trio_d + 2, S.stream);
-        read_back(3, mx);
+        // s = m - x_old, y = grad - grad_old, max|grad|, max|s|, max|m| and the three dot
+        // products of the update (unused if the run ends here): one launch, one synchronisation
+        lb_pair(S.m64.as<double>(), h->x_old.as<double>(), h->grad.as<double>(), h->grad_old.as<double>(),
+                h->s.as<double>(), h->y.as<double>(), n3, c.red(), c.counter(), coef + kLbSix, S.stream);
+        double mx[6];
+        MAF_CUDA(cudaMemcpyAsync(mx, coef + kLbSix, sizeof(mx), cudaMemcpyDeviceToHost, S.stream));
+        MAF_CUDA(cudaStreamSynchronize(S.stream));
         gradNorm = mx[0];
         h->last_gradnorm = gradNorm;
         if (gradNorm < (epsr * f1)) {
@@ -896,14 +946,8 @@ double lbfgs_minimize(maf_lbfgs_s* h, maf_state_s* st) {
         }
         const double smax = mx[1], mmax = mx[2];
         if (((f_old - f) < (h->tolerance * f1)) && (smax < (tolf2 * (1 + mmax))) && (gradNorm <= (tolf3 * f1))) break;
-        axpby(h->y.as<double>(), 1.0, h->grad.as<double>(), -1.0, h->grad_old.as<double>(), n3, S.stream);
-        double d3[3];
-        dot_dev(h->y.as<double>(), h->s.as<double>(), n3, c.red(), trio_d, S.stream);
-        dot_dev(h->y.as<double>(), h->y.as<double>(), n3, c.red(), trio_d + 1, S.stream);
-        dot_dev(h->s.as<double>(), h->s.as<double>(), n3, c.red(), trio_d + 2, S.stream);
-        read_back(3, d3);
-        const double ys = d3[0], yy = d3[1];
-        if (ys <= eps2 * std::sqrt(yy) * std::sqrt(d3[2])) {
+        const double ys = mx[3], yy = mx[4];
+        if (ys <= eps2 * std::sqrt(yy) * std::sqrt(mx[5])) {
             // Dennis, Schnabel 9.4.1: skip the update
         } else {
             int slot;
@@ -915,8 +959,8 @@ double lbfgs_minimize(maf_lbfgs_s* h, maf_state_s* st) {
                 order[4] = first;
                 slot = first;
             }
-            MAF_CUDA(cudaMemcpyAsync(h->sV[slot].p, h->s.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
-            MAF_CUDA(cudaMemcpyAsync(h->yV[slot].p, h->y.p, sizeof(double) * n3, cudaMemcpyDeviceToDevice, S.stream));
+            std::swap(h->sV[slot], h->s);  // h->s and h->y are rewritten by the next iteration
+            std::swap(h->yV[slot], h->y);
             h->rho[slot] = 1.0 / ys;  // = 1 / (s . y): the products commute exactly, same partial-sum order
             H0k = ys / yy;
             iter++;

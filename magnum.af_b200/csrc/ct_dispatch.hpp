@@ -17,10 +17,19 @@ bool ct_convz(cplx_t<R>* S, const R* Nred, int nz, int ny, int nxh, int pitch, T
               cudaStream_t st);
 template <typename R>
 bool ct_convy(cplx_t<R>* S, const R* Nred, int ny, int nxh, int pitch, Twiddles& tw, cudaStream_t st);
+// (the lengths are instantiated in three groups G)
+template <typename R, int G>
+bool ct_xinv_group(const cplx_t<R>* S1, int pitch, int Px, Twiddles& tw, const Geom& g, R scale, const R* m,
+                   const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep, const TuneChoice& tc, cudaStream_t st,
+                   int* nblocks);
 template <typename R>
 bool ct_xinv(const cplx_t<R>* S1, int pitch, int Px, Twiddles& tw, const Geom& g, R scale, const R* m,
              const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep, const TuneChoice& tc, cudaStream_t st,
-             int* nblocks);
+             int* nblocks) {
+    return ct_xinv_group<R, 0>(S1, pitch, Px, tw, g, scale, m, ms, tl, ep, tc, st, nblocks) ||
+           ct_xinv_group<R, 1>(S1, pitch, Px, tw, g, scale, m, ms, tl, ep, tc, st, nblocks) ||
+           ct_xinv_group<R, 2>(S1, pitch, Px, tw, g, scale, m, ms, tl, ep, tc, st, nblocks);
+}
 
 // Batched compile-time passes: one launch runs the (item, tile) pairs of a
 // device work table, every item of a launch with the same transform length
@@ -63,8 +72,16 @@ void ct_batch_xfwd(const CtXfwdItem<R>* items, const int2* work, int nwork, int 
                    cudaStream_t st);
 template <typename R>
 void ct_batch_convy(const CtConvyItem<R>* items, const int2* work, int nwork, int L, const void* tw, cudaStream_t st);
+template <typename R, int G>
+bool ct_batch_xinv_group(const CtXinvItem<R>* items, const int2* work, int nwork, int L, int run, const void* tw,
+                         const void* twP, cudaStream_t st);
 template <typename R>
 void ct_batch_xinv(const CtXinvItem<R>* items, const int2* work, int nwork, int L, int run, const void* tw,
-                   const void* twP, cudaStream_t st);
+                   const void* twP, cudaStream_t st) {
+    if (nwork <= 0) return;
+    ct_batch_xinv_group<R, 0>(items, work, nwork, L, run, tw, twP, st) ||
+        ct_batch_xinv_group<R, 1>(items, work, nwork, L, run, tw, twP, st) ||
+        ct_batch_xinv_group<R, 2>(items, work, nwork, L, run, tw, twP, st);
+}
 
 }  // namespace mafb

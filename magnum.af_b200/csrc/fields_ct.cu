@@ -878,13 +878,13 @@ static void xinv_L(const cplx_t<R>* S1, int pitch, const void* tw, const void* t
             break;
         }
         case EPI_EGRAD: {
-            auto k = k_xinv_ct<R, EPI_EGRAD, LC, NBR, NT, RN>;
+            auto k = k_xinv_ct<R, EPI_EGRAD, LC, NBR, NT, 2>;
             ct_smem(k, smem);
             k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run4);
             break;
         }
         default: {
-            auto k = k_xinv_ct<R, EPI_EDENS, LC, NBR, NT, RN>;
+            auto k = k_xinv_ct<R, EPI_EDENS, LC, NBR, NT, 2>;
             ct_smem(k, smem);
             k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run4);
             break;
@@ -1079,10 +1079,39 @@ bool ct_convy(cplx_t<R>* S, const R* Nred, int ny, int nxh, int pitch, Twiddles&
 #undef X
 }
 
-template <typename R>
-bool ct_xinv(const cplx_t<R>* S1, int pitch, int Px, Twiddles& tw, const Geom& g, R scale, const R* m,
-             const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep, const TuneChoice& tc, cudaStream_t st,
-             int* nblocks) {
+// The x-inverse lengths in three groups, instantiated by separate compilations.
+#define MAF_CT_XINV_SWITCH(G, L, CALL)              \
+    if constexpr (G == 0) {                         \
+        switch (L) {                                \
+            case 16: CALL(16); return true;         \
+            case 32: CALL(32); return true;         \
+            case 64: CALL(64); return true;         \
+            case 128: CALL(128); return true;       \
+            case 256: CALL(256); return true;       \
+            default: return false;                  \
+        }                                           \
+    } else if constexpr (G == 1) {                  \
+        switch (L) {                                \
+            case 512: CALL(512); return true;       \
+            case 1024: CALL(1024); return true;     \
+            case 2048: CALL(2048); return true;     \
+            default: return false;                  \
+        }                                           \
+    } else {                                        \
+        switch (L) {                                \
+            case 96: CALL(96); return true;         \
+            case 192: CALL(192); return true;       \
+            case 384: CALL(384); return true;       \
+            case 768: CALL(768); return true;       \
+            case 1536: CALL(1536); return true;     \
+            default: return false;                  \
+        }                                           \
+    }
+
+template <typename R, int G>
+bool ct_xinv_group(const cplx_t<R>* S1, int pitch, int Px, Twiddles& tw, const Geom& g, R scale, const R* m,
+                   const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep, const TuneChoice& tc, cudaStream_t st,
+                   int* nblocks) {
     const int LC = Px / 2;
     if (g.nx != LC) return false;  // the kernels take the row length from LC
     const bool f64 = sizeof(R) == 8;
@@ -1094,22 +1123,7 @@ bool ct_xinv(const cplx_t<R>* S1, int pitch, int Px, Twiddles& tw, const Geom& g
         else                                                                                                    \
             xinv_L<R, N, 2>(S1, pitch, ct_tw<N>(tw, f64), tw.get(Px, f64), g, scale, m, ms, tl, ep, st, nblocks);  \
     } while (0)
-    switch (LC) {
-        case 16: X(16); return true;
-        case 32: X(32); return true;
-        case 64: X(64); return true;
-        case 128: X(128); return true;
-        case 256: X(256); return true;
-        case 512: X(512); return true;
-        case 1024: X(1024); return true;
-        case 2048: X(2048); return true;
-        case 96: X(96); return true;
-        case 192: X(192); return true;
-        case 384: X(384); return true;
-        case 768: X(768); return true;
-        case 1536: X(1536); return true;
-        default: return false;
-    }
+    MAF_CT_XINV_SWITCH(G, LC, X)
 #undef X
 }
 
@@ -1172,10 +1186,9 @@ void ct_batch_convy(const CtConvyItem<R>* items, const int2* work, int nwork, in
 #undef X
 }
 
-template <typename R>
-void ct_batch_xinv(const CtXinvItem<R>* items, const int2* work, int nwork, int L, int run, const void* tw,
-                   const void* twP, cudaStream_t st) {
-    if (nwork <= 0) return;
+template <typename R, int G>
+bool ct_batch_xinv_group(const CtXinvItem<R>* items, const int2* work, int nwork, int L, int run, const void* tw,
+                         const void* twP, cudaStream_t st) {
 #define X(N)                                                        \
     do {                                                            \
         if (run == 4)                                               \
@@ -1183,12 +1196,12 @@ void ct_batch_xinv(const CtXinvItem<R>* items, const int2* work, int nwork, int 
         else                                                        \
             batch_xinv_L<R, N, 2>(items, work, nwork, tw, twP, st); \
     } while (0)
-    MAF_CT_BATCH_SWITCH(L, X)
+    MAF_CT_XINV_SWITCH(G, L, X)
 #undef X
 }
 
 // The instantiations are split over several compilations of this file
-// (MAF_CT_PART = 1: x forward and convolutions, 2: y passes, 3: x inverse;
+// (MAF_CT_PART = 1: x forward and convolutions, 2: y passes, 3..5: x inverse, by length group;
 // MAF_CT_REAL = 4 or 8 selects FP32 or FP64), so that the build compiles them
 // in parallel; without the macros every instantiation is made here.
 #if !defined(MAF_CT_PART) || MAF_CT_PART == 1
@@ -1216,16 +1229,27 @@ void ct_batch_xinv(const CtXinvItem<R>* items, const int2* work, int nwork, int 
 #else
 #define MAF_INST2(R)
 #endif
+#define MAF_INST_XINV(R, G)                                                                                           \
+    template bool ct_xinv_group<R, G>(const cplx_t<R>*, int, int, Twiddles&, const Geom&, R, const R*, const MsInfo&, \
+                                      const TermList&, const EpilogueArgs&, const TuneChoice&, cudaStream_t, int*);   \
+    template bool ct_batch_xinv_group<R, G>(const CtXinvItem<R>*, const int2*, int, int, int, const void*,            \
+                                            const void*, cudaStream_t);
 #if !defined(MAF_CT_PART) || MAF_CT_PART == 3
-#define MAF_INST3(R)                                                                                                  \
-    template bool ct_xinv<R>(const cplx_t<R>*, int, int, Twiddles&, const Geom&, R, const R*, const MsInfo&,          \
-                             const TermList&, const EpilogueArgs&, const TuneChoice&, cudaStream_t, int*);        \
-    template void ct_batch_xinv<R>(const CtXinvItem<R>*, const int2*, int, int, int, const void*, const void*,      \
-                                   cudaStream_t);
+#define MAF_INST3(R) MAF_INST_XINV(R, 0)
 #else
 #define MAF_INST3(R)
 #endif
-#define MAF_INST(R) MAF_INST1(R) MAF_INST2(R) MAF_INST3(R)
+#if !defined(MAF_CT_PART) || MAF_CT_PART == 4
+#define MAF_INST4(R) MAF_INST_XINV(R, 1)
+#else
+#define MAF_INST4(R)
+#endif
+#if !defined(MAF_CT_PART) || MAF_CT_PART == 5
+#define MAF_INST5(R) MAF_INST_XINV(R, 2)
+#else
+#define MAF_INST5(R)
+#endif
+#define MAF_INST(R) MAF_INST1(R) MAF_INST2(R) MAF_INST3(R) MAF_INST4(R) MAF_INST5(R)
 #if !defined(MAF_CT_REAL) || MAF_CT_REAL == 4
 MAF_INST(float)
 #endif

@@ -350,15 +350,16 @@ __global__ void k_mean_partials(const double* __restrict__ m, int64_t N, double*
     }
 }
 
+// one warp per sum (the three components and the cell count)
 __global__ void k_mean_final(const double* __restrict__ part, int nb, double* __restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s[4] = {0, 0, 0, 0};
-        for (int b = 0; b < nb; ++b)
-            for (int q = 0; q < 4; ++q) s[q] += part[4 * b + q];
-        out[0] = s[0] / s[3];
-        out[1] = s[1] / s[3];
-        out[2] = s[2] / s[3];
-    }
+    __shared__ double tot[4];
+    const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+    double s = 0;
+    for (int b = lane; b < nb; b += 32) s += part[4 * b + q];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) tot[q] = s;
+    __syncthreads();
+    if (threadIdx.x < 3) out[threadIdx.x] = tot[threadIdx.x] / tot[3];
 }
 
 int mean_m_blocks() { return 2 * sm_count(); }
@@ -367,7 +368,7 @@ void mean_m(const double* m, int64_t N, double* scratch, double* out_dev, cudaSt
     const int blocks = (int)std::min<int64_t>(ceil_div(N, 256), mean_m_blocks());
     k_mean_partials<<<blocks, 256, 0, st>>>(m, N, scratch);
     MAF_LAUNCH_CHECK();
-    k_mean_final<<<1, 32, 0, st>>>(scratch, blocks, out_dev);
+    k_mean_final<<<1, 128, 0, st>>>(scratch, blocks, out_dev);
     MAF_LAUNCH_CHECK();
 }
 
@@ -424,10 +425,21 @@ __global__ void k_red_partials(const double* __restrict__ a, const double* __res
     }
 }
 
+// one block, 256 threads: the partials in a fixed tree (one thread adding the 192-296
+// partials in a chain took 10.9 us, longer than the reduction itself)
 __global__ void k_red_final(const double* __restrict__ part, int nb, int mode, double* __restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int i = 0; i < nb; ++i) s = mode != 1 ? s + part[i] : nanmax(s, part[i]);
+    __shared__ double red[8];
+    double v = 0.0;
+    for (int i = threadIdx.x; i < nb; i += 256) v = mode != 1 ? v + part[i] : nanmax(v, part[i]);
+    for (int o = 16; o > 0; o >>= 1) {
+        const double w = __shfl_down_sync(0xffffffffu, v, o);
+        v = mode != 1 ? v + w : nanmax(v, w);
+    }
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = red[0];
+        for (int i = 1; i < 8; ++i) s = mode != 1 ? s + red[i] : nanmax(s, red[i]);
         *out = s;
     }
 }
@@ -437,7 +449,7 @@ double reduce_host(const double* a, const double* b, int64_t n, int mode, double
     const int blocks = (int)std::min<int64_t>(ceil_div(n, 256), nred);
     k_red_partials<<<blocks, 256, 0, st>>>(a, b, n, mode, scratch);
     MAF_LAUNCH_CHECK();
-    k_red_final<<<1, 32, 0, st>>>(scratch, blocks, mode, scratch + nred);
+    k_red_final<<<1, 256, 0, st>>>(scratch, blocks, mode, scratch + nred);
     MAF_LAUNCH_CHECK();
     double v = 0;
     MAF_CUDA(cudaMemcpyAsync(&v, scratch + nred, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -447,19 +459,6 @@ double reduce_host(const double* a, const double* b, int64_t n, int mode, double
 
 double dot_host(const double* a, const double* b, int64_t n, double* scratch, cudaStream_t st) {
     return reduce_host(a, b, n, 0, scratch, st);
-}
-
-void reduce_dev(const double* a, const double* b, int64_t n, int mode, double* scratch, double* out, cudaStream_t st) {
-    const int nred = red_blocks();
-    const int blocks = (int)std::min<int64_t>(ceil_div(n, 256), nred);
-    k_red_partials<<<blocks, 256, 0, st>>>(a, b, n, mode, scratch);
-    MAF_LAUNCH_CHECK();
-    k_red_final<<<1, 32, 0, st>>>(scratch, blocks, mode, out);
-    MAF_LAUNCH_CHECK();
-}
-
-void dot_dev(const double* a, const double* b, int64_t n, double* scratch, double* out, cudaStream_t st) {
-    reduce_dev(a, b, n, 0, scratch, out, st);
 }
 
 double maxabs_host(const double* a, int64_t n, double* scratch, cudaStream_t st) {
@@ -506,24 +505,154 @@ void axpby(double* out, double a, const double* x, double b, const double* y, in
     MAF_LAUNCH_CHECK();
 }
 
-// k_axpby with a = 1 and the coefficient formed on the device from the dot
-// product *d (every thread forms the same value)
-__global__ void k_axpby_rho(double* q, const double* __restrict__ y, const double* __restrict__ d, double rho,
-                            const double* __restrict__ alpha_in, double* __restrict__ alpha_out, int64_t n) {
-    const double t = rho * *d;
-    const double b = alpha_in ? *alpha_in - t : -t;
-    if (alpha_out && blockIdx.x == 0 && threadIdx.x == 0) *alpha_out = t;
-    const double a = 1.0;
+// ---------------------------------------------------------------------------
+// LBFGS iteration kernels: an update and the reductions that follow it in one
+// launch.  A film of 128x128 cells is 0.4 MB per vector, so an iteration is bound
+// by the number of dependent launches (2.5-3.5 us each), not by bandwidth: with an
+// update, a partial and a final kernel per dot product an iteration of 20 took
+// 72 launches, 0.47 ms; with the last block of the update's grid forming the
+// reduction's result it takes about 18.
+// ---------------------------------------------------------------------------
+constexpr int kLbThreads = 256;
+
+// Block sums (or, bit r of maxmask, NaN-propagating maxima) of v[0..NR) to
+// part[r * gridDim.x + block]; the block that arrives last combines every block's
+// partials in a fixed tree, whatever the arrival order, and writes out[0..NR).
+// *counter is zero before and after the launch.  Returns whether this is that block.
+template <int NR>
+__device__ __forceinline__ bool reduce_last_block(double (&v)[NR], unsigned maxmask, double* part, unsigned* counter,
+                                                  double* out) {
+    __shared__ double red[NR][kLbThreads / 32];
+    __shared__ bool last;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    auto block_combine = [&](double (&x)[NR]) {  // the result in thread r < NR, x[0]
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+            for (int o = 16; o > 0; o >>= 1) {
+                const double w = __shfl_down_sync(0xffffffffu, x[r], o);
+                x[r] = (maxmask >> r) & 1u ? nanmax(x[r], w) : x[r] + w;
+            }
+            if (lane == 0) red[r][wid] = x[r];
+        }
+        __syncthreads();
+        if (threadIdx.x < NR) {
+            const int r = threadIdx.x;
+            double s = red[r][0];
+            for (int k = 1; k < kLbThreads / 32; ++k) s = (maxmask >> r) & 1u ? nanmax(s, red[r][k]) : s + red[r][k];
+            x[0] = s;
+        }
+    };
+    block_combine(v);
+    if (threadIdx.x < NR) {
+        part[threadIdx.x * gridDim.x + blockIdx.x] = v[0];
+        __threadfence();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return false;
+    __threadfence();
+    double t[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+        t[r] = 0.0;
+        for (unsigned b = threadIdx.x; b < gridDim.x; b += kLbThreads) {
+            const double w = __ldcg(part + r * gridDim.x + b);
+            t[r] = (maxmask >> r) & 1u ? nanmax(t[r], w) : t[r] + w;
+        }
+    }
+    block_combine(t);
+    if (threadIdx.x < NR) out[threadIdx.x] = t[0];
+    return true;
+}
+
+// One step of the two-loop recursion (lbfgs_minimizer.cpp:96-130):
+//   q <- scale (q_in + b u),  b = -rho *d (first loop) or *alpha_in - rho *d (second),
+// *alpha_out = rho *d, dir <- -q, and *d <- w . q for the next step.  u, alpha_*, dir
+// and the copies (x_copy <- x, g_copy <- q_in) are optional.  The product order is
+// that of separate kernels; *d is read by every thread before its block arrives, and
+// written by the last block only.
+__global__ void __launch_bounds__(kLbThreads) k_lb_recur(LbRecur a, int64_t n, double* part, unsigned* counter) {
+    double b = 0.0;
+    if (a.u) {
+        const double t = a.rho * *a.d;
+        b = a.alpha_in ? *a.alpha_in - t : -t;
+        if (a.alpha_out && blockIdx.x == 0 && threadIdx.x == 0) *a.alpha_out = t;
+    }
+    double v[1] = {0.0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double v = a * q[i];
-        q[i] = v + b * y[i];
+        double q = a.q_in[i];
+        if (a.g_copy) a.g_copy[i] = q;
+        if (a.x_copy) a.x_copy[i] = a.x[i];
+        if (a.u) q = q + b * a.u[i];
+        if (a.scaled) q = a.scale * q;
+        a.q[i] = q;
+        if (a.dir) a.dir[i] = -q;
+        v[0] += a.w[i] * q;
+    }
+    reduce_last_block<1>(v, 0u, part, counter, a.d);
+}
+
+void lb_recur(const LbRecur& a, int64_t n, double* part, unsigned* counter, cudaStream_t st) {
+    const int blocks = (int)std::min<int64_t>(ceil_div(n, kLbThreads), red_blocks());
+    k_lb_recur<<<blocks, kLbThreads, 0, st>>>(a, n, part, counter);
+    MAF_LAUNCH_CHECK();
+}
+
+// out[1] = g . s, and out[0] = the sum of the energy partials e[0, ne) in the order
+// of k_sum_partials (one block of 256 threads)
+__global__ void __launch_bounds__(kLbThreads) k_lb_slope(const double* __restrict__ g, const double* __restrict__ s,
+                                                         int64_t n, const double* __restrict__ e, int ne, double* part,
+                                                         unsigned* counter, double* out) {
+    double v[1] = {0.0};
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+        v[0] += g[i] * s[i];
+    if (!reduce_last_block<1>(v, 0u, part, counter, out + 1)) return;
+    __shared__ double red[kLbThreads / 32];
+    double t = 0.0;
+    for (int i = threadIdx.x; i < ne; i += kLbThreads) t += e[i];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        double x = threadIdx.x < kLbThreads / 32 ? red[threadIdx.x] : 0.0;
+        for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+        if (threadIdx.x == 0) out[0] = x;
     }
 }
 
-void axpby_rho(double* q, const double* y, const double* d, double rho, const double* alpha_in, double* alpha_out,
-               int64_t n, cudaStream_t st) {
-    const int64_t blocks = std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16);
-    k_axpby_rho<<<(unsigned)blocks, 256, 0, st>>>(q, y, d, rho, alpha_in, alpha_out, n);
+void lb_slope(const double* g, const double* s, int64_t n, const double* e, int ne, double* part, unsigned* counter,
+              double* out, cudaStream_t st) {
+    const int blocks = (int)std::min<int64_t>(ceil_div(n, kLbThreads), red_blocks());
+    k_lb_slope<<<blocks, kLbThreads, 0, st>>>(g, s, n, e, ne, part, counter, out);
+    MAF_LAUNCH_CHECK();
+}
+
+// s = x - x_old, y = g - g_old; out = max|g|, max|s|, max|x|, y . s, y . y, s . s
+__global__ void __launch_bounds__(kLbThreads) k_lb_pair(const double* __restrict__ x, const double* __restrict__ x_old,
+                                                        const double* __restrict__ g, const double* __restrict__ g_old,
+                                                        double* __restrict__ s, double* __restrict__ y, int64_t n,
+                                                        double* part, unsigned* counter, double* out) {
+    double v[6] = {0, 0, 0, 0, 0, 0};
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double xi = x[i], gi = g[i];
+        const double si = xi - x_old[i], yi = gi - g_old[i];
+        s[i] = si;
+        y[i] = yi;
+        v[0] = nanmax(v[0], fabs(gi));
+        v[1] = nanmax(v[1], fabs(si));
+        v[2] = nanmax(v[2], fabs(xi));
+        v[3] += yi * si;
+        v[4] += yi * yi;
+        v[5] += si * si;
+    }
+    reduce_last_block<6>(v, 7u, part, counter, out);
+}
+
+void lb_pair(const double* x, const double* x_old, const double* g, const double* g_old, double* s, double* y,
+             int64_t n, double* part, unsigned* counter, double* out, cudaStream_t st) {
+    const int blocks = (int)std::min<int64_t>(ceil_div(n, kLbThreads), red_blocks());
+    k_lb_pair<<<blocks, kLbThreads, 0, st>>>(x, x_old, g, g_old, s, y, n, part, counter, out);
     MAF_LAUNCH_CHECK();
 }
 

@@ -27,16 +27,29 @@ int red_blocks();
 double dot_host(const double* a, const double* b, int64_t n, double* scratch, cudaStream_t st);
 double maxabs_host(const double* a, int64_t n, double* scratch, cudaStream_t st);
 void axpby(double* out, double a, const double* x, double b, const double* y, int64_t n, cudaStream_t st);
-// Device-resident steps of the LBFGS two-loop recursion (no host synchronisation):
-// *out = a . b (the same partial sums and order as dot_host), and
-// q = 1 q + c y with c = -(rho *d) (alpha_out: t = rho *d, written by one thread)
-// or c = *alpha_in - rho *d (the reference's operations; the multiply-add may round
-// differently in the last bit from axpby's).
-void dot_dev(const double* a, const double* b, int64_t n, double* scratch, double* out, cudaStream_t st);
-// reduce_host's mode (0 dot, 1 NaN-propagating max |a|, 2 squared difference) into a device scalar
-void reduce_dev(const double* a, const double* b, int64_t n, int mode, double* scratch, double* out, cudaStream_t st);
-void axpby_rho(double* q, const double* y, const double* d, double rho, const double* alpha_in, double* alpha_out,
-               int64_t n, cudaStream_t st);
+// Device-resident LBFGS iteration kernels (no host synchronisation; llg.cu).  part:
+// 6 red_blocks() doubles; counter: one zeroed word that every launch leaves zero.
+struct LbRecur {
+    const double* q_in = nullptr;   // q of the previous step, or the gradient
+    double* q = nullptr;
+    const double* u = nullptr;      // vector added with the coefficient formed from *d
+    double* d = nullptr;            // in: the dot product of the previous step; out: w . q
+    const double* w = nullptr;
+    double rho = 0.0;
+    const double* alpha_in = nullptr;
+    double* alpha_out = nullptr;
+    int scaled = 0;
+    double scale = 1.0;
+    double* dir = nullptr;          // -q
+    const double* x = nullptr;      // copied to x_copy
+    double* x_copy = nullptr;
+    double* g_copy = nullptr;       // copy of q_in
+};
+void lb_recur(const LbRecur& a, int64_t n, double* part, unsigned* counter, cudaStream_t st);
+void lb_slope(const double* g, const double* s, int64_t n, const double* e, int ne, double* part, unsigned* counter,
+              double* out, cudaStream_t st);
+void lb_pair(const double* x, const double* x_old, const double* g, const double* g_old, double* s, double* y,
+             int64_t n, double* part, unsigned* counter, double* out, cudaStream_t st);
 void normalize_combine(double* m, const double* wa, double stp, const double* s, int64_t N, cudaStream_t st);
 // string method: sum (a-b)^2 over n values (synchronises), out = a + (c1 (b - a)) / c2
 double sqdiff_host(const double* a, const double* b, int64_t n, double* scratch, cudaStream_t st);
