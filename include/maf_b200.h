@@ -405,6 +405,26 @@ int maf_nn_colsum(const float* dY, long long P, int C, float* db, void* st);
  * weight gradient [Cout][9][Cin] from a GEMM result [Cout][9 Cp] */
 int maf_nn_wcast(const float* W32, int Cout, int Cin, int Cp, int CoutP, void* Wb, void* WtB, void* st);
 int maf_nn_wgrad(const float* g, int Cout, int Cin, int Cp, float* dW, void* st);
+/* 3x3 convolution as an implicit GEMM on the tensor cores (zero padding, no im2col):
+ * out [P][ldo] (FP32, channels 0 .. N-1) = relu?(bias + taps of act [P][Cp] . w [N][9 Cp]^T) and, when
+ * outb, its BF16 copy [P][ldb]; bias may be NULL.  The data gradient is the same call on dY with the
+ * weights Wd below.  Buffers 16-byte aligned. */
+int maf_nn_conv(const void* act, int B, int H, int W, int Cp, const void* w, int N, const float* bias, int relu,
+                float* out, int ldo, void* outb, int ldb, void* st);
+/* weight gradient dW [Cout][9][Cin] of that convolution from act [P][Cp] and dY [P][CoutP] (BF16); the
+ * pixels are split over at most max_splits partial slabs work [.][9 Cp][CoutP], summed in a fixed order */
+int maf_nn_conv_wgrad(const void* act, int B, int H, int W, int Cp, int Cin, const void* dy, int Cout, int CoutP,
+                      float* work, int max_splits, float* dW, void* st);
+/* FP32 weights W [Cout][9][Cin] -> BF16 Wf [Cout][9 Cp] (forward) and Wd [Cin][9 CoutP] (data gradient) */
+int maf_nn_wcast_conv(const float* W32, int Cout, int Cin, int Cp, int CoutP, void* Wf, void* Wd, void* st);
+/* dYb [P][Cp] = BF16(dA relu'(A)) and db [C] = its column sums before rounding (FP64, fixed order); part:
+ * maf_nn_relu_bias_bwd_parts() x C doubles of scratch */
+int maf_nn_relu_bias_bwd(const float* dA, const float* A, long long P, int C, int relu, void* dYb, int Cp, float* db,
+                         double* part, void* st);
+int maf_nn_relu_bias_bwd_parts(int* n);
+/* maf_nn_up_cat_bwd with ds = instead of ds += */
+int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
+                          void* st);
 /* y = normalize(m + d) [P][3]; with a target t: per-pixel |y - t|^2, its mean in *loss (device) and
  * dL/dd [P][3] in gd */
 int maf_nn_head(const float* m, const float* d, int ldd, const float* t, long long P, float* y, float* gd,

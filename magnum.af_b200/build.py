@@ -38,6 +38,7 @@ SOURCES = {
     "batch.o": ("batch.cu", []),
     "umma.o": ("umma.cu", []),
     "nn.o": ("nn.cu", []),
+    "conv.o": ("conv.cu", []),
 }
 for _part in (1, 2, 3, 4, 5):
     for _real in (4, 8):

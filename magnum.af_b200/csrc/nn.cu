@@ -157,12 +157,14 @@ __global__ void k_up_cat_bwd_a(const float* __restrict__ dcat, int Cp, int Ca, i
     }
 }
 
+// dst (+)= channels off .. off + C - 1 of src
 __global__ void k_add_channels(const float* __restrict__ src, int lds, int off, int64_t P, int C,
-                               float* __restrict__ dst) {
+                               float* __restrict__ dst, int accumulate) {
     GRID_STRIDE(i, P * C) {
         const int64_t p = i / C;
         const int c = (int)(i - p * C);
-        dst[i] += src[p * lds + off + c];
+        const float v = src[p * lds + off + c];
+        dst[i] = accumulate ? dst[i] + v : v;
     }
 }
 
@@ -293,16 +295,27 @@ __global__ void k_head(const float* __restrict__ m, const float* __restrict__ d,
     }
 }
 
-__global__ void k_mean(const float* __restrict__ v, int64_t n, float* __restrict__ out) {
-    __shared__ double red[kT / 32];
+// one block of kMeanT threads, sixteen values in flight per thread (a block of 256 with one
+// load in flight took longer than the head itself)
+constexpr int kMeanT = 1024;
+__global__ void __launch_bounds__(kMeanT) k_mean(const float* __restrict__ v, int64_t n, float* __restrict__ out) {
+    __shared__ double red[kMeanT / 32];
     double s = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s += v[i];
+    int64_t i = threadIdx.x;
+    for (; i + 15 * kMeanT < n; i += 16 * kMeanT) {
+        float x[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) x[k] = v[i + k * kMeanT];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) s += x[k];
+    }
+    for (; i < n; i += kMeanT) s += v[i];
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
         double t = 0.0;
-        for (int k = 0; k < kT / 32; ++k) t += red[k];
+        for (int k = 0; k < kMeanT / 32; ++k) t += red[k];
         *out = (float)(t / (double)n);
     }
 }
@@ -402,14 +415,25 @@ int maf_nn_up_cat(const float* a, int Ca, const float* s, int Cs, int B, int H, 
     });
 }
 
-int maf_nn_up_cat_bwd(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
-                      void* st) {
+static int up_cat_bwd(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
+                      int accumulate, void* st) {
     return run([&] {
         k_up_cat_bwd_a<<<grid_for((int64_t)B * (H / 2) * (W / 2) * Ca), kT, 0, S(st)>>>(dcat, Cp, Ca, B, H, W, da);
         MAF_LAUNCH_CHECK();
-        k_add_channels<<<grid_for((int64_t)B * H * W * Cs), kT, 0, S(st)>>>(dcat, Cp, Ca, (int64_t)B * H * W, Cs, ds);
+        k_add_channels<<<grid_for((int64_t)B * H * W * Cs), kT, 0, S(st)>>>(dcat, Cp, Ca, (int64_t)B * H * W, Cs, ds,
+                                                                            accumulate);
         MAF_LAUNCH_CHECK();
     });
+}
+
+int maf_nn_up_cat_bwd(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
+                      void* st) {
+    return up_cat_bwd(dcat, Cp, Ca, Cs, B, H, W, da, ds, 1, st);
+}
+
+int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
+                          void* st) {
+    return up_cat_bwd(dcat, Cp, Ca, Cs, B, H, W, da, ds, 0, st);
 }
 
 int maf_nn_relu_bwd(const float* dA, const float* A, long long P, int C, int relu, float* dY, void* dYb, int Cp,
@@ -464,7 +488,7 @@ int maf_nn_head(const float* m, const float* d, int ldd, const float* tgt, long 
         k_head<<<grid_for(P), kT, 0, S(st)>>>(m, d, ldd, tgt, P, y, gd, cell_loss);
         MAF_LAUNCH_CHECK();
         if (tgt && loss) {
-            k_mean<<<1, kT, 0, S(st)>>>(cell_loss, P, loss);
+            k_mean<<<1, kMeanT, 0, S(st)>>>(cell_loss, P, loss);
             MAF_LAUNCH_CHECK();
         }
     });

@@ -175,6 +175,15 @@ DevBuf g_umma_err;  // device error flag of the tensor-core GEMM (one per proces
 
 }  // namespace
 
+// The error flag, zeroed on first use.
+int* umma_error_flag() {
+    if (!g_umma_err.p) {
+        g_umma_err.alloc(sizeof(int));
+        MAF_CUDA(cudaMemset(g_umma_err.p, 0, sizeof(int)));
+    }
+    return g_umma_err.as<int>();
+}
+
 // Host launcher (nn.cu and the C ABI): the tile width follows N; with splits > 1
 // the K range is cut into that many chunks whose partial products land in
 // consecutive slabs C + s M ldc (the caller sums them).
@@ -186,11 +195,7 @@ void umma_gemm(const void* A, int lda, const void* B, int ldb, float* C, int ldc
     splits = (int)ceil_div(K, kchunk);
     if (K % 8 || lda % 8 || ldb % 8 || lda < K || ldb < K || ldc < N || ((uintptr_t)A | (uintptr_t)B) % 16)
         throw Error(1, "bf16 gemm: K and the row strides must be multiples of 8 elements, rows 16-byte aligned");
-    if (!g_umma_err.p) {
-        g_umma_err.alloc(sizeof(int));
-        MAF_CUDA(cudaMemset(g_umma_err.p, 0, sizeof(int)));
-    }
-    int* err = g_umma_err.as<int>();
+    int* err = umma_error_flag();
     const auto* a = static_cast<const __nv_bfloat16*>(A);
     const auto* b = static_cast<const __nv_bfloat16*>(B);
     const unsigned gx = (unsigned)ceil_div(M, kBM);

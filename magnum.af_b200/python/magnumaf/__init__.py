@@ -154,6 +154,12 @@ _SIGS = {
     "maf_nn_colsum": (_I, [_P, C.c_longlong, _I, _P, _P]),
     "maf_nn_wcast": (_I, [_P, _I, _I, _I, _I, _P, _P, _P]),
     "maf_nn_wgrad": (_I, [_P, _I, _I, _I, _P, _P]),
+    "maf_nn_conv": (_I, [_P, _I, _I, _I, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P]),
+    "maf_nn_conv_wgrad": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _I, _P, _I, _P, _P]),
+    "maf_nn_wcast_conv": (_I, [_P, _I, _I, _I, _I, _P, _P, _P]),
+    "maf_nn_relu_bias_bwd": (_I, [_P, _P, C.c_longlong, _I, _I, _P, _I, _P, _P, _P]),
+    "maf_nn_relu_bias_bwd_parts": (_I, [C.POINTER(_I)]),
+    "maf_nn_up_cat_bwd_set": (_I, [_P, _I, _I, _I, _I, _I, _I, _P, _P, _P]),
     "maf_nn_head": (_I, [_P, _P, _I, _P, C.c_longlong, _P, _P, _P, _P, _P]),
     "maf_nn_adam": (_I, [_P, _P, _P, _P, C.c_longlong, C.c_float, _I, _P]),
     "maf_stoch_batch_is_fused": (_I, [_P, C.POINTER(_I)]),

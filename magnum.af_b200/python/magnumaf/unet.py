@@ -1,10 +1,11 @@
 """U-net of the learned warm start, on the library's own CUDA kernels.
 
-Convolutions are implicit GEMMs: an im2col tile and the weights in BF16 go
-through the tensor-core GEMM (tcgen05.mma, FP32 accumulation in tensor memory,
-``maf_nn_gemm``); bias, ReLU, pooling, upsampling, the skip concatenations, the
-normalising head, every backward pass and Adam are the hand-written kernels of
-``nn.cu``.  Master weights are FP32 (Adam updates them); the GEMMs read their
+Convolutions are implicit GEMMs (``conv.cu``): the taps are gathered from the BF16
+activations into shared memory and multiplied on the tensor cores (tcgen05.mma, FP32
+accumulation in tensor memory), bias, ReLU and the next layer's BF16 input in the
+epilogue; the data and weight gradients are the same gather.  Pooling, upsampling, the
+skip concatenations, the normalising head, their backward passes and Adam are the
+hand-written kernels of ``nn.cu``.  Master weights are FP32 (Adam updates them); the GEMMs read their
 BF16 copies.  PyTorch only holds the device buffers (allocation, views); no
 torch operation computes anything here.
 
@@ -44,8 +45,8 @@ class _Conv:
 
     def __init__(self, cin, cout, level, relu, off):
         self.cin, self.cout, self.level, self.relu = cin, cout, level, relu
-        self.cp = _r8(cin)          # padded input channels of the im2col tile
-        self.coutp = _r8(cout)      # padded output channels of the data-gradient GEMM
+        self.cp = _r8(cin)          # padded input channels
+        self.coutp = _r8(cout)      # padded output channels of the gradients
         self.woff = off             # offset of W [cout][9][cin] in the flat parameters
         self.boff = off + cout * 9 * cin
         self.n = cout * 9 * cin + cout
@@ -105,16 +106,16 @@ class UNet:
         return _P(self.torch.cuda.current_stream().cuda_stream)
 
     def _cast_weights(self):
-        """BF16 copies of every layer's weights: Wb [cout][9 cp] and WtB [9 cp][coutp]."""
+        """BF16 copies of every layer's weights: [cout][9 cp] (forward) and [cin][9 coutp] (data gradient)."""
         torch = self.torch
         st = self._stream()
         for i, L in enumerate(self.layers):
             if self._wb[i] is None:
                 self._wb[i] = (torch.empty((L.cout, 9 * L.cp), dtype=torch.bfloat16, device="cuda"),
-                               torch.empty((9 * L.cp, L.coutp), dtype=torch.bfloat16, device="cuda"))
-            wb, wtb = self._wb[i]
-            _ck(lib.maf_nn_wcast(_P(_p(self.params) + 4 * L.woff), L.cout, L.cin, L.cp, L.coutp, _P(_p(wb)),
-                                 _P(_p(wtb)), st))
+                               torch.empty((L.cin, 9 * L.coutp), dtype=torch.bfloat16, device="cuda"))
+            wf, wd = self._wb[i]
+            _ck(lib.maf_nn_wcast_conv(_P(_p(self.params) + 4 * L.woff), L.cout, L.cin, L.cp, L.coutp, _P(_p(wf)),
+                                      _P(_p(wd)), st))
         self._dirty = False
 
     # ------------------------------------------------------------ buffers
@@ -134,41 +135,34 @@ class UNet:
         self.m_in = z(P[0], 3)
         self.pool1 = z(P[1], self.widths[0])
         self.pool2 = z(P[2], self.widths[1])
-        kmax = max(9 * L.cp * P[L.level] for L in self.layers)
-        self.col = torch.zeros(kmax, dtype=b16, device="cuda")
-        self.colT = torch.zeros(kmax, dtype=b16, device="cuda")
-        self.gemm = torch.zeros(max(max(P[L.level] * L.coutp, P[L.level] * 9 * L.cp) for L in self.layers),
-                                dtype=f32, device="cuda")
         self.y = z(P[0], 3)
         # backward
         self.dA = [z(P[L.level], L.cout) for L in self.layers]
-        self.dY = z(max(P[L.level] * L.cout for L in self.layers))
         self.dYb = torch.zeros(max(P[L.level] * L.coutp for L in self.layers), dtype=b16, device="cuda")
-        self.dYbT = torch.zeros_like(self.dYb)
         self.dX = z(max(P[L.level] * L.cp for L in self.layers))
         self.gd = z(P[0], 3)
         self.cell_loss = z(P[0])
         self.loss = z(1)
-        self.splits = 64
-        self.work = z(self.splits * max(L.cout * 9 * L.cp for L in self.layers))
-        self.wg = z(max(L.cout * 9 * L.cp for L in self.layers))
+        # the weight gradients' partial sums: about 592 CTAs of 128 x 128, at least 256 pixels each
+        tiles = lambda L: -(-9 * L.cp // 128) * -(-L.coutp // 128)
+        self.splits = [max(1, min(-(-592 // tiles(L)), -(-P[L.level] // 256))) for L in self.layers]
+        self.work = z(max(s * 9 * L.cp * L.coutp for s, L in zip(self.splits, self.layers)))
+        n = C.c_int()
+        _ck(lib.maf_nn_relu_bias_bwd_parts(C.byref(n)))
+        self.bpart = torch.zeros(n.value * max(L.cout for L in self.layers), dtype=torch.float64, device="cuda")
         self._shape = (B, H, W)
 
     # ------------------------------------------------------------ forward
     def _conv_fwd(self, i, B):
         L = self.layers[i]
-        P = self.P[L.level]
         h, w = self.dims[L.level]
         st = self._stream()
-        wb, _ = self._wb[i]
-        _ck(lib.maf_nn_im2col(_P(_p(self.inb[i])), B, h, w, L.cp, _P(_p(self.col)), 0, st))
-        _ck(lib.maf_nn_gemm(_P(_p(self.col)), 9 * L.cp, _P(_p(wb)), 9 * L.cp, _P(_p(self.gemm)), L.cout, P, L.cout,
-                            9 * L.cp, st))
+        wf, _ = self._wb[i]
         nxt = self.inb[i + 1] if i + 1 < len(self.layers) and self.layers[i + 1].cin == L.cout and \
             self.layers[i + 1].level == L.level else None
-        _ck(lib.maf_nn_bias_act(_P(_p(self.gemm)), L.cout, _P(_p(self.params) + 4 * L.boff), P, L.cout,
-                                int(L.relu), _P(_p(self.out[i])), _P(_p(nxt)) if nxt is not None else None,
-                                self.layers[i + 1].cp if nxt is not None else L.coutp, st))
+        _ck(lib.maf_nn_conv(_P(_p(self.inb[i])), B, h, w, L.cp, _P(_p(wf)), L.cout, _P(_p(self.params) + 4 * L.boff),
+                            int(L.relu), _P(_p(self.out[i])), L.cout, _P(_p(nxt)) if nxt is not None else None,
+                            self.layers[i + 1].cp if nxt is not None else 0, st))
 
     def _forward(self, x_ptr, B, H, W):
         self._buffers(B, H, W)
@@ -211,26 +205,19 @@ class UNet:
     def _conv_bwd(self, i, B, dx=None, dx_channels=0):
         """dA[i] (FP32 [P][cout]) -> parameter gradients of layer i and, when dx is
         given, the gradient of its input into dx (FP32 [P][dx_channels], the first
-        dx_channels of the cp im2col channels)."""
+        dx_channels of the layer's input channels)."""
         L = self.layers[i]
         P = self.P[L.level]
         h, w = self.dims[L.level]
         st = self._stream()
-        _, wtb = self._wb[i]
-        _ck(lib.maf_nn_relu_bwd(_P(_p(self.dA[i])), _P(_p(self.out[i])), P, L.cout, int(L.relu), _P(_p(self.dY)),
-                                _P(_p(self.dYb)), L.coutp, st))
-        _ck(lib.maf_nn_colsum(_P(_p(self.dY)), P, L.cout, _P(_p(self.grad) + 4 * L.boff), st))
-        # dW [cout][9 cp] = dY^T . col: both operands with the pixels contiguous
-        _ck(lib.maf_nn_transpose(_P(_p(self.dYb)), P, L.coutp, _P(_p(self.dYbT)), st))
-        _ck(lib.maf_nn_im2col(_P(_p(self.inb[i])), B, h, w, L.cp, _P(_p(self.colT)), 1, st))
-        _ck(lib.maf_nn_gemm_splitk(_P(_p(self.dYbT)), P, _P(_p(self.colT)), P, _P(_p(self.wg)), L.cout, 9 * L.cp, P,
-                                   self.splits, _P(_p(self.work)), st))
-        _ck(lib.maf_nn_wgrad(_P(_p(self.wg)), L.cout, L.cin, L.cp, _P(_p(self.grad) + 4 * L.woff), st))
+        _, wd = self._wb[i]
+        _ck(lib.maf_nn_relu_bias_bwd(_P(_p(self.dA[i])), _P(_p(self.out[i])), P, L.cout, int(L.relu),
+                                     _P(_p(self.dYb)), L.coutp, _P(_p(self.grad) + 4 * L.boff), _P(_p(self.bpart)), st))
+        _ck(lib.maf_nn_conv_wgrad(_P(_p(self.inb[i])), B, h, w, L.cp, L.cin, _P(_p(self.dYb)), L.cout, L.coutp,
+                                  _P(_p(self.work)), self.splits[i], _P(_p(self.grad) + 4 * L.woff), st))
         if dx is not None:
-            # dcol [P][9 cp] = dY . W, then col2im
-            _ck(lib.maf_nn_gemm(_P(_p(self.dYb)), L.coutp, _P(_p(wtb)), L.coutp, _P(_p(self.gemm)), 9 * L.cp, P,
-                                9 * L.cp, L.coutp, st))
-            _ck(lib.maf_nn_col2im(_P(_p(self.gemm)), B, h, w, L.cp, dx_channels, _P(_p(dx)), 0, st))
+            _ck(lib.maf_nn_conv(_P(_p(self.dYb)), B, h, w, L.coutp, _P(_p(wd)), dx_channels, None, 0, _P(_p(dx)),
+                                dx_channels, None, 0, st))
 
     def _backward(self, B):
         st = self._stream()
@@ -238,13 +225,13 @@ class UNet:
         H, W = self.dims[0]
         H1, W1 = self.dims[1]
         self._conv_bwd(8, B, self.dA[7], w1)
-        self._conv_bwd(7, B, self.dX, self.layers[7].cp)   # d cat(up(u2), e1) [P0][w2 + w1]
+        self._conv_bwd(7, B, self.dX, self.layers[7].cin)   # d cat(up(u2), e1) [P0][w2 + w1]
         # e1 = out[1] gets its skip part here and its pooled-path part below
-        _ck(lib.maf_nn_up_cat_bwd(_P(_p(self.dX)), self.layers[7].cp, w2, w1, B, H, W, _P(_p(self.dA[6])),
-                                  _P(_p(self.dA[1].zero_())), st))
-        self._conv_bwd(6, B, self.dX, self.layers[6].cp)   # d cat(up(b), e2) [P1][w3 + w2]
-        _ck(lib.maf_nn_up_cat_bwd(_P(_p(self.dX)), self.layers[6].cp, w3, w2, B, H1, W1, _P(_p(self.dA[5])),
-                                  _P(_p(self.dA[3].zero_())), st))
+        _ck(lib.maf_nn_up_cat_bwd_set(_P(_p(self.dX)), self.layers[7].cin, w2, w1, B, H, W, _P(_p(self.dA[6])),
+                                      _P(_p(self.dA[1])), st))
+        self._conv_bwd(6, B, self.dX, self.layers[6].cin)   # d cat(up(b), e2) [P1][w3 + w2]
+        _ck(lib.maf_nn_up_cat_bwd_set(_P(_p(self.dX)), self.layers[6].cin, w3, w2, B, H1, W1, _P(_p(self.dA[5])),
+                                      _P(_p(self.dA[3])), st))
         self._conv_bwd(5, B, self.dA[4], w3)
         self._conv_bwd(4, B, self.dX, w2)                   # d pool2 [P2][w2]
         _ck(lib.maf_nn_pool_bwd(_P(_p(self.dX)), B, H1, W1, w2, _P(_p(self.dA[3])), 1, st))
