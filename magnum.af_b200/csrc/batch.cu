@@ -283,7 +283,8 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
     for (int i = 0; i < M; ++i) {
         Demag* dm = mem[i].demag;
         if (dm->tune.generic) continue;
-        const int Lc = dm->Px() / 2, Py = dm->Py();
+        const DemagPlan<R> pl = dm->plan<R>(st);
+        const int Lc = pl.Px / 2, Py = pl.Py;
         const int run = dm->tune.xinv_run ? dm->tune.xinv_run : 2;
         if (ct_batch_tile<R>(0, Lc) > 0) {
             CtClass& c = ct_class(cx, Lc, 0);
@@ -297,7 +298,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
             pos_c[i] = (int)c.members.size();
             c.members.push_back(i);
         }
-        if (ct_batch_tile<R>(2, Lc) > 0 && mem[i].md.nx == Lc) {
+        if (ct_batch_tile<R>(2, Lc) > 0) {
             CtClass& c = ct_class(ci, Lc, run);
             ci_of[i] = (int)(&c - ci.data());
             pos_i[i] = (int)c.members.size();
@@ -316,8 +317,9 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
         Demag* dm = f.demag;
         const int nx = f.md.nx, ny = f.md.ny;
         const int64_t N = f.md.N(), rows_pc = (int64_t)ny * f.md.nz;
-        const int Px = dm->Px(), Py = dm->Py(), Lc = Px / 2, nxh = dm->nxh(), pitch = dm->pitch();
-        C* s1 = dm->spectrum<R>();
+        const DemagPlan<R> pl = dm->plan<R>(st);
+        const int Px = pl.Px, Py = pl.Py, Lc = Px / 2, nxh = pl.nxh, pitch = pl.pitch;
+        C* s1 = pl.s1;
         if (cx_of[i] >= 0) {
             CtClass& c = cx[cx_of[i]];
             if (!c.tw) {
@@ -330,7 +332,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
             CtClass& c = cc[cc_of[i]];
             if (!c.tw) c.tw = ct_batch_twiddles<R>(1, Py, dm->twiddle_tables());
             add_items(wcc[cc_of[i]], pos_c[i], ceil_div(nxh, ct_batch_tile<R>(1, Py)));
-            icv[cc_of[i]][pos_c[i]] = CtConvyItem<R>{s1, dm->tensor_data<R>(), nxh, pitch};
+            icv[cc_of[i]][pos_c[i]] = CtConvyItem<R>{s1, pl.tensor, ny, nxh, pitch};
         }
         if (ci_of[i] >= 0) {
             CtClass& c = ci[ci_of[i]];
@@ -368,7 +370,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
             g.smem = std::max(g.smem, sizeof(C) * (size_t)3 * nbc * spad_len(Py));
             add_items(g.w, i, ceil_div(nxh, nbc));
         }
-        cv[i] = ConvA<R>{s1, dm->tensor_data<R>(), py, ny, (int64_t)pitch, (int64_t)ny * pitch, nxh, nbc, ny, 1, nxh};
+        cv[i] = ConvA<R>{s1, pl.tensor, py, ny, (int64_t)pitch, (int64_t)ny * pitch, nxh, nbc, ny, 1, nxh};
         // x inverse + LLG epilogue (inverse_x_epilogue's generic shape)
         int nbr = pick_nb(3 * Lc, tile_target<R>(), (int)std::min<int64_t>(rows_pc, 1 << 20), 32);
         while (true) {
@@ -389,7 +391,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
         MsInfo ms;
         ms.Ms = f.Ms;
         const C* twP = static_cast<const C*>(dm->twiddles(Px, f64));
-        const R scale = (R)(1.0 / ((double)Px * Py * dm->Pz()));
+        const R scale = (R)(1.0 / ((double)Px * Py * pl.Pz));
         for (int p = 0; p < 2; ++p) {
             const double* mp = f.m[p];
             double* mo = f.m[1 - p];
@@ -425,7 +427,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
                 if (ci_of[i] >= 0) {
                     const size_t nc = ci[ci_of[i]].members.size();
                     CtXinvItem<R> it{s1, pitch, f.md.geom(), scale, in, ms, tl, ep, 0};
-                    ct_batch_xinv_prepare<R>(it);
+                    ct_batch_xinv_prepare<R>(it, ci[ci_of[i]].run);
                     ixi[ci_of[i]][((size_t)p * S + s) * nc + pos_i[i]] = it;
                 }
                 CombA c{};

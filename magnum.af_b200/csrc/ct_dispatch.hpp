@@ -1,6 +1,8 @@
 // Compile-time specialised demag passes (fields_ct.cu).  Each returns false when
 // no specialisation exists for the transform length; the caller then runs the
-// generic kernel of fields.cu.
+// generic kernel of fields.cu.  The transform may be longer than twice the mesh:
+// n_in or n_out of the y passes below L/2, nz (ny) planes (rows) of a z (y)
+// convolution of length L with ny = Py/2, and rows of fewer than Px/2 cells.
 #pragma once
 #include "engine.hpp"
 
@@ -13,10 +15,10 @@ template <typename R, int DIR>
 bool ct_cols(const cplx_t<R>* in, cplx_t<R>* out, int L, int n_in, int n_out, int ncols, int64_t in_si, int64_t out_si,
              int64_t in_sbat, int64_t out_sbat, int nbat, Twiddles& tw, const TuneChoice& tc, cudaStream_t st);
 template <typename R>
-bool ct_convz(cplx_t<R>* S, const R* Nred, int nz, int ny, int nxh, int pitch, Twiddles& tw, const TuneChoice& tc,
-              cudaStream_t st);
+bool ct_convz(cplx_t<R>* S, const R* Nred, int nz, int L, int ny, int nxh, int pitch, Twiddles& tw,
+              const TuneChoice& tc, cudaStream_t st);
 template <typename R>
-bool ct_convy(cplx_t<R>* S, const R* Nred, int ny, int nxh, int pitch, Twiddles& tw, cudaStream_t st);
+bool ct_convy(cplx_t<R>* S, const R* Nred, int ny, int L, int nxh, int pitch, Twiddles& tw, cudaStream_t st);
 // (the lengths are instantiated in three groups G)
 template <typename R, int G>
 bool ct_xinv_group(const cplx_t<R>* S1, int pitch, int Px, Twiddles& tw, const Geom& g, R scale, const R* m,
@@ -46,7 +48,7 @@ template <typename R> struct CtXfwdItem {
 template <typename R> struct CtConvyItem {
     cplx_t<R>* S;
     const R* Nred;
-    int nxh, pitch;
+    int ny, nxh, pitch;
 };
 template <typename R> struct CtXinvItem {
     const cplx_t<R>* S1;
@@ -57,7 +59,7 @@ template <typename R> struct CtXinvItem {
     MsInfo ms;
     TermList tl;
     EpilogueArgs ep;  // EPI_LLG
-    int run4;
+    int run;  // run_mode
 };
 // pass: 0 x forward (L = Px / 2), 1 y convolution (L = Py), 2 x inverse (L = Px / 2).
 // Rows (x passes) or kx columns (y convolution) per tile; 0: no compile-time kernel.
@@ -65,7 +67,7 @@ template <typename R> int ct_batch_tile(int pass, int L);
 // The twiddle table the pass's kernel of length L reads (created on first use).
 template <typename R> const void* ct_batch_twiddles(int pass, int L, Twiddles& tw);
 // The run-epilogue flag and constants of an x-inverse item (as the per-state launch prepares them).
-template <typename R> void ct_batch_xinv_prepare(CtXinvItem<R>& it);
+template <typename R> void ct_batch_xinv_prepare(CtXinvItem<R>& it, int run);
 // Launches; tw from ct_batch_twiddles, twP the length-Px table (Twiddles::get).
 template <typename R>
 void ct_batch_xfwd(const CtXfwdItem<R>* items, const int2* work, int nwork, int L, const void* tw, const void* twP,

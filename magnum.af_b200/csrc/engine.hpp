@@ -142,6 +142,15 @@ struct TuneChoice {
     int generic = 0;    // 1: the run-time-plan kernels for every pass (as the batched passes run)
 };
 
+// Transform lengths, buffers and tensor that an evaluation runs with.
+template <typename R> struct DemagPlan {
+    int Px = 0, Py = 0, Pz = 0, nxh = 0, pitch = 0;
+    bool padded = false;      // longer than twice the mesh (Demag::padded_)
+    const R* tensor = nullptr;  // [ncomp][Pz/2+1][Py/2+1][nxh]
+    cplx_t<R>* s1 = nullptr;
+    cplx_t<R>* s2 = nullptr;
+};
+
 // Demag plan: the symmetry-reduced real spectral Newell tensor and the
 // spectral work buffers for one mesh.
 class Demag {
@@ -174,24 +183,32 @@ class Demag {
     size_t tensor_elems() const { return (size_t)ncomp() * (md_.nz == 1 ? 1 : md_.nz + 1) * (md_.ny + 1) * nxh(); }
     int pitch() const { return pitch_; }
     template <typename R> int edens_blocks() const;
-    // buffers and tables of the generic passes, for the batched passes (batch.cu)
-    template <typename R> cplx_t<R>* spectrum() { return S1<R>(); }
-    template <typename R> const R* tensor_data() { return tensor<R>(); }
+    // the plan of an evaluation at the current kernel choices; its tensor and buffers are made on first use
+    template <typename R> DemagPlan<R> plan(cudaStream_t st);
     const void* twiddles(int L, bool fp64) { return tw_.get(L, fp64); }
     Twiddles& twiddle_tables() { return tw_; }
 
   private:
     template <typename R> const R* tensor() ;
-    template <typename R> cplx_t<R>* S1();
-    template <typename R> cplx_t<R>* S2();
+    template <typename R> cplx_t<R>* S1(int pitch);
+    template <typename R> cplx_t<R>* S2(int Py, int pitch);
     void build_tensor(cudaStream_t st);
-    void transform_octant(const double* oct, int comp, int Lx, int Ly, int Lz, double* quad, double scale, DevBuf* work,
-                          cudaStream_t st);
+    void build_padded_tensor(double* out64, float* out32, cudaStream_t st);
+    void transform_octant(const double* oct, int o0, int o1, int o2, int comp, int Lx, int Ly, int Lz, double* quad,
+                          double scale, char* work, cudaStream_t st);
+    size_t padded_elems() const {
+        return (size_t)ncomp() * (pad_z_ == 1 ? 1 : pad_z_ / 2 + 1) * (pad_y_ / 2 + 1) * (pad_x_ / 2 + 1);
+    }
 
     MeshDims md_;
     bool pbc_ = false;
     int pitch_;  // complex row pitch of the half spectrum (>= nxh)
-    DevBuf Nred64_, Nred32_;
+    // Zero padding to any length of at least 2n - 1 gives the same linear convolution, so
+    // a mesh whose doubled sizes have no compile-time kernels is padded to the next lengths
+    // that have them; the tensor at those lengths is made from Nred64_ on first use.
+    bool padded_ = false;
+    int pad_x_ = 0, pad_y_ = 0, pad_z_ = 0;
+    DevBuf Nred64_, Nred32_, Npad64_, Npad32_;
     DevBuf S1_64_, S2_64_, S1_32_, S2_32_;
     Twiddles tw_;
 };

@@ -199,13 +199,14 @@ __global__ void __launch_bounds__(256) k_local_epi(Geom g, const R* __restrict__
 }
 
 // Local terms only, in runs of RN consecutive cells along x: the x-inverse's
-// run epilogue with a zero demag contribution (eligibility: run4_eligible).
+// run epilogue with a zero demag contribution (eligibility: run_mode).
 // Thread q takes run q of the flattened (row, run) index (fewer than 2^31 runs).
 // FP32: capped for two CTAs per SM (128 registers); FP64 uncapped (it would spill).
-template <typename R, int EPI, int RN>
-__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_local_run(Geom g, const R* __restrict__ m, TermList tl, EpilogueArgs ep,
-                                                   int nruns) {
+template <typename R, int EPI, int RN, bool MSF>
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_local_run(Geom g, const R* __restrict__ m, MsInfo ms, TermList tl,
+                                                                           EpilogueArgs ep, int nruns) {
     const int runs_row = g.nx / RN;
+    double eacc = 0;
     R hd[RN][3];
 #pragma unroll
     for (int i = 0; i < RN; ++i) hd[i][0] = hd[i][1] = hd[i][2] = (R)0;
@@ -217,8 +218,15 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_local_run(Geom 
         const int64_t cell0 = (int64_t)row * g.nx + x0;
         RunN<R, RN> r;
         runN_load<R, RN>(m, g, x0, y, z, cell0, r);
-        runN_epilogue<R, EPI, RN>(tl, g, r, cell0, hd, ep);
+        double Ms = ms.Ms;
+        if constexpr (MSF) {
+            Ms = ms.field64[cell0];
+            r.ms = cell_Ms<R>(ms, cell0);
+            r.inv = (R)1 / r.ms;
+        }
+        eacc += runN_epilogue<R, EPI, RN, MSF>(tl, g, r, cell0, hd, ep, Ms);
     }
+    if constexpr (EPI == EPI_EDENS || EPI == EPI_EGRAD) block_sum_store(eacc, ep.partials);
 }
 
 __global__ void k_sum_partials(const double* __restrict__ p, int n, double* out) {
@@ -280,10 +288,10 @@ __device__ __forceinline__ int wrap_offset(int i, int L, bool odd, bool& neg, bo
     return j;
 }
 
-// rows [nz][ny][L] of real values from the octant [nz][ny][o0]: the x axis
-// completed by parity; rows on the zero planes of the other axes are zero
-__global__ void k_tensor_rows(const double* __restrict__ oct, double* __restrict__ out, int comp, int o0, int ny,
-                              int nz, int Ly, int Lz, int L) {
+// rows [nz][ny][L] of real values from the octant [o2][o1][o0] (zero beyond it): the
+// x axis completed by parity; rows on the zero planes of the other axes are zero
+__global__ void k_tensor_rows(const double* __restrict__ oct, double* __restrict__ out, int comp, int o0, int o1,
+                              int o2, int ny, int nz, int Ly, int Lz, int L) {
     const int64_t total = (int64_t)L * ny * nz;
     const bool ox = tensor_odd(comp, 0), oy = tensor_odd(comp, 1), oz = tensor_odd(comp, 2);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -292,7 +300,7 @@ __global__ void k_tensor_rows(const double* __restrict__ oct, double* __restrict
         const int y = (int)(r % ny), z = (int)(r / ny);
         bool neg = false, zero = (oy && (y == 0 || 2 * y == Ly)) || (oz && (z == 0 || 2 * z == Lz));
         const int j = wrap_offset(x, L, ox, neg, zero);
-        const double v = zero || j >= o0 ? 0.0 : oct[r * o0 + j];
+        const double v = zero || j >= o0 || y >= o1 || z >= o2 ? 0.0 : oct[((int64_t)z * o1 + y) * o0 + j];
         out[i] = neg ? -v : v;
     }
 }
@@ -411,6 +419,20 @@ static void launch_cols(const cplx_t<R>* in, cplx_t<R>* out, int L, int n_in, in
 // ---------------------------------------------------------------------------
 // Demag
 // ---------------------------------------------------------------------------
+// Lengths of the compile-time passes: packed x rows, y convolutions (2-D meshes), y
+// passes (3-D) and z convolutions.
+static const int kCtX[] = {16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 0};
+static const int kCtY2[] = {16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 0};
+static const int kCtY3[] = {16, 32, 64, 96, 128, 192, 256, 384, 512, 768, 1024, 1536, 2048, 4096, 0};
+static const int kCtZ[] = {8, 16, 32, 64, 96, 128, 0};
+
+// the smallest length of the list that is at least n, 0 if there is none
+static int ct_length(const int* list, int n) {
+    for (; *list; ++list)
+        if (*list >= n) return *list;
+    return 0;
+}
+
 Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, bool pbc) : md_(md), pbc_(pbc) {
     if (md.nx < 1 || md.ny < 1 || md.nz < 1) throw Error(1, "DemagField: empty mesh");
     if (pbc) {
@@ -425,6 +447,10 @@ Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, boo
     }
     // complex pitch: multiple of 4 so that tiles of 4 complex values start on 32 B
     pitch_ = (nxh() + 3) / 4 * 4;
+    pad_x_ = 2 * ct_length(kCtX, md.nx);
+    pad_y_ = md.nz == 1 ? ct_length(kCtY2, 2 * md.ny - 1) : ct_length(kCtY3, 2 * md.ny - 1);
+    pad_z_ = md.nz == 1 ? 1 : ct_length(kCtZ, 2 * md.nz - 1);
+    padded_ = pad_x_ && pad_y_ && pad_z_ && (pad_x_ != Px() || pad_y_ != Py() || pad_z_ != Pz());
     // validate all FFT lengths early
     make_fft_plan(Px() / 2, nullptr);
     make_fft_plan(Py(), nullptr);
@@ -440,23 +466,33 @@ Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, boo
 
 // Real spectrum (times scale) on the quadrant [Lz/2+1][Ly/2+1][Lx/2+1] (Lz = 1: one
 // plane) of the periodic function of lengths (Lx, Ly, Lz) that a tensor component's
-// octant `oct` [z][y][x] (the same quadrant of offsets) completes by parity.  Each
+// octant `oct` [o2][o1][o0] completes by parity.  The spectrum has the component's
+// parity, so the transform of its quadrant over L values, divided by L, is the octant.  Each
 // axis is completed just before its transform, so the x transforms run on a quarter
 // of the rows, the y transforms on half of the planes and the z transforms on half of
-// the rows.  work: two buffers kept between calls.
-void Demag::transform_octant(const double* oct, int comp, int Lx, int Ly, int Lz, double* quad, double scale,
-                             DevBuf* work, cudaStream_t st) {
+// the rows.  work: octant_work bytes.
+static size_t octant_work_a(int Lx, int Ly, int Lz) {
+    // the completed real rows, then the completed y columns
+    const int Ky = Ly / 2 + 1, Kz = Lz == 1 ? 1 : Lz / 2 + 1, pitch = (Lx / 2 + 4) / 4 * 4;
+    return (std::max(sizeof(double) * (size_t)Lx * Ky * Kz, sizeof(double2) * (size_t)Kz * Ly * pitch) + 255) / 256 * 256;
+}
+static size_t octant_work(int Lx, int Ly, int Lz) {
+    // and the x spectra, then the completed z columns
+    const int Ky = Ly / 2 + 1, Kz = Lz == 1 ? 1 : Lz / 2 + 1, pitch = (Lx / 2 + 4) / 4 * 4;
+    const size_t b = sizeof(double2) * (size_t)std::max<int64_t>((int64_t)Ky * Kz, Lz > 1 ? (int64_t)Lz * Ky : 0) * pitch;
+    return octant_work_a(Lx, Ly, Lz) + (b + 255) / 256 * 256;
+}
+
+void Demag::transform_octant(const double* oct, int o0, int o1, int o2, int comp, int Lx, int Ly, int Lz, double* quad,
+                             double scale, char* work, cudaStream_t st) {
     const int nxh = Lx / 2 + 1, Ky = Ly / 2 + 1, Kz = Lz == 1 ? 1 : Lz / 2 + 1;
     const int pitch = (nxh + 3) / 4 * 4;
-    const size_t csz = sizeof(double2);
-    // A: the completed real rows, then the completed y columns; B: the x spectra, then the completed z columns
-    work[0].ensure(std::max(sizeof(double) * (size_t)Lx * Ky * Kz, csz * (size_t)Kz * Ly * pitch));
-    work[1].ensure(csz * (size_t)std::max<int64_t>((int64_t)Ky * Kz, Lz > 1 ? (int64_t)Lz * Ky : 0) * pitch);
+    char* work_b = work + octant_work_a(Lx, Ly, Lz);
     auto grid = [](int64_t n) { return (unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16); };
-    double* rows = work[0].as<double>();
-    double2* ycol = work[0].as<double2>();
-    double2* xs = work[1].as<double2>();
-    k_tensor_rows<<<grid((int64_t)Lx * Ky * Kz), 256, 0, st>>>(oct, rows, comp, nxh, Ky, Kz, Ly, Lz, Lx);
+    double* rows = reinterpret_cast<double*>(work);
+    double2* ycol = reinterpret_cast<double2*>(work);
+    double2* xs = reinterpret_cast<double2*>(work_b);
+    k_tensor_rows<<<grid((int64_t)Lx * Ky * Kz), 256, 0, st>>>(oct, rows, comp, o0, o1, o2, Ky, Kz, Ly, Lz, Lx);
     MAF_LAUNCH_CHECK();
     launch_xfwd<double>(rows, Lx, (int64_t)Ky * Kz, (int64_t)Ky * Kz, nullptr, 1.0, xs, pitch, Lx, tw_, st);
     k_tensor_wrap<<<grid((int64_t)Kz * Ly * nxh), 256, 0, st>>>(xs, ycol, Kz, Ly, 1, Ky, 1, tensor_odd(comp, 1),
@@ -465,7 +501,7 @@ void Demag::transform_octant(const double* oct, int comp, int Lx, int Ly, int Lz
     launch_cols<double, -1>(ycol, ycol, Ly, Ly, Ly, nxh, pitch, pitch, (int64_t)Ly * pitch, (int64_t)Ly * pitch, Kz,
                             tw_, tune, st);
     if (Lz > 1) {
-        double2* zcol = work[1].as<double2>();
+        double2* zcol = reinterpret_cast<double2*>(work_b);
         k_tensor_wrap<<<grid((int64_t)Lz * Ky * nxh), 256, 0, st>>>(ycol, zcol, 1, Lz, Ky, 0, Ly,
                                                                     tensor_odd(comp, 2), pitch, nxh);
         MAF_LAUNCH_CHECK();
@@ -479,18 +515,52 @@ void Demag::transform_octant(const double* oct, int comp, int Lx, int Ly, int Lz
     MAF_LAUNCH_CHECK();
 }
 
+// tensor components that are stored, in order
+static const int kComps6[6] = {0, 1, 2, 3, 4, 5};
+static const int kComps4[4] = {0, 1, 3, 5};
+
 void Demag::build_tensor(cudaStream_t st) {
     const int Kx = md_.nx + 1, Ky = md_.ny + 1, Kz = md_.nz == 1 ? 1 : md_.nz + 1;
     const int64_t cstride = (int64_t)Kz * Ky * Kx;
+    const int* comps = md_.nz == 1 ? kComps4 : kComps6;
     Nred64_.alloc(sizeof(double) * cstride * ncomp());
-    DevBuf oct(sizeof(double) * cstride), work[2];
-    const int comps6[6] = {0, 1, 2, 3, 4, 5};
-    const int comps4[4] = {0, 1, 3, 5};
-    const int* comps = md_.nz == 1 ? comps4 : comps6;
+    // one allocation for the octant and the work buffers (each takes 0.5-1 ms above 2 MB)
+    const size_t oct_bytes = (sizeof(double) * cstride + 255) / 256 * 256;
+    DevBuf scratch(oct_bytes + octant_work(Px(), Py(), Pz()));
+    double* oct = scratch.as<double>();
     for (int ci = 0; ci < ncomp(); ++ci) {
-        newell_octant(oct.as<double>(), comps[ci], md_, Kx, Ky, Kz, st);
-        transform_octant(oct.as<double>(), comps[ci], Px(), Py(), Pz(), Nred64_.as<double>() + ci * cstride, 1.0, work,
+        newell_octant(oct, comps[ci], md_, Kx, Ky, Kz, st);
+        transform_octant(oct, Kx, Ky, Kz, comps[ci], Px(), Py(), Pz(), Nred64_.as<double>() + ci * cstride, 1.0,
+                         scratch.as<char>() + oct_bytes, st);
+    }
+    MAF_CUDA(cudaStreamSynchronize(st));
+}
+
+// The tensor at the padded lengths (FP64 or FP32), from the one at twice the mesh
+// (assembled or read from a file: the same values either way): back to its octant of
+// offsets, then forward at the other lengths.
+void Demag::build_padded_tensor(double* out64, float* out32, cudaStream_t st) {
+    const int Kx = md_.nx + 1, Ky = md_.ny + 1, Kz = md_.nz == 1 ? 1 : md_.nz + 1;
+    const int64_t cstride = (int64_t)Kz * Ky * Kx, pstride = (int64_t)padded_elems() / ncomp();
+    const int* comps = md_.nz == 1 ? kComps4 : kComps6;
+    const size_t oct_bytes = (sizeof(double) * cstride + 255) / 256 * 256;
+    const size_t quad_bytes = out32 ? (sizeof(double) * pstride + 255) / 256 * 256 : 0;
+    DevBuf scratch(oct_bytes + quad_bytes +
+                   std::max(octant_work(Px(), Py(), Pz()), octant_work(pad_x_, pad_y_, pad_z_)));
+    double* oct = scratch.as<double>();
+    double* quad = reinterpret_cast<double*>(scratch.as<char>() + oct_bytes);
+    char* work = scratch.as<char>() + oct_bytes + quad_bytes;
+    const double scale = 1.0 / ((double)Px() * Py() * Pz());
+    for (int ci = 0; ci < ncomp(); ++ci) {
+        transform_octant(Nred64_.as<double>() + ci * cstride, Kx, Ky, Kz, comps[ci], Px(), Py(), Pz(), oct, scale, work,
                          st);
+        transform_octant(oct, Kx, Ky, Kz, comps[ci], pad_x_, pad_y_, pad_z_, out32 ? quad : out64 + ci * pstride, 1.0,
+                         work, st);
+        if (out32) {
+            k_d2f<<<(unsigned)std::min<int64_t>(ceil_div(pstride, 256), (int64_t)sm_count() * 16), 256, 0, st>>>(
+                quad, out32 + ci * pstride, pstride);
+            MAF_LAUNCH_CHECK();
+        }
     }
     MAF_CUDA(cudaStreamSynchronize(st));
 }
@@ -532,21 +602,64 @@ template <> const float* Demag::tensor<float>() {
     return Nred32_.as<float>();
 }
 
-template <> cplx_t<double>* Demag::S1<double>() {
-    S1_64_.ensure(sizeof(double2) * 3 * md_.N() / md_.nx * pitch_);
+template <> cplx_t<double>* Demag::S1<double>(int pitch) {
+    S1_64_.ensure(sizeof(double2) * 3 * md_.N() / md_.nx * pitch);
     return S1_64_.as<double2>();
 }
-template <> cplx_t<float>* Demag::S1<float>() {
-    S1_32_.ensure(sizeof(float2) * 3 * md_.N() / md_.nx * pitch_);
+template <> cplx_t<float>* Demag::S1<float>(int pitch) {
+    S1_32_.ensure(sizeof(float2) * 3 * md_.N() / md_.nx * pitch);
     return S1_32_.as<float2>();
 }
-template <> cplx_t<double>* Demag::S2<double>() {
-    S2_64_.ensure(sizeof(double2) * 3 * (int64_t)md_.nz * Py() * pitch_);
+template <> cplx_t<double>* Demag::S2<double>(int Py, int pitch) {
+    S2_64_.ensure(sizeof(double2) * 3 * (int64_t)md_.nz * Py * pitch);
     return S2_64_.as<double2>();
 }
-template <> cplx_t<float>* Demag::S2<float>() {
-    S2_32_.ensure(sizeof(float2) * 3 * (int64_t)md_.nz * Py() * pitch_);
+template <> cplx_t<float>* Demag::S2<float>(int Py, int pitch) {
+    S2_32_.ensure(sizeof(float2) * 3 * (int64_t)md_.nz * Py * pitch);
     return S2_32_.as<float2>();
+}
+
+template <typename R> DemagPlan<R> Demag::plan(cudaStream_t st) {
+    DemagPlan<R> p;
+    if (padded_ && !tune.generic) {
+        p.Px = pad_x_;
+        p.Py = pad_y_;
+        p.Pz = pad_z_;
+        p.nxh = pad_x_ / 2 + 1;
+        p.pitch = (p.nxh + 3) / 4 * 4;
+        DevBuf& N = sizeof(R) == 8 ? Npad64_ : Npad32_;
+        try {
+            if (!N.p) {
+                DevBuf t(sizeof(R) * padded_elems());
+                if constexpr (sizeof(R) == 8)
+                    build_padded_tensor(t.as<double>(), nullptr, st);
+                else
+                    build_padded_tensor(nullptr, t.as<float>(), st);
+                N = std::move(t);
+            }
+            p.s1 = S1<R>(p.pitch);
+            p.s2 = md_.nz > 1 ? S2<R>(p.Py, p.pitch) : nullptr;
+            p.tensor = N.as<R>();
+            p.padded = true;
+            return p;
+        } catch (const Error& e) {
+            if (e.code != 3) throw;
+            // no memory for the longer transforms: the mesh's own lengths from here on
+            cudaGetLastError();
+            N.release();
+            padded_ = false;
+        }
+    }
+    p.Px = Px();
+    p.Py = Py();
+    p.Pz = Pz();
+    p.nxh = nxh();
+    p.pitch = pitch_;
+    p.s1 = S1<R>(pitch_);
+    p.s2 = md_.nz > 1 ? S2<R>(Py(), pitch_) : nullptr;
+    // the periodic form has no tensor and runs the run-time plans only
+    p.tensor = pbc_ ? nullptr : tensor<R>();
+    return p;
 }
 
 template <typename R> void Demag::forward_conv(const R* m, const MsInfo& ms, cudaStream_t st, PassMarks* marks) {
@@ -559,26 +672,27 @@ template <typename R> void Demag::forward_conv(const R* m, const MsInfo& ms, cud
         if constexpr (sizeof(R) == 4) msf = reinterpret_cast<const R*>(ms.field32);
         else msf = reinterpret_cast<const R*>(ms.field64);
     }
-    C* s1 = S1<R>();
-    // the periodic form has no tensor and runs the run-time plans only
-    const R* Nr = pbc_ ? nullptr : tensor<R>();
     const bool ct = !pbc_ && !tune.generic;
+    const DemagPlan<R> pl = plan<R>(st);
+    C* s1 = pl.s1;
+    const R* Nr = pl.tensor;
+    const int Py_ = pl.Py, nxh_ = pl.nxh, pitch = pl.pitch;
     const PbcOp pop{nx, ny, nz, md_.dx, md_.dy, md_.dz};
     // pass 1: x forward (zero pad fused)
-    launch_xfwd<R>(m, nx, 3 * rows_pc, rows_pc, msf, (R)ms.Ms, s1, pitch_, Px(), tw_, st, ct);
+    launch_xfwd<R>(m, nx, 3 * rows_pc, rows_pc, msf, (R)ms.Ms, s1, pitch, pl.Px, tw_, st, ct);
     if (marks) marks->mark(st, "x_fwd");
     if (nz > 1) {
-        C* s2 = S2<R>();
+        C* s2 = pl.s2;
         // pass 2: y forward, S1 [3*nz][ny][pitch] -> S2 [3*nz][Py][pitch]
-        launch_cols<R, -1>(s1, s2, Py(), ny, Py(), nxh(), pitch_, pitch_, (int64_t)ny * pitch_,
-                           (int64_t)Py() * pitch_, 3 * nz, tw_, tune, st, ct);
+        launch_cols<R, -1>(s1, s2, Py_, ny, Py_, nxh_, pitch, pitch, (int64_t)ny * pitch,
+                           (int64_t)Py_ * pitch, 3 * nz, tw_, tune, st, ct);
         if (marks) marks->mark(st, "y_fwd");
         // pass 3: z forward . tensor . z inverse, in place on S2
-        if (!ct || !ct_convz<R>(s2, Nr, nz, ny, nxh(), pitch_, tw_, tune, st)) {
-            const int L = Pz();
+        if (!ct || !ct_convz<R>(s2, Nr, nz, pl.Pz, Py_ / 2, nxh_, pitch, tw_, tune, st)) {
+            const int L = pl.Pz;
             FFTPlan fp = make_fft_plan(L, tw_.get(L, f64));
             FFTPlan ip = fp;
-            int nb = pick_nb(3 * L, tile_target<R>(), nxh(), 64);
+            int nb = pick_nb(3 * L, tile_target<R>(), nxh_, 64);
             int threads;
             while (true) {
                 threads = std::max(fft_threads_needed(fp, 3 * nb), std::min(256, 3 * nb * L));
@@ -587,34 +701,34 @@ template <typename R> void Demag::forward_conv(const R* m, const MsInfo& ms, cud
             }
             threads = round_threads(threads);
             const size_t smem = sizeof(C) * (size_t)3 * nb * spad_len(L);
-            dim3 grid((unsigned)ceil_div(nxh(), nb), (unsigned)Py());
+            dim3 grid((unsigned)ceil_div(nxh_, nb), (unsigned)Py_);
             if (pbc_) {
                 set_smem(k_conv<R, true>, smem);
-                k_conv<R, true><<<grid, threads, smem, st>>>(s2, Nr, fp, ip, nz, (int64_t)Py() * pitch_,
-                                                             (int64_t)nz * Py() * pitch_, pitch_, nxh(), nb, 1, ny,
-                                                             nz, nxh(), pop);
+                k_conv<R, true><<<grid, threads, smem, st>>>(s2, Nr, fp, ip, nz, (int64_t)Py_ * pitch,
+                                                             (int64_t)nz * Py_ * pitch, pitch, nxh_, nb, 1, ny,
+                                                             nz, nxh_, pop);
             } else {
                 set_smem(k_conv<R, false>, smem);
-                k_conv<R, false><<<grid, threads, smem, st>>>(s2, Nr, fp, ip, nz, (int64_t)Py() * pitch_,
-                                                              (int64_t)nz * Py() * pitch_, pitch_, nxh(), nb, 1, ny,
-                                                              nz, nxh(), pop);
+                k_conv<R, false><<<grid, threads, smem, st>>>(s2, Nr, fp, ip, nz, (int64_t)Py_ * pitch,
+                                                              (int64_t)nz * Py_ * pitch, pitch, nxh_, nb, 1, ny,
+                                                              nz, nxh_, pop);
             }
             MAF_LAUNCH_CHECK();
         }
         if (marks) marks->mark(st, "z_conv");
         // pass 4: y inverse, S2 -> S1, keep ky rows [0, ny)
-        launch_cols<R, 1>(s2, s1, Py(), Py(), ny, nxh(), pitch_, pitch_, (int64_t)Py() * pitch_,
-                          (int64_t)ny * pitch_, 3 * nz, tw_, tune, st, ct);
+        launch_cols<R, 1>(s2, s1, Py_, Py_, ny, nxh_, pitch, pitch, (int64_t)Py_ * pitch,
+                          (int64_t)ny * pitch, 3 * nz, tw_, tune, st, ct);
         if (marks) marks->mark(st, "y_inv");
     } else {
         // pass 2 (2-D): y forward . tensor . y inverse, in place on S1
-        if (ct && ct_convy<R>(s1, Nr, ny, nxh(), pitch_, tw_, st)) {
+        if (ct && ct_convy<R>(s1, Nr, ny, Py_, nxh_, pitch, tw_, st)) {
             if (marks) marks->mark(st, "y_conv");
             return;
         }
-        const int L = Py();
+        const int L = Py_;
         FFTPlan fp = make_fft_plan(L, tw_.get(L, f64));
-        int nb = pick_nb(3 * L, tile_target<R>(), nxh(), 64);
+        int nb = pick_nb(3 * L, tile_target<R>(), nxh_, 64);
         int threads;
         while (true) {
             threads = std::max(fft_threads_needed(fp, 3 * nb), std::min(256, 3 * nb * L));
@@ -623,15 +737,15 @@ template <typename R> void Demag::forward_conv(const R* m, const MsInfo& ms, cud
         }
         threads = round_threads(threads);
         const size_t smem = sizeof(C) * (size_t)3 * nb * spad_len(L);
-        dim3 grid((unsigned)ceil_div(nxh(), nb), 1);
+        dim3 grid((unsigned)ceil_div(nxh_, nb), 1);
         if (pbc_) {
             set_smem(k_conv<R, true>, smem);
-            k_conv<R, true><<<grid, threads, smem, st>>>(s1, Nr, fp, fp, ny, pitch_, (int64_t)ny * pitch_, 0, nxh(),
-                                                         nb, 0, ny, nz, nxh(), pop);
+            k_conv<R, true><<<grid, threads, smem, st>>>(s1, Nr, fp, fp, ny, pitch, (int64_t)ny * pitch, 0, nxh_,
+                                                         nb, 0, ny, nz, nxh_, pop);
         } else {
             set_smem(k_conv<R, false>, smem);
-            k_conv<R, false><<<grid, threads, smem, st>>>(s1, Nr, fp, fp, ny, pitch_, (int64_t)ny * pitch_, 0, nxh(),
-                                                          nb, 0, ny, nz, nxh(), pop);
+            k_conv<R, false><<<grid, threads, smem, st>>>(s1, Nr, fp, fp, ny, pitch, (int64_t)ny * pitch, 0, nxh_,
+                                                          nb, 0, ny, nz, nxh_, pop);
         }
         MAF_LAUNCH_CHECK();
         if (marks) marks->mark(st, "y_conv");
@@ -645,9 +759,10 @@ void Demag::inverse_x_epilogue(const R* m, const MsInfo& ms, const TermList& tl,
                                cudaStream_t st, int* nblocks_out, PassMarks* marks) {
     const bool f64 = sizeof(R) == 8;
     const int Lc = Px() / 2;
+    const DemagPlan<R> pl = plan<R>(st);
     if (!pbc_ && !tune.generic) {
-        const R scale = (R)(1.0 / ((double)Px() * Py() * Pz()));
-        if (ct_xinv<R>(S1<R>(), pitch_, Px(), tw_, md_.geom(), scale, m, ms, tl, ep, tune, st, nblocks_out)) {
+        const R scale = (R)(1.0 / ((double)pl.Px * pl.Py * pl.Pz));
+        if (ct_xinv<R>(pl.s1, pl.pitch, pl.Px, tw_, md_.geom(), scale, m, ms, tl, ep, tune, st, nblocks_out)) {
             if (marks) marks->mark(st, "x_inv_local");
             return;
         }
@@ -671,22 +786,22 @@ void Demag::inverse_x_epilogue(const R* m, const MsInfo& ms, const TermList& tl,
     switch (ep.kind) {
         case EPI_H:
             set_smem(k_xinv_epi<R, EPI_H>, smem);
-            k_xinv_epi<R, EPI_H><<<(unsigned)blocks, threads, smem, st>>>(S1<R>(), pitch_, plan, tP, g, scale, m, ms,
+            k_xinv_epi<R, EPI_H><<<(unsigned)blocks, threads, smem, st>>>(pl.s1, pl.pitch, plan, tP, g, scale, m, ms,
                                                                           tl, ep, nbr);
             break;
         case EPI_LLG:
             set_smem(k_xinv_epi<R, EPI_LLG>, smem);
-            k_xinv_epi<R, EPI_LLG><<<(unsigned)blocks, threads, smem, st>>>(S1<R>(), pitch_, plan, tP, g, scale, m,
+            k_xinv_epi<R, EPI_LLG><<<(unsigned)blocks, threads, smem, st>>>(pl.s1, pl.pitch, plan, tP, g, scale, m,
                                                                             ms, tl, ep, nbr);
             break;
         case EPI_EGRAD:
             set_smem(k_xinv_epi<R, EPI_EGRAD>, smem);
-            k_xinv_epi<R, EPI_EGRAD><<<(unsigned)blocks, threads, smem, st>>>(S1<R>(), pitch_, plan, tP, g, scale, m,
+            k_xinv_epi<R, EPI_EGRAD><<<(unsigned)blocks, threads, smem, st>>>(pl.s1, pl.pitch, plan, tP, g, scale, m,
                                                                               ms, tl, ep, nbr);
             break;
         default:
             set_smem(k_xinv_epi<R, EPI_EDENS>, smem);
-            k_xinv_epi<R, EPI_EDENS><<<(unsigned)blocks, threads, smem, st>>>(S1<R>(), pitch_, plan, tP, g, scale, m,
+            k_xinv_epi<R, EPI_EDENS><<<(unsigned)blocks, threads, smem, st>>>(pl.s1, pl.pitch, plan, tP, g, scale, m,
                                                                               ms, tl, ep, nbr);
             break;
     }
@@ -694,6 +809,8 @@ void Demag::inverse_x_epilogue(const R* m, const MsInfo& ms, const TermList& tl,
     if (marks) marks->mark(st, "x_inv_local");
 }
 
+template DemagPlan<float> Demag::plan<float>(cudaStream_t);
+template DemagPlan<double> Demag::plan<double>(cudaStream_t);
 template void Demag::forward_conv<float>(const float*, const MsInfo&, cudaStream_t, PassMarks*);
 template void Demag::forward_conv<double>(const double*, const MsInfo&, cudaStream_t, PassMarks*);
 template void Demag::inverse_x_epilogue<float>(const float*, const MsInfo&, const TermList&, const EpilogueArgs&,
@@ -741,20 +858,40 @@ void eval_terms(const std::vector<Term*>& terms, const MeshDims& md, const R* m,
         if (marks) marks->mark(st, "start");
         demag->forward_conv<R>(m, ms, st, marks);
         demag->inverse_x_epilogue<R>(m, ms, tl, ep, st, &nblocks, marks);
-    } else if (run4_eligible(md.geom(), m, ms, tl, ep) && md.N() / 4 < (int64_t)INT32_MAX) {
-        // scalar parameters, no Ms field, nx % 4 == 0: runs of four cells with
-        // per-launch term constants (no division in the cell loop)
-        constexpr int RN = 4;
+    } else if (const int run = md.N() < (int64_t)INT32_MAX ? run_mode(md.geom(), m, ms, tl, ep, 2) : 0) {
+        // scalar parameters: runs of cells with per-launch term constants
+        // (no division in the cell loop); four cells per run where the rows allow it, two
+        // for the energies (the energy and the field of four do not fit the registers)
         const Geom g = md.geom();
-        prepare_run4(tl, g, ms.Ms);
-        const int nruns = (int)(md.N() / RN);
+        prepare_run(tl, g, ms);
+        const bool four = run == 1 && g.nx % 4 == 0 && (ep.kind == EPI_H || ep.kind == EPI_LLG);
+        const int nruns = (int)(md.N() / (four ? 4 : run == 1 ? 2 : 1));
         const int threads = 256;
         const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(nruns, threads), (int64_t)sm_count() * 16);
+        nblocks = (int)blocks;
         if (marks) marks->mark(st, "start");
-        if (ep.kind == EPI_H)
-            k_local_run<R, EPI_H, RN><<<blocks, threads, 0, st>>>(g, m, tl, ep, nruns);
+#define MAF_LOCAL_RUN(EPI)                                                                                        \
+    do {                                                                                                         \
+        if (run == 1)                                                                                            \
+            k_local_run<R, EPI, 2, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                  \
+        else if (run == 2)                                                                                       \
+            k_local_run<R, EPI, 1, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                  \
+        else                                                                                                     \
+            k_local_run<R, EPI, 1, true><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                   \
+    } while (0)
+        if (four && ep.kind == EPI_H)
+            k_local_run<R, EPI_H, 4, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);
+        else if (four)
+            k_local_run<R, EPI_LLG, 4, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);
+        else if (ep.kind == EPI_H)
+            MAF_LOCAL_RUN(EPI_H);
+        else if (ep.kind == EPI_LLG)
+            MAF_LOCAL_RUN(EPI_LLG);
+        else if (ep.kind == EPI_EGRAD)
+            MAF_LOCAL_RUN(EPI_EGRAD);
         else
-            k_local_run<R, EPI_LLG, RN><<<blocks, threads, 0, st>>>(g, m, tl, ep, nruns);
+            MAF_LOCAL_RUN(EPI_EDENS);
+#undef MAF_LOCAL_RUN
         MAF_LAUNCH_CHECK();
         if (marks) marks->mark(st, "local");
     } else {

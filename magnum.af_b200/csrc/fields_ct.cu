@@ -53,7 +53,7 @@ template <typename R, int LC, int NB> constexpr size_t xfwd_pipe_smem() {
 // HIN: n_in <= LC, so the packed values k >= LC/2 are the zero padding (pruned
 // from the first stage)
 // (tile body: rows [tile NB, tile NB + NB); k_xfwd_ct runs tile blockIdx.x, the
-// batched kernel the tile of its work item)
+// batched kernel the tile of its work item; rows shorter than LC are padded in the load)
 template <typename R, int LC, int NB, int NT, bool HIN>
 __device__ __forceinline__ void xfwd_ct_tile(const R* __restrict__ in, int n_in, int64_t rows, int64_t rows_pc,
                                              const R* __restrict__ msf, R ms, cplx_t<R>* __restrict__ out,
@@ -65,7 +65,8 @@ __device__ __forceinline__ void xfwd_ct_tile(const R* __restrict__ in, int n_in,
     constexpr int SB = (LC - 1) + ((LC - 1) >> 4) + 1;
     static_assert(LC * NB % NT == 0, "tile");
     const int64_t r0 = tile * NB;
-    const bool even = (n_in & 1) == 0;
+    // (pairs are loaded as one value where every row starts on a pair's boundary)
+    const bool even = (n_in & 1) == 0 && (uintptr_t)in % sizeof(C) == 0;
     // packed pair (in[2k], in[2k+1]) * Ms of row b, k = j + dk, loaded straight into the first stage
     auto ld = [&](int b, int j, int dk) -> C {
         const int k = j + dk;
@@ -128,8 +129,8 @@ __global__ void __launch_bounds__(NT) k_xfwd_ct(const R* __restrict__ in, int n_
 // x forward, persistent and pipelined: each CTA walks tiles of NB rows; the m rows
 // of the next tile are copied into a shared-memory staging buffer with cp.async
 // while the current tile's transform runs (issued right after the first stage,
-// the staging buffer's only reader).  For a scalar Ms, n_in <= LC (zero-padded
-// half pruned) and rows of whole 16-byte chunks; the same arithmetic as k_xfwd_ct.
+// the staging buffer's only reader).  For a scalar Ms, n_in = LC (RAG: n_in <= LC; the
+// zero-padded half is pruned) and rows of whole 16-byte chunks; the same arithmetic as k_xfwd_ct.
 // CTAs per SM the kernel is compiled for: 1024 (FP32) / 512 (FP64) resident threads for
 // power-of-two lengths, 576 / 288 for three times a power of two, whose radix-3 stage
 // holds more values per thread
@@ -137,7 +138,7 @@ template <typename R, int NT>
 constexpr int kXfwdPipeBlocks = ((sizeof(R) == 4 ? (NT % 3 == 0 ? 576 : 1024) : (NT % 3 == 0 ? 288 : 512)) / NT > 1)
                                     ? (sizeof(R) == 4 ? (NT % 3 == 0 ? 576 : 1024) : (NT % 3 == 0 ? 288 : 512)) / NT
                                     : 1;
-template <typename R, int LC, int NB, int NT>
+template <typename R, int LC, int NB, int NT, bool RAG>
 __global__ void __launch_bounds__(NT, (kXfwdPipeBlocks<R, NT>)) k_xfwd_pipe(const R* __restrict__ in, int n_in, int64_t rows, R ms,
                                                   cplx_t<R>* __restrict__ out, int pitch,
                                                   const cplx_t<R>* __restrict__ tw,
@@ -168,7 +169,7 @@ __global__ void __launch_bounds__(NT, (kXfwdPipeBlocks<R, NT>)) k_xfwd_pipe(cons
         __syncthreads();
         // the packed values k = j + dk < LC/2 of a pruned first stage are all inside the row (n_in = LC)
         auto ld = [&](int b, int j, int dk) -> C {
-            if (r0 + b >= rows) return mk((R)0, (R)0);
+            if (r0 + b >= rows || (RAG && 2 * (j + dk) >= n_in)) return mk((R)0, (R)0);
             const C v = reinterpret_cast<const C*>(stage + b * n_in)[j + dk];
             return mk(v.x * ms, v.y * ms);
         };
@@ -201,8 +202,9 @@ __global__ void __launch_bounds__(NT, (kXfwdPipeBlocks<R, NT>)) k_xfwd_pipe(cons
 // are not read), the last stage stores straight to global memory (rows >=
 // n_out are truncated and not written).
 // HIN: n_in <= L/2 (zero-padded input), HOUT: n_out <= L/2 (truncated output);
-// both prune the transform at compile time
-template <typename R, int DIR, int L, int NB, int NT, bool HIN, bool HOUT, int PV>
+// both prune the transform at compile time.  RAG: n_in or n_out is below L/2 (a
+// transform longer than twice the mesh), checked per row.
+template <typename R, int DIR, int L, int NB, int NT, bool HIN, bool HOUT, int PV, bool RAG>
 __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT * (L * NB / kE > NT ? L * NB / kE / NT : 1), 1024, 512>)) k_cols_ct(const cplx_t<R>* in, cplx_t<R>* out, int n_in, int n_out, int ncols,
                                                 int64_t in_si, int64_t out_si, int64_t in_sbat, int64_t out_sbat,
                                                 const cplx_t<R>* __restrict__ tw) {
@@ -213,13 +215,13 @@ __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT * (L * NB / kE > NT ? L 
     const C* ib = in + (int64_t)blockIdx.y * in_sbat + c0;
     C* ob = out + (int64_t)blockIdx.y * out_sbat + c0;
     const int ncv = min(NB, ncols - c0);
-    // element i = j + di of column b; the host guarantees n_in = L/2 (HIN) or L and
+    // element i = j + di of column b; without RAG n_in = L/2 (HIN) or L and
     // n_out = L/2 (HOUT) or L, so every element the stages touch is in range
     auto ld = [&](int b, int j, int di) -> C {
-        return b < ncv ? ib[(int64_t)j * in_si + b + (int64_t)di * in_si] : mk((R)0, (R)0);
+        return b < ncv && (!RAG || j + di < n_in) ? ib[(int64_t)j * in_si + b + (int64_t)di * in_si] : mk((R)0, (R)0);
     };
     auto st = [&](int b, int j, int di, C v) {
-        if (b < ncv) ob[(int64_t)j * out_si + b + (int64_t)di * out_si] = v;
+        if (b < ncv && (!RAG || j + di < n_out)) ob[(int64_t)j * out_si + b + (int64_t)di * out_si] = v;
     };
     ct_fft_io<R, DIR, true, L, NB, NT, HIN, HOUT>(s, 0, tw, ld, st, typename CtPlanV<L, PV>::T());
 }
@@ -238,8 +240,8 @@ template <typename R, int L, int NB, bool HIN> constexpr size_t cols_pipe_smem()
     return cols_stage_offset<R, L, NB>() + sizeof(cplx_t<R>) * NB * (HIN ? L / 2 : L);
 }
 
-template <typename R, int DIR, int L, int NB, int NT, bool HIN, bool HOUT, int PV>
-__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_cols_pipe(const cplx_t<R>* in, cplx_t<R>* out, int ncols, int64_t in_si,
+template <typename R, int DIR, int L, int NB, int NT, bool HIN, bool HOUT, int PV, bool RAG>
+__global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_cols_pipe(const cplx_t<R>* in, cplx_t<R>* out, int n_in, int ncols, int64_t in_si,
                                                    int64_t out_si, int64_t in_sbat, int64_t out_sbat, int nbat,
                                                    int pitch, const cplx_t<R>* __restrict__ tw) {
     using C = cplx_t<R>;
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_cols_pipe(const cplx_
 #pragma unroll 4
         for (int q = threadIdx.x; q < NIN * CPR; q += NT) {
             const int i = q / CPR, c = q - i * CPR;
-            if (c >= cmax) continue;
+            if (c >= cmax || (RAG && i >= n_in)) continue;
             const unsigned char* src = src0 + (int64_t)i * in_si * (int64_t)sizeof(C) + c * 16;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst0 + (unsigned)q * 16u), "l"(src));
         }
@@ -278,7 +280,9 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_cols_pipe(const cplx_
         asm volatile("cp.async.wait_all;\n" ::);
         __syncthreads();
         // element i = j + di of column b, from the staging buffer
-        auto ld = [&](int b, int j, int di) -> C { return stage[(j + di) * NB + b]; };
+        auto ld = [&](int b, int j, int di) -> C {
+            return !RAG || j + di < n_in ? stage[(j + di) * NB + b] : mk((R)0, (R)0);
+        };
         auto st = [&](int b, int j, int di, C v) {
             if (b < ncv) ob[(int64_t)j * out_si + b + (int64_t)di * out_si] = v;
         };
@@ -290,9 +294,9 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_cols_pipe(const cplx_
 }
 
 // -------------------------------------------------- z convolution (3-D meshes)
-// CTA (kx tile, ky) with ky in [0, ny]: rows ky and Py - ky (same tensor quadrant
-// row, sign of Nxy and Nyz flipped for the second); ky = 0 and ky = ny are
-// their own mirrors and run alone.
+// CTA (kx tile, ky) with ky in [0, ny], ny = Py/2: rows ky and Py - ky (same tensor
+// quadrant row, sign of Nxy and Nyz flipped for the second); ky = 0 and ky = ny are
+// their own mirrors and run alone.  The spectra have nz <= L/2 planes.
 template <typename R, int L, int NB, int NT>
 __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT, 768, 512>)) k_convz_ct(cplx_t<R>* S, const R* __restrict__ Nred, int nz, int ny, int nxh,
                                                  int pitch, const cplx_t<R>* __restrict__ tw) {
@@ -322,16 +326,15 @@ __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT, 768, 512>)) k_convz_ct(
         const int64_t o = at(col, j + di, ok);
         return ok ? S[o] : mk((R)0, (R)0);
     };
-    // L = 2 nz: the upper half of the input is the padding, of the output the truncation
+    // L >= 2 nz: the upper half of the input is padding, of the output truncation
     ct_fft_in<R, -1, true, L, NC, NT, true>(s, 0, tw, ld, typename CtPlan<L>::T());
-    const int Pz = 2 * nz;
-    const int64_t tcs = (int64_t)(nz + 1) * (ny + 1) * nxh;
+    const int64_t tcs = (int64_t)(L / 2 + 1) * (ny + 1) * nxh;
     for (int idx = threadIdx.x; idx < L * NB; idx += NT) {
         const int kz = idx / NB;
         const int b = idx % NB;
         if (b >= ncv) continue;
-        const int kzr = kz <= nz ? kz : Pz - kz;
-        const R sz = kz <= nz ? (R)1 : (R)-1;
+        const int kzr = kz <= L / 2 ? kz : L - kz;
+        const R sz = kz <= L / 2 ? (R)1 : (R)-1;
         const int64_t o = ((int64_t)kzr * (ny + 1) + ky) * nxh + c0 + b;
         const R Nxx = Nred[o], Nxy = Nred[tcs + o], Nxz = sz * Nred[2 * tcs + o];
         const R Nyy = Nred[3 * tcs + o], Nyz = sz * Nred[4 * tcs + o], Nzz = Nred[5 * tcs + o];
@@ -393,9 +396,10 @@ template <typename R, int NZ> __device__ __forceinline__ cplx_t<R> wz_const(int 
 // so only the padded half's zeros are skipped for free, no shared-memory stage
 // is needed inside the transforms, and shared memory carries only the spectra
 // between the transforms and the 3-component tensor product.
-template <typename R, int NZ, int NB>
+// RAG: the spectra have nz < NZ planes (the missing ones are zero).
+template <typename R, int NZ, int NB, bool RAG>
 __global__ void __launch_bounds__(6 * NB, (kMinBlocks<R, 6 * NB, 576, 288>))
-    k_convz_reg(cplx_t<R>* S, const R* __restrict__ Nred, int ny, int nxh, int pitch,
+    k_convz_reg(cplx_t<R>* S, const R* __restrict__ Nred, int nz, int ny, int nxh, int pitch,
                 const cplx_t<R>* __restrict__ tw) {
     using C = cplx_t<R>;
     constexpr int L = 2 * NZ;
@@ -410,7 +414,7 @@ __global__ void __launch_bounds__(6 * NB, (kMinBlocks<R, 6 * NB, 576, 288>))
     const int c0 = blockIdx.x * NB;
     const int ncv = min(NB, nxh - c0);
     const int64_t si = (int64_t)Py * pitch;       // z stride
-    const int64_t cs = (int64_t)NZ * Py * pitch;  // component stride
+    const int64_t cs = (int64_t)(RAG ? nz : NZ) * Py * pitch;  // component stride
     const int col = threadIdx.x;
     const int64_t tcs = (int64_t)(NZ + 1) * (ny + 1) * nxh;
     // the tensor rows of this tile go to shared memory asynchronously, under the
@@ -441,7 +445,7 @@ __global__ void __launch_bounds__(6 * NB, (kMinBlocks<R, 6 * NB, 576, 288>))
         const C* src = S + comp * cs + (int64_t)(row ? Py - ky : ky) * pitch + c0 + b;
         C e[NZ], o[NZ];
 #pragma unroll
-        for (int n = 0; n < NZ; ++n) e[n] = ok ? src[n * si] : mk((R)0, (R)0);
+        for (int n = 0; n < NZ; ++n) e[n] = ok && (!RAG || n < nz) ? src[n * si] : mk((R)0, (R)0);
         // the twiddles W_L^n: immediates in FP32, the correctly rounded table in FP64
         auto wz = [&](int n) -> C {
             if constexpr (sizeof(R) == 4) return wz_const<R, NZ>(n);
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(6 * NB, (kMinBlocks<R, 6 * NB, 576, 288>))
                 C w;
                 if constexpr (sizeof(R) == 4) w = wz_const<R, NZ>(n);
                 else w = tw[n];
-                dst[n * si] = cadd(e[n], cmulc(o[n], w));
+                if (!RAG || n < nz) dst[n * si] = cadd(e[n], cmulc(o[n], w));
             }
         }
     }
@@ -527,15 +531,15 @@ __device__ __forceinline__ void convy_ct_tile(cplx_t<R>* S, const R* __restrict_
         const int i = j + di;
         return (i < ny && b < ncv) ? S[comp * cs + (int64_t)i * pitch + c0 + b] : mk((R)0, (R)0);
     };
-    // L = 2 ny: zero-padded input, truncated output
+    // L >= 2 ny: zero-padded input, truncated output
     ct_fft_in<R, -1, true, L, NC, NT, true>(s, 0, tw, ld, typename CtPlan<L>::T());
-    const int64_t tcs = (int64_t)(ny + 1) * nxh;
+    const int64_t tcs = (int64_t)(L / 2 + 1) * nxh;
     for (int idx = threadIdx.x; idx < L * NB; idx += NT) {
         const int ky = idx / NB;
         const int b = idx % NB;
         if (b >= ncv) continue;
-        const int kyr = ky <= ny ? ky : L - ky;
-        const R sy = ky <= ny ? (R)1 : (R)-1;
+        const int kyr = ky <= L / 2 ? ky : L - ky;
+        const R sy = ky <= L / 2 ? (R)1 : (R)-1;
         const int64_t o = (int64_t)kyr * nxh + c0 + b;
         const R Nxx = Nred[o], Nxy = sy * Nred[tcs + o], Nyy = Nred[2 * tcs + o], Nzz = Nred[3 * tcs + o];
         const int base = spad(ky) * NC + b;
@@ -560,12 +564,65 @@ __global__ void __launch_bounds__(NT) k_convy_ct(cplx_t<R>* S, const R* __restri
 }
 
 // --------------------------------------------------- x inverse + epilogue
-// (tile body: (y, z) rows [tile NBR, tile NBR + NBR))
+// The run epilogue on the tile's rows, whose demag values sit in s.  Rows have up
+// to LC cells: the run index arithmetic is compile-time, runs beyond a shorter row
+// are skipped.  Returns the thread's energy density.
+template <typename R, int EPI, int LC, int NBR, int NT, int N, bool MSF>
+__device__ __forceinline__ double xinv_runs(const cplx_t<R>* s, const Geom& g, R scale, const R* __restrict__ m,
+                                            const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep, int ry0) {
+    constexpr int SB = (LC - 1) + ((LC - 1) >> 4) + 1;
+    constexpr int runs = LC / N;
+    const int rows_pc = g.ny * g.nz;
+    // (y, z) of the CTA's first row once
+    const int z0 = ry0 / g.ny;
+    const int y0 = ry0 - z0 * g.ny;
+    double eacc = 0;
+    for (int idx = threadIdx.x; idx < NBR * runs; idx += NT) {
+        const int b = idx / runs;
+        const int x0 = (idx - b * runs) * N;
+        const int ry = ry0 + b;
+        if (ry >= rows_pc || x0 >= g.nx) continue;
+        int y = y0 + b, z = z0;
+        while (y >= g.ny) {
+            y -= g.ny;
+            ++z;
+        }
+        const int64_t cell0 = (int64_t)ry * g.nx + x0;
+        RunN<R, N> r;
+        runN_load<R, N>(m, g, x0, y, z, cell0, r);
+        double Ms = ms.Ms;
+        if constexpr (MSF) {
+            Ms = ms.field64[cell0];
+            r.ms = cell_Ms<R>(ms, cell0);
+            r.inv = (R)1 / r.ms;
+        }
+        R hd[N][3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            if constexpr (N == 1) {
+                const cplx_t<R> val = s[spad(x0 >> 1) + (c * NBR + b) * SB];
+                hd[0][c] = scale * ((x0 & 1) ? val.y : val.x);
+            } else {
+#pragma unroll
+                for (int i = 0; i < N; i += 2) {
+                    // cells x0 + i and x0 + i + 1 are the two halves of one packed value
+                    const cplx_t<R> val = s[spad((x0 + i) >> 1) + (c * NBR + b) * SB];
+                    hd[i][c] = scale * val.x;
+                    hd[i + 1][c] = scale * val.y;
+                }
+            }
+        }
+        eacc += runN_epilogue<R, EPI, N, MSF>(tl, g, r, cell0, hd, ep, Ms);
+    }
+    return eacc;
+}
+
+// (tile body: (y, z) rows [tile NBR, tile NBR + NBR); run: run_mode's answer)
 template <typename R, int EPI, int LC, int NBR, int NT, int RN>
 __device__ __forceinline__ void xinv_ct_tile(const cplx_t<R>* __restrict__ S1, int pitch,
                                              const cplx_t<R>* __restrict__ tw, const cplx_t<R>* __restrict__ twP,
                                              const Geom& g, R scale, const R* __restrict__ m, const MsInfo& ms,
-                                             const TermList& tl, const EpilogueArgs& ep, int run4, int tile) {
+                                             const TermList& tl, const EpilogueArgs& ep, int run, int tile) {
     using C = cplx_t<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);
@@ -587,48 +644,20 @@ __device__ __forceinline__ void xinv_ct_tile(const cplx_t<R>* __restrict__ S1, i
         const C O = cmulc(csub(Xk, cconj(Xm)), (twP + j)[dk]);
         return cadd(E_, cmul_i<1>(O));
     };
-    // only the first nx of the 2 LC real outputs (packed values k < LC/2) are kept
+    // only the first nx <= LC of the 2 LC real outputs (packed values k < LC/2) are kept
     if constexpr (LC >= 32)
         ct_fft_in<R, 1, false, LC, NC, NT, false, true>(s, SB, tw, ld, typename CtPlan<LC>::T());
     else
         ct_fft_in<R, 1, false, LC, NC, NT>(s, SB, tw, ld, typename CtPlan<LC>::T());
-    if constexpr (EPI == EPI_H || EPI == EPI_LLG) {
-        if (run4) {
-            // the rows are nx = LC cells long (the x padding doubles nx), so the run
-            // index arithmetic is compile-time; (y, z) of the CTA's first row once
-            constexpr int runs = LC / RN;
-            const int z0 = ry0 / g.ny;
-            const int y0 = ry0 - z0 * g.ny;
-            for (int idx = threadIdx.x; idx < NBR * runs; idx += NT) {
-                const int b = idx / runs;
-                const int x0 = (idx - b * runs) * RN;
-                const int ry = ry0 + b;
-                if (ry >= rows_pc) continue;
-                int y = y0 + b, z = z0;
-                while (y >= g.ny) {
-                    y -= g.ny;
-                    ++z;
-                }
-                const int64_t cell0 = (int64_t)ry * LC + x0;
-                RunN<R, RN> r;
-                runN_load<R, RN>(m, g, x0, y, z, cell0, r);
-                R hd[RN][3];
-#pragma unroll
-                for (int i = 0; i < RN; i += 2) {
-#pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        // cells x0 + i and x0 + i + 1 are the two halves of one packed value
-                        const C val = s[spad((x0 + i) >> 1) + (c * NBR + b) * SB];
-                        hd[i][c] = scale * val.x;
-                        hd[i + 1][c] = scale * val.y;
-                    }
-                }
-                runN_epilogue<R, EPI, RN>(tl, g, r, cell0, hd, ep);
-            }
-            return;
-        }
-    }
     double eacc = 0;
+    if constexpr (sizeof(R) == 4 && EPI == EPI_EGRAD) run = 0;  // as run_mode
+    if (run) {
+        eacc = run == 1   ? xinv_runs<R, EPI, LC, NBR, NT, RN, false>(s, g, scale, m, ms, tl, ep, ry0)
+               : run == 2 ? xinv_runs<R, EPI, LC, NBR, NT, 1, false>(s, g, scale, m, ms, tl, ep, ry0)
+                          : xinv_runs<R, EPI, LC, NBR, NT, 1, true>(s, g, scale, m, ms, tl, ep, ry0);
+        if constexpr (EPI == EPI_EDENS || EPI == EPI_EGRAD) block_sum_store(eacc, ep.partials);
+        return;
+    }
     for (int idx = threadIdx.x; idx < NBR * g.nx; idx += NT) {
         const int b = idx / g.nx;
         const int x = idx - b * g.nx;
@@ -652,8 +681,8 @@ template <typename R, int EPI, int LC, int NBR, int NT, int RN>
 __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT, (RN == 2 ? (NT == 192 ? MAF_XINV_THREADS_192 : MAF_XINV_THREADS) : 384), MAF_XINV_THREADS_F64>)) k_xinv_ct(const cplx_t<R>* __restrict__ S1, int pitch,
                                                 const cplx_t<R>* __restrict__ tw, const cplx_t<R>* __restrict__ twP,
                                                 Geom g, R scale, const R* __restrict__ m, MsInfo ms, TermList tl,
-                                                EpilogueArgs ep, int run4) {
-    xinv_ct_tile<R, EPI, LC, NBR, NT, RN>(S1, pitch, tw, twP, g, scale, m, ms, tl, ep, run4, blockIdx.x);
+                                                EpilogueArgs ep, int run) {
+    xinv_ct_tile<R, EPI, LC, NBR, NT, RN>(S1, pitch, tw, twP, g, scale, m, ms, tl, ep, run, blockIdx.x);
 }
 
 // ---------------------------------------------- batched (work-table) passes
@@ -672,7 +701,7 @@ __global__ void __launch_bounds__(NT) kbt_convy(const CtConvyItem<R>* __restrict
                                                 const cplx_t<R>* __restrict__ tw) {
     const int2 w = work[blockIdx.x];
     const CtConvyItem<R> d = items[w.x];
-    convy_ct_tile<R, L, NB, NT>(d.S, d.Nred, L / 2, d.nxh, d.pitch, tw, w.y);
+    convy_ct_tile<R, L, NB, NT>(d.S, d.Nred, d.ny, d.nxh, d.pitch, tw, w.y);
 }
 
 template <typename R, int LC, int NBR, int NT, int RN>
@@ -681,7 +710,7 @@ __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT, (RN == 2 ? (NT == 192 ?
              const cplx_t<R>* __restrict__ twP) {
     const int2 w = work[blockIdx.x];
     const CtXinvItem<R>& d = items[w.x];
-    xinv_ct_tile<R, EPI_LLG, LC, NBR, NT, RN>(d.S1, d.pitch, tw, twP, d.g, d.scale, d.m, d.ms, d.tl, d.ep, d.run4, w.y);
+    xinv_ct_tile<R, EPI_LLG, LC, NBR, NT, RN>(d.S1, d.pitch, tw, twP, d.g, d.scale, d.m, d.ms, d.tl, d.ep, d.run, w.y);
 }
 
 // ------------------------------------------------------------------ launches
@@ -743,11 +772,12 @@ static void xfwd_L(const R* in, int n_in, int64_t rows, int64_t rows_pc, const R
         constexpr int NT = LC * NB / kE;
         constexpr int E16 = 16 / (int)sizeof(R);
         if (!msf && n_in % E16 == 0 && (uintptr_t)in % 16 == 0) {
-            auto kp = k_xfwd_pipe<R, LC, NB, NT>;
+            const bool rag = n_in != LC;
+            auto kp = rag ? k_xfwd_pipe<R, LC, NB, NT, true> : k_xfwd_pipe<R, LC, NB, NT, false>;
             const size_t smem_p = xfwd_pipe_smem<R, LC, NB>();
             ct_smem(kp, smem_p);
-            static int per_sm[2] = {0, 0}, sms = 0;  // per precision, measured once per process
-            int& ps = per_sm[sizeof(R) == 8];
+            static int per_sm[2] = {0, 0}, sms = 0;  // exact and shorter rows, measured once per process
+            int& ps = per_sm[rag];
             if (!ps) {
                 MAF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, kp, NT, smem_p));
                 int dev = 0;
@@ -771,7 +801,7 @@ static void xfwd_L(const R* in, int n_in, int64_t rows, int64_t rows_pc, const R
     MAF_LAUNCH_CHECK();
 }
 
-template <typename R, int DIR, int L, int TILE, bool HIN, bool HOUT, int PV>
+template <typename R, int DIR, int L, int TILE, bool HIN, bool HOUT, int PV, bool RAG = false>
 static void cols_L(const cplx_t<R>* in, cplx_t<R>* out, int n_in, int n_out, int ncols, int64_t in_si, int64_t out_si,
                    int64_t in_sbat, int64_t out_sbat, int nbat, const void* tw, int pipe, int pitch, cudaStream_t st) {
     constexpr int NB = pow2floor(cmin(32, cmax(1, TILE / L)));
@@ -786,20 +816,20 @@ static void cols_L(const cplx_t<R>* in, cplx_t<R>* out, int n_in, int n_out, int
                         (in_si * (int64_t)sizeof(cplx_t<R>)) % 16 == 0 &&
                         (in_sbat * (int64_t)sizeof(cplx_t<R>)) % 16 == 0;
         if (ok) {
-            auto kp = k_cols_pipe<R, DIR, L, NB, NT, HIN, HOUT, PV>;
+            auto kp = k_cols_pipe<R, DIR, L, NB, NT, HIN, HOUT, PV, RAG>;
             const size_t smem_p = cols_pipe_smem<R, L, NB, HIN>();
             ct_smem(kp, smem_p);
             int per_sm = 0;
             MAF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp, NT, smem_p));
             const int64_t ntiles = (int64_t)ntx * nbat;
             const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)std::max(per_sm, 1) * sm_count());
-            kp<<<grid, NT, smem_p, st>>>(in, out, ncols, in_si, out_si, in_sbat, out_sbat, nbat, pitch,
+            kp<<<grid, NT, smem_p, st>>>(in, out, n_in, ncols, in_si, out_si, in_sbat, out_sbat, nbat, pitch,
                                          static_cast<const cplx_t<R>*>(tw));
             MAF_LAUNCH_CHECK();
             return;
         }
     }
-    auto k = k_cols_ct<R, DIR, L, NB, NT, HIN, HOUT, PV>;
+    auto k = k_cols_ct<R, DIR, L, NB, NT, HIN, HOUT, PV, RAG>;
     ct_smem(k, smem);
     dim3 grid((unsigned)ceil_div(ncols, NB), (unsigned)nbat);
     k<<<grid, NT, smem, st>>>(in, out, n_in, n_out, ncols, in_si, out_si, in_sbat, out_sbat,
@@ -820,10 +850,10 @@ static void convz_L(cplx_t<R>* S, const R* Nred, int nz, int ny, int nxh, int pi
         constexpr int NBR = 16;
         // spectra [L][6 NBR] plus the tensor slice [6][L/2 + 1][NBR]
         constexpr size_t smem_r = sizeof(cplx_t<R>) * (size_t)L * 6 * NBR + sizeof(R) * (size_t)6 * (L / 2 + 1) * NBR;
-        auto kr = k_convz_reg<R, L / 2, NBR>;
+        auto kr = 2 * nz == L ? k_convz_reg<R, L / 2, NBR, false> : k_convz_reg<R, L / 2, NBR, true>;
         ct_smem(kr, smem_r);
         dim3 grid((unsigned)ceil_div(nxh, NBR), (unsigned)(ny + 1));
-        kr<<<grid, 6 * NBR, smem_r, st>>>(S, Nred, ny, nxh, pitch, static_cast<const cplx_t<R>*>(tw));
+        kr<<<grid, 6 * NBR, smem_r, st>>>(S, Nred, nz, ny, nxh, pitch, static_cast<const cplx_t<R>*>(tw));
     } else {
         auto k = k_convz_ct<R, L, NB, NT>;
         ct_smem(k, smem);
@@ -858,9 +888,9 @@ static void xinv_L(const cplx_t<R>* S1, int pitch, const void* tw, const void* t
     const size_t smem = sizeof(cplx_t<R>) * (size_t)NC * SB;
     const int64_t rows_pc = (int64_t)g.ny * g.nz;
     const unsigned blocks = (unsigned)ceil_div(rows_pc, NBR);
-    const int run4 = run4_eligible(g, m, ms, tl_in, ep) ? 1 : 0;
+    const int run = run_mode(g, m, ms, tl_in, ep, RN);
     TermList tl = tl_in;
-    if (run4) prepare_run4(tl, g, ms.Ms);
+    if (run) prepare_run(tl, g, ms);
     if (nblocks) *nblocks = (int)blocks;
     const auto* t = static_cast<const cplx_t<R>*>(tw);
     const auto* tp = static_cast<const cplx_t<R>*>(twP);
@@ -868,25 +898,25 @@ static void xinv_L(const cplx_t<R>* S1, int pitch, const void* tw, const void* t
         case EPI_H: {
             auto k = k_xinv_ct<R, EPI_H, LC, NBR, NT, RN>;
             ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run4);
+            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
             break;
         }
         case EPI_LLG: {
             auto k = k_xinv_ct<R, EPI_LLG, LC, NBR, NT, RN>;
             ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run4);
+            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
             break;
         }
         case EPI_EGRAD: {
             auto k = k_xinv_ct<R, EPI_EGRAD, LC, NBR, NT, 2>;
             ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run4);
+            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
             break;
         }
         default: {
             auto k = k_xinv_ct<R, EPI_EDENS, LC, NBR, NT, 2>;
             ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run4);
+            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
             break;
         }
     }
@@ -988,8 +1018,10 @@ bool ct_cols(const cplx_t<R>* in, cplx_t<R>* out, int L, int n_in, int n_out, in
     // (truncated output); the tensor's full transforms (FP64) run unpruned
     const bool hin = 2 * n_in <= L, hout = 2 * n_out <= L;
     if (hin && hout) return false;
-    // the kernels read exactly L/2 (pruned) or L rows and write L/2 or L
-    if ((hin ? 2 * n_in : n_in) != L || (hout ? 2 * n_out : n_out) != L) return false;
+    // the kernels read L/2 (pruned) or L rows and write L/2 or L; the RAG ones read or
+    // write fewer than L/2
+    if ((!hin && n_in != L) || (!hout && n_out != L)) return false;
+    const bool rag = (hin && 2 * n_in < L) || (hout && 2 * n_out < L);
     // the row stride bounds the column tiles the pipelined kernel copies whole
     const int pitch = (int)std::min<int64_t>(in_si, 1 << 30);
     if (!hin && !hout && !f64) return false;
@@ -1019,9 +1051,18 @@ bool ct_cols(const cplx_t<R>* in, cplx_t<R>* out, int L, int n_in, int n_out, in
         else if constexpr (sizeof(R) == 8)                      \
             C2(N, T, false, false);                             \
     } while (0)
+// (RAG: one tile width and the 16 16 R plan; the autotuner's choices are for the others)
+#define CR(N, HI, HO)                                                                                       \
+    cols_L<R, DIR, N, kTileCols<R>, HI, HO, 0, true>(in, out, n_in, n_out, ncols, in_si, out_si, in_sbat,    \
+                                                     out_sbat, nbat, ct_tw<N>(tw, f64), tc.cols_pipe, pitch, st)
 #define X(N)                                                    \
     do {                                                        \
-        if (tc.cols_wide)                                       \
+        if (rag) {                                              \
+            if (hin)                                            \
+                CR(N, true, false);                             \
+            else                                                \
+                CR(N, false, true);                             \
+        } else if (tc.cols_wide)                                \
             C1(N, 2 * kTileCols<R>);                            \
         else                                                    \
             C1(N, kTileCols<R>);                                \
@@ -1031,13 +1072,14 @@ bool ct_cols(const cplx_t<R>* in, cplx_t<R>* out, int L, int n_in, int n_out, in
 #undef C1
 #undef C2
 #undef C3
+#undef CR
 }
 
 template <typename R>
-bool ct_convz(cplx_t<R>* S, const R* Nred, int nz, int ny, int nxh, int pitch, Twiddles& tw, const TuneChoice& tc,
-              cudaStream_t st) {
+bool ct_convz(cplx_t<R>* S, const R* Nred, int nz, int L, int ny, int nxh, int pitch, Twiddles& tw,
+              const TuneChoice& tc, cudaStream_t st) {
     const bool f64 = sizeof(R) == 8;
-    const int L = 2 * nz;
+    if (2 * nz > L) return false;
 #define X(N)                                                                 \
     do {                                                                     \
         if (tc.convz_reg)                                                    \
@@ -1050,15 +1092,17 @@ bool ct_convz(cplx_t<R>* S, const R* Nred, int nz, int ny, int nxh, int pitch, T
         case 16: X(16); return true;
         case 32: X(32); return true;
         case 64: X(64); return true;
+        case 96: X(96); return true;
+        case 128: X(128); return true;
         default: return false;
     }
 #undef X
 }
 
 template <typename R>
-bool ct_convy(cplx_t<R>* S, const R* Nred, int ny, int nxh, int pitch, Twiddles& tw, cudaStream_t st) {
+bool ct_convy(cplx_t<R>* S, const R* Nred, int ny, int L, int nxh, int pitch, Twiddles& tw, cudaStream_t st) {
     const bool f64 = sizeof(R) == 8;
-    const int L = 2 * ny;
+    if (2 * ny > L) return false;
 #define X(N) convy_L<R, N>(S, Nred, ny, nxh, pitch, ct_tw<N>(tw, f64), st)
     switch (L) {
         case 16: X(16); return true;
@@ -1113,7 +1157,7 @@ bool ct_xinv_group(const cplx_t<R>* S1, int pitch, int Px, Twiddles& tw, const G
                    const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep, const TuneChoice& tc, cudaStream_t st,
                    int* nblocks) {
     const int LC = Px / 2;
-    if (g.nx != LC) return false;  // the kernels take the row length from LC
+    if (g.nx > LC) return false;
     const bool f64 = sizeof(R) == 8;
     const int run = tc.xinv_run ? tc.xinv_run : kRunCells;
 #define X(N)                                                                                                    \
@@ -1164,9 +1208,9 @@ template <typename R> const void* ct_batch_twiddles(int pass, int L, Twiddles& t
     return p;
 }
 
-template <typename R> void ct_batch_xinv_prepare(CtXinvItem<R>& it) {
-    it.run4 = run4_eligible(it.g, it.m, it.ms, it.tl, it.ep) ? 1 : 0;
-    if (it.run4) prepare_run4(it.tl, it.g, it.ms.Ms);
+template <typename R> void ct_batch_xinv_prepare(CtXinvItem<R>& it, int run) {
+    it.run = run_mode(it.g, it.m, it.ms, it.tl, it.ep, run);
+    if (it.run) prepare_run(it.tl, it.g, it.ms);
 }
 
 template <typename R>
@@ -1208,12 +1252,12 @@ bool ct_batch_xinv_group(const CtXinvItem<R>* items, const int2* work, int nwork
 #define MAF_INST1(R)                                                                                                  \
     template bool ct_xfwd<R>(const R*, int, int64_t, int64_t, const R*, R, cplx_t<R>*, int, int, Twiddles&,          \
                              cudaStream_t);                                                                          \
-    template bool ct_convz<R>(cplx_t<R>*, const R*, int, int, int, int, Twiddles&, const TuneChoice&,                \
+    template bool ct_convz<R>(cplx_t<R>*, const R*, int, int, int, int, int, Twiddles&, const TuneChoice&,           \
                               cudaStream_t);                                                                         \
-    template bool ct_convy<R>(cplx_t<R>*, const R*, int, int, int, Twiddles&, cudaStream_t);                    \
+    template bool ct_convy<R>(cplx_t<R>*, const R*, int, int, int, int, Twiddles&, cudaStream_t);               \
     template int ct_batch_tile<R>(int, int);                                                                      \
     template const void* ct_batch_twiddles<R>(int, int, Twiddles&);                                               \
-    template void ct_batch_xinv_prepare<R>(CtXinvItem<R>&);                                                       \
+    template void ct_batch_xinv_prepare<R>(CtXinvItem<R>&, int);                                                    \
     template void ct_batch_xfwd<R>(const CtXfwdItem<R>*, const int2*, int, int, const void*, const void*,        \
                                    cudaStream_t);                                                                \
     template void ct_batch_convy<R>(const CtConvyItem<R>*, const int2*, int, int, const void*, cudaStream_t);
