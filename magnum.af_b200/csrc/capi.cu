@@ -212,6 +212,23 @@ struct maf_state_s {
     }
 };
 
+// A pinned host double that kernels write directly: read after the stream's
+// synchronisation, without a copy of its own (a copy to pageable memory was another
+// 8-10 us per step).
+struct HostWord {
+    double* p = nullptr;
+    HostWord() = default;
+    HostWord(const HostWord&) = delete;
+    HostWord& operator=(const HostWord&) = delete;
+    ~HostWord() { if (p) cudaFreeHost(p); }
+    void ensure() { if (!p) MAF_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable)); }
+    double* device() const {
+        void* d = nullptr;
+        MAF_CUDA(cudaHostGetDevicePointer(&d, p, 0));
+        return static_cast<double*>(d);
+    }
+};
+
 struct maf_term_s {
     std::shared_ptr<Term> t;
 };
@@ -227,8 +244,12 @@ struct maf_llg_s {
     Controller ctrl;
     double h = 1.01e-15;
     bool dissipation_only = false;
-    DevBuf k[8];
-    DevBuf mstage64, mstage32, mcand, partials, errbuf, h32out;
+    // the k's and one stage buffer in one allocation (rk_work: each allocation above 2 MB costs
+    // 0.5-1 ms of a first step); the stages' m goes to that stage buffer and mcand in turn (an
+    // epilogue reads one and writes the other), its FP32 copy likewise; mcand and mcand32 then
+    // take the candidate and are swapped with the state's m
+    DevBuf work, mcand, mcand32, partials;
+    HostWord err;
     unsigned long long accumulated_steps = 0;
     std::vector<std::string> prof_names;  // interval names of the last maf_llg_attempt_profile
 };
@@ -264,8 +285,8 @@ void eval_on_state(maf_state_s* st, const std::vector<Term*>& terms, EpilogueArg
     }
 }
 
-// interval names of the attempt profile that carry the number of FP64 k
-// buffers a Runge-Kutta kernel reads (its algorithmic bytes depend on it)
+// interval names of the attempt profile that carry the number of FP64 k buffers a
+// Runge-Kutta kernel reads (its algorithmic bytes depend on it)
 const char* const kCombineNames[8] = {"rk_combine_k0", "rk_combine_k1", "rk_combine_k2", "rk_combine_k3",
                                       "rk_combine_k4", "rk_combine_k5", "rk_combine_k6", "rk_combine_k7"};
 const char* const kFinalizeNames[9] = {"rk_finalize_k0", "rk_finalize_k1", "rk_finalize_k2",
@@ -283,73 +304,108 @@ LLGParams llg_params(const maf_llg_s* l, double scale) {
     return p;
 }
 
+// Cells up to which a stage's epilogue writes the next stage's m.  A DP45 step, separate
+// combine kernels -> fused (FP64 / FP32 field): 185 -> 170 / 178 -> 171 us at 64x64 cells,
+// 237 -> 218 / 215 -> 214 at 256x256, 489 -> 485 / 328 -> 327 at 512x512 (launches saved);
+// 1096 -> 1120 / 686 -> 702 at 512x512x2 and 1678 -> 1728 / 1042 -> 1086 at 512x512x4: there
+// the combine streams at HBM speed, which the epilogue's fewer warps do not reach.
+constexpr int64_t kFusedStageCells = 1 << 18;
+
+// partials and block counter of rk_finalize
+void ensure_finalize_scratch(DevBuf& partials, cudaStream_t st) {
+    const size_t n = sizeof(double) * (rk_finalize_blocks() + 1);
+    if (partials.bytes >= n) return;
+    partials.alloc(n);
+    MAF_CUDA(cudaMemsetAsync(partials.p, 0, n, st));
+}
+
 // One RK attempt of `sch` with step dt; leaves m + sumbk (normalised per
-// norm_mode) in l->mcand and returns the error norm.
+// norm_mode) in l->mcand (FP32 copy: l->mcand32) and returns the error norm.
+// On small meshes (kFusedStageCells) the epilogue that computes a stage's k also writes
+// the next stage's m (NextStage); on large ones rk_combine does.
 double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, int norm_mode,
                   PassMarks* marks = nullptr) {
     StateD& s = st->s;
     const int64_t N = s.md.N();
     const int64_t n3 = 3 * N;
     const bool f32 = s.precision == PREC_FP32_FIELD;
-    for (int i = 0; i < sch.stages; ++i) l->k[i].ensure(sizeof(double) * n3);
-    l->mstage64.ensure(sizeof(double) * n3);
-    if (f32) l->mstage32.ensure(sizeof(float) * n3);
+    const int64_t np = (n3 + 31) / 32 * 32;  // 256-byte aligned buffers
+    l->work.ensure(sizeof(double) * np * (sch.stages + 1) + (f32 ? sizeof(float) * np : 0));
+    double* const kbuf = l->work.as<double>();
+    double* const mstage64 = kbuf + np * sch.stages;
+    float* const mstage32 = f32 ? reinterpret_cast<float*>(mstage64 + np) : nullptr;
     l->mcand.ensure(sizeof(double) * n3);
-    l->partials.ensure(sizeof(double) * sm_count() * 8 + 64);
-    l->errbuf.ensure(sizeof(double) * 4);
+    if (f32) l->mcand32.ensure(sizeof(float) * n3);
+    ensure_finalize_scratch(l->partials, s.stream);
+    l->err.ensure();
     auto terms = raw_terms(l->terms);
     const double kscale = sch.dt_in_k ? dt : 1.0;
     const double cmul = sch.dt_in_k ? 1.0 : dt;
+    const bool fused = N <= kFusedStageCells;
+    if (marks) marks->mark(s.stream, "attempt");
+    if (f32) {  // the FP64 form has no FP32 copy
+        ensure_m32(st);
+        if (marks) marks->mark(s.stream, "stage_m32");
+    }
     for (int stg = 0; stg < sch.stages; ++stg) {
-        EpilogueArgs ep;
-        ep.kind = EPI_LLG;
-        ep.out = l->k[stg].p;
-        ep.llg = llg_params(l, kscale);
-        if (stg == 0) {
-            ep.llg.m64 = s.m64.as<double>();
-            if (marks) {
-                marks->mark(s.stream, "attempt");
-                if (s.precision == PREC_FP32_FIELD) {  // the FP64 form has no FP32 copy
-                    ensure_m32(st);
-                    marks->mark(s.stream, "stage_m32");
-                }
-            }
-            eval_on_state(st, terms, ep, nullptr, nullptr, marks);
-        } else {
+        const bool other = fused && !(stg & 1);
+        const double* in64 = stg == 0 ? s.m64.as<double>() : other ? l->mcand.as<double>() : mstage64;
+        const float* in32 = stg == 0 ? s.m32.as<float>() : other ? l->mcand32.as<float>() : mstage32;
+        if (stg > 0 && !fused) {
             KList kl;
             for (int j = 0; j < stg; ++j) {
                 if (sch.a[stg][j] == 0.0) continue;
-                kl.k[kl.n] = l->k[j].as<double>();
+                kl.k[kl.n] = kbuf + np * j;
                 kl.c[kl.n] = sch.dt_in_k ? sch.a[stg][j] : dt * sch.a[stg][j];
                 ++kl.n;
             }
-            rk_combine(s.m64.as<double>(), kl, l->mstage64.as<double>(), f32 ? l->mstage32.as<float>() : nullptr, n3,
-                       s.stream);
+            rk_combine(s.m64.as<double>(), kl, mstage64, mstage32, n3, s.stream);
             if (marks) marks->mark(s.stream, kCombineNames[kl.n]);
-            ep.llg.m64 = l->mstage64.as<double>();
-            if (f32)
-                eval_terms<float>(terms, s.md, l->mstage32.as<float>(), s.msinfo(), ep, s.stream, st->scratch, nullptr,
-                                  marks);
-            else
-                eval_terms<double>(terms, s.md, l->mstage64.as<double>(), s.msinfo(), ep, s.stream, st->scratch,
-                                   nullptr, marks);
         }
+        EpilogueArgs ep;
+        ep.kind = EPI_LLG;
+        ep.out = kbuf + np * stg;
+        ep.llg = llg_params(l, kscale);
+        ep.llg.m64 = in64;
+        if (fused && stg + 1 < sch.stages) {
+            NextStage& ns = ep.llg.next;
+            ns.out64 = ((stg + 1) & 1) ? mstage64 : l->mcand.as<double>();
+            ns.out32 = !f32 ? nullptr : ((stg + 1) & 1) ? mstage32 : l->mcand32.as<float>();
+            ns.base = s.m64.as<double>();
+            for (int j = 0; j <= stg; ++j) {
+                if (sch.a[stg + 1][j] == 0.0) continue;
+                const double c = sch.dt_in_k ? sch.a[stg + 1][j] : dt * sch.a[stg + 1][j];
+                if (j == stg) {
+                    ns.with_cur = 1;
+                    ns.cur = c;
+                } else {
+                    ns.k[ns.n] = kbuf + np * j;
+                    ns.c[ns.n] = c;
+                    ++ns.n;
+                }
+            }
+        }
+        if (f32)
+            eval_terms<float>(terms, s.md, in32, s.msinfo(), ep, s.stream, st->scratch, nullptr, marks);
+        else
+            eval_terms<double>(terms, s.md, in64, s.msinfo(), ep, s.stream, st->scratch, nullptr, marks);
     }
     KList kb, ke;
     for (int j = 0; j < sch.stages; ++j) {
         if (sch.b[j] != 0.0) {
-            kb.k[kb.n] = l->k[j].as<double>();
+            kb.k[kb.n] = kbuf + np * j;
             kb.c[kb.n] = sch.b[j] * cmul;
             ++kb.n;
         }
         if (sch.e[j] != 0.0) {
-            ke.k[ke.n] = l->k[j].as<double>();
+            ke.k[ke.n] = kbuf + np * j;
             ke.c[ke.n] = sch.e[j] * cmul;
             ++ke.n;
         }
     }
-    rk_finalize(s.m64.as<double>(), kb, ke, sch.form, l->ctrl.atol, l->ctrl.rtol, l->mcand.as<double>(), norm_mode, N,
-                l->partials.as<double>(), l->errbuf.as<double>(), s.stream);
+    rk_finalize(s.m64.as<double>(), kb, ke, sch.form, l->ctrl.atol, l->ctrl.rtol, l->mcand.as<double>(),
+                f32 ? l->mcand32.as<float>() : nullptr, norm_mode, N, l->partials.as<double>(), l->err.device(),
+                s.stream);
     if (marks) {
         std::vector<const double*> uniq;
         for (int j = 0; j < kb.n; ++j) uniq.push_back(kb.k[j]);
@@ -357,15 +413,17 @@ double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, i
             if (std::find(uniq.begin(), uniq.end(), ke.k[j]) == uniq.end()) uniq.push_back(ke.k[j]);
         marks->mark(s.stream, kFinalizeNames[std::min<size_t>(uniq.size(), 8)]);
     }
-    double err = 0;
-    MAF_CUDA(cudaMemcpyAsync(&err, l->errbuf.p, sizeof(double), cudaMemcpyDeviceToHost, s.stream));
     MAF_CUDA(cudaStreamSynchronize(s.stream));
-    return err;
+    return *l->err.p;
 }
 
 void accept_candidate(maf_llg_s* l, maf_state_s* st) {
     std::swap(st->s.m64, l->mcand);
     st->m32_valid = false;
+    if (st->s.precision == PREC_FP32_FIELD) {  // the candidate's FP32 copy (as ensure_m32 would make it)
+        std::swap(st->s.m32, l->mcand32);
+        st->m32_valid = true;
+    }
 }
 
 void llg_step(maf_llg_s* l, maf_state_s* st) {
@@ -517,7 +575,7 @@ void stoch_step(maf_stoch_s* h, maf_state_s* st, unsigned long long* q_dev = nul
     h->mstage64.ensure(sizeof(double) * n3);
     if (f32) h->mstage32.ensure(sizeof(float) * n3);
     h->mcand.ensure(sizeof(double) * n3);
-    h->partials.ensure(sizeof(double) * sm_count() * 8 + 64);
+    ensure_finalize_scratch(h->partials, s.stream);
     h->errbuf.ensure(sizeof(double) * 4);
     std::vector<Term*> terms;
     for (auto& t : h->terms) terms.push_back(t.get());
@@ -568,8 +626,8 @@ void stoch_step(maf_stoch_s* h, maf_state_s* st, unsigned long long* q_dev = nul
     dummy.n = 1;
     dummy.k[0] = fin.k[0];
     dummy.c[0] = 0.0;
-    rk_finalize(s.m64.as<double>(), fin, dummy, 0, 1.0, 0.0, h->mcand.as<double>(), 2, N, h->partials.as<double>(),
-                h->errbuf.as<double>(), s.stream);
+    rk_finalize(s.m64.as<double>(), fin, dummy, 0, 1.0, 0.0, h->mcand.as<double>(), nullptr, 2, N,
+                h->partials.as<double>(), h->errbuf.as<double>(), s.stream);
     std::swap(s.m64, h->mcand);
     if (q_dev) inc_counter(q_dev, s.stream);
     st->m32_valid = false;
@@ -1923,13 +1981,13 @@ int maf_llg_dmdt(maf_llg l, maf_state s, double* out) {
         check_llg_state(l, s);
         check(out, "NULL argument");
         const int64_t n3 = 3 * s->s.md.N();
-        l->k[0].ensure(sizeof(double) * n3);
+        l->work.ensure(sizeof(double) * n3);
         EpilogueArgs ep;
         ep.kind = EPI_LLG;
-        ep.out = l->k[0].p;
+        ep.out = l->work.p;
         ep.llg = llg_params(l, 1.0);
         eval_on_state(s, raw_terms(l->terms), ep);
-        MAF_CUDA(cudaMemcpyAsync(out, l->k[0].p, sizeof(double) * n3, cudaMemcpyDeviceToHost, s->s.stream));
+        MAF_CUDA(cudaMemcpyAsync(out, l->work.p, sizeof(double) * n3, cudaMemcpyDeviceToHost, s->s.stream));
         MAF_CUDA(cudaStreamSynchronize(s->s.stream));
     });
 }
@@ -2741,6 +2799,8 @@ void batch_capture(maf_stoch_batch_s* b) {
     b->fb.reset();
     b->fused_active = false;
     if (b->fused) b->fb = make_fused(b);
+    // every replay stages the FP32 copy of m itself (the per-member steps skip it when it is valid)
+    for (auto* st : b->sts) st->m32_valid = false;
     // host-side state advances while the work is only recorded: restore it
     std::vector<double> t(n);
     std::vector<unsigned long long> steps(n), calls(n);

@@ -70,6 +70,20 @@ enum Epilogue : int {
     EPI_EGRAD = 3,  // energy partials and the LBFGS gradient m x (m x H) (double) to out[3][N]
 };
 
+// The next Runge-Kutta stage's magnetisation, written by the epilogue that computes a
+// stage's k: out = base + sum_j c[j] k[j] + cur k (in that order), and its FP32 copy.
+// out must not be the buffer the epilogue reads m from.
+struct NextStage {
+    double* out64 = nullptr;      // null: nothing to write
+    float* out32 = nullptr;
+    const double* base = nullptr;
+    const double* k[6] = {};      // earlier k's
+    double c[6] = {};
+    int n = 0;
+    int with_cur = 0;             // whether this stage's k enters
+    double cur = 0;
+};
+
 struct LLGParams {
     double c_prec = 0;             // -gamma/(1+alpha^2)
     double c_damp = 0;             // -alpha*gamma/(1+alpha^2)
@@ -86,6 +100,7 @@ struct LLGParams {
     // the device: a captured CUDA graph replays with the step counter it advances
     const unsigned long long* noise_base = nullptr;
     unsigned noise_mul = 0;
+    NextStage next;
     __host__ __device__ unsigned long long stream_index() const {
 #ifdef __CUDA_ARCH__
         return noise_base ? noise_mul * (*noise_base) + noise_index : noise_index;

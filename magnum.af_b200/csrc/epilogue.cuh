@@ -16,6 +16,43 @@ __device__ __forceinline__ R cell_Ms(const MsInfo& ms, int64_t cell) {
     return (R)ms.Ms;
 }
 
+template <typename R, int N> __device__ __forceinline__ void loadN(const R* __restrict__ p, R out[N]);
+template <typename R, int N> __device__ __forceinline__ void storeN(R* p, const R v[N]);
+
+// The next stage's magnetisation at N cells whose k is kc (NextStage).  One component
+// at a time with its up to seven loads issued together: a chain of one load per k costs a
+// round trip each, all components at once 72 registers.  Same order of operations as
+// k_combine.
+template <int N>
+__device__ __forceinline__ void next_stage(const NextStage& ns, int64_t stride, int64_t cell0, const double kc[3][N]) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const int64_t i = c * stride + cell0;
+        double acc[N], kv[6][N];
+        loadN<double, N>(ns.base + i, acc);
+#pragma unroll
+        for (int j = 0; j < 6; ++j)
+            if (j < ns.n) loadN<double, N>(ns.k[j] + i, kv[j]);
+#pragma unroll
+        for (int j = 0; j < 6; ++j)
+            if (j < ns.n) {
+#pragma unroll
+                for (int e = 0; e < N; ++e) acc[e] = acc[e] + ns.c[j] * kv[j][e];
+            }
+        if (ns.with_cur) {
+#pragma unroll
+            for (int e = 0; e < N; ++e) acc[e] = acc[e] + ns.cur * kc[c][e];
+        }
+        storeN<double, N>(ns.out64 + i, acc);
+        if (ns.out32) {
+            float f[N];
+#pragma unroll
+            for (int e = 0; e < N; ++e) f[e] = (float)acc[e];
+            storeN<float, N>(ns.out32 + i, f);
+        }
+    }
+}
+
 template <typename R, int EPI>
 __device__ __forceinline__ void epilogue_cell(const Geom& g, int x, int y, int z, int64_t cell,
                                               const R* __restrict__ m, const MsInfo& ms, const TermList& tl,
@@ -116,9 +153,11 @@ __device__ __forceinline__ void epilogue_cell(const Geom& g, int x, int y, int z
             }
             double* o = static_cast<double*>(ep.out);
             const double sc = ep.llg.scale;
-            o[cell] = sc * k0;
-            o[g.N + cell] = sc * k1;
-            o[2 * g.N + cell] = sc * k2;
+            const double kc[3][1] = {{sc * k0}, {sc * k1}, {sc * k2}};
+            o[cell] = kc[0][0];
+            o[g.N + cell] = kc[1][0];
+            o[2 * g.N + cell] = kc[2][0];
+            if (ep.llg.next.out64) next_stage<1>(ep.llg.next, g.N, cell, kc);
         }
     }
 }
@@ -475,6 +514,9 @@ __device__ __forceinline__ double runN_epilogue(const TermList& tl, const Geom& 
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) storeN<double, N>(o + c * g.N + cell0, out[c]);
+        if constexpr (EPI == EPI_LLG) {
+            if (ep.llg.next.out64) next_stage<N>(ep.llg.next, g.N, cell0, out);
+        }
     }
     return e;
 }
@@ -509,6 +551,11 @@ inline int run_mode(const Geom& g, const R* m, const MsInfo& ms, const TermList&
     uintptr_t a = (uintptr_t)m;
     if (ep.kind != EPI_EDENS) a |= (uintptr_t)ep.out;
     if (ep.kind == EPI_LLG || ep.kind == EPI_EGRAD) a |= (uintptr_t)ep.llg.m64;
+    if (ep.kind == EPI_LLG && ep.llg.next.out64) {
+        const NextStage& ns = ep.llg.next;
+        a |= (uintptr_t)ns.out64 | (uintptr_t)ns.out32 | (uintptr_t)ns.base;
+        for (int j = 0; j < ns.n; ++j) a |= (uintptr_t)ns.k[j];
+    }
     return g.nx % run == 0 && a % 16 == 0 ? 1 : 2;
 }
 

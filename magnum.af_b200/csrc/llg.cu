@@ -80,23 +80,43 @@ __device__ __forceinline__ double nanmax(double a, double b) {
     return a > b ? a : b;
 }
 
-__device__ __forceinline__ void block_max_store(double v, double* partials) {
+// The block's maximum to partials[block]; the block that arrives last writes the maximum
+// over all blocks to *err (a kernel of its own for it was one more dependent launch per
+// step).  *counter is zero before and after the launch.
+__device__ __forceinline__ void block_max_final(double v, double* partials, unsigned* counter, double* err) {
     __shared__ double red[32];
     for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     if (lane == 0) red[wid] = v;
     __syncthreads();
-    if (wid == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        double s = lane < nw ? red[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) s = nanmax(s, __shfl_down_sync(0xffffffffu, s, o));
-        if (lane == 0) partials[blockIdx.x] = s;
+    __shared__ bool last;
+    const int nw = (blockDim.x + 31) >> 5;
+    if (threadIdx.x == 0) {
+        double s = red[0];
+        for (int k = 1; k < nw; ++k) s = nanmax(s, red[k]);
+        partials[blockIdx.x] = s;
+        __threadfence();
+        last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    v = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) v = nanmax(v, __ldcg(partials + b));
+    for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
+    if (lane == 0) red[wid] = v;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = red[0];
+        for (int k = 1; k < nw; ++k) s = nanmax(s, red[k]);
+        *err = s;
     }
 }
 
 // sumbk = sum bs_j k_j ; rk_error = (form 0) sum e_j k_j  or (form 1) sumbk - sum e_j k_j
 __global__ void k_finalize(const double* __restrict__ m, KList kb, KList ke, int form, double atol, double rtol,
-                           double* __restrict__ mcand, int norm_mode, int64_t N, double* __restrict__ partials) {
+                           double* __restrict__ mcand, float* __restrict__ mcand32, int norm_mode, int64_t N,
+                           double* partials, unsigned* counter, double* errout) {
     double vmax = 0.0;
     for (int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; cell < N;
          cell += (int64_t)gridDim.x * blockDim.x) {
@@ -124,25 +144,13 @@ __global__ void k_finalize(const double* __restrict__ m, KList kb, KList ke, int
             if (nrm != 0) { out[0] /= nrm; out[1] /= nrm; out[2] /= nrm; }
             else { out[0] = 0; out[1] = 0; out[2] = 0; }
         }
-        mcand[cell] = out[0];
-        mcand[N + cell] = out[1];
-        mcand[2 * N + cell] = out[2];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            mcand[c * N + cell] = out[c];
+            if (mcand32) mcand32[c * N + cell] = (float)out[c];
+        }
     }
-    block_max_store(vmax, partials);
-}
-
-__global__ void k_max_partials(const double* __restrict__ p, int n, double* out) {
-    double v = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) v = nanmax(v, p[i]);
-    __shared__ double red[32];
-    for (int o = 16; o > 0; o >>= 1) v = nanmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        double s = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) s = nanmax(s, __shfl_down_sync(0xffffffffu, s, o));
-        if (threadIdx.x == 0) *out = s;
-    }
+    block_max_final(vmax, partials, counter, errout);
 }
 
 // The union of the b- and e-lists' k buffers, each loaded once: k[j] enters
@@ -182,8 +190,9 @@ __device__ __forceinline__ void fin_norm(double* o, int norm_mode) {
 // arithmetic as k_finalize, bit-identical results.
 template <int NU>
 __global__ void __launch_bounds__(256) k_finalize_v(const double* __restrict__ m, KUnion ku, int form, double atol,
-                                                    double rtol, double* __restrict__ mcand, int norm_mode, int64_t N,
-                                                    double* __restrict__ partials) {
+                                                    double rtol, double* __restrict__ mcand,
+                                                    float* __restrict__ mcand32, int norm_mode, int64_t N,
+                                                    double* partials, unsigned* counter, double* errout) {
     const int64_t N2 = N / 2;
     double vmax = 0.0;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N2; p += (int64_t)gridDim.x * blockDim.x) {
@@ -213,9 +222,12 @@ __global__ void __launch_bounds__(256) k_finalize_v(const double* __restrict__ m
         fin_norm(o0, norm_mode);
         fin_norm(o1, norm_mode);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) reinterpret_cast<double2*>(mcand)[c * N2 + p] = make_double2(o0[c], o1[c]);
+        for (int c = 0; c < 3; ++c) {
+            reinterpret_cast<double2*>(mcand)[c * N2 + p] = make_double2(o0[c], o1[c]);
+            if (mcand32) reinterpret_cast<float2*>(mcand32)[c * N2 + p] = make_float2((float)o0[c], (float)o1[c]);
+        }
     }
-    block_max_store(vmax, partials);
+    block_max_final(vmax, partials, counter, errout);
 }
 
 // Union of the two lists with each list's order preserved, or false.
@@ -244,32 +256,35 @@ static bool make_union(const KList& kb, const KList& ke, KUnion& u) {
     return u.n >= 1 && u.n <= 7;
 }
 
-int rk_finalize(const double* m, const KList& kb, const KList& ke, int form, double atol, double rtol, double* mcand,
-                int norm_mode, int64_t N, double* partials, double* err_dev, cudaStream_t st) {
+int rk_finalize_blocks() { return 8 * sm_count(); }
+
+void rk_finalize(const double* m, const KList& kb, const KList& ke, int form, double atol, double rtol, double* mcand,
+                 float* mcand32, int norm_mode, int64_t N, double* partials, double* err, cudaStream_t st) {
     const int threads = 256;
     KUnion u;
-    bool vec = N % 2 == 0 && aligned16(m) && aligned16(mcand) && make_union(kb, ke, u);
+    bool vec = N % 2 == 0 && aligned16(m) && aligned16(mcand) && ((uintptr_t)mcand32 & 7) == 0 && make_union(kb, ke, u);
     for (int j = 0; vec && j < u.n; ++j) vec = aligned16(u.k[j]);
-    int blocks;
+    const int blocks = (int)std::min<int64_t>(ceil_div(vec ? N / 2 : N, threads), rk_finalize_blocks());
+    unsigned* counter = reinterpret_cast<unsigned*>(partials + rk_finalize_blocks());
     if (vec) {
-        blocks = (int)std::min<int64_t>(ceil_div(N / 2, threads), (int64_t)sm_count() * 8);
+#define MAF_FIN(NU)                                                                                                  \
+    k_finalize_v<NU><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, mcand32, norm_mode, N, partials, counter, \
+                                                 err)
         switch (u.n) {
-            case 1: k_finalize_v<1><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, norm_mode, N, partials); break;
-            case 2: k_finalize_v<2><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, norm_mode, N, partials); break;
-            case 3: k_finalize_v<3><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, norm_mode, N, partials); break;
-            case 4: k_finalize_v<4><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, norm_mode, N, partials); break;
-            case 5: k_finalize_v<5><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, norm_mode, N, partials); break;
-            case 6: k_finalize_v<6><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, norm_mode, N, partials); break;
-            default: k_finalize_v<7><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, norm_mode, N, partials); break;
+            case 1: MAF_FIN(1); break;
+            case 2: MAF_FIN(2); break;
+            case 3: MAF_FIN(3); break;
+            case 4: MAF_FIN(4); break;
+            case 5: MAF_FIN(5); break;
+            case 6: MAF_FIN(6); break;
+            default: MAF_FIN(7); break;
         }
+#undef MAF_FIN
     } else {
-        blocks = (int)std::min<int64_t>(ceil_div(N, threads), (int64_t)sm_count() * 8);
-        k_finalize<<<blocks, threads, 0, st>>>(m, kb, ke, form, atol, rtol, mcand, norm_mode, N, partials);
+        k_finalize<<<blocks, threads, 0, st>>>(m, kb, ke, form, atol, rtol, mcand, mcand32, norm_mode, N, partials,
+                                               counter, err);
     }
     MAF_LAUNCH_CHECK();
-    k_max_partials<<<1, 256, 0, st>>>(partials, blocks, err_dev);
-    MAF_LAUNCH_CHECK();
-    return blocks;
 }
 
 // normalize_handle_zero_vectors (util.cpp:37-42); counts cells of zero norm
