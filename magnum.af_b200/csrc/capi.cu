@@ -933,7 +933,22 @@ double lbfgs_minimize(maf_lbfgs_s* h, maf_state_s* st) {
         // the pair was stored: the same value as recomputing it).  Step 0 copies x and the
         // gradient; steps 1 .. k are the first loop and k+1 .. 2k the second; each forms the
         // dot product of the next, the last one grad . q and the search direction s = -q.
-        for (int step = 0; step <= 2 * k; ++step) {
+        LbLoop lp;
+        lp.grad = h->grad.as<double>();
+        lp.k = k;
+        for (int i = 0; i < k; ++i) {
+            lp.s[i] = h->sV[order[i]].as<double>();
+            lp.y[i] = h->yV[order[i]].as<double>();
+            lp.rho[i] = h->rho[order[i]];
+        }
+        lp.scale = H0k;
+        lp.x = S.m64.as<double>();
+        lp.x_copy = h->x_old.as<double>();
+        lp.g_copy = h->grad_old.as<double>();
+        lp.dir = h->s.as<double>();
+        lp.d = coef + kLbDot;
+        const bool looped = lb_loop(lp, n3, S.stream);  // small films: the same steps in one launch
+        for (int step = 0; !looped && step <= 2 * k; ++step) {
             LbRecur a;
             a.q_in = step == 0 ? h->grad.as<double>() : h->q.as<double>();
             a.q = h->q.as<double>();

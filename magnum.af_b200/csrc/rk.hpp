@@ -49,6 +49,22 @@ struct LbRecur {
     double* g_copy = nullptr;       // copy of q_in
 };
 void lb_recur(const LbRecur& a, int64_t n, double* part, unsigned* counter, cudaStream_t st);
+// The recursion over k stored pairs (s[0..k), y[0..k), oldest first) in one launch: dir = -q,
+// *d = grad . q, the copies as above; false (nothing done) when n is too large for it.
+struct LbLoop {
+    const double* grad = nullptr;
+    const double* s[5] = {};
+    const double* y[5] = {};
+    double rho[5] = {};
+    int k = 0;
+    double scale = 1.0;
+    const double* x = nullptr;
+    double* x_copy = nullptr;
+    double* g_copy = nullptr;
+    double* dir = nullptr;
+    double* d = nullptr;
+};
+bool lb_loop(const LbLoop& a, int64_t n, cudaStream_t st);
 void lb_slope(const double* g, const double* s, int64_t n, const double* e, int ne, double* part, unsigned* counter,
               double* out, cudaStream_t st);
 void lb_pair(const double* x, const double* x_old, const double* g, const double* g_old, double* s, double* y,
