@@ -448,14 +448,22 @@ __global__ void __launch_bounds__(kRT) k_relu_bias_bwd(const float* __restrict__
     }
 }
 
-// db[c] = sum of part[0..nb)[c], one warp per channel in a fixed order
-__global__ void k_bias_final(const double* __restrict__ part, int nb, int C, float* __restrict__ db) {
-    const int c = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
-    if (c >= C) return;
+// db[c] = sum of part[0..nb)[c] in a fixed order: a block takes 32 channels, eight
+// groups of threads every eighth row of partials
+__global__ void __launch_bounds__(256) k_bias_final(const double* __restrict__ part, int nb, int C, float* __restrict__ db) {
+    __shared__ double red[8][32];
+    const int l = threadIdx.x & 31, g = threadIdx.x >> 5, c = blockIdx.x * 32 + l;
     double s = 0.0;
-    for (int b = threadIdx.x & 31; b < nb; b += 32) s += part[(int64_t)b * C + c];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) db[c] = (float)s;
+    if (c < C) {
+#pragma unroll 8
+        for (int b = g; b < nb; b += 8) s += part[(int64_t)b * C + c];
+    }
+    red[g][l] = s;
+    __syncthreads();
+    if (g == 0 && c < C) {
+        for (int k = 1; k < 8; ++k) s += red[k][l];
+        db[c] = (float)s;
+    }
 }
 
 constexpr int kReluBlocks = 592;  // 4 per SM
@@ -557,7 +565,7 @@ int maf_nn_relu_bias_bwd(const float* dA, const float* A, long long P, int C, in
         k_relu_bias_bwd<<<dim3((unsigned)nb, (unsigned)ceil_div(Cp, kRT)), kRT, 0, s>>>(
             dA, A, P, C, relu, static_cast<__nv_bfloat16*>(dYb), Cp, part);
         MAF_LAUNCH_CHECK();
-        k_bias_final<<<(unsigned)ceil_div(C, 8), 256, 0, s>>>(part, nb, C, db);
+        k_bias_final<<<(unsigned)ceil_div(C, 32), 256, 0, s>>>(part, nb, C, db);
         MAF_LAUNCH_CHECK();
     });
 }
