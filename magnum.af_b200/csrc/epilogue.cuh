@@ -448,7 +448,9 @@ __device__ __forceinline__ double runN_energy(const TermList& tl, const RunN<R, 
 
 // Writes the epilogue output (H, dt*LLG or the LBFGS gradient) of the run; returns
 // the run's energy density for EPI_EDENS and EPI_EGRAD (0 otherwise).
-template <typename R, int EPI, int N, bool MSF>
+// NEXT: also the next stage's m where one is asked for (its loads' registers are kept
+// out of the kernels for large meshes, which never ask).
+template <typename R, int EPI, int N, bool MSF, bool NEXT>
 __device__ __forceinline__ double runN_epilogue(const TermList& tl, const Geom& g, const RunN<R, N>& r, int64_t cell0,
                                                 const R hd[N][3], const EpilogueArgs& ep, double Ms) {
     R h[N][3];
@@ -514,7 +516,7 @@ __device__ __forceinline__ double runN_epilogue(const TermList& tl, const Geom& 
         }
 #pragma unroll
         for (int c = 0; c < 3; ++c) storeN<double, N>(o + c * g.N + cell0, out[c]);
-        if constexpr (EPI == EPI_LLG) {
+        if constexpr (EPI == EPI_LLG && NEXT) {
             if (ep.llg.next.out64) next_stage<N>(ep.llg.next, g.N, cell0, out);
         }
     }

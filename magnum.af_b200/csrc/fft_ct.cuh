@@ -100,6 +100,50 @@ template <int DIR, typename R> __host__ __device__ __forceinline__ void bfly3(cp
     v[2] = csub(t2, t3);
 }
 
+// 6-point DFT as 2 x 3 and 12-point DFT as 4 x 3: one stage where a radix-3 stage and a
+// radix-2 or -4 stage exchanged through shared memory.
+template <int DIR, typename R> __host__ __device__ __forceinline__ void bfly6(cplx_t<R>* v) {
+    using C = cplx_t<R>;
+    const R h3 = (R)0.86602540378443864676, h = (R)0.5;  // sin, cos (pi/3)
+    C e[3] = {v[0], v[2], v[4]}, o[3] = {v[1], v[3], v[5]};
+    bfly3<DIR, R>(e);
+    bfly3<DIR, R>(o);
+    const C o1 = cmul(o[1], mk(h, (R)DIR * h3)), o2 = cmul(o[2], mk(-h, (R)DIR * h3));  // W6, W6^2
+    v[0] = cadd(e[0], o[0]);
+    v[1] = cadd(e[1], o1);
+    v[2] = cadd(e[2], o2);
+    v[3] = csub(e[0], o[0]);
+    v[4] = csub(e[1], o1);
+    v[5] = csub(e[2], o2);
+}
+
+template <int DIR, typename R> __host__ __device__ __forceinline__ void bfly12(cplx_t<R>* v) {
+    using C = cplx_t<R>;
+    const R h3 = (R)0.86602540378443864676, h = (R)0.5, sd = (R)DIR;
+    C a[3][4];  // a[n2][k1] = sum over n1 of v[3 n1 + n2] W4^(n1 k1)
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) {
+        C t[4] = {v[n2], v[3 + n2], v[6 + n2], v[9 + n2]};
+        bfly4<DIR>(t);
+#pragma unroll
+        for (int k1 = 0; k1 < 4; ++k1) a[n2][k1] = t[k1];
+    }
+    // a[n2][k1] *= W12^(n2 k1)
+    a[1][1] = cmul(a[1][1], mk(h3, sd * h));
+    a[1][2] = cmul(a[1][2], mk(h, sd * h3));
+    a[1][3] = cmul_i<DIR>(a[1][3]);
+    a[2][1] = cmul(a[2][1], mk(h, sd * h3));
+    a[2][2] = cmul(a[2][2], mk(-h, sd * h3));
+    a[2][3] = mk(-a[2][3].x, -a[2][3].y);
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1) {
+        C t[3] = {a[0][k1], a[1][k1], a[2][k1]};
+        bfly3<DIR, R>(t);
+#pragma unroll
+        for (int k2 = 0; k2 < 3; ++k2) v[k1 + 4 * k2] = t[k2];
+    }
+}
+
 template <int RAD, int DIR, typename R> __device__ __forceinline__ void bfly_ct(cplx_t<R>* v) {
     if constexpr (RAD == 2) {
         bfly2<DIR>(v[0], v[1]);
@@ -107,10 +151,14 @@ template <int RAD, int DIR, typename R> __device__ __forceinline__ void bfly_ct(
         bfly3<DIR, R>(v);
     } else if constexpr (RAD == 4) {
         bfly4<DIR>(v);
+    } else if constexpr (RAD == 6) {
+        bfly6<DIR, R>(v);
     } else if constexpr (RAD == 8) {
         bfly8<DIR, R>(v);
+    } else if constexpr (RAD == 12) {
+        bfly12<DIR, R>(v);
     } else {
-        static_assert(RAD == 16, "radix 2, 3, 4, 8 or 16");
+        static_assert(RAD == 16, "radix 2, 3, 4, 6, 8, 12 or 16");
         bfly16<DIR, R>(v);
     }
 }
@@ -161,8 +209,8 @@ template <typename R, int RAD, int NS, int L, int NB, int NT, bool BFAST, int TW
     static constexpr int NBF = L / RAD;
     static constexpr int TOTAL = NBF * NB;
     static constexpr int BPT = (TOTAL + NT - 1) / NT;
-    // (a radix-3 stage loads both of its twiddles)
-    static constexpr bool FULL = tw_mode<R>() == 0 || RAD == 3;
+    // (the stages with a factor 3 load all of their twiddles)
+    static constexpr bool FULL = tw_mode<R>() == 0 || RAD % 3 == 0;
     static constexpr int NBASE = NS == 1 ? 0 : FULL ? RAD - 1 : (RAD == 16 ? 4 : RAD == 8 ? 3 : RAD == 4 ? 2 : 1);
     C w[BPT][NBASE > 0 ? NBASE : 1];
     __device__ __forceinline__ void load(const C* __restrict__ tw) {
@@ -522,10 +570,10 @@ template <> struct CtPlan<512> { using T = Radices<16, 16, 2>; };
 template <> struct CtPlan<1024> { using T = Radices<16, 16, 4>; };
 template <> struct CtPlan<2048> { using T = Radices<16, 16, 8>; };
 template <> struct CtPlan<4096> { using T = Radices<16, 16, 16>; };
-// three times a power of two: the radix-3 stage second (after the pruned radix-16
-// first stage, before an even last stage that output pruning can halve)
-template <> struct CtPlan<96> { using T = Radices<16, 3, 2>; };
-template <> struct CtPlan<192> { using T = Radices<16, 3, 4>; };
+// three times a power of two: the factor 3 in the second stage (after the pruned
+// radix-16 first stage; the last stage is even, so that output pruning can halve it)
+template <> struct CtPlan<96> { using T = Radices<16, 6>; };
+template <> struct CtPlan<192> { using T = Radices<16, 12>; };
 template <> struct CtPlan<384> { using T = Radices<16, 3, 8>; };
 template <> struct CtPlan<768> { using T = Radices<16, 3, 16>; };
 template <> struct CtPlan<1536> { using T = Radices<16, 3, 16, 2>; };

@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(256) k_local_epi(Geom g, const R* __restrict__
 // run epilogue with a zero demag contribution (eligibility: run_mode).
 // Thread q takes run q of the flattened (row, run) index (fewer than 2^31 runs).
 // FP32: capped for two CTAs per SM (128 registers); FP64 uncapped (it would spill).
-template <typename R, int EPI, int RN, bool MSF>
+template <typename R, int EPI, int RN, bool MSF, bool NEXT>
 __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_local_run(Geom g, const R* __restrict__ m, MsInfo ms, TermList tl,
                                                                            EpilogueArgs ep, int nruns) {
     const int runs_row = g.nx / RN;
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_local_run(Geom 
             r.ms = cell_Ms<R>(ms, cell0);
             r.inv = (R)1 / r.ms;
         }
-        eacc += runN_epilogue<R, EPI, RN, MSF>(tl, g, r, cell0, hd, ep, Ms);
+        eacc += runN_epilogue<R, EPI, RN, MSF, NEXT>(tl, g, r, cell0, hd, ep, Ms);
     }
     if constexpr (EPI == EPI_EDENS || EPI == EPI_EGRAD) block_sum_store(eacc, ep.partials);
 }
@@ -864,7 +864,8 @@ void eval_terms(const std::vector<Term*>& terms, const MeshDims& md, const R* m,
         // for the energies (the energy and the field of four do not fit the registers)
         const Geom g = md.geom();
         prepare_run(tl, g, ms);
-        const bool four = run == 1 && g.nx % 4 == 0 && (ep.kind == EPI_H || ep.kind == EPI_LLG);
+        // (and with the next Runge-Kutta stage)
+        const bool four = run == 1 && g.nx % 4 == 0 && (ep.kind == EPI_H || (ep.kind == EPI_LLG && !ep.llg.next.out64));
         const int nruns = (int)(md.N() / (four ? 4 : run == 1 ? 2 : 1));
         const int threads = 256;
         const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(nruns, threads), (int64_t)sm_count() * 16);
@@ -873,16 +874,16 @@ void eval_terms(const std::vector<Term*>& terms, const MeshDims& md, const R* m,
 #define MAF_LOCAL_RUN(EPI)                                                                                        \
     do {                                                                                                         \
         if (run == 1)                                                                                            \
-            k_local_run<R, EPI, 2, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                  \
+            k_local_run<R, EPI, 2, false, true><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                  \
         else if (run == 2)                                                                                       \
-            k_local_run<R, EPI, 1, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                  \
+            k_local_run<R, EPI, 1, false, true><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                  \
         else                                                                                                     \
-            k_local_run<R, EPI, 1, true><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                   \
+            k_local_run<R, EPI, 1, true, true><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);                   \
     } while (0)
         if (four && ep.kind == EPI_H)
-            k_local_run<R, EPI_H, 4, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);
+            k_local_run<R, EPI_H, 4, false, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);
         else if (four)
-            k_local_run<R, EPI_LLG, 4, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);
+            k_local_run<R, EPI_LLG, 4, false, false><<<blocks, threads, 0, st>>>(g, m, ms, tl, ep, nruns);
         else if (ep.kind == EPI_H)
             MAF_LOCAL_RUN(EPI_H);
         else if (ep.kind == EPI_LLG)

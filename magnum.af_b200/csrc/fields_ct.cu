@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(NT) k_convy_ct(cplx_t<R>* S, const R* __restri
 // The run epilogue on the tile's rows, whose demag values sit in s.  Rows have up
 // to LC cells: the run index arithmetic is compile-time, runs beyond a shorter row
 // are skipped.  Returns the thread's energy density.
-template <typename R, int EPI, int LC, int NBR, int NT, int N, bool MSF>
+template <typename R, int EPI, int LC, int NBR, int NT, int N, bool MSF, bool NEXT>
 __device__ __forceinline__ double xinv_runs(const cplx_t<R>* s, const Geom& g, R scale, const R* __restrict__ m,
                                             const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep, int ry0) {
     constexpr int SB = (LC - 1) + ((LC - 1) >> 4) + 1;
@@ -612,13 +612,20 @@ __device__ __forceinline__ double xinv_runs(const cplx_t<R>* s, const Geom& g, R
                 }
             }
         }
-        eacc += runN_epilogue<R, EPI, N, MSF>(tl, g, r, cell0, hd, ep, Ms);
+        eacc += runN_epilogue<R, EPI, N, MSF, NEXT>(tl, g, r, cell0, hd, ep, Ms);
     }
     return eacc;
 }
 
-// (tile body: (y, z) rows [tile NBR, tile NBR + NBR); run: run_mode's answer)
-template <typename R, int EPI, int LC, int NBR, int NT, int RN>
+// What an x-inverse kernel's epilogue is compiled for (run_mode's answer `run`): runs of
+// RN cells only (1), the same with the next Runge-Kutta stage, the other modes of a single
+// state (0, 2 and 3), or the modes of a batch item (0, 1 and 2).  One kernel for all of
+// them needed the registers of the widest: at the FP32 cap of 80 it spilled 208 bytes, and
+// the FP64 pass at 512x512x16 took 160 us instead of 150.
+enum XinvMode { XM_RUN, XM_RUN_NEXT, XM_OTHER, XM_BATCH };
+
+// (tile body: (y, z) rows [tile NBR, tile NBR + NBR))
+template <typename R, int EPI, int LC, int NBR, int NT, int RN, XinvMode XM>
 __device__ __forceinline__ void xinv_ct_tile(const cplx_t<R>* __restrict__ S1, int pitch,
                                              const cplx_t<R>* __restrict__ tw, const cplx_t<R>* __restrict__ twP,
                                              const Geom& g, R scale, const R* __restrict__ m, const MsInfo& ms,
@@ -650,39 +657,45 @@ __device__ __forceinline__ void xinv_ct_tile(const cplx_t<R>* __restrict__ S1, i
     else
         ct_fft_in<R, 1, false, LC, NC, NT>(s, SB, tw, ld, typename CtPlan<LC>::T());
     double eacc = 0;
-    if constexpr (sizeof(R) == 4 && EPI == EPI_EGRAD) run = 0;  // as run_mode
-    if (run) {
-        eacc = run == 1   ? xinv_runs<R, EPI, LC, NBR, NT, RN, false>(s, g, scale, m, ms, tl, ep, ry0)
-               : run == 2 ? xinv_runs<R, EPI, LC, NBR, NT, 1, false>(s, g, scale, m, ms, tl, ep, ry0)
-                          : xinv_runs<R, EPI, LC, NBR, NT, 1, true>(s, g, scale, m, ms, tl, ep, ry0);
-        if constexpr (EPI == EPI_EDENS || EPI == EPI_EGRAD) block_sum_store(eacc, ep.partials);
-        return;
-    }
-    for (int idx = threadIdx.x; idx < NBR * g.nx; idx += NT) {
-        const int b = idx / g.nx;
-        const int x = idx - b * g.nx;
-        const int ry = ry0 + b;
-        if (ry >= rows_pc) continue;
-        const int z = ry / g.ny;
-        const int y = ry - z * g.ny;
-        const int64_t cell = (int64_t)ry * g.nx + x;
-        R hd[3];
+    if constexpr (XM == XM_RUN || XM == XM_RUN_NEXT) {
+        eacc = xinv_runs<R, EPI, LC, NBR, NT, RN, false, XM == XM_RUN_NEXT>(s, g, scale, m, ms, tl, ep, ry0);
+    } else if (XM == XM_BATCH && run == 1) {
+        eacc = xinv_runs<R, EPI, LC, NBR, NT, RN, false, false>(s, g, scale, m, ms, tl, ep, ry0);
+    } else if (run == 2) {
+        eacc = xinv_runs<R, EPI, LC, NBR, NT, 1, false, XM != XM_BATCH>(s, g, scale, m, ms, tl, ep, ry0);
+    } else if (XM != XM_BATCH && run == 3) {
+        eacc = xinv_runs<R, EPI, LC, NBR, NT, 1, true, true>(s, g, scale, m, ms, tl, ep, ry0);
+    } else {
+        for (int idx = threadIdx.x; idx < NBR * g.nx; idx += NT) {
+            const int b = idx / g.nx;
+            const int x = idx - b * g.nx;
+            const int ry = ry0 + b;
+            if (ry >= rows_pc) continue;
+            const int z = ry / g.ny;
+            const int y = ry - z * g.ny;
+            const int64_t cell = (int64_t)ry * g.nx + x;
+            R hd[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const C val = s[spad(x >> 1) + (c * NBR + b) * SB];
-            hd[c] = scale * ((x & 1) ? val.y : val.x);
+            for (int c = 0; c < 3; ++c) {
+                const C val = s[spad(x >> 1) + (c * NBR + b) * SB];
+                hd[c] = scale * ((x & 1) ? val.y : val.x);
+            }
+            epilogue_cell<R, EPI>(g, x, y, z, cell, m, ms, tl, ep, hd, eacc);
         }
-        epilogue_cell<R, EPI>(g, x, y, z, cell, m, ms, tl, ep, hd, eacc);
     }
     if constexpr (EPI == EPI_EDENS || EPI == EPI_EGRAD) block_sum_store(eacc, ep.partials);
 }
 
-template <typename R, int EPI, int LC, int NBR, int NT, int RN>
-__global__ void __launch_bounds__(NT, (kMinBlocks<R, NT, (RN == 2 ? (NT == 192 ? MAF_XINV_THREADS_192 : MAF_XINV_THREADS) : 384), MAF_XINV_THREADS_F64>)) k_xinv_ct(const cplx_t<R>* __restrict__ S1, int pitch,
+template <typename R, int NT, int RN>
+constexpr int kXinvBlocks =
+    kMinBlocks<R, NT, (RN == 2 ? (NT == 192 || NT == 96 ? MAF_XINV_THREADS_192 : MAF_XINV_THREADS) : 384), MAF_XINV_THREADS_F64>;
+
+template <typename R, int EPI, int LC, int NBR, int NT, int RN, XinvMode XM>
+__global__ void __launch_bounds__(NT, (kXinvBlocks<R, NT, RN>)) k_xinv_ct(const cplx_t<R>* __restrict__ S1, int pitch,
                                                 const cplx_t<R>* __restrict__ tw, const cplx_t<R>* __restrict__ twP,
                                                 Geom g, R scale, const R* __restrict__ m, MsInfo ms, TermList tl,
                                                 EpilogueArgs ep, int run) {
-    xinv_ct_tile<R, EPI, LC, NBR, NT, RN>(S1, pitch, tw, twP, g, scale, m, ms, tl, ep, run, blockIdx.x);
+    xinv_ct_tile<R, EPI, LC, NBR, NT, RN, XM>(S1, pitch, tw, twP, g, scale, m, ms, tl, ep, run, blockIdx.x);
 }
 
 // ---------------------------------------------- batched (work-table) passes
@@ -705,12 +718,12 @@ __global__ void __launch_bounds__(NT) kbt_convy(const CtConvyItem<R>* __restrict
 }
 
 template <typename R, int LC, int NBR, int NT, int RN>
-__global__ void __launch_bounds__(NT, (kMinBlocks<R, NT, (RN == 2 ? (NT == 192 ? MAF_XINV_THREADS_192 : MAF_XINV_THREADS) : 384), MAF_XINV_THREADS_F64>))
+__global__ void __launch_bounds__(NT, (kXinvBlocks<R, NT, RN>))
     kbt_xinv(const CtXinvItem<R>* __restrict__ items, const int2* __restrict__ work, const cplx_t<R>* __restrict__ tw,
              const cplx_t<R>* __restrict__ twP) {
     const int2 w = work[blockIdx.x];
     const CtXinvItem<R>& d = items[w.x];
-    xinv_ct_tile<R, EPI_LLG, LC, NBR, NT, RN>(d.S1, d.pitch, tw, twP, d.g, d.scale, d.m, d.ms, d.tl, d.ep, d.run, w.y);
+    xinv_ct_tile<R, EPI_LLG, LC, NBR, NT, RN, XM_BATCH>(d.S1, d.pitch, tw, twP, d.g, d.scale, d.m, d.ms, d.tl, d.ep, d.run, w.y);
 }
 
 // ------------------------------------------------------------------ launches
@@ -875,12 +888,17 @@ static void convy_L(cplx_t<R>* S, const R* Nred, int ny, int nxh, int pitch, con
     MAF_LAUNCH_CHECK();
 }
 
+// Rows per x-inverse CTA: 4096 values per component triple, 96 threads up to 512 cells
+// per row, so that many CTAs in different phases share an SM (FP32, 512x512x4: 37.9 ->
+// 36.4 us against 192-thread CTAs of two rows); FP32 lengths of three times a power of
+// two take twice as many (their 72-thread CTAs were slower, 17.4 -> 20.4 us at 384x192x4).
+template <typename R, int LC>
+constexpr int kXinvRows = pow2floor(cmax(1, (sizeof(R) == 4 && LC % 3 == 0 ? 8192 : 4096) / (6 * LC)));
+
 template <typename R, int LC, int RN>
 static void xinv_L(const cplx_t<R>* S1, int pitch, const void* tw, const void* twP, const Geom& g, R scale, const R* m,
                    const MsInfo& ms, const TermList& tl_in, const EpilogueArgs& ep, cudaStream_t st, int* nblocks) {
-    // half the column-pass tile: the epilogue's register demand allows one
-    // 384-thread CTA per SM, two CTAs of half the rows overlap their phases
-    constexpr int NBR = pow2floor(cmax(1, kTileC<R> / (6 * LC)));
+    constexpr int NBR = kXinvRows<R, LC>;
     constexpr int NC = 3 * NBR;
     constexpr int NT = LC * NC / kE;
     static_assert(NT <= kMaxFftThreads, "CTA size");
@@ -894,31 +912,33 @@ static void xinv_L(const cplx_t<R>* S1, int pitch, const void* tw, const void* t
     if (nblocks) *nblocks = (int)blocks;
     const auto* t = static_cast<const cplx_t<R>*>(tw);
     const auto* tp = static_cast<const cplx_t<R>*>(twP);
+    auto go = [&](auto k) {
+        ct_smem(k, smem);
+        k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
+    };
     switch (ep.kind) {
-        case EPI_H: {
-            auto k = k_xinv_ct<R, EPI_H, LC, NBR, NT, RN>;
-            ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
+        case EPI_H:
+            if (run == 1) go(k_xinv_ct<R, EPI_H, LC, NBR, NT, RN, XM_RUN>);
+            else go(k_xinv_ct<R, EPI_H, LC, NBR, NT, 2, XM_OTHER>);
             break;
-        }
-        case EPI_LLG: {
-            auto k = k_xinv_ct<R, EPI_LLG, LC, NBR, NT, RN>;
-            ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
+        case EPI_LLG:
+            if (run == 1 && ep.llg.next.out64) go(k_xinv_ct<R, EPI_LLG, LC, NBR, NT, 2, XM_RUN_NEXT>);
+            else if (run == 1) go(k_xinv_ct<R, EPI_LLG, LC, NBR, NT, RN, XM_RUN>);
+            else go(k_xinv_ct<R, EPI_LLG, LC, NBR, NT, 2, XM_OTHER>);
             break;
-        }
-        case EPI_EGRAD: {
-            auto k = k_xinv_ct<R, EPI_EGRAD, LC, NBR, NT, 2>;
-            ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
+        case EPI_EGRAD:
+            if constexpr (sizeof(R) == 8) {  // (run_mode: FP32 gradients go cell by cell)
+                if (run == 1) {
+                    go(k_xinv_ct<R, EPI_EGRAD, LC, NBR, NT, 2, XM_RUN>);
+                    break;
+                }
+            }
+            go(k_xinv_ct<R, EPI_EGRAD, LC, NBR, NT, 2, XM_OTHER>);
             break;
-        }
-        default: {
-            auto k = k_xinv_ct<R, EPI_EDENS, LC, NBR, NT, 2>;
-            ct_smem(k, smem);
-            k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
+        default:
+            if (run == 1) go(k_xinv_ct<R, EPI_EDENS, LC, NBR, NT, 2, XM_RUN>);
+            else go(k_xinv_ct<R, EPI_EDENS, LC, NBR, NT, 2, XM_OTHER>);
             break;
-        }
     }
     MAF_LAUNCH_CHECK();
 }
@@ -935,7 +955,7 @@ template <typename R, int L> struct ConvyShape {
     static constexpr size_t smem = sizeof(cplx_t<R>) * (size_t)3 * NB * ((L - 1) + ((L - 1) >> 4) + 1);
 };
 template <typename R, int LC> struct XinvShape {
-    static constexpr int NBR = pow2floor(cmax(1, kTileC<R> / (6 * LC)));
+    static constexpr int NBR = kXinvRows<R, LC>;
     static constexpr int NT = LC * 3 * NBR / kE;
     static constexpr size_t smem = sizeof(cplx_t<R>) * (size_t)3 * NBR * ((LC - 1) + ((LC - 1) >> 4) + 1);
 };

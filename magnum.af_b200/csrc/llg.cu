@@ -164,13 +164,20 @@ struct KUnion {
     int n = 0;
 };
 
+// vmax <- max(vmax, |err / sc|), NaN-propagating.  The FP64 division is skipped where the
+// quotient, rounded, cannot exceed vmax (the finalize kernels are bound on FP64 division
+// and square root as much as on HBM); a NaN fails the comparison and is divided.
+__device__ __forceinline__ void err_max(double err, double sc, double& vmax) {
+    if (!(fabs(err) <= vmax * sc * (1.0 - 1e-12))) vmax = nanmax(vmax, fabs(err / sc));
+}
+
 __device__ __forceinline__ double fin_one(double sumbk, double e, int form, double mi, double atol, double rtol,
                                           double& vmax) {
     const double err = form == 0 ? e : sumbk - e;
     const double mn = mi + sumbk;
     const double mx = mi > mn ? mi : mn;  // af::max(m, m + sumbk)
     const double sc = atol + rtol * fabs(mx);
-    vmax = nanmax(vmax, fabs(err / sc));
+    err_max(err, sc, vmax);
     return mn;
 }
 
@@ -189,7 +196,7 @@ __device__ __forceinline__ void fin_norm(double* o, int norm_mode) {
 // thread through 16-byte loads (N even, 16-byte aligned buffers); same
 // arithmetic as k_finalize, bit-identical results.
 template <int NU>
-__global__ void __launch_bounds__(256) k_finalize_v(const double* __restrict__ m, KUnion ku, int form, double atol,
+__global__ void __launch_bounds__(256, 4) k_finalize_v(const double* __restrict__ m, KUnion ku, int form, double atol,
                                                     double rtol, double* __restrict__ mcand,
                                                     float* __restrict__ mcand32, int norm_mode, int64_t N,
                                                     double* partials, unsigned* counter, double* errout) {
@@ -256,7 +263,7 @@ static bool make_union(const KList& kb, const KList& ke, KUnion& u) {
     return u.n >= 1 && u.n <= 7;
 }
 
-int rk_finalize_blocks() { return 8 * sm_count(); }
+int rk_finalize_blocks() { return 32 * sm_count(); }
 
 void rk_finalize(const double* m, const KList& kb, const KList& ke, int form, double atol, double rtol, double* mcand,
                  float* mcand32, int norm_mode, int64_t N, double* partials, double* err, cudaStream_t st) {
