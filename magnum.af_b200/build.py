@@ -39,6 +39,7 @@ SOURCES = {
     "umma.o": ("umma.cu", []),
     "nn.o": ("nn.cu", []),
     "conv.o": ("conv.cu", []),
+    "alloc.o": ("alloc.cu", []),
 }
 for _part in (1, 2, 3, 4, 5):
     for _real in (4, 8):

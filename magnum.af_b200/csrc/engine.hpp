@@ -14,6 +14,11 @@ namespace mafb {
 
 enum Precision : int { PREC_FP64 = 0, PREC_FP32_FIELD = 1 };
 
+// Device memory (alloc.cu): dev_alloc throws, dev_free(p, the size asked for) waits for
+// the device's work, as cudaFree does.
+void* dev_alloc(size_t n);
+void dev_free(void* p, size_t n);
+
 // Owning device allocation.
 struct DevBuf {
     void* p = nullptr;
@@ -30,11 +35,11 @@ struct DevBuf {
     ~DevBuf() { release(); }
     void alloc(size_t n) {
         release();
-        if (n) MAF_CUDA(cudaMalloc(&p, n));
+        if (n) p = dev_alloc(n);
         bytes = n;
     }
     void ensure(size_t n) { if (bytes < n) alloc(n); }
-    void release() { if (p) cudaFree(p); p = nullptr; bytes = 0; }
+    void release() { if (p) dev_free(p, bytes); p = nullptr; bytes = 0; }
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
