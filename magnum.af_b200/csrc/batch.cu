@@ -279,7 +279,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
     // compile-time kernel per pass and member (the per-state path's choice: ct_xfwd,
     // ct_convy and ct_xinv run for these lengths unless the DemagField is set to the
     // run-time-plan kernels); cx_of[i] etc.: the member's class, -1 for generic
-    std::vector<int> cx_of(M, -1), cc_of(M, -1), ci_of(M, -1), pos_x(M), pos_c(M), pos_i(M);
+    std::vector<int> cx_of(M, -1), cc_of(M, -1), ci_of(M, -1), pos_x(M), pos_c(M), pos_i(M), run_of(M, 2);
     for (int i = 0; i < M; ++i) {
         Demag* dm = mem[i].demag;
         if (dm->tune.generic) continue;
@@ -299,7 +299,14 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
             c.members.push_back(i);
         }
         if (ct_batch_tile<R>(2, Lc) > 0) {
-            CtClass& c = ct_class(ci, Lc, run);
+            // (the buffers are DevBufs: aligned alike, so the mesh and the terms decide)
+            CtXinvItem<R> it{};
+            it.g = mem[i].md.geom();
+            it.ms.Ms = mem[i].Ms;
+            for (const TermDesc& t : mem[i].terms) it.tl.t[it.tl.n++] = t;
+            it.ep.kind = EPI_LLG;
+            run_of[i] = run;
+            CtClass& c = ct_class(ci, Lc, ct_batch_xinv_class<R>(it, run));
             ci_of[i] = (int)(&c - ci.data());
             pos_i[i] = (int)c.members.size();
             c.members.push_back(i);
@@ -427,7 +434,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
                 if (ci_of[i] >= 0) {
                     const size_t nc = ci[ci_of[i]].members.size();
                     CtXinvItem<R> it{s1, pitch, f.md.geom(), scale, in, ms, tl, ep, 0};
-                    ct_batch_xinv_prepare<R>(it, ci[ci_of[i]].run);
+                    ct_batch_xinv_prepare<R>(it, run_of[i]);
                     ixi[ci_of[i]][((size_t)p * S + s) * nc + pos_i[i]] = it;
                 }
                 CombA c{};

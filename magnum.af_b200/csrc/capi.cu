@@ -246,9 +246,9 @@ struct maf_llg_s {
     bool dissipation_only = false;
     // the k's and one stage buffer in one allocation (rk_work: each allocation above 2 MB costs
     // 0.5-1 ms of a first step); the stages' m goes to that stage buffer and mcand in turn (an
-    // epilogue reads one and writes the other), its FP32 copy likewise; mcand and mcand32 then
-    // take the candidate and are swapped with the state's m
-    DevBuf work, mcand, mcand32, partials;
+    // epilogue reads one and writes the other), its FP32 copy to two buffers likewise; mcand
+    // then takes the candidate and is swapped with the state's m
+    DevBuf work, mcand, partials;
     HostWord err;
     unsigned long long accumulated_steps = 0;
     std::vector<std::string> prof_names;  // interval names of the last maf_llg_attempt_profile
@@ -320,7 +320,7 @@ void ensure_finalize_scratch(DevBuf& partials, cudaStream_t st) {
 }
 
 // One RK attempt of `sch` with step dt; leaves m + sumbk (normalised per
-// norm_mode) in l->mcand (FP32 copy: l->mcand32) and returns the error norm.
+// norm_mode) in l->mcand and returns the error norm.
 // On small meshes (kFusedStageCells) the epilogue that computes a stage's k also writes
 // the next stage's m (NextStage); on large ones rk_combine does.
 double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, int norm_mode,
@@ -330,12 +330,12 @@ double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, i
     const int64_t n3 = 3 * N;
     const bool f32 = s.precision == PREC_FP32_FIELD;
     const int64_t np = (n3 + 31) / 32 * 32;  // 256-byte aligned buffers
-    l->work.ensure(sizeof(double) * np * (sch.stages + 1) + (f32 ? sizeof(float) * np : 0));
+    l->work.ensure(sizeof(double) * np * (sch.stages + 1) + (f32 ? 2 * sizeof(float) * np : 0));
     double* const kbuf = l->work.as<double>();
     double* const mstage64 = kbuf + np * sch.stages;
     float* const mstage32 = f32 ? reinterpret_cast<float*>(mstage64 + np) : nullptr;
+    float* const mother32 = f32 ? mstage32 + np : nullptr;
     l->mcand.ensure(sizeof(double) * n3);
-    if (f32) l->mcand32.ensure(sizeof(float) * n3);
     ensure_finalize_scratch(l->partials, s.stream);
     l->err.ensure();
     auto terms = raw_terms(l->terms);
@@ -350,7 +350,7 @@ double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, i
     for (int stg = 0; stg < sch.stages; ++stg) {
         const bool other = fused && !(stg & 1);
         const double* in64 = stg == 0 ? s.m64.as<double>() : other ? l->mcand.as<double>() : mstage64;
-        const float* in32 = stg == 0 ? s.m32.as<float>() : other ? l->mcand32.as<float>() : mstage32;
+        const float* in32 = stg == 0 ? s.m32.as<float>() : other ? mother32 : mstage32;
         if (stg > 0 && !fused) {
             KList kl;
             for (int j = 0; j < stg; ++j) {
@@ -370,7 +370,7 @@ double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, i
         if (fused && stg + 1 < sch.stages) {
             NextStage& ns = ep.llg.next;
             ns.out64 = ((stg + 1) & 1) ? mstage64 : l->mcand.as<double>();
-            ns.out32 = !f32 ? nullptr : ((stg + 1) & 1) ? mstage32 : l->mcand32.as<float>();
+            ns.out32 = ((stg + 1) & 1) ? mstage32 : mother32;
             ns.base = s.m64.as<double>();
             for (int j = 0; j <= stg; ++j) {
                 if (sch.a[stg + 1][j] == 0.0) continue;
@@ -404,8 +404,7 @@ double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, i
         }
     }
     rk_finalize(s.m64.as<double>(), kb, ke, sch.form, l->ctrl.atol, l->ctrl.rtol, l->mcand.as<double>(),
-                f32 ? l->mcand32.as<float>() : nullptr, norm_mode, N, l->partials.as<double>(), l->err.device(),
-                s.stream);
+                norm_mode, N, l->partials.as<double>(), l->err.device(), s.stream);
     if (marks) {
         std::vector<const double*> uniq;
         for (int j = 0; j < kb.n; ++j) uniq.push_back(kb.k[j]);
@@ -420,10 +419,6 @@ double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, i
 void accept_candidate(maf_llg_s* l, maf_state_s* st) {
     std::swap(st->s.m64, l->mcand);
     st->m32_valid = false;
-    if (st->s.precision == PREC_FP32_FIELD) {  // the candidate's FP32 copy (as ensure_m32 would make it)
-        std::swap(st->s.m32, l->mcand32);
-        st->m32_valid = true;
-    }
 }
 
 void llg_step(maf_llg_s* l, maf_state_s* st) {
@@ -626,7 +621,7 @@ void stoch_step(maf_stoch_s* h, maf_state_s* st, unsigned long long* q_dev = nul
     dummy.n = 1;
     dummy.k[0] = fin.k[0];
     dummy.c[0] = 0.0;
-    rk_finalize(s.m64.as<double>(), fin, dummy, 0, 1.0, 0.0, h->mcand.as<double>(), nullptr, 2, N,
+    rk_finalize(s.m64.as<double>(), fin, dummy, 0, 1.0, 0.0, h->mcand.as<double>(), 2, N,
                 h->partials.as<double>(), h->errbuf.as<double>(), s.stream);
     std::swap(s.m64, h->mcand);
     if (q_dev) inc_counter(q_dev, s.stream);

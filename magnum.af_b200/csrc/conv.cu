@@ -239,6 +239,7 @@ __global__ void __launch_bounds__(128) k_conv(ConvArgs a) {
 #pragma unroll 1
         for (int c0 = 0; c0 < BN && n0 + c0 < nout; c0 += 16) {
             uint32_t u[16];
+            __syncwarp();
             tmem_ld16(cta.tmem + ((uint32_t)(tid & ~31) << 16) + (uint32_t)c0, u);
             if (p >= a.P) continue;
             float v[16];
@@ -360,6 +361,7 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(WgradArgs a) {
 #pragma unroll 1
         for (int c0 = 0; c0 < BN && n0 + c0 < a.Np; c0 += 16) {
             uint32_t u[16];
+            __syncwarp();
             tmem_ld16(cta.tmem + ((uint32_t)(tid & ~31) << 16) + (uint32_t)c0, u);
             if (m >= M) continue;
 #pragma unroll

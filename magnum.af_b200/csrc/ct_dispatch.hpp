@@ -66,7 +66,11 @@ template <typename R> struct CtXinvItem {
 template <typename R> int ct_batch_tile(int pass, int L);
 // The twiddle table the pass's kernel of length L reads (created on first use).
 template <typename R> const void* ct_batch_twiddles(int pass, int L, Twiddles& tw);
-// The run-epilogue flag and constants of an x-inverse item (as the per-state launch prepares them).
+// The launch class of an x-inverse item: `run` when its rows go in runs of that many cells,
+// 0 for the other forms (the `run` argument of ct_batch_xinv).
+template <typename R> int ct_batch_xinv_class(const CtXinvItem<R>& it, int run);
+// The run-epilogue flag and constants of an x-inverse item (as the per-state launch prepares
+// them for runs of `run` cells).
 template <typename R> void ct_batch_xinv_prepare(CtXinvItem<R>& it, int run);
 // Launches; tw from ct_batch_twiddles, twP the length-Px table (Twiddles::get).
 template <typename R>

@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(NT) k_xfwd_ct(const R* __restrict__ in, int n_
                                                 const R* __restrict__ msf, R ms, cplx_t<R>* __restrict__ out,
                                                 int pitch, const cplx_t<R>* __restrict__ tw,
                                                 const cplx_t<R>* __restrict__ twP) {
+    pdl_begin();
     xfwd_ct_tile<R, LC, NB, NT, HIN>(in, n_in, rows, rows_pc, msf, ms, out, pitch, tw, twP, blockIdx.x);
 }
 
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(NT, (kXfwdPipeBlocks<R, NT>)) k_xfwd_pipe(cons
                                                   const cplx_t<R>* __restrict__ tw,
                                                   const cplx_t<R>* __restrict__ twP) {
     using C = cplx_t<R>;
+    pdl_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);
     constexpr int SB = (LC - 1) + ((LC - 1) >> 4) + 1;
@@ -209,6 +211,7 @@ __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT * (L * NB / kE > NT ? L 
                                                 int64_t in_si, int64_t out_si, int64_t in_sbat, int64_t out_sbat,
                                                 const cplx_t<R>* __restrict__ tw) {
     using C = cplx_t<R>;
+    pdl_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);
     const int c0 = blockIdx.x * NB;
@@ -248,6 +251,7 @@ __global__ void __launch_bounds__(NT, NT >= 512 ? 1 : 2) k_cols_pipe(const cplx_
     constexpr int NIN = HIN ? L / 2 : L;
     constexpr int CPR = NB * (int)sizeof(C) / 16;  // 16-byte chunks per staged row
     static_assert(NB * sizeof(C) % 16 == 0, "16-byte row segments");
+    pdl_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);
     C* stage = reinterpret_cast<C*>(smem_raw + cols_stage_offset<R, L, NB>());
@@ -301,6 +305,7 @@ template <typename R, int L, int NB, int NT>
 __global__ void __launch_bounds__(NT, (kMinBlocks<R, NT, 768, 512>)) k_convz_ct(cplx_t<R>* S, const R* __restrict__ Nred, int nz, int ny, int nxh,
                                                  int pitch, const cplx_t<R>* __restrict__ tw) {
     using C = cplx_t<R>;
+    pdl_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);
     constexpr int NC = 6 * NB;  // columns: (row, comp, b)
@@ -405,6 +410,7 @@ __global__ void __launch_bounds__(6 * NB, (kMinBlocks<R, 6 * NB, 576, 288>))
     constexpr int L = 2 * NZ;
     constexpr int NC = 6 * NB;  // columns (row, comp, b) = threads
     constexpr int NT6 = 6 * (NZ + 1) * NB;  // tensor slice: [6][NZ+1][NB]
+    pdl_begin();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);  // [L][NC]
     R* tsl = reinterpret_cast<R*>(s + L * NC);
@@ -560,6 +566,7 @@ __device__ __forceinline__ void convy_ct_tile(cplx_t<R>* S, const R* __restrict_
 template <typename R, int L, int NB, int NT>
 __global__ void __launch_bounds__(NT) k_convy_ct(cplx_t<R>* S, const R* __restrict__ Nred, int ny, int nxh, int pitch,
                                                  const cplx_t<R>* __restrict__ tw) {
+    pdl_begin();
     convy_ct_tile<R, L, NB, NT>(S, Nred, ny, nxh, pitch, tw, blockIdx.x);
 }
 
@@ -619,7 +626,7 @@ __device__ __forceinline__ double xinv_runs(const cplx_t<R>* s, const Geom& g, R
 
 // What an x-inverse kernel's epilogue is compiled for (run_mode's answer `run`): runs of
 // RN cells only (1), the same with the next Runge-Kutta stage, the other modes of a single
-// state (0, 2 and 3), or the modes of a batch item (0, 1 and 2).  One kernel for all of
+// state (0, 2 and 3), or the other modes of a batch item (0 and 2).  One kernel for all of
 // them needed the registers of the widest: at the FP32 cap of 80 it spilled 208 bytes, and
 // the FP64 pass at 512x512x16 took 160 us instead of 150.
 enum XinvMode { XM_RUN, XM_RUN_NEXT, XM_OTHER, XM_BATCH };
@@ -659,8 +666,6 @@ __device__ __forceinline__ void xinv_ct_tile(const cplx_t<R>* __restrict__ S1, i
     double eacc = 0;
     if constexpr (XM == XM_RUN || XM == XM_RUN_NEXT) {
         eacc = xinv_runs<R, EPI, LC, NBR, NT, RN, false, XM == XM_RUN_NEXT>(s, g, scale, m, ms, tl, ep, ry0);
-    } else if (XM == XM_BATCH && run == 1) {
-        eacc = xinv_runs<R, EPI, LC, NBR, NT, RN, false, false>(s, g, scale, m, ms, tl, ep, ry0);
     } else if (run == 2) {
         eacc = xinv_runs<R, EPI, LC, NBR, NT, 1, false, XM != XM_BATCH>(s, g, scale, m, ms, tl, ep, ry0);
     } else if (XM != XM_BATCH && run == 3) {
@@ -695,6 +700,7 @@ __global__ void __launch_bounds__(NT, (kXinvBlocks<R, NT, RN>)) k_xinv_ct(const 
                                                 const cplx_t<R>* __restrict__ tw, const cplx_t<R>* __restrict__ twP,
                                                 Geom g, R scale, const R* __restrict__ m, MsInfo ms, TermList tl,
                                                 EpilogueArgs ep, int run) {
+    pdl_begin();
     xinv_ct_tile<R, EPI, LC, NBR, NT, RN, XM>(S1, pitch, tw, twP, g, scale, m, ms, tl, ep, run, blockIdx.x);
 }
 
@@ -717,13 +723,13 @@ __global__ void __launch_bounds__(NT) kbt_convy(const CtConvyItem<R>* __restrict
     convy_ct_tile<R, L, NB, NT>(d.S, d.Nred, d.ny, d.nxh, d.pitch, tw, w.y);
 }
 
-template <typename R, int LC, int NBR, int NT, int RN>
+template <typename R, int LC, int NBR, int NT, int RN, XinvMode XM>
 __global__ void __launch_bounds__(NT, (kXinvBlocks<R, NT, RN>))
     kbt_xinv(const CtXinvItem<R>* __restrict__ items, const int2* __restrict__ work, const cplx_t<R>* __restrict__ tw,
              const cplx_t<R>* __restrict__ twP) {
     const int2 w = work[blockIdx.x];
     const CtXinvItem<R>& d = items[w.x];
-    xinv_ct_tile<R, EPI_LLG, LC, NBR, NT, RN, XM_BATCH>(d.S1, d.pitch, tw, twP, d.g, d.scale, d.m, d.ms, d.tl, d.ep, d.run, w.y);
+    xinv_ct_tile<R, EPI_LLG, LC, NBR, NT, RN, XM>(d.S1, d.pitch, tw, twP, d.g, d.scale, d.m, d.ms, d.tl, d.ep, d.run, w.y);
 }
 
 // ------------------------------------------------------------------ launches
@@ -800,18 +806,15 @@ static void xfwd_L(const R* in, int n_in, int64_t rows, int64_t rows_pc, const R
             }
             const int64_t ntiles = ceil_div(rows, NB);
             const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)ps * sms);
-            kp<<<grid, NT, smem_p, st>>>(in, n_in, rows, ms, out, pitch, static_cast<const cplx_t<R>*>(tw),
-                                         static_cast<const cplx_t<R>*>(twP));
-            MAF_LAUNCH_CHECK();
+            launch_chain(kp, dim3(grid), NT, smem_p, st, in, n_in, rows, ms, out, pitch,
+                         static_cast<const cplx_t<R>*>(tw), static_cast<const cplx_t<R>*>(twP));
             return;
         }
     }
     auto k = k_xfwd_ct<R, LC, NB, NT, HIN>;
     ct_smem(k, smem);
-    k<<<(unsigned)ceil_div(rows, NB), NT, smem, st>>>(in, n_in, rows, rows_pc, msf, ms, out, pitch,
-                                                       static_cast<const cplx_t<R>*>(tw),
-                                                       static_cast<const cplx_t<R>*>(twP));
-    MAF_LAUNCH_CHECK();
+    launch_chain(k, dim3((unsigned)ceil_div(rows, NB)), NT, smem, st, in, n_in, rows, rows_pc, msf, ms, out, pitch,
+                 static_cast<const cplx_t<R>*>(tw), static_cast<const cplx_t<R>*>(twP));
 }
 
 template <typename R, int DIR, int L, int TILE, bool HIN, bool HOUT, int PV, bool RAG = false>
@@ -836,18 +839,16 @@ static void cols_L(const cplx_t<R>* in, cplx_t<R>* out, int n_in, int n_out, int
             MAF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kp, NT, smem_p));
             const int64_t ntiles = (int64_t)ntx * nbat;
             const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)std::max(per_sm, 1) * sm_count());
-            kp<<<grid, NT, smem_p, st>>>(in, out, n_in, ncols, in_si, out_si, in_sbat, out_sbat, nbat, pitch,
-                                         static_cast<const cplx_t<R>*>(tw));
-            MAF_LAUNCH_CHECK();
+            launch_chain(kp, dim3(grid), NT, smem_p, st, in, out, n_in, ncols, in_si, out_si, in_sbat, out_sbat, nbat,
+                         pitch, static_cast<const cplx_t<R>*>(tw));
             return;
         }
     }
     auto k = k_cols_ct<R, DIR, L, NB, NT, HIN, HOUT, PV, RAG>;
     ct_smem(k, smem);
     dim3 grid((unsigned)ceil_div(ncols, NB), (unsigned)nbat);
-    k<<<grid, NT, smem, st>>>(in, out, n_in, n_out, ncols, in_si, out_si, in_sbat, out_sbat,
-                              static_cast<const cplx_t<R>*>(tw));
-    MAF_LAUNCH_CHECK();
+    launch_chain(k, grid, NT, smem, st, in, out, n_in, n_out, ncols, in_si, out_si, in_sbat, out_sbat,
+                 static_cast<const cplx_t<R>*>(tw));
 }
 
 template <typename R, int L, bool REG>
@@ -866,14 +867,13 @@ static void convz_L(cplx_t<R>* S, const R* Nred, int nz, int ny, int nxh, int pi
         auto kr = 2 * nz == L ? k_convz_reg<R, L / 2, NBR, false> : k_convz_reg<R, L / 2, NBR, true>;
         ct_smem(kr, smem_r);
         dim3 grid((unsigned)ceil_div(nxh, NBR), (unsigned)(ny + 1));
-        kr<<<grid, 6 * NBR, smem_r, st>>>(S, Nred, nz, ny, nxh, pitch, static_cast<const cplx_t<R>*>(tw));
+        launch_chain(kr, grid, 6 * NBR, smem_r, st, S, Nred, nz, ny, nxh, pitch, static_cast<const cplx_t<R>*>(tw));
     } else {
         auto k = k_convz_ct<R, L, NB, NT>;
         ct_smem(k, smem);
         dim3 grid((unsigned)ceil_div(nxh, NB), (unsigned)(ny + 1));
-        k<<<grid, NT, smem, st>>>(S, Nred, nz, ny, nxh, pitch, static_cast<const cplx_t<R>*>(tw));
+        launch_chain(k, grid, NT, smem, st, S, Nred, nz, ny, nxh, pitch, static_cast<const cplx_t<R>*>(tw));
     }
-    MAF_LAUNCH_CHECK();
 }
 
 template <typename R, int L>
@@ -884,8 +884,8 @@ static void convy_L(cplx_t<R>* S, const R* Nred, int ny, int nxh, int pitch, con
     const size_t smem = sizeof(cplx_t<R>) * (size_t)3 * NB * ((L - 1) + ((L - 1) >> 4) + 1);
     auto k = k_convy_ct<R, L, NB, NT0>;
     ct_smem(k, smem);
-    k<<<(unsigned)ceil_div(nxh, NB), NT0, smem, st>>>(S, Nred, ny, nxh, pitch, static_cast<const cplx_t<R>*>(tw));
-    MAF_LAUNCH_CHECK();
+    launch_chain(k, dim3((unsigned)ceil_div(nxh, NB)), NT0, smem, st, S, Nred, ny, nxh, pitch,
+                 static_cast<const cplx_t<R>*>(tw));
 }
 
 // Rows per x-inverse CTA: 4096 values per component triple, 96 threads up to 512 cells
@@ -914,7 +914,7 @@ static void xinv_L(const cplx_t<R>* S1, int pitch, const void* tw, const void* t
     const auto* tp = static_cast<const cplx_t<R>*>(twP);
     auto go = [&](auto k) {
         ct_smem(k, smem);
-        k<<<blocks, NT, smem, st>>>(S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
+        launch_chain(k, dim3(blocks), NT, smem, st, S1, pitch, t, tp, g, scale, m, ms, tl, ep, run);
     };
     switch (ep.kind) {
         case EPI_H:
@@ -980,15 +980,19 @@ static void batch_convy_L(const CtConvyItem<R>* items, const int2* work, int nwo
     MAF_LAUNCH_CHECK();
 }
 
-template <typename R, int LC, int RN>
-static void batch_xinv_L(const CtXinvItem<R>* items, const int2* work, int nwork, const void* tw, const void* twP,
-                         cudaStream_t st) {
+template <typename R, int LC>
+static void batch_xinv_L(const CtXinvItem<R>* items, const int2* work, int nwork, int run, const void* tw,
+                         const void* twP, cudaStream_t st) {
     using S = XinvShape<R, LC>;
-    auto k = kbt_xinv<R, LC, S::NBR, S::NT, RN>;
-    ct_smem(k, S::smem);
-    k<<<(unsigned)nwork, S::NT, S::smem, st>>>(items, work, static_cast<const cplx_t<R>*>(tw),
-                                                static_cast<const cplx_t<R>*>(twP));
-    MAF_LAUNCH_CHECK();
+    auto go = [&](auto k) {
+        ct_smem(k, S::smem);
+        k<<<(unsigned)nwork, S::NT, S::smem, st>>>(items, work, static_cast<const cplx_t<R>*>(tw),
+                                                    static_cast<const cplx_t<R>*>(twP));
+        MAF_LAUNCH_CHECK();
+    };
+    if (run == 4) go(kbt_xinv<R, LC, S::NBR, S::NT, 4, XM_RUN>);
+    else if (run == 2) go(kbt_xinv<R, LC, S::NBR, S::NT, 2, XM_RUN>);
+    else go(kbt_xinv<R, LC, S::NBR, S::NT, 2, XM_BATCH>);
 }
 
 #define MAF_CT_SWITCH(L, CALL) \
@@ -1228,6 +1232,10 @@ template <typename R> const void* ct_batch_twiddles(int pass, int L, Twiddles& t
     return p;
 }
 
+template <typename R> int ct_batch_xinv_class(const CtXinvItem<R>& it, int run) {
+    return run_mode(it.g, it.m, it.ms, it.tl, it.ep, run) == 1 ? run : 0;
+}
+
 template <typename R> void ct_batch_xinv_prepare(CtXinvItem<R>& it, int run) {
     it.run = run_mode(it.g, it.m, it.ms, it.tl, it.ep, run);
     if (it.run) prepare_run(it.tl, it.g, it.ms);
@@ -1253,13 +1261,7 @@ void ct_batch_convy(const CtConvyItem<R>* items, const int2* work, int nwork, in
 template <typename R, int G>
 bool ct_batch_xinv_group(const CtXinvItem<R>* items, const int2* work, int nwork, int L, int run, const void* tw,
                          const void* twP, cudaStream_t st) {
-#define X(N)                                                        \
-    do {                                                            \
-        if (run == 4)                                               \
-            batch_xinv_L<R, N, 4>(items, work, nwork, tw, twP, st); \
-        else                                                        \
-            batch_xinv_L<R, N, 2>(items, work, nwork, tw, twP, st); \
-    } while (0)
+#define X(N) batch_xinv_L<R, N>(items, work, nwork, run, tw, twP, st)
     MAF_CT_XINV_SWITCH(G, L, X)
 #undef X
 }
@@ -1277,6 +1279,7 @@ bool ct_batch_xinv_group(const CtXinvItem<R>* items, const int2* work, int nwork
     template bool ct_convy<R>(cplx_t<R>*, const R*, int, int, int, int, Twiddles&, cudaStream_t);               \
     template int ct_batch_tile<R>(int, int);                                                                      \
     template const void* ct_batch_twiddles<R>(int, int, Twiddles&);                                               \
+    template int ct_batch_xinv_class<R>(const CtXinvItem<R>&, int);                                               \
     template void ct_batch_xinv_prepare<R>(CtXinvItem<R>&, int);                                                    \
     template void ct_batch_xfwd<R>(const CtXfwdItem<R>*, const int2*, int, int, const void*, const void*,        \
                                    cudaStream_t);                                                                \

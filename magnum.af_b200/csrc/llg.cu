@@ -31,6 +31,7 @@ __global__ void k_combine(const double* __restrict__ m, KList kl, double* __rest
 template <int NK>
 __global__ void __launch_bounds__(256) k_combine_v(const double* __restrict__ m, KList kl, double* __restrict__ out64,
                                                    float* __restrict__ out32, int64_t n2) {
+    pdl_begin();
     const double2* m2 = reinterpret_cast<const double2*>(m);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += (int64_t)gridDim.x * blockDim.x) {
         double2 kv[NK];
@@ -57,13 +58,13 @@ void rk_combine(const double* m, const KList& kl, double* out64, float* out32, i
         const int64_t n2 = n / 2;
         const unsigned blocks = (unsigned)std::min<int64_t>(ceil_div(n2, 256), (int64_t)sm_count() * 16);
         switch (kl.n) {
-            case 1: k_combine_v<1><<<blocks, 256, 0, st>>>(m, kl, out64, out32, n2); break;
-            case 2: k_combine_v<2><<<blocks, 256, 0, st>>>(m, kl, out64, out32, n2); break;
-            case 3: k_combine_v<3><<<blocks, 256, 0, st>>>(m, kl, out64, out32, n2); break;
-            case 4: k_combine_v<4><<<blocks, 256, 0, st>>>(m, kl, out64, out32, n2); break;
-            case 5: k_combine_v<5><<<blocks, 256, 0, st>>>(m, kl, out64, out32, n2); break;
-            case 6: k_combine_v<6><<<blocks, 256, 0, st>>>(m, kl, out64, out32, n2); break;
-            default: k_combine_v<7><<<blocks, 256, 0, st>>>(m, kl, out64, out32, n2); break;
+            case 1: launch_chain(k_combine_v<1>, dim3(blocks), 256, 0, st, m, kl, out64, out32, n2); break;
+            case 2: launch_chain(k_combine_v<2>, dim3(blocks), 256, 0, st, m, kl, out64, out32, n2); break;
+            case 3: launch_chain(k_combine_v<3>, dim3(blocks), 256, 0, st, m, kl, out64, out32, n2); break;
+            case 4: launch_chain(k_combine_v<4>, dim3(blocks), 256, 0, st, m, kl, out64, out32, n2); break;
+            case 5: launch_chain(k_combine_v<5>, dim3(blocks), 256, 0, st, m, kl, out64, out32, n2); break;
+            case 6: launch_chain(k_combine_v<6>, dim3(blocks), 256, 0, st, m, kl, out64, out32, n2); break;
+            default: launch_chain(k_combine_v<7>, dim3(blocks), 256, 0, st, m, kl, out64, out32, n2); break;
         }
         MAF_LAUNCH_CHECK();
         return;
@@ -115,8 +116,7 @@ __device__ __forceinline__ void block_max_final(double v, double* partials, unsi
 
 // sumbk = sum bs_j k_j ; rk_error = (form 0) sum e_j k_j  or (form 1) sumbk - sum e_j k_j
 __global__ void k_finalize(const double* __restrict__ m, KList kb, KList ke, int form, double atol, double rtol,
-                           double* __restrict__ mcand, float* __restrict__ mcand32, int norm_mode, int64_t N,
-                           double* partials, unsigned* counter, double* errout) {
+                           double* __restrict__ mcand, int norm_mode, int64_t N, double* partials, unsigned* counter, double* errout) {
     double vmax = 0.0;
     for (int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; cell < N;
          cell += (int64_t)gridDim.x * blockDim.x) {
@@ -145,10 +145,7 @@ __global__ void k_finalize(const double* __restrict__ m, KList kb, KList ke, int
             else { out[0] = 0; out[1] = 0; out[2] = 0; }
         }
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            mcand[c * N + cell] = out[c];
-            if (mcand32) mcand32[c * N + cell] = (float)out[c];
-        }
+        for (int c = 0; c < 3; ++c) mcand[c * N + cell] = out[c];
     }
     block_max_final(vmax, partials, counter, errout);
 }
@@ -197,9 +194,9 @@ __device__ __forceinline__ void fin_norm(double* o, int norm_mode) {
 // arithmetic as k_finalize, bit-identical results.
 template <int NU>
 __global__ void __launch_bounds__(256, 4) k_finalize_v(const double* __restrict__ m, KUnion ku, int form, double atol,
-                                                    double rtol, double* __restrict__ mcand,
-                                                    float* __restrict__ mcand32, int norm_mode, int64_t N,
+                                                    double rtol, double* __restrict__ mcand, int norm_mode, int64_t N,
                                                     double* partials, unsigned* counter, double* errout) {
+    pdl_begin();
     const int64_t N2 = N / 2;
     double vmax = 0.0;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N2; p += (int64_t)gridDim.x * blockDim.x) {
@@ -229,10 +226,7 @@ __global__ void __launch_bounds__(256, 4) k_finalize_v(const double* __restrict_
         fin_norm(o0, norm_mode);
         fin_norm(o1, norm_mode);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            reinterpret_cast<double2*>(mcand)[c * N2 + p] = make_double2(o0[c], o1[c]);
-            if (mcand32) reinterpret_cast<float2*>(mcand32)[c * N2 + p] = make_float2((float)o0[c], (float)o1[c]);
-        }
+        for (int c = 0; c < 3; ++c) reinterpret_cast<double2*>(mcand)[c * N2 + p] = make_double2(o0[c], o1[c]);
     }
     block_max_final(vmax, partials, counter, errout);
 }
@@ -266,17 +260,17 @@ static bool make_union(const KList& kb, const KList& ke, KUnion& u) {
 int rk_finalize_blocks() { return 32 * sm_count(); }
 
 void rk_finalize(const double* m, const KList& kb, const KList& ke, int form, double atol, double rtol, double* mcand,
-                 float* mcand32, int norm_mode, int64_t N, double* partials, double* err, cudaStream_t st) {
+                 int norm_mode, int64_t N, double* partials, double* err, cudaStream_t st) {
     const int threads = 256;
     KUnion u;
-    bool vec = N % 2 == 0 && aligned16(m) && aligned16(mcand) && ((uintptr_t)mcand32 & 7) == 0 && make_union(kb, ke, u);
+    bool vec = N % 2 == 0 && aligned16(m) && aligned16(mcand) && make_union(kb, ke, u);
     for (int j = 0; vec && j < u.n; ++j) vec = aligned16(u.k[j]);
     const int blocks = (int)std::min<int64_t>(ceil_div(vec ? N / 2 : N, threads), rk_finalize_blocks());
     unsigned* counter = reinterpret_cast<unsigned*>(partials + rk_finalize_blocks());
     if (vec) {
-#define MAF_FIN(NU)                                                                                                  \
-    k_finalize_v<NU><<<blocks, threads, 0, st>>>(m, u, form, atol, rtol, mcand, mcand32, norm_mode, N, partials, counter, \
-                                                 err)
+#define MAF_FIN(NU)                                                                                                 \
+    launch_chain(k_finalize_v<NU>, dim3(blocks), threads, 0, st, m, u, form, atol, rtol, mcand, norm_mode, N, \
+                 partials, counter, err)
         switch (u.n) {
             case 1: MAF_FIN(1); break;
             case 2: MAF_FIN(2); break;
@@ -288,7 +282,7 @@ void rk_finalize(const double* m, const KList& kb, const KList& ke, int form, do
         }
 #undef MAF_FIN
     } else {
-        k_finalize<<<blocks, threads, 0, st>>>(m, kb, ke, form, atol, rtol, mcand, mcand32, norm_mode, N, partials,
+        k_finalize<<<blocks, threads, 0, st>>>(m, kb, ke, form, atol, rtol, mcand, norm_mode, N, partials,
                                                counter, err);
     }
     MAF_LAUNCH_CHECK();
@@ -766,6 +760,7 @@ bool lb_loop(const LbLoop& a, int64_t n, cudaStream_t st) {
 __global__ void __launch_bounds__(kLbThreads) k_lb_slope(const double* __restrict__ g, const double* __restrict__ s,
                                                          int64_t n, const double* __restrict__ e, int ne, double* part,
                                                          unsigned* counter, double* out) {
+    pdl_begin();
     double v[1] = {0.0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         v[0] += g[i] * s[i];
@@ -786,8 +781,7 @@ __global__ void __launch_bounds__(kLbThreads) k_lb_slope(const double* __restric
 void lb_slope(const double* g, const double* s, int64_t n, const double* e, int ne, double* part, unsigned* counter,
               double* out, cudaStream_t st) {
     const int blocks = (int)std::min<int64_t>(ceil_div(n, kLbThreads), red_blocks());
-    k_lb_slope<<<blocks, kLbThreads, 0, st>>>(g, s, n, e, ne, part, counter, out);
-    MAF_LAUNCH_CHECK();
+    launch_chain(k_lb_slope, dim3(blocks), kLbThreads, 0, st, g, s, n, e, ne, part, counter, out);
 }
 
 // s = x - x_old, y = g - g_old; out = max|g|, max|s|, max|x|, y . s, y . y, s . s
@@ -795,6 +789,7 @@ __global__ void __launch_bounds__(kLbThreads) k_lb_pair(const double* __restrict
                                                         const double* __restrict__ g, const double* __restrict__ g_old,
                                                         double* __restrict__ s, double* __restrict__ y, int64_t n,
                                                         double* part, unsigned* counter, double* out) {
+    pdl_begin();
     double v[6] = {0, 0, 0, 0, 0, 0};
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         const double xi = x[i], gi = g[i];
@@ -814,13 +809,13 @@ __global__ void __launch_bounds__(kLbThreads) k_lb_pair(const double* __restrict
 void lb_pair(const double* x, const double* x_old, const double* g, const double* g_old, double* s, double* y,
              int64_t n, double* part, unsigned* counter, double* out, cudaStream_t st) {
     const int blocks = (int)std::min<int64_t>(ceil_div(n, kLbThreads), red_blocks());
-    k_lb_pair<<<blocks, kLbThreads, 0, st>>>(x, x_old, g, g_old, s, y, n, part, counter, out);
-    MAF_LAUNCH_CHECK();
+    launch_chain(k_lb_pair, dim3(blocks), kLbThreads, 0, st, x, x_old, g, g_old, s, y, n, part, counter, out);
 }
 
 // m = normalize(wa + stp * s) with the zero-safe normalize (lbfgs_minimizer.cpp:274-275)
 __global__ void k_normalize_combine(double* __restrict__ m, const double* __restrict__ wa, double stp,
                                     const double* __restrict__ s, int64_t N) {
+    pdl_begin();
     for (int64_t cell = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; cell < N;
          cell += (int64_t)gridDim.x * blockDim.x) {
         double v[3];
@@ -834,8 +829,7 @@ __global__ void k_normalize_combine(double* __restrict__ m, const double* __rest
 
 void normalize_combine(double* m, const double* wa, double stp, const double* s, int64_t N, cudaStream_t st) {
     const int64_t blocks = std::min<int64_t>(ceil_div(N, 256), (int64_t)sm_count() * 8);
-    k_normalize_combine<<<(unsigned)blocks, 256, 0, st>>>(m, wa, stp, s, N);
-    MAF_LAUNCH_CHECK();
+    launch_chain(k_normalize_combine, dim3((unsigned)blocks), 256, 0, st, m, wa, stp, s, N);
 }
 
 // thermal field sigma * xi(seed, member, index, cell) [3][N] (the h_th of

@@ -11,12 +11,12 @@ struct KList {
 };
 
 void rk_combine(const double* m, const KList& kl, double* out64, float* out32, int64_t n, cudaStream_t st);
-// Candidate m (FP64 and, when mcand32, its FP32 copy) and the error norm: *err receives
+// Candidate m and the error norm: *err receives
 // the NaN-propagating max (device-accessible memory).  partials: rk_finalize_blocks() doubles
 // and, behind them, one zeroed word, the block counter, which every launch leaves zero.
 int rk_finalize_blocks();
 void rk_finalize(const double* m, const KList& kb, const KList& ke, int form, double atol, double rtol, double* mcand,
-                 float* mcand32, int norm_mode, int64_t N, double* partials, double* err, cudaStream_t st);
+                 int norm_mode, int64_t N, double* partials, double* err, cudaStream_t st);
 void normalize_m(double* m, int64_t N, int mode, unsigned long long* zero_count_dev, cudaStream_t st);
 void ms_field_from_m(const double* m, double Ms, double* msf, float* msf32, int64_t N, cudaStream_t st);
 // partial-sum blocks of mean_m (its scratch needs 4 per block; out_dev may sit behind them)
