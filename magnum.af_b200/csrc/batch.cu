@@ -1,14 +1,20 @@
-// Batched passes of an ensemble of 2-D states (batch.hpp): every pass of a
-// fixed-step stochastic / RK4 step is one launch per transform length over a
-// device work table of (member, tile) pairs, the launches of a pass on
-// parallel graph branches.  Members whose lengths have compile-time kernels run
-// those kernels' tile bodies (fields_ct.cu), the others the generic kernels'
-// (run-time FFT plans, passes_generic.cuh); members of a DemagField set to the
-// run-time-plan kernels run those.  The element-wise kernels repeat the
-// arithmetic of llg.cu's, so a member's trajectory is bit-identical to the one
-// the per-state path computes with the same kernels.
+// Batched passes of an ensemble of 2-D states (batch.hpp): the members go in chains by
+// transform lengths; every pass of a chain is one launch over a device work table of
+// (member, tile) pairs.  Chains whose lengths have compile-time kernels run those
+// kernels' tile bodies (fields_ct.cu), the others the generic kernels' (run-time FFT
+// plans, passes_generic.cuh); members of a DemagField set to the run-time-plan kernels
+// run those.  The element-wise kernels repeat the arithmetic of llg.cu's, so a member's
+// trajectory is bit-identical to the one the per-state path computes with the same
+// kernels.
+//
+// Members do not depend on one another, so a chain joins the others only after the last
+// recorded step: with a fork and a join around the launches of each pass 16 films up to
+// 512 x 512 (15 pairs of lengths; FP32, Heun) took 320 us a step, in chains 259.
 #include <algorithm>
 #include <cstring>
+#include <map>
+#include <memory>
+#include <tuple>
 
 #include "batch.hpp"
 #include "ct_dispatch.hpp"
@@ -204,7 +210,7 @@ struct GenClass {
     size_t smem = 0;
 };
 
-struct FusedBatch::Impl {
+struct FusedBatch::Chain {
     bool f32 = false;
     int M = 0, S = 0;
     FusedScheme scheme;
@@ -221,7 +227,7 @@ struct FusedBatch::Impl {
     std::vector<cudaEvent_t> ev;
     cudaEvent_t fork_ev = nullptr;
 
-    ~Impl() {
+    ~Chain() {
         for (cudaStream_t q : side) cudaStreamDestroy(q);
         for (cudaEvent_t e : ev) cudaEventDestroy(e);
         if (fork_ev) cudaEventDestroy(fork_ev);
@@ -232,7 +238,7 @@ struct FusedBatch::Impl {
     template <typename F> void branches(cudaStream_t st, int n, F&& launch);
 };
 
-template <typename F> void FusedBatch::Impl::branches(cudaStream_t st, int n, F&& launch) {
+template <typename F> void FusedBatch::Chain::branches(cudaStream_t st, int n, F&& launch) {
     if (n <= 1) {
         if (n == 1) launch(0, st);
         return;
@@ -265,7 +271,7 @@ static GenClass& gen_class(std::vector<GenClass>& cls, int L) {
     return cls.back();
 }
 
-template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
+template <typename R> void FusedBatch::Chain::build(cudaStream_t st) {
     using C = cplx_t<R>;
     const bool f64 = sizeof(R) == 8;
     std::vector<XfwdA<R>> xf((size_t)2 * S * M);
@@ -507,8 +513,12 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
     MAF_CUDA(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
     n_el3 = (int)we.size();
     n_cell = (int)wn.size();
+    // (only raised: another chain's launches may need the larger one)
     auto smem_attr = [](auto k, size_t bytes) {
-        if (bytes > 32 * 1024) MAF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        cudaFuncAttributes a;
+        MAF_CUDA(cudaFuncGetAttributes(&a, k));
+        if (bytes > 32 * 1024 && (int)bytes > a.maxDynamicSharedSizeBytes)
+            MAF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };
     smem_attr(kb_xfwd<R>, s_xfwd);
     smem_attr(kb_conv<R>, s_conv);
@@ -516,7 +526,7 @@ template <typename R> void FusedBatch::Impl::build(cudaStream_t st) {
     MAF_CUDA(cudaStreamSynchronize(st));
 }
 
-template <typename R> void FusedBatch::Impl::record(cudaStream_t st, int p) {
+template <typename R> void FusedBatch::Chain::record(cudaStream_t st, int p) {
     const size_t psm = (size_t)p * S * M;
     if (f32) {
         kb_stage32<<<n_el3, kElemThreads, 0, st>>>(stage32.as<StageA>() + (size_t)p * M, w_el3.as<int2>());
@@ -568,37 +578,92 @@ template <typename R> void FusedBatch::Impl::record(cudaStream_t st, int p) {
     MAF_LAUNCH_CHECK();
 }
 
-FusedBatch::FusedBatch(std::vector<FusedMember> members, FusedScheme scheme, bool f32, cudaStream_t st)
-    : impl_(new Impl) {
-    impl_->f32 = f32;
-    impl_->M = (int)members.size();
-    impl_->S = (int)scheme.stages.size();
-    impl_->scheme = scheme;
-    impl_->mem = std::move(members);
-    try {
-        if (f32)
-            impl_->build<float>(st);
-        else
-            impl_->build<double>(st);
-    } catch (...) {
-        delete impl_;
-        throw;
+// The chains at most; further keys share chains, whose passes then have a launch per key.
+// The same ensemble in 1, 2, 4, 8, 15 chains: 320, 297, 272, 268, 259 us a step.
+constexpr size_t kMaxChains = 16;
+
+struct FusedBatch::Impl {
+    bool f32 = false;
+    std::vector<std::unique_ptr<Chain>> chains;
+    std::vector<cudaStream_t> side;  // of the chains after the first
+    std::vector<cudaEvent_t> ev;
+    cudaEvent_t fork_ev = nullptr;
+
+    ~Impl() {
+        for (cudaStream_t q : side) cudaStreamDestroy(q);
+        for (cudaEvent_t e : ev) cudaEventDestroy(e);
+        if (fork_ev) cudaEventDestroy(fork_ev);
     }
+};
+
+// What the members of a chain share: the transform lengths (largest first, so that the
+// longest chains start first) and the form of the x inverse.
+template <typename R> static std::tuple<int64_t, int, int> chain_key(const FusedMember& f, cudaStream_t st) {
+    const DemagPlan<R> pl = f.demag->plan<R>(st);
+    CtXinvItem<R> it{};
+    it.g = f.md.geom();
+    it.ms.Ms = f.Ms;
+    for (const TermDesc& t : f.terms) it.tl.t[it.tl.n++] = t;
+    it.ep.kind = EPI_LLG;
+    const int run = f.demag->tune.xinv_run ? f.demag->tune.xinv_run : 2;
+    const int form = f.demag->tune.generic ? -1 : ct_batch_xinv_class<R>(it, run);
+    return {-(int64_t)pl.Px * pl.Py, pl.Px, form};
+}
+
+FusedBatch::FusedBatch(std::vector<FusedMember> members, FusedScheme scheme, bool f32, cudaStream_t st)
+    : impl_(nullptr) {
+    auto impl = std::make_unique<Impl>();
+    impl->f32 = f32;
+    std::map<std::tuple<int64_t, int, int>, std::vector<FusedMember>> keyed;
+    for (FusedMember& f : members)
+        keyed[f32 ? chain_key<float>(f, st) : chain_key<double>(f, st)].push_back(std::move(f));
+    const size_t n = std::min(keyed.size(), kMaxChains);
+    size_t rank = 0;
+    for (auto& [key, v] : keyed) {
+        if (impl->chains.size() <= rank * n / keyed.size()) {
+            impl->chains.push_back(std::make_unique<Chain>());
+            impl->chains.back()->scheme = scheme;
+        }
+        auto& mem = impl->chains.back()->mem;
+        for (FusedMember& f : v) mem.push_back(std::move(f));
+        ++rank;
+    }
+    for (size_t c = 0; c < impl->chains.size(); ++c) {
+        Chain& ch = *impl->chains[c];
+        ch.f32 = f32;
+        ch.M = (int)ch.mem.size();
+        ch.S = (int)scheme.stages.size();
+        if (f32) ch.build<float>(st);
+        else ch.build<double>(st);
+        if (c == 0) continue;
+        cudaStream_t q;
+        MAF_CUDA(cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking));
+        impl->side.push_back(q);
+        cudaEvent_t e;
+        MAF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        impl->ev.push_back(e);
+    }
+    MAF_CUDA(cudaEventCreateWithFlags(&impl->fork_ev, cudaEventDisableTiming));
+    impl_ = impl.release();
 }
 
 FusedBatch::~FusedBatch() { delete impl_; }
 
-void FusedBatch::record_step(cudaStream_t st, int parity) {
-    if (impl_->f32)
-        impl_->record<float>(st, parity & 1);
-    else
-        impl_->record<double>(st, parity & 1);
-}
-
-int FusedBatch::launches_per_step() const {
-    const Impl& b = *impl_;
-    const int per_stage = (int)(b.gx.size() + b.gc.size() + b.gi.size() + b.cx.size() + b.cc.size() + b.ci.size());
-    return (b.f32 ? 1 : 0) + b.S * (per_stage + 1) - 1 + 2;
+void FusedBatch::record_steps(cudaStream_t st, int parity, int n) {
+    Impl& b = *impl_;
+    MAF_CUDA(cudaEventRecord(b.fork_ev, st));
+    for (cudaStream_t q : b.side) MAF_CUDA(cudaStreamWaitEvent(q, b.fork_ev, 0));
+    for (size_t c = 0; c < b.chains.size(); ++c) {
+        cudaStream_t q = c ? b.side[c - 1] : st;
+        for (int i = 0; i < n; ++i) {
+            if (b.f32) b.chains[c]->record<float>(q, (parity + i) & 1);
+            else b.chains[c]->record<double>(q, (parity + i) & 1);
+        }
+    }
+    for (size_t c = 0; c < b.side.size(); ++c) {
+        MAF_CUDA(cudaEventRecord(b.ev[c], b.side[c]));
+        MAF_CUDA(cudaStreamWaitEvent(st, b.ev[c], 0));
+    }
 }
 
 bool fused_supported(const std::vector<FusedMember>& members, const FusedScheme& scheme) {

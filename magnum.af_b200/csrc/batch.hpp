@@ -1,9 +1,9 @@
 // Batched passes of an ensemble of small states (stochastic LLG members,
-// string-method images): one kernel launch per pass covers every member.  Each
-// CTA of a launch reads its (member, tile) pair from a device work table and
-// the member's parameters from a device array, and runs that tile of the
-// member's pass (the generic kernels' tile bodies, passes_generic.cuh), so a
-// step of M members of uneven sizes costs the launches of one member.
+// string-method images).  The members with the same transform lengths form a
+// chain: one kernel launch per pass covers all of them (each CTA reads its
+// (member, tile) pair from a device work table and the member's parameters from
+// a device array, and runs that tile of the member's pass), and the chains run
+// beside each other from their first pass to their last.
 //
 // Reference: the ensemble and the string images are stepped one after another
 // in magnumaf/src/integrators/stochastic_integrator.cpp:42-57 and
@@ -59,12 +59,13 @@ class FusedBatch {
     // All members share the scheme and the precision (f32: FP32 field, FP64 state).
     FusedBatch(std::vector<FusedMember> members, FusedScheme scheme, bool f32, cudaStream_t st);
     ~FusedBatch();
-    // Records one step of every member on st; parity p reads m[p] and writes the
-    // new state to m[1 - p].  Also advances every member's counter q.
-    void record_step(cudaStream_t st, int parity);
-    int launches_per_step() const;
+    // Records n steps of every member, ordered with st; the first reads m[parity] and
+    // writes the new state to m[1 - parity], and they swap every step.  Also advances
+    // every member's counter q.
+    void record_steps(cudaStream_t st, int parity, int n);
 
   private:
+    struct Chain;
     struct Impl;
     Impl* impl_;
 };

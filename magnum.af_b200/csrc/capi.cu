@@ -2824,8 +2824,7 @@ void batch_capture(maf_stoch_batch_s* b) {
         if (b->fb) {
             // two steps of every member: the first writes the candidates, the second
             // the states again, so the graph leaves the buffers where it found them
-            b->fb->record_step(b->root, 0);
-            b->fb->record_step(b->root, 1);
+            b->fb->record_steps(b->root, 0, 2);
             b->fused_active = true;
         } else {
             MAF_CUDA(cudaEventRecord(b->fork, b->root));

@@ -2,7 +2,8 @@
 Runge-Kutta stage writes the next stage's magnetisation, above a combine kernel does; up
 to 196608 values per vector the LBFGS recursion is one cluster launch, above a chain of
 launches.  Both sides of each line against the oracle (1e-12 for an attempt, 1e-9 relative
-for the energy after a few iterations), local terms only."""
+for the energy after a few iterations), local terms only.  Ensembles: members of more
+transform lengths than there are chains share chains, bit for bit their own trajectories."""
 import numpy as np
 import pytest
 
@@ -55,3 +56,24 @@ def test_minimiser_on_both_sides_of_the_recursion_rule(shape):
     assert abs(E - E_ref) <= 1e-9 * abs(E_ref)
     assert mini.stats()["iterations"] == it_ref
     assert np.abs(gs.m - os_.m).max() < 1e-8
+
+
+@pytest.mark.parametrize("prec", ["fp32_field", "fp64"])
+@pytest.mark.parametrize("members", [1, 16, 17, 23])
+def test_ensemble_chains_on_both_sides_of_their_bound(members, prec):
+    sides = [(nx, ny) for nx in (10, 33, 66, 100, 130) for ny in (6, 20, 35, 65, 99)][:members]
+    made = []
+    for _ in range(2):
+        group = []
+        for i, (nx, ny) in enumerate(sides):
+            mesh = M.Mesh(nx, ny, 1, 2e-9, 2e-9, 1e-9)
+            st = M.State(mesh, 7e5, random_m((nx, ny, 1), 60 + i), precision=prec)
+            terms = [M.DemagField(mesh), M.ExchangeField(1.5e-11), M.UniaxialAnisotropyField(6e5)]
+            group.append((M.Stochastic_LLG(0.1, 300.0, 5e-14, st, terms, "Heun", seed=11, member=i), st))
+        made.append(group)
+    batch = M.StochasticBatch(made[0], fused=True)
+    batch.steps(5)
+    assert batch.fused_active
+    for (_, sb), (it, ss) in zip(*made):
+        it.steps(ss, 5)
+        assert np.array_equal(np.asarray(sb.m), np.asarray(ss.m))
