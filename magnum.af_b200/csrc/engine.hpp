@@ -214,8 +214,8 @@ class Demag {
     template <typename R> cplx_t<R>* S2(int Py, int pitch);
     void build_tensor(cudaStream_t st);
     void build_padded_tensor(double* out64, float* out32, cudaStream_t st);
-    void transform_octant(const double* oct, int o0, int o1, int o2, int comp, int Lx, int Ly, int Lz, double* quad,
-                          double scale, char* work, cudaStream_t st);
+    void transform_octants(const double* oct, int o0, int o1, int o2, const int* comps, int nc, int Lx, int Ly, int Lz,
+                           double* quad, double scale, char* work, cudaStream_t st);
     size_t padded_elems() const {
         return (size_t)ncomp() * (pad_z_ == 1 ? 1 : pad_z_ / 2 + 1) * (pad_y_ / 2 + 1) * (pad_x_ / 2 + 1);
     }
@@ -287,6 +287,8 @@ void widen_m(const float* m32, double* m64, int64_t n, cudaStream_t st);  // FP3
 // assembles it, and its entries at the offsets 0 <= j < (o0, o1, o2), [o2][o1][o0]
 // (newell.cu).
 void newell_component(double* out, int comp, const MeshDims& md, int Px, int Py, int Pz, cudaStream_t st);
-void newell_octant(double* out, int comp, const MeshDims& md, int o0, int o1, int o2, cudaStream_t st);
+// ncomp components, one [o2][o1][o0] array after the other
+void newell_octants(double* out, const int* comps, int ncomp, const MeshDims& md, int o0, int o1, int o2,
+                    cudaStream_t st);
 
 }  // namespace mafb

@@ -288,11 +288,19 @@ __device__ __forceinline__ int wrap_offset(int i, int L, bool odd, bool& neg, bo
     return j;
 }
 
+// The components a launch completes (blockIdx.y), one array after the other.
+struct TensorComps {
+    int c[6];
+};
+
 // rows [nz][ny][L] of real values from the octant [o2][o1][o0] (zero beyond it): the
 // x axis completed by parity; rows on the zero planes of the other axes are zero
-__global__ void k_tensor_rows(const double* __restrict__ oct, double* __restrict__ out, int comp, int o0, int o1,
-                              int o2, int ny, int nz, int Ly, int Lz, int L) {
+__global__ void k_tensor_rows(const double* __restrict__ oct, double* __restrict__ out, TensorComps comps, int o0,
+                              int o1, int o2, int ny, int nz, int Ly, int Lz, int L) {
     const int64_t total = (int64_t)L * ny * nz;
+    const int comp = comps.c[blockIdx.y];
+    oct += (int64_t)blockIdx.y * o0 * o1 * o2;
+    out += blockIdx.y * total;
     const bool ox = tensor_odd(comp, 0), oy = tensor_odd(comp, 1), oz = tensor_odd(comp, 2);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int x = (int)(i % L);
@@ -306,10 +314,15 @@ __global__ void k_tensor_rows(const double* __restrict__ oct, double* __restrict
 }
 
 // spectrum rows completed along one axis by parity: out [A][L][B][pitch] from the
-// rows a sa + j sj + b of in, j <= L/2 (y: A = z planes, B = 1; z: A = 1, B = ky rows)
-__global__ void k_tensor_wrap(const double2* __restrict__ in, double2* __restrict__ out, int64_t A, int L, int64_t B,
-                              int64_t sa, int64_t sj, int odd, int pitch, int nxh) {
+// rows a sa + j sj + b of in (rows_in of them per component), j <= L/2 (y: A = z planes,
+// B = 1; z: A = 1, B = ky rows)
+__global__ void k_tensor_wrap(const double2* __restrict__ in, double2* __restrict__ out, int64_t rows_in, int64_t A,
+                              int L, int64_t B, int64_t sa, int64_t sj, TensorComps comps, int axis, int pitch,
+                              int nxh) {
     const int64_t total = A * L * B * nxh;
+    const bool odd = tensor_odd(comps.c[blockIdx.y], axis);
+    in += blockIdx.y * rows_in * pitch;
+    out += blockIdx.y * A * L * B * pitch;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int x = (int)(i % nxh);
         int64_t r = i / nxh;
@@ -319,17 +332,19 @@ __global__ void k_tensor_wrap(const double2* __restrict__ in, double2* __restric
         const int l = (int)(r % L);
         const int64_t a = r / L;
         bool neg = false, zero = false;
-        const int j = wrap_offset(l, L, odd != 0, neg, zero);
+        const int j = wrap_offset(l, L, odd, neg, zero);
         double2 v = make_double2(0.0, 0.0);
         if (!zero) v = in[(a * sa + j * sj + b) * pitch + x];
         out[o] = neg ? make_double2(-v.x, -v.y) : v;
     }
 }
 
-// scaled real part of the spectrum on the stored quadrant
-__global__ void k_tensor_real(const double2* __restrict__ spec, double* __restrict__ dst, int64_t rows, int nxh,
-                              int pitch, double scale, int Ky, int spec_ky) {
+// scaled real part of the spectrum (rows_in rows per component) on the stored quadrant
+__global__ void k_tensor_real(const double2* __restrict__ spec, int64_t rows_in, double* __restrict__ dst, int64_t rows,
+                              int nxh, int pitch, double scale, int Ky, int spec_ky) {
     const int64_t total = rows * nxh;
+    spec += blockIdx.y * rows_in * pitch;
+    dst += blockIdx.y * total;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
         const int kx = (int)(i % nxh);
         const int64_t r = i / nxh;
@@ -464,53 +479,67 @@ Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, boo
     }
 }
 
-// Real spectrum (times scale) on the quadrant [Lz/2+1][Ly/2+1][Lx/2+1] (Lz = 1: one
-// plane) of the periodic function of lengths (Lx, Ly, Lz) that a tensor component's
-// octant `oct` [o2][o1][o0] completes by parity.  The spectrum has the component's
-// parity, so the transform of its quadrant over L values, divided by L, is the octant.  Each
-// axis is completed just before its transform, so the x transforms run on a quarter
-// of the rows, the y transforms on half of the planes and the z transforms on half of
-// the rows.  work: octant_work bytes.
-static size_t octant_work_a(int Lx, int Ly, int Lz) {
+// Real spectra (times scale) on the quadrant [Lz/2+1][Ly/2+1][Lx/2+1] (Lz = 1: one
+// plane) of the periodic functions of lengths (Lx, Ly, Lz) that the octants `oct`
+// [o2][o1][o0] of nc tensor components complete by parity (oct and quad: one component
+// after the other).  The spectrum has the component's parity, so the transform of its
+// quadrant over L values, divided by L, is the octant.  Each axis is completed just before
+// its transform, so the x transforms run on a quarter of the rows, the y transforms on half
+// of the planes and the z transforms on half of the rows.  The octants are read before the
+// quadrants are written.  work: octant_work bytes.
+static size_t octant_work_a(int Lx, int Ly, int Lz, int nc) {
     // the completed real rows, then the completed y columns
     const int Ky = Ly / 2 + 1, Kz = Lz == 1 ? 1 : Lz / 2 + 1, pitch = (Lx / 2 + 4) / 4 * 4;
-    return (std::max(sizeof(double) * (size_t)Lx * Ky * Kz, sizeof(double2) * (size_t)Kz * Ly * pitch) + 255) / 256 * 256;
+    return (nc * std::max(sizeof(double) * (size_t)Lx * Ky * Kz, sizeof(double2) * (size_t)Kz * Ly * pitch) + 255) / 256 *
+           256;
 }
-static size_t octant_work(int Lx, int Ly, int Lz) {
+static size_t octant_work(int Lx, int Ly, int Lz, int nc) {
     // and the x spectra, then the completed z columns
     const int Ky = Ly / 2 + 1, Kz = Lz == 1 ? 1 : Lz / 2 + 1, pitch = (Lx / 2 + 4) / 4 * 4;
-    const size_t b = sizeof(double2) * (size_t)std::max<int64_t>((int64_t)Ky * Kz, Lz > 1 ? (int64_t)Lz * Ky : 0) * pitch;
-    return octant_work_a(Lx, Ly, Lz) + (b + 255) / 256 * 256;
+    const size_t b =
+        sizeof(double2) * nc * (size_t)std::max<int64_t>((int64_t)Ky * Kz, Lz > 1 ? (int64_t)Lz * Ky : 0) * pitch;
+    return octant_work_a(Lx, Ly, Lz, nc) + (b + 255) / 256 * 256;
 }
 
-void Demag::transform_octant(const double* oct, int o0, int o1, int o2, int comp, int Lx, int Ly, int Lz, double* quad,
-                             double scale, char* work, cudaStream_t st) {
+// Components that are transformed together: all of them while the work buffers stay
+// within kTensorBatch, else one by one: small tensors are launches of 3-15 us one after the
+// other, 24 for the four components of a film.  A new tensor one by one and together: 24 x
+// 24 x 1 302 and 184 us, 250 x 240 x 1 583 and 384, 66 x 91 x 6 816 and 501, 200 x 120 x 10
+// (99 MB) 1947 and 1772.
+constexpr size_t kTensorBatch = 128u << 20;
+static int octant_batch(size_t work_all, int ncomp) { return work_all <= kTensorBatch ? ncomp : 1; }
+
+void Demag::transform_octants(const double* oct, int o0, int o1, int o2, const int* comps, int nc, int Lx, int Ly,
+                              int Lz, double* quad, double scale, char* work, cudaStream_t st) {
     const int nxh = Lx / 2 + 1, Ky = Ly / 2 + 1, Kz = Lz == 1 ? 1 : Lz / 2 + 1;
     const int pitch = (nxh + 3) / 4 * 4;
-    char* work_b = work + octant_work_a(Lx, Ly, Lz);
-    auto grid = [](int64_t n) { return (unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16); };
+    TensorComps c = {};
+    for (int i = 0; i < nc; ++i) c.c[i] = comps[i];
+    char* work_b = work + octant_work_a(Lx, Ly, Lz, nc);
+    auto grid = [nc](int64_t n) {
+        return dim3((unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16), (unsigned)nc);
+    };
     double* rows = reinterpret_cast<double*>(work);
     double2* ycol = reinterpret_cast<double2*>(work);
     double2* xs = reinterpret_cast<double2*>(work_b);
-    k_tensor_rows<<<grid((int64_t)Lx * Ky * Kz), 256, 0, st>>>(oct, rows, comp, o0, o1, o2, Ky, Kz, Ly, Lz, Lx);
+    const int64_t xrows = (int64_t)Ky * Kz, yrows = (int64_t)Kz * Ly, zrows = (int64_t)Lz * Ky;
+    k_tensor_rows<<<grid(Lx * xrows), 256, 0, st>>>(oct, rows, c, o0, o1, o2, Ky, Kz, Ly, Lz, Lx);
     MAF_LAUNCH_CHECK();
-    launch_xfwd<double>(rows, Lx, (int64_t)Ky * Kz, (int64_t)Ky * Kz, nullptr, 1.0, xs, pitch, Lx, tw_, st);
-    k_tensor_wrap<<<grid((int64_t)Kz * Ly * nxh), 256, 0, st>>>(xs, ycol, Kz, Ly, 1, Ky, 1, tensor_odd(comp, 1),
-                                                                pitch, nxh);
+    launch_xfwd<double>(rows, Lx, nc * xrows, nc * xrows, nullptr, 1.0, xs, pitch, Lx, tw_, st);
+    k_tensor_wrap<<<grid(yrows * nxh), 256, 0, st>>>(xs, ycol, xrows, Kz, Ly, 1, Ky, 1, c, 1, pitch, nxh);
     MAF_LAUNCH_CHECK();
-    launch_cols<double, -1>(ycol, ycol, Ly, Ly, Ly, nxh, pitch, pitch, (int64_t)Ly * pitch, (int64_t)Ly * pitch, Kz,
-                            tw_, tune, st);
+    launch_cols<double, -1>(ycol, ycol, Ly, Ly, Ly, nxh, pitch, pitch, (int64_t)Ly * pitch, (int64_t)Ly * pitch,
+                            nc * Kz, tw_, tune, st);
     if (Lz > 1) {
+        // a component's columns are its rows of ky one after the other, the pitch's padding too
         double2* zcol = reinterpret_cast<double2*>(work_b);
-        k_tensor_wrap<<<grid((int64_t)Lz * Ky * nxh), 256, 0, st>>>(ycol, zcol, 1, Lz, Ky, 0, Ly,
-                                                                    tensor_odd(comp, 2), pitch, nxh);
+        k_tensor_wrap<<<grid(zrows * nxh), 256, 0, st>>>(ycol, zcol, yrows, 1, Lz, Ky, 0, Ly, c, 2, pitch, nxh);
         MAF_LAUNCH_CHECK();
-        launch_cols<double, -1>(zcol, zcol, Lz, Lz, Lz, nxh, (int64_t)Ky * pitch, (int64_t)Ky * pitch, pitch, pitch,
-                                Ky, tw_, tune, st);
-        k_tensor_real<<<grid((int64_t)Kz * Ky * nxh), 256, 0, st>>>(zcol, quad, (int64_t)Kz * Ky, nxh, pitch, scale,
-                                                                    Ky, Ky);
+        launch_cols<double, -1>(zcol, zcol, Lz, Lz, Lz, Ky * pitch, (int64_t)Ky * pitch, (int64_t)Ky * pitch,
+                                zrows * pitch, zrows * pitch, nc, tw_, tune, st);
+        k_tensor_real<<<grid(xrows * nxh), 256, 0, st>>>(zcol, zrows, quad, xrows, nxh, pitch, scale, Ky, Ky);
     } else {
-        k_tensor_real<<<grid((int64_t)Ky * nxh), 256, 0, st>>>(ycol, quad, Ky, nxh, pitch, scale, Ky, Ly);
+        k_tensor_real<<<grid((int64_t)Ky * nxh), 256, 0, st>>>(ycol, yrows, quad, Ky, nxh, pitch, scale, Ky, Ly);
     }
     MAF_LAUNCH_CHECK();
 }
@@ -524,14 +553,13 @@ void Demag::build_tensor(cudaStream_t st) {
     const int64_t cstride = (int64_t)Kz * Ky * Kx;
     const int* comps = md_.nz == 1 ? kComps4 : kComps6;
     Nred64_.alloc(sizeof(double) * cstride * ncomp());
-    // one allocation for the octant and the work buffers (each takes 0.5-1 ms above 2 MB)
-    const size_t oct_bytes = (sizeof(double) * cstride + 255) / 256 * 256;
-    DevBuf scratch(oct_bytes + octant_work(Px(), Py(), Pz()));
-    double* oct = scratch.as<double>();
-    for (int ci = 0; ci < ncomp(); ++ci) {
-        newell_octant(oct, comps[ci], md_, Kx, Ky, Kz, st);
-        transform_octant(oct, Kx, Ky, Kz, comps[ci], Px(), Py(), Pz(), Nred64_.as<double>() + ci * cstride, 1.0,
-                         scratch.as<char>() + oct_bytes, st);
+    // the octants where the transforms replace them
+    newell_octants(Nred64_.as<double>(), comps, ncomp(), md_, Kx, Ky, Kz, st);
+    const int nb = octant_batch(octant_work(Px(), Py(), Pz(), ncomp()), ncomp());
+    DevBuf work(octant_work(Px(), Py(), Pz(), nb));
+    for (int ci = 0; ci < ncomp(); ci += nb) {
+        double* t = Nred64_.as<double>() + ci * cstride;
+        transform_octants(t, Kx, Ky, Kz, comps + ci, nb, Px(), Py(), Pz(), t, 1.0, work.as<char>(), st);
     }
     MAF_CUDA(cudaStreamSynchronize(st));
 }
@@ -543,22 +571,27 @@ void Demag::build_padded_tensor(double* out64, float* out32, cudaStream_t st) {
     const int Kx = md_.nx + 1, Ky = md_.ny + 1, Kz = md_.nz == 1 ? 1 : md_.nz + 1;
     const int64_t cstride = (int64_t)Kz * Ky * Kx, pstride = (int64_t)padded_elems() / ncomp();
     const int* comps = md_.nz == 1 ? kComps4 : kComps6;
-    const size_t oct_bytes = (sizeof(double) * cstride + 255) / 256 * 256;
-    const size_t quad_bytes = out32 ? (sizeof(double) * pstride + 255) / 256 * 256 : 0;
-    DevBuf scratch(oct_bytes + quad_bytes +
-                   std::max(octant_work(Px(), Py(), Pz()), octant_work(pad_x_, pad_y_, pad_z_)));
+    auto oct_bytes = [&](int nc) { return (sizeof(double) * nc * cstride + 255) / 256 * 256; };
+    auto quad_bytes = [&](int nc) { return out32 ? (sizeof(double) * nc * pstride + 255) / 256 * 256 : (size_t)0; };
+    auto bytes = [&](int nc) {
+        return oct_bytes(nc) + quad_bytes(nc) +
+               std::max(octant_work(Px(), Py(), Pz(), nc), octant_work(pad_x_, pad_y_, pad_z_, nc));
+    };
+    const int nb = octant_batch(bytes(ncomp()), ncomp());
+    DevBuf scratch(bytes(nb));
     double* oct = scratch.as<double>();
-    double* quad = reinterpret_cast<double*>(scratch.as<char>() + oct_bytes);
-    char* work = scratch.as<char>() + oct_bytes + quad_bytes;
+    double* quad = reinterpret_cast<double*>(scratch.as<char>() + oct_bytes(nb));
+    char* work = scratch.as<char>() + oct_bytes(nb) + quad_bytes(nb);
     const double scale = 1.0 / ((double)Px() * Py() * Pz());
-    for (int ci = 0; ci < ncomp(); ++ci) {
-        transform_octant(Nred64_.as<double>() + ci * cstride, Kx, Ky, Kz, comps[ci], Px(), Py(), Pz(), oct, scale, work,
-                         st);
-        transform_octant(oct, Kx, Ky, Kz, comps[ci], pad_x_, pad_y_, pad_z_, out32 ? quad : out64 + ci * pstride, 1.0,
-                         work, st);
+    for (int ci = 0; ci < ncomp(); ci += nb) {
+        transform_octants(Nred64_.as<double>() + ci * cstride, Kx, Ky, Kz, comps + ci, nb, Px(), Py(), Pz(), oct, scale,
+                          work, st);
+        transform_octants(oct, Kx, Ky, Kz, comps + ci, nb, pad_x_, pad_y_, pad_z_, out32 ? quad : out64 + ci * pstride,
+                          1.0, work, st);
         if (out32) {
-            k_d2f<<<(unsigned)std::min<int64_t>(ceil_div(pstride, 256), (int64_t)sm_count() * 16), 256, 0, st>>>(
-                quad, out32 + ci * pstride, pstride);
+            const int64_t n = nb * pstride;
+            k_d2f<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16), 256, 0, st>>>(
+                quad, out32 + ci * pstride, n);
             MAF_LAUNCH_CHECK();
         }
     }
@@ -577,7 +610,7 @@ void Demag::download_real_tensor(double* host, bool symmetric, cudaStream_t st) 
     if (symmetric) oct.alloc(sizeof(double) * Kx * Ky * Kz);
     for (int c = 0; c < 6; ++c) {
         if (symmetric) {
-            newell_octant(oct.as<double>(), c, md_, Kx, Ky, Kz, st);
+            newell_octants(oct.as<double>(), &c, 1, md_, Kx, Ky, Kz, st);
             k_tensor_full<<<(unsigned)std::min<int64_t>(ceil_div(nreal, 256), (int64_t)sm_count() * 16), 256, 0, st>>>(
                 oct.as<double>(), real.as<double>(), c, Kx, Ky, Px(), Py(), Pz());
             MAF_LAUNCH_CHECK();

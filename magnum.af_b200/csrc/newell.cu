@@ -90,20 +90,61 @@ __global__ void k_newell(double* __restrict__ out, int comp, int Px, int Py, int
     }
 }
 
-// The component at the offsets 0 <= j < (o0, o1, o2) only, one thread per entry.
-// The parity-exact tensor that the spectral pipeline transforms is even or odd
-// along each axis, so these entries carry all of it (fields.cu, tensor_odd)
-// and the 27 evaluations of f or g per entry (FP64 asinh and atan: the kernel is
-// bound on the FP64 pipe) are made for an eighth of the padded grid.
-__global__ void k_newell_octant(double* __restrict__ out, int comp, int o0, int o1, int o2, double dx, double dy,
-                                double dz) {
+// The stored components (blockIdx.y) at the offsets 0 <= j < (o0, o1, o2) only.  The
+// parity-exact tensor that the spectral pipeline transforms is even or odd along each
+// axis, so these entries carry all of it (fields.cu, tensor_odd).  The kernel is bound on
+// the FP64 pipe (27 evaluations of f or g with asinh and atan per entry) or, for small
+// meshes, on their chain: a CTA takes 32 entries, lane = entry, and each of its 9 warps
+// makes 3 of the 27 evaluations (so the offsets are uniform in a warp); the terms are added
+// in newell_27's order, so the entries are the same bit for bit.  A new tensor (create,
+// allocation and transforms included) with a thread for all 27, a warp per entry (lane =
+// evaluation) and this split: 33 x 50 x 1 429, 373, 370 us; 400 x 400 x 1 1117, 1265, 858;
+// 200 x 120 x 10 3118, 2762, 1952 (the evaluations of one offset branch alike).
+struct NewellComps {
+    int c[6];
+};
+constexpr int kOctWarps = 9;
+// newell_27's order: centre, the 6 faces, the 12 edges, the 8 corners
+__constant__ signed char kStencil[27][3] = {
+    {0, 0, 0},   {1, 0, 0},  {-1, 0, 0},  {0, 1, 0},   {0, -1, 0},  {0, 0, 1},  {0, 0, -1},
+    {1, 1, 0},   {1, -1, 0}, {-1, 1, 0},  {-1, -1, 0}, {1, 0, 1},   {1, 0, -1}, {-1, 0, 1},
+    {-1, 0, -1}, {0, 1, 1},  {0, 1, -1},  {0, -1, 1},  {0, -1, -1}, {1, 1, 1},  {1, 1, -1},
+    {1, -1, 1},  {1, -1, -1}, {-1, 1, 1}, {-1, 1, -1}, {-1, -1, 1}, {-1, -1, -1}};
+
+__global__ void __launch_bounds__(32 * kOctWarps)
+    k_newell_octant(double* __restrict__ out, NewellComps comps, int o0, int o1, int o2, double dx, double dy, double dz) {
+    __shared__ double terms[27][32];
     const int64_t total = (int64_t)o0 * o1 * o2;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
-         idx += (int64_t)gridDim.x * blockDim.x) {
+    const int comp = comps.c[blockIdx.y], lane = threadIdx.x & 31, warp = threadIdx.x / 32;
+    const bool is_f = comp == 0 || comp == 3 || comp == 5;
+    for (int64_t base = (int64_t)blockIdx.x * 32; base < total; base += (int64_t)gridDim.x * 32) {
+        const int64_t idx = base + lane < total ? base + lane : total - 1;
         const int j0 = (int)(idx % o0);
         const int j1 = (int)((idx / o0) % o1);
         const int j2 = (int)(idx / ((int64_t)o0 * o1));
-        out[idx] = newell_comp(comp, j0, j1, j2, dx, dy, dz);
+        // newell_comp's mapping of the axes
+        int ix = j0, iy = j1, iz = j2;
+        double hx = dx, hy = dy, hz = dz;
+        if (comp == 2) {
+            iy = j2, iz = j1, hy = dz, hz = dy;
+        } else if (comp == 3 || comp == 4) {
+            ix = j1, iy = j2, iz = j0, hx = dy, hy = dz, hz = dx;
+        } else if (comp == 5) {
+            ix = j2, iy = j0, iz = j1, hx = dz, hy = dx, hz = dy;
+        }
+        for (int t = warp; t < 27; t += kOctWarps) {
+            const double x = hx * ix + kStencil[t][0] * hx, y = hy * iy + kStencil[t][1] * hy,
+                         z = hz * iz + kStencil[t][2] * hz;
+            const double w = t == 0 ? 8.0 : t < 7 ? -4.0 : t < 19 ? 2.0 : -1.0;
+            terms[t][lane] = w * (is_f ? newell_f(x, y, z) : newell_g(x, y, z));
+        }
+        __syncthreads();
+        if (warp == 0 && base + lane < total) {
+            double sum = terms[0][lane];
+            for (int t = 1; t < 27; ++t) sum += terms[t][lane];
+            out[blockIdx.y * total + base + lane] = -sum / (4.0 * 3.14159265358979323846 * hx * hy * hz);
+        }
+        __syncthreads();
     }
 }
 
@@ -116,8 +157,13 @@ void newell_component(double* out, int comp, const MeshDims& md, int Px, int Py,
     MAF_LAUNCH_CHECK();
 }
 
-void newell_octant(double* out, int comp, const MeshDims& md, int o0, int o1, int o2, cudaStream_t st) {
-    k_newell_octant<<<newell_blocks((int64_t)o0 * o1 * o2), 128, 0, st>>>(out, comp, o0, o1, o2, md.dx, md.dy, md.dz);
+void newell_octants(double* out, const int* comps, int ncomp, const MeshDims& md, int o0, int o1, int o2,
+                    cudaStream_t st) {
+    NewellComps c = {};
+    for (int i = 0; i < ncomp; ++i) c.c[i] = comps[i];
+    const int64_t blocks = std::min<int64_t>(ceil_div((int64_t)o0 * o1 * o2, 32), (int64_t)sm_count() * 256);
+    k_newell_octant<<<dim3((unsigned)blocks, (unsigned)ncomp), 32 * kOctWarps, 0, st>>>(out, c, o0, o1, o2, md.dx, md.dy,
+                                                                                     md.dz);
     MAF_LAUNCH_CHECK();
 }
 
