@@ -9,7 +9,7 @@
 //
 // Members do not depend on one another, so a chain joins the others only after the last
 // recorded step: with a fork and a join around the launches of each pass 16 films up to
-// 512 x 512 (15 pairs of lengths; FP32, Heun) took 320 us a step, in chains 259.
+// 512 x 512 (15 pairs of lengths; FP32, Heun) took 300 us a step, in chains 253.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -187,8 +187,8 @@ int tile_threads(const FFTPlan& p, int ncols, int elems) {
 
 }  // namespace
 
-// The members of one compile-time kernel of a pass (same transform length L and,
-// for the x inverse, run length): their argument items, [parity][stage][member
+// The members of one compile-time kernel of a pass (same transform length L and run:
+// for the x inverse the run length, for the convolution whether rows are padded): their argument items, [parity][stage][member
 // of the class] for the x passes and [member of the class] for the convolution,
 // and the work table of (member of the class, tile).
 struct CtClass {
@@ -299,7 +299,7 @@ template <typename R> void FusedBatch::Chain::build(cudaStream_t st) {
             c.members.push_back(i);
         }
         if (ct_batch_tile<R>(1, Py) > 0) {
-            CtClass& c = ct_class(cc, Py, 0);
+            CtClass& c = ct_class(cc, Py, Py != 2 * mem[i].md.ny);
             cc_of[i] = (int)(&c - cc.data());
             pos_c[i] = (int)c.members.size();
             c.members.push_back(i);
@@ -557,7 +557,7 @@ template <typename R> void FusedBatch::Chain::record(cudaStream_t st, int p) {
                 MAF_LAUNCH_CHECK();
             } else {
                 const CtClass& c = cc[b - ngc];
-                ct_batch_convy<R>(c.items.as<CtConvyItem<R>>(), c.work.as<int2>(), c.nwork, c.L, c.tw, q);
+                ct_batch_convy<R>(c.items.as<CtConvyItem<R>>(), c.work.as<int2>(), c.nwork, c.L, c.run != 0, c.tw, q);
             }
         });
         branches(st, ngi + (int)ci.size(), [&](int b, cudaStream_t q) {
@@ -579,8 +579,11 @@ template <typename R> void FusedBatch::Chain::record(cudaStream_t st, int p) {
 }
 
 // The chains at most; further keys share chains, whose passes then have a launch per key.
-// The same ensemble in 1, 2, 4, 8, 15 chains: 320, 297, 272, 268, 259 us a step.
-constexpr size_t kMaxChains = 16;
+// Up to 2^20 cells as many as the keys need, above fewer: the members of more chains no
+// longer fit the L2 cache side by side.  FP32, Heun, us a step in 1, 2, 4 and 16 chains: 16
+// films of 0.63 M cells (15 keys) 300, -, 265, 253; 24 of 1.75 M (19 keys) 651, 612, 585,
+// 604; 64 of 3.1 M (40 keys) 1059, 1015, 1066, 1109.
+static size_t max_chains(int64_t cells) { return cells <= (1 << 20) ? 16 : cells <= (1 << 21) ? 4 : 2; }
 
 struct FusedBatch::Impl {
     bool f32 = false;
@@ -597,7 +600,7 @@ struct FusedBatch::Impl {
 };
 
 // What the members of a chain share: the transform lengths (largest first, so that the
-// longest chains start first) and the form of the x inverse.
+// longest chains start first) and the forms of the convolution and the x inverse.
 template <typename R> static std::tuple<int64_t, int, int> chain_key(const FusedMember& f, cudaStream_t st) {
     const DemagPlan<R> pl = f.demag->plan<R>(st);
     CtXinvItem<R> it{};
@@ -606,7 +609,7 @@ template <typename R> static std::tuple<int64_t, int, int> chain_key(const Fused
     for (const TermDesc& t : f.terms) it.tl.t[it.tl.n++] = t;
     it.ep.kind = EPI_LLG;
     const int run = f.demag->tune.xinv_run ? f.demag->tune.xinv_run : 2;
-    const int form = f.demag->tune.generic ? -1 : ct_batch_xinv_class<R>(it, run);
+    const int form = f.demag->tune.generic ? -1 : 2 * ct_batch_xinv_class<R>(it, run) + (pl.Py != 2 * f.md.ny);
     return {-(int64_t)pl.Px * pl.Py, pl.Px, form};
 }
 
@@ -615,9 +618,11 @@ FusedBatch::FusedBatch(std::vector<FusedMember> members, FusedScheme scheme, boo
     auto impl = std::make_unique<Impl>();
     impl->f32 = f32;
     std::map<std::tuple<int64_t, int, int>, std::vector<FusedMember>> keyed;
+    int64_t cells = 0;
+    for (const FusedMember& f : members) cells += f.md.N();
     for (FusedMember& f : members)
         keyed[f32 ? chain_key<float>(f, st) : chain_key<double>(f, st)].push_back(std::move(f));
-    const size_t n = std::min(keyed.size(), kMaxChains);
+    const size_t n = std::min(keyed.size(), max_chains(cells));
     size_t rank = 0;
     for (auto& [key, v] : keyed) {
         if (impl->chains.size() <= rank * n / keyed.size()) {

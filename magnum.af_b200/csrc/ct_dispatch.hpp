@@ -77,7 +77,8 @@ template <typename R>
 void ct_batch_xfwd(const CtXfwdItem<R>* items, const int2* work, int nwork, int L, const void* tw, const void* twP,
                    cudaStream_t st);
 template <typename R>
-void ct_batch_convy(const CtConvyItem<R>* items, const int2* work, int nwork, int L, const void* tw, cudaStream_t st);
+void ct_batch_convy(const CtConvyItem<R>* items, const int2* work, int nwork, int L, bool rag, const void* tw,
+                    cudaStream_t st);
 template <typename R, int G>
 bool ct_batch_xinv_group(const CtXinvItem<R>* items, const int2* work, int nwork, int L, int run, const void* tw,
                          const void* twP, cudaStream_t st);

@@ -519,10 +519,13 @@ __global__ void __launch_bounds__(6 * NB, (kMinBlocks<R, 6 * NB, 576, 288>))
 }
 
 // -------------------------------------------------- y convolution (nz == 1)
-// (tile body: kx columns [tile NB, tile NB + NB))
-template <typename R, int L, int NB, int NT>
-__device__ __forceinline__ void convy_ct_tile(cplx_t<R>* S, const R* __restrict__ Nred, int ny, int nxh, int pitch,
+// (tile body: kx columns [tile NB, tile NB + NB)).  RAG: ny < L / 2 rows; a kernel of its
+// own, since the compares cost the exact lengths 16-30 % (8 films, FP32, batched: L = 768
+// 101 -> 120 us, L = 384 20 -> 27).
+template <typename R, int L, int NB, int NT, bool RAG>
+__device__ __forceinline__ void convy_ct_tile(cplx_t<R>* S, const R* __restrict__ Nred, int rows, int nxh, int pitch,
                                               const cplx_t<R>* __restrict__ tw, int tile) {
+    const int ny = RAG ? rows : L / 2;
     using C = cplx_t<R>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     C* s = reinterpret_cast<C*>(smem_raw);
@@ -563,11 +566,11 @@ __device__ __forceinline__ void convy_ct_tile(cplx_t<R>* S, const R* __restrict_
     ct_fft_out<R, 1, true, L, NC, NT, true>(s, 0, tw, st, typename CtPlan<L>::T());
 }
 
-template <typename R, int L, int NB, int NT>
+template <typename R, int L, int NB, int NT, bool RAG>
 __global__ void __launch_bounds__(NT) k_convy_ct(cplx_t<R>* S, const R* __restrict__ Nred, int ny, int nxh, int pitch,
                                                  const cplx_t<R>* __restrict__ tw) {
     pdl_begin();
-    convy_ct_tile<R, L, NB, NT>(S, Nred, ny, nxh, pitch, tw, blockIdx.x);
+    convy_ct_tile<R, L, NB, NT, RAG>(S, Nred, ny, nxh, pitch, tw, blockIdx.x);
 }
 
 // --------------------------------------------------- x inverse + epilogue
@@ -715,12 +718,12 @@ __global__ void __launch_bounds__(NT) kbt_xfwd(const CtXfwdItem<R>* __restrict__
     xfwd_ct_tile<R, LC, NB, NT, true>(d.in, d.n_in, d.rows, d.rows, nullptr, d.ms, d.out, d.pitch, tw, twP, w.y);
 }
 
-template <typename R, int L, int NB, int NT>
+template <typename R, int L, int NB, int NT, bool RAG>
 __global__ void __launch_bounds__(NT) kbt_convy(const CtConvyItem<R>* __restrict__ items, const int2* __restrict__ work,
                                                 const cplx_t<R>* __restrict__ tw) {
     const int2 w = work[blockIdx.x];
     const CtConvyItem<R> d = items[w.x];
-    convy_ct_tile<R, L, NB, NT>(d.S, d.Nred, d.ny, d.nxh, d.pitch, tw, w.y);
+    convy_ct_tile<R, L, NB, NT, RAG>(d.S, d.Nred, d.ny, d.nxh, d.pitch, tw, w.y);
 }
 
 template <typename R, int LC, int NBR, int NT, int RN, XinvMode XM>
@@ -882,10 +885,13 @@ static void convy_L(cplx_t<R>* S, const R* Nred, int ny, int nxh, int pitch, con
     constexpr int NT0 = L * 3 * NB / kE;
     static_assert(NT0 >= 1 && NT0 <= kMaxFftThreads, "CTA size");
     const size_t smem = sizeof(cplx_t<R>) * (size_t)3 * NB * ((L - 1) + ((L - 1) >> 4) + 1);
-    auto k = k_convy_ct<R, L, NB, NT0>;
-    ct_smem(k, smem);
-    launch_chain(k, dim3((unsigned)ceil_div(nxh, NB)), NT0, smem, st, S, Nred, ny, nxh, pitch,
-                 static_cast<const cplx_t<R>*>(tw));
+    auto go = [&](auto k) {
+        ct_smem(k, smem);
+        launch_chain(k, dim3((unsigned)ceil_div(nxh, NB)), NT0, smem, st, S, Nred, ny, nxh, pitch,
+                     static_cast<const cplx_t<R>*>(tw));
+    };
+    if (2 * ny == L) go(k_convy_ct<R, L, NB, NT0, false>);
+    else go(k_convy_ct<R, L, NB, NT0, true>);
 }
 
 // Rows per x-inverse CTA: 4096 values per component triple, 96 threads up to 512 cells
@@ -972,9 +978,10 @@ static void batch_xfwd_L(const CtXfwdItem<R>* items, const int2* work, int nwork
 }
 
 template <typename R, int L>
-static void batch_convy_L(const CtConvyItem<R>* items, const int2* work, int nwork, const void* tw, cudaStream_t st) {
+static void batch_convy_L(const CtConvyItem<R>* items, const int2* work, int nwork, bool rag, const void* tw,
+                          cudaStream_t st) {
     using S = ConvyShape<R, L>;
-    auto k = kbt_convy<R, L, S::NB, S::NT>;
+    auto k = rag ? kbt_convy<R, L, S::NB, S::NT, true> : kbt_convy<R, L, S::NB, S::NT, false>;
     ct_smem(k, S::smem);
     k<<<(unsigned)nwork, S::NT, S::smem, st>>>(items, work, static_cast<const cplx_t<R>*>(tw));
     MAF_LAUNCH_CHECK();
@@ -1251,9 +1258,10 @@ void ct_batch_xfwd(const CtXfwdItem<R>* items, const int2* work, int nwork, int 
 }
 
 template <typename R>
-void ct_batch_convy(const CtConvyItem<R>* items, const int2* work, int nwork, int L, const void* tw, cudaStream_t st) {
+void ct_batch_convy(const CtConvyItem<R>* items, const int2* work, int nwork, int L, bool rag, const void* tw,
+                    cudaStream_t st) {
     if (nwork <= 0) return;
-#define X(N) batch_convy_L<R, N>(items, work, nwork, tw, st)
+#define X(N) batch_convy_L<R, N>(items, work, nwork, rag, tw, st)
     MAF_CT_BATCH_SWITCH(L, X)
 #undef X
 }
@@ -1283,7 +1291,7 @@ bool ct_batch_xinv_group(const CtXinvItem<R>* items, const int2* work, int nwork
     template void ct_batch_xinv_prepare<R>(CtXinvItem<R>&, int);                                                    \
     template void ct_batch_xfwd<R>(const CtXfwdItem<R>*, const int2*, int, int, const void*, const void*,        \
                                    cudaStream_t);                                                                \
-    template void ct_batch_convy<R>(const CtConvyItem<R>*, const int2*, int, int, const void*, cudaStream_t);
+    template void ct_batch_convy<R>(const CtConvyItem<R>*, const int2*, int, int, bool, const void*, cudaStream_t);
 #else
 #define MAF_INST1(R)
 #endif
