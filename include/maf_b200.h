@@ -229,7 +229,8 @@ int maf_llg_pass_name(maf_llg l, maf_state s, int index, char* buf, int buflen);
  * (AdaptiveRungeKutta's stage loop, adaptive_runge_kutta.cpp:113-173; the state is not
  * changed) with a CUDA event after every kernel: synchronises and returns the duration in
  * ms of each interval -- the FP32 copy of m ("stage_m32"), every stage's combine
- * ("rk_combine_kN": N = FP64 k buffers read) and field passes, and the finalize
+ * ("rk_combine_kN": N = FP64 k buffers read; only above 2^18 cells, below the previous
+ * stage's last pass does it) and field passes, and the finalize
  * ("rk_finalize_kN": sumbk, error norm and candidate from N distinct k buffers).  Names
  * come from maf_llg_profile_name (valid until the next profile on this integrator). */
 int maf_llg_attempt_profile(maf_llg l, maf_state s, double dt, double* ms_out, int max_entries, int* n_entries);
