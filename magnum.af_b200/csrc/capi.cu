@@ -531,6 +531,18 @@ struct StochStage {
     double scale = 0;
 };
 
+// The work buffers of a step (Heun 2, SemiHeun 6, detRK4 4 stages).
+void stoch_buffers(maf_stoch_s* h, maf_state_s* st) {
+    const size_t n3 = 3 * (size_t)st->s.md.N();
+    const int stages = h->mode == 0 ? 2 : h->mode == 1 ? 6 : 4;
+    for (int i = 0; i < stages; ++i) h->k[i].ensure(sizeof(double) * n3);
+    h->mstage64.ensure(sizeof(double) * n3);
+    if (st->s.precision == PREC_FP32_FIELD) h->mstage32.ensure(sizeof(float) * n3);
+    h->mcand.ensure(sizeof(double) * n3);
+    ensure_finalize_scratch(h->partials, st->s.stream);
+    h->errbuf.ensure(sizeof(double) * 4);
+}
+
 // One step.  With q_dev (a device copy of h->calls) the noise stream indices are
 // read from q_dev on the device and q_dev is advanced by a device kernel, so the
 // step can be captured in a CUDA graph and replayed.
@@ -566,12 +578,7 @@ void stoch_step(maf_stoch_s* h, maf_state_s* st, unsigned long long* q_dev = nul
         stages = {a, b, c, d};
         fin.n = 4; fin.c[0] = 1. / 6.; fin.c[1] = 2. / 6.; fin.c[2] = 2. / 6.; fin.c[3] = 1. / 6.;
     }
-    for (size_t i = 0; i < stages.size(); ++i) h->k[i].ensure(sizeof(double) * n3);
-    h->mstage64.ensure(sizeof(double) * n3);
-    if (f32) h->mstage32.ensure(sizeof(float) * n3);
-    h->mcand.ensure(sizeof(double) * n3);
-    ensure_finalize_scratch(h->partials, s.stream);
-    h->errbuf.ensure(sizeof(double) * 4);
+    stoch_buffers(h, st);
     std::vector<Term*> terms;
     for (auto& t : h->terms) terms.push_back(t.get());
     for (size_t i = 0; i < stages.size(); ++i) {
@@ -2700,8 +2707,10 @@ struct maf_stoch_batch_s {
     DevBuf q;  // per-member step counters (device)
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    std::vector<const void*> m_at_capture;  // state buffers the graph was captured with
+    // what the last eager step ran with, and what the graph was captured with (batch_plans, batch_buffers)
     bool warm = false;
+    std::vector<unsigned long long> warm_plans, plans_at_capture;
+    std::vector<const void*> buffers_at_capture;
     ~maf_stoch_batch_s() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
@@ -2720,6 +2729,43 @@ void batch_drop_graph(maf_stoch_batch_s* b) {
     b->exec = nullptr;
     b->graph = nullptr;
     b->fused_active = false;
+}
+
+// The demag plans that the members' next steps run with: object, kernel choices, lengths and the
+// addresses a graph records.  A plan's tensor and spectra are made here if they are missing.
+std::vector<unsigned long long> batch_plans(maf_stoch_batch_s* b) {
+    std::vector<unsigned long long> v;
+    auto add = [&](const Demag& d, const auto& p) {
+        const TuneChoice& c = d.tune;
+        for (int x : {c.cols_wide, c.convz_reg, c.xinv_run, c.cols_pipe, c.cols_plan, c.generic, p.Px, p.Py, p.Pz})
+            v.push_back((unsigned long long)x);
+        for (const void* q : {(const void*)p.s1, (const void*)p.s2, (const void*)p.tensor})
+            v.push_back((unsigned long long)(uintptr_t)q);
+        v.push_back(d.id());
+    };
+    for (size_t i = 0; i < b->its.size(); ++i) {
+        const StateD& s = b->sts[i]->s;
+        for (auto& t : b->its[i]->terms) {
+            if (t->kind != TK_DEMAG) continue;
+            Demag* d = term_demag(*t, s.md, s.stream);
+            if (s.precision == PREC_FP32_FIELD) add(*d, d->plan<float>(s.stream));
+            else add(*d, d->plan<double>(s.stream));
+        }
+    }
+    return v;
+}
+
+// The members' other buffers whose addresses a graph records.
+std::vector<const void*> batch_buffers(maf_stoch_batch_s* b) {
+    std::vector<const void*> v;
+    for (size_t i = 0; i < b->its.size(); ++i) {
+        const maf_stoch_s* h = b->its[i];
+        const StateD& s = b->sts[i]->s;
+        for (const DevBuf* d : {&s.m64, &s.m32, &h->mcand, &h->mstage64, &h->mstage32, &h->partials, &h->errbuf})
+            v.push_back(d->p);
+        for (const DevBuf& k : h->k) v.push_back(k.p);
+    }
+    return v;
 }
 
 // device counters <- host step counts
@@ -2846,13 +2892,13 @@ void batch_capture(maf_stoch_batch_s* b) {
     }
     MAF_CUDA(cudaStreamEndCapture(b->root, &b->graph));
     MAF_CUDA(cudaGraphInstantiate(&b->exec, b->graph, 0));
-    b->m_at_capture.clear();
     for (size_t i = 0; i < n; ++i) {
         b->sts[i]->s.t = t[i];
         b->sts[i]->s.steps = steps[i];
         b->its[i]->calls = calls[i];
-        b->m_at_capture.push_back(b->sts[i]->s.m64.p);
     }
+    b->plans_at_capture = b->warm_plans;
+    b->buffers_at_capture = batch_buffers(b);
 }
 
 }  // namespace
@@ -2916,15 +2962,22 @@ int maf_stoch_batch_steps(maf_stoch_batch b, int nsteps) {
         const size_t n = b->its.size();
         int left = nsteps;
         for (auto* st : b->sts) MAF_CUDA(cudaStreamSynchronize(st->s.stream));
-        // the first step runs eagerly: it sizes every work buffer before a capture
-        if (left > 0 && !b->warm) {
-            for (size_t i = 0; i < n; ++i) stoch_step(b->its[i], b->sts[i]);
-            --left;
-            b->warm = true;
+        // The first step with a set of demag plans runs eagerly: it makes every buffer, twiddle table
+        // and kernel attribute before a capture.  The plans change with DemagField.generic and the tuned
+        // choices, which the user and the autotuner set at any time.
+        if (left > 0) {
+            for (size_t i = 0; i < n; ++i) stoch_buffers(b->its[i], b->sts[i]);
+            std::vector<unsigned long long> plans = batch_plans(b);
+            if (!b->warm || plans != b->warm_plans) {
+                for (size_t i = 0; i < n; ++i) stoch_step(b->its[i], b->sts[i]);
+                --left;
+                b->warm = true;
+                b->warm_plans = std::move(plans);
+            }
         }
         if (left >= 2) {
-            bool stale = !b->exec;
-            for (size_t i = 0; i < n && !stale; ++i) stale = b->sts[i]->s.m64.p != b->m_at_capture[i];
+            // a graph replays the addresses it recorded: captured again when one of them changed
+            const bool stale = !b->exec || b->plans_at_capture != b->warm_plans || b->buffers_at_capture != batch_buffers(b);
             for (auto* st : b->sts) MAF_CUDA(cudaStreamSynchronize(st->s.stream));
             batch_upload_counters(b);
             if (stale) batch_capture(b);

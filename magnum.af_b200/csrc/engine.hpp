@@ -203,8 +203,11 @@ class Demag {
     size_t tensor_elems() const { return (size_t)ncomp() * (md_.nz == 1 ? 1 : md_.nz + 1) * (md_.ny + 1) * nxh(); }
     int pitch() const { return pitch_; }
     template <typename R> int edens_blocks() const;
-    // the plan of an evaluation at the current kernel choices; its tensor and buffers are made on first use
+    // the plan of an evaluation at the current kernel choices; its tensor and buffers are made on first use.
+    // The spectra grow when a plan needs longer rows: whoever keeps their addresses (a captured
+    // graph) compares them, and id(), with the plan's before every use.
     template <typename R> DemagPlan<R> plan(cudaStream_t st);
+    unsigned long long id() const { return id_; }  // of this object, never given twice in a process
     const void* twiddles(int L, bool fp64) { return tw_.get(L, fp64); }
     Twiddles& twiddle_tables() { return tw_; }
 
@@ -220,6 +223,8 @@ class Demag {
         return (size_t)ncomp() * (pad_z_ == 1 ? 1 : pad_z_ / 2 + 1) * (pad_y_ / 2 + 1) * (pad_x_ / 2 + 1);
     }
 
+    unsigned long long id_ = next_id();
+    static unsigned long long next_id();
     MeshDims md_;
     bool pbc_ = false;
     int pitch_;  // complex row pitch of the half spectrum (>= nxh)
@@ -272,6 +277,9 @@ struct StateD {
         return mi;
     }
 };
+
+// The Demag of a TK_DEMAG term on a mesh (DemagFieldPBC: planned on first use).
+Demag* term_demag(Term& t, const MeshDims& md, cudaStream_t st);
 
 // Field evaluation of a list of terms on m (precision R), with one epilogue.
 template <typename R>

@@ -20,6 +20,7 @@
 //   fused into the store) -> x-inv C2R + local terms + epilogue.
 // Passes (nz == 1): x-fwd -> y-fwd . tensor . y-inv (in place) -> x-inv + epilogue.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 
 #include "engine.hpp"
@@ -448,6 +449,11 @@ static int ct_length(const int* list, int n) {
     return 0;
 }
 
+unsigned long long Demag::next_id() {
+    static std::atomic<unsigned long long> n{0};
+    return ++n;
+}
+
 Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, bool pbc) : md_(md), pbc_(pbc) {
     if (md.nx < 1 || md.ny < 1 || md.nz < 1) throw Error(1, "DemagField: empty mesh");
     if (pbc) {
@@ -854,6 +860,16 @@ template void Demag::inverse_x_epilogue<double>(const double*, const MsInfo&, co
 // ---------------------------------------------------------------------------
 // field evaluation of a term list
 // ---------------------------------------------------------------------------
+Demag* term_demag(Term& t, const MeshDims& md, cudaStream_t st) {
+    if (t.demag_pbc() && !(t.demag && t.demag_mesh == md)) {
+        // DemagFieldPBC takes its mesh from the state: plan it on first use
+        t.demag = std::make_unique<Demag>(md, st, nullptr, true);
+        t.demag_mesh = md;
+    }
+    if (!(t.demag_mesh == md)) throw Error(1, "DemagField mesh differs from the state's mesh");
+    return t.demag.get();
+}
+
 template <typename R>
 void eval_terms(const std::vector<Term*>& terms, const MeshDims& md, const R* m, const MsInfo& ms,
                 const EpilogueArgs& ep_in, cudaStream_t st, DevBuf& scratch, double* energy_out,
@@ -865,13 +881,7 @@ void eval_terms(const std::vector<Term*>& terms, const MeshDims& md, const R* m,
     for (Term* t : terms) {
         if (t->kind == TK_DEMAG) {
             if (demag) throw Error(1, "at most one DemagField per term list");
-            if (t->demag_pbc() && !(t->demag && t->demag_mesh == md)) {
-                // DemagFieldPBC takes its mesh from the state: plan it on first use
-                t->demag = std::make_unique<Demag>(md, st, nullptr, true);
-                t->demag_mesh = md;
-            }
-            if (!(t->demag_mesh == md)) throw Error(1, "DemagField mesh differs from the state's mesh");
-            demag = t->demag.get();
+            demag = term_demag(*t, md, st);
         }
         if (t->field_cells && t->field_cells != md.N())
             throw Error(1, "field-term parameter array does not match the state's mesh");

@@ -87,3 +87,50 @@ def test_fused_batch_falls_back_for_3d_members():
     batch = M.StochasticBatch([(it, st)], fused=True)
     batch.steps(3)
     assert not batch.fused_active
+
+
+@pytest.mark.parametrize("fused", [True, False])
+@pytest.mark.parametrize("prec", ["fp32_field", "fp64"])
+def test_kernel_choice_changed_between_batch_steps(prec, fused):
+    """DemagField.generic switched while the batch holds a captured graph, on meshes whose
+    two forms have spectra of different lengths (the buffers move): the graph is captured
+    again, and every member's trajectory stays its own integrator's."""
+    bm = _members(prec, "Heun", generic=True, sides=[(40, 24), (33, 15), (100, 25)])
+    sm = _members(prec, "Heun", generic=True, sides=[(40, 24), (33, 15), (100, 25)])
+    batch = M.StochasticBatch([(it, st) for it, st, _ in bm], fused=fused)
+    for generic, n in ((True, 5), (False, 5), (False, 4), (True, 3), (False, 2), (False, 2)):
+        for group in (bm, sm):
+            for _, st, terms in group:
+                if terms[0].generic != generic:
+                    terms[0].generic = generic
+                    terms[0].H_in_Apm(st)  # an evaluation in between: the spectra are those of the new choice
+        batch.steps(n)
+        for (itb, stb, _), (its, sts, _) in zip(bm, sm):
+            its.steps(sts, n)
+            assert np.array_equal(np.asarray(stb.m), np.asarray(sts.m))
+            assert stb.t == sts.t and itb.calls == its.calls
+
+
+def test_integrator_used_elsewhere_between_batch_steps():
+    """A member's integrator steps larger and smaller states of its own (its work buffers
+    move) while the batch holds a captured graph."""
+    def terms(mesh):
+        return [M.ExchangeField(1.5e-11), M.UniaxialAnisotropyField(6e5)]
+
+    made = []
+    for _ in range(2):
+        group = []
+        for i, (nx, ny) in enumerate([(40, 24), (33, 15)]):
+            mesh = M.Mesh(nx, ny, 1, 2e-9, 2e-9, 1e-9)
+            st = M.State(mesh, 7e5, random_m((nx, ny, 1), 60 + i))
+            group.append((M.Stochastic_LLG(0.1, 300.0, 5e-14, st, terms(mesh), "Heun", seed=11, member=i), st))
+        made.append(group)
+    batch = M.StochasticBatch(made[0])
+    for shape in ((200, 100, 1), (8, 6, 1), (64, 64, 1)):
+        batch.steps(4)
+        for (_, sb), (it, ss) in zip(*made):
+            it.steps(ss, 4)
+            assert np.array_equal(np.asarray(sb.m), np.asarray(ss.m))
+        for group in made:
+            other = M.State(M.Mesh(*shape, 2e-9, 2e-9, 1e-9), 7e5, random_m(shape, 5))
+            group[0][0].steps(other, 3)
