@@ -368,6 +368,12 @@ typedef struct maf_cnn_s* maf_cnn;
  * returns after the stream finished it.  MAF_ERR_TIMEOUT if a bounded tensor-core wait gave up. */
 int maf_bf16_gemm(const void* A_dev, int lda, const void* B_dev, int ldb, float* C_dev, int ldc, int M, int N, int K,
                   void* stream);
+/* The waits of the tensor-core kernels (maf_bf16_gemm, maf_nn_conv*) are bounded.  A kernel whose wait gives
+ * up stores nothing and raises a flag of its device.  maf_nn_check returns MAF_ERR_TIMEOUT and lowers the flag
+ * if it is up (wait: after the stream's work has finished).  maf_nn_flag_timeout raises the flag from the stream
+ * as such a kernel does, for tests of the callers. */
+int maf_nn_check(void* stream, int wait);
+int maf_nn_flag_timeout(void* stream);
 /* Layer kernels of the warm-start U-net (magnumaf/unet.py; no counterpart in the reference).  Device
  * pointers; activations pixel-major ([pixels][channels], pixel (b, y, x) at row (b H + y) W + x); BF16
  * tensors that feed a GEMM have their channels padded with zeros to Cp, a multiple of 8; every call is
@@ -427,7 +433,7 @@ int maf_nn_relu_bias_bwd_parts(int* n);
 int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
                           void* st);
 /* y = normalize(m + d) [P][3]; with a target t: per-pixel |y - t|^2, its mean in *loss (device) and
- * dL/dd [P][3] in gd */
+ * dL/dd [P][3] in gd.  While the timeout flag (maf_nn_check) is up, y is NaN. */
 int maf_nn_head(const float* m, const float* d, int ldd, const float* t, long long P, float* y, float* gd,
                 float* cell_loss, float* loss, void* st);
 /* one Adam step (beta 0.9 / 0.999, eps 1e-8), step = the 1-based step count for the bias corrections */

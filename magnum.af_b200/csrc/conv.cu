@@ -14,8 +14,8 @@
 // Pipeline: kStages shared-memory stages of 64 K values; per stage one barrier, four
 // MMAs issued by thread 0 and committed to the stage's mbarrier; a stage is refilled
 // when the MMA that read it has completed, so up to kStages - 1 copies are in flight
-// under the MMAs.  Every wait is bounded: a wait that gives up sets *err and the CTA
-// leaves through its epilogue, freeing its tensor memory.
+// under the MMAs.  Every wait is bounded: a wait that gives up raises the device's flag
+// (tc_error.hpp) and the CTA leaves without storing, freeing its tensor memory.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -23,6 +23,7 @@
 #include "../../include/maf_b200.h"
 #include "capi_internal.hpp"
 #include "engine.hpp"
+#include "tc_error.hpp"
 
 namespace mafb {
 
@@ -165,7 +166,7 @@ struct ConvArgs {
     bf16* outb;         // [P][ldb] (zero beyond N) or null
     int H, W, Cp, N, ldo, ldb, relu;
     int64_t P;
-    int* err;
+    TcError err;
 };
 
 // out[p][n] = relu?(bias[n] + sum_{t, c} act[tap t of p][c] w[n][t Cp + c]): CTA =
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(128) k_conv(ConvArgs a) {
             }
         }
     } else if (tid == 0) {
-        atomicExch(a.err, 1);
+        tc_raise(a.err);
     }
     cta_end<BN>(cta);
 }
@@ -289,7 +290,7 @@ struct WgradArgs {
     float* work;      // [splits][9 Cp][Np]
     int H, W, Cp, Np;
     int64_t P, chunk;  // pixels per split, a multiple of kBK
-    int* err;
+    TcError err;
 };
 
 // work[s][t Cp + c][n] = sum over the split's pixels of act[tap t of p][c] dy[p][n]:
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(128) k_conv_wgrad(WgradArgs a) {
                                     __uint_as_float(u[j + 3]));
         }
     } else if (tid == 0) {
-        atomicExch(a.err, 1);
+        tc_raise(a.err);
     }
     cta_end<BN>(cta);
 }
@@ -472,8 +473,6 @@ constexpr int kReluBlocks = 592;  // 4 per SM
 
 }  // namespace
 
-int* umma_error_flag();  // umma.cu
-
 template <int BN> static void launch_conv(const ConvArgs& a, cudaStream_t st) {
     constexpr size_t smem = (size_t)kStages * (kBM + BN) * 128 + 1024;
     MAF_CUDA(cudaFuncSetAttribute(k_conv<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -506,7 +505,7 @@ int maf_nn_conv(const void* act, int B, int H, int W, int Cp, const void* w, int
             throw Error(1, "maf_nn_conv: 16-byte aligned buffers expected");
         ConvArgs a{static_cast<const __nv_bfloat16*>(act), static_cast<const __nv_bfloat16*>(w), bias, out,
                    static_cast<__nv_bfloat16*>(outb), H, W, Cp, N, ldo, ldb, relu, (int64_t)B * H * W,
-                   umma_error_flag()};
+                   tc_error()};
         cudaStream_t s = static_cast<cudaStream_t>(st);
         // the widest tile that the channels fill, so that a pixel's taps are gathered once;
         // narrower when the tiles would leave SMs idle (a single film's deeper levels)
@@ -530,7 +529,7 @@ int maf_nn_conv_wgrad(const void* act, int B, int H, int W, int Cp, int Cin, con
             throw Error(1, "maf_nn_conv_wgrad: 16-byte aligned buffers expected");
         cudaStream_t s = static_cast<cudaStream_t>(st);
         WgradArgs a{static_cast<const __nv_bfloat16*>(act), static_cast<const __nv_bfloat16*>(dy), work, H, W, Cp,
-                    CoutP, (int64_t)B * H * W, 0, umma_error_flag()};
+                    CoutP, (int64_t)B * H * W, 0, tc_error()};
         const int bn = CoutP <= 32 ? 32 : CoutP <= 64 ? 64 : 128;
         // about four CTAs per SM, at least four K blocks each
         const int64_t tiles = ceil_div(9 * Cp, kBM) * ceil_div(CoutP, bn);

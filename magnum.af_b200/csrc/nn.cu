@@ -13,6 +13,7 @@
 #include "../../include/maf_b200.h"
 #include "capi_internal.hpp"
 #include "engine.hpp"
+#include "tc_error.hpp"
 
 namespace mafb {
 void umma_gemm(const void* A, int lda, const void* B, int ldb, float* C, int ldc, int M, int N, int K,
@@ -334,15 +335,17 @@ __global__ void k_wgrad(const float* __restrict__ g, int Cout, int Cin, int Cp, 
 }
 
 // head: v = m + d, y = v / |v|; per-pixel loss |y - t|^2 and dL/dd (L = mean over
-// pixels of |y - t|^2; t may be null: inference)
+// pixels of |y - t|^2; t may be null: inference).  Where a convolution's wait gave up, y is
+// NaN: its tiles hold another call's values, and an inference returns before the host could ask.
 __global__ void k_head(const float* __restrict__ m, const float* __restrict__ d, int ldd,
                        const float* __restrict__ tgt, int64_t P, float* __restrict__ y, float* __restrict__ gd,
-                       float* __restrict__ cell_loss) {
+                       float* __restrict__ cell_loss, const int* __restrict__ failed) {
     const float inv = 1.f / (float)P;
+    const bool bad = *failed != 0;
     GRID_STRIDE(p, P) {
         float v[3];
 #pragma unroll
-        for (int c = 0; c < 3; ++c) v[c] = m[p * 3 + c] + d[p * ldd + c];
+        for (int c = 0; c < 3; ++c) v[c] = bad ? __int_as_float(0x7fc00000) : m[p * 3 + c] + d[p * ldd + c];
         const float n = sqrtf(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
         const float in_ = n > 0.f ? 1.f / n : 0.f;
         float yy[3];
@@ -574,7 +577,7 @@ int maf_nn_wgrad(const float* g, int Cout, int Cin, int Cp, float* dW, void* st)
 int maf_nn_head(const float* m, const float* d, int ldd, const float* tgt, long long P, float* y, float* gd,
                 float* cell_loss, float* loss, void* st) {
     return run([&] {
-        k_head<<<grid_for(P), kT, 0, S(st)>>>(m, d, ldd, tgt, P, y, gd, cell_loss);
+        k_head<<<grid_for(P), kT, 0, S(st)>>>(m, d, ldd, tgt, P, y, gd, cell_loss, tc_error().dev);
         MAF_LAUNCH_CHECK();
         if (tgt && loss) {
             k_mean<<<1, kMeanT, 0, S(st)>>>(cell_loss, P, loss);

@@ -15,12 +15,16 @@
 // the CTA waits for that barrier before the tiles are overwritten.  The
 // epilogue reads the accumulator with tcgen05.ld (warp w owns TMEM lanes
 // 32w .. 32w + 31, i.e. rows 32w .. of the tile).  Every wait is bounded: a
-// wait that gives up sets *err and the CTA skips to freeing its TMEM.
+// wait that gives up raises the device's flag (tc_error.hpp) and the CTA skips to
+// freeing its TMEM.
 #include <cuda_bf16.h>
+
+#include <mutex>
 
 #include "../../include/maf_b200.h"
 #include "capi_internal.hpp"
 #include "engine.hpp"
+#include "tc_error.hpp"
 
 namespace mafb {
 
@@ -66,7 +70,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
 template <int BN>
 __global__ void __launch_bounds__(128) k_umma_gemm(const __nv_bfloat16* __restrict__ A, int lda,
                                                    const __nv_bfloat16* __restrict__ B, int ldb, float* __restrict__ C,
-                                                   int ldc, int M, int N, int K, int kchunk, int* err) {
+                                                   int ldc, int M, int N, int K, int kchunk, TcError err) {
     static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "tile width");
     constexpr uint32_t A_KC = (kBM / 8) * 128;  // bytes between the K chunks of the A tile (LBO)
     constexpr uint32_t B_KC = (BN / 8) * 128;   // of the B tile
@@ -164,24 +168,54 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __nv_bfloat16* __restri
             }
         }
     } else if (tid == 0) {
-        atomicExch(err, 1);
+        tc_raise(err);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(BN));
 }
 
-DevBuf g_umma_err;  // device error flag of the tensor-core GEMM (one per process)
+// the flag as a wait that gave up raises it (maf_nn_flag_timeout)
+__global__ void k_tc_raise(TcError e) { tc_raise(e); }
+
+constexpr int kMaxOrdinals = 64;
+struct DeviceFlag {
+    TcError e;
+    volatile int* host = nullptr;  // host address of the host word
+};
+
+DeviceFlag& device_flag() {
+    static std::mutex mu;
+    static DeviceFlag flags[kMaxOrdinals];
+    int dev = 0;
+    MAF_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kMaxOrdinals) throw Error(6, "tensor-core kernels: device ordinal too large");
+    std::lock_guard<std::mutex> lock(mu);
+    DeviceFlag& f = flags[dev];
+    if (!f.host) {
+        void *d = nullptr, *h = nullptr, *hd = nullptr;
+        MAF_CUDA(cudaMalloc(&d, sizeof(int)));
+        MAF_CUDA(cudaMemset(d, 0, sizeof(int)));
+        MAF_CUDA(cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped));
+        MAF_CUDA(cudaHostGetDevicePointer(&hd, h, 0));
+        *static_cast<int*>(h) = 0;
+        f.e = TcError{static_cast<int*>(d), static_cast<int*>(hd)};
+        f.host = static_cast<volatile int*>(h);
+    }
+    return f;
+}
 
 }  // namespace
 
-// The error flag, zeroed on first use.
-int* umma_error_flag() {
-    if (!g_umma_err.p) {
-        g_umma_err.alloc(sizeof(int));
-        MAF_CUDA(cudaMemset(g_umma_err.p, 0, sizeof(int)));
-    }
-    return g_umma_err.as<int>();
+TcError tc_error() { return device_flag().e; }
+
+void tc_check(cudaStream_t st, bool wait) {
+    DeviceFlag& f = device_flag();
+    if (wait) MAF_CUDA(cudaStreamSynchronize(st));
+    if (!*f.host) return;
+    *f.host = 0;
+    MAF_CUDA(cudaMemsetAsync(f.e.dev, 0, sizeof(int), st));
+    throw Error(5, "a tensor-core kernel's wait timed out: its outputs are not valid");
 }
 
 // Host launcher (nn.cu and the C ABI): the tile width follows N; with splits > 1
@@ -195,7 +229,7 @@ void umma_gemm(const void* A, int lda, const void* B, int ldb, float* C, int ldc
     splits = (int)ceil_div(K, kchunk);
     if (K % 8 || lda % 8 || ldb % 8 || lda < K || ldb < K || ldc < N || ((uintptr_t)A | (uintptr_t)B) % 16)
         throw Error(1, "bf16 gemm: K and the row strides must be multiples of 8 elements, rows 16-byte aligned");
-    int* err = umma_error_flag();
+    const TcError err = tc_error();
     const auto* a = static_cast<const __nv_bfloat16*>(A);
     const auto* b = static_cast<const __nv_bfloat16*>(B);
     const unsigned gx = (unsigned)ceil_div(M, kBM);
@@ -209,15 +243,7 @@ void umma_gemm(const void* A, int lda, const void* B, int ldb, float* C, int ldc
                                                                                     kchunk, err);
     }
     MAF_LAUNCH_CHECK();
-    if (check) {
-        int e = 0;
-        MAF_CUDA(cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        MAF_CUDA(cudaStreamSynchronize(st));
-        if (e) {
-            MAF_CUDA(cudaMemset(err, 0, sizeof(int)));
-            throw Error(5, "bf16 gemm: a tensor-core wait timed out");
-        }
-    }
+    if (check) tc_check(st, true);
 }
 
 }  // namespace mafb
@@ -227,5 +253,16 @@ extern "C" int maf_bf16_gemm(const void* A_dev, int lda, const void* B_dev, int 
     return mafb::capi_run([&] {
         if (!A_dev || !B_dev || !C_dev) throw mafb::Error(1, "maf_bf16_gemm: NULL argument");
         mafb::umma_gemm(A_dev, lda, B_dev, ldb, C_dev, ldc, M, N, K, static_cast<cudaStream_t>(stream), true);
+    });
+}
+
+extern "C" int maf_nn_check(void* stream, int wait) {
+    return mafb::capi_run([&] { mafb::tc_check(static_cast<cudaStream_t>(stream), wait != 0); });
+}
+
+extern "C" int maf_nn_flag_timeout(void* stream) {
+    return mafb::capi_run([&] {
+        mafb::k_tc_raise<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(mafb::tc_error());
+        MAF_LAUNCH_CHECK();
     });
 }

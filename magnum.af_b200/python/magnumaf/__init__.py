@@ -154,6 +154,8 @@ _SIGS = {
     "maf_nn_colsum": (_I, [_P, C.c_longlong, _I, _P, _P]),
     "maf_nn_wcast": (_I, [_P, _I, _I, _I, _I, _P, _P, _P]),
     "maf_nn_wgrad": (_I, [_P, _I, _I, _I, _P, _P]),
+    "maf_nn_check": (_I, [_P, _I]),
+    "maf_nn_flag_timeout": (_I, [_P]),
     "maf_nn_conv": (_I, [_P, _I, _I, _I, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P]),
     "maf_nn_conv_wgrad": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _I, _P, _I, _P, _P]),
     "maf_nn_wcast_conv": (_I, [_P, _I, _I, _I, _I, _P, _P, _P]),

@@ -105,6 +105,12 @@ class UNet:
     def _stream(self):
         return _P(self.torch.cuda.current_stream().cuda_stream)
 
+    def check(self, wait: bool = True) -> None:
+        """Raises (MAF_ERR_TIMEOUT) when a convolution's bounded wait gave up since the last check; wait: once
+        the current stream's work has finished.  forward() returns before that, with y NaN in such a case;
+        loss_grad and train_step check themselves, and every call first reports an earlier one's."""
+        _ck(lib.maf_nn_check(self._stream(), int(wait)))
+
     def _cast_weights(self):
         """BF16 copies of every layer's weights: [cout][9 cp] (forward) and [cin][9 coutp] (data gradient)."""
         torch = self.torch
@@ -165,6 +171,7 @@ class UNet:
                             self.layers[i + 1].cp if nxt is not None else 0, st))
 
     def _forward(self, x_ptr, B, H, W):
+        self.check(wait=False)
         self._buffers(B, H, W)
         if self._dirty:
             self._cast_weights()
@@ -251,7 +258,9 @@ class UNet:
                             _P(_p(self.dA[8])), _P(_p(self.cell_loss)), _P(_p(self.loss)), st))
         if want_grad:
             self._backward(B)
-        return float(self.loss.item())
+        loss = float(self.loss.item())
+        self.check(wait=False)  # item() has waited for the stream
+        return loss
 
     def train_step(self, x_ptr: int, t_ptr: int, B: int, H: int, W: int, lr: float) -> float:
         loss = self.loss_grad(x_ptr, t_ptr, B, H, W, True)

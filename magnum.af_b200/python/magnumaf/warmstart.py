@@ -115,8 +115,9 @@ def propose(net, m0: np.ndarray, p: Dict[str, float]) -> np.ndarray:
         y = torch.empty((1, 3, ny, nx), dtype=torch.float32, device="cuda")
         net.forward(x.data_ptr(), 1, ny, nx, y.data_ptr())
         return from_chw(y[0].double().cpu().numpy())
-    y = net.forward(x.data_ptr(), 1, ny, nx)  # U-net: [ny nx][3], pixel-major
-    return np.ascontiguousarray(np.transpose(y.double().cpu().numpy().reshape(ny, nx, 3), (1, 0, 2))[:, :, None, :])
+    y = net.forward(x.data_ptr(), 1, ny, nx).double().cpu().numpy()  # U-net: [ny nx][3], pixel-major
+    net.check(wait=False)
+    return np.ascontiguousarray(np.transpose(y.reshape(ny, nx, 3), (1, 0, 2))[:, :, None, :])
 
 
 def relax(m0: np.ndarray, p: Dict[str, float], cnn=None, tol: float = 1e-6, maxiter: int = 1000):

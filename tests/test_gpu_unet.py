@@ -104,3 +104,47 @@ def test_unet_training_lowers_the_loss():
     losses = [net.train_step(xd.data_ptr(), td.data_ptr(), B, H, W, 2e-3) for _ in range(150)]
     assert np.all(np.isfinite(losses))
     assert np.mean(losses[-10:]) < 0.5 * np.mean(losses[:5])
+
+
+def test_timed_out_wait_is_reported():
+    """The flag that a convolution's bounded wait raises (here raised from the stream, no
+    kernel times out): a training step stops before Adam, an inference gives NaN and its
+    caller or the next call raises; once reported, the same calls work again."""
+    rng = np.random.default_rng(6)
+    B, H, W, cin = 1, 16, 16, 8
+    net = UNet(cin, seed=2, widths=(16, 32, 64))
+    x, t = _sample(rng, B, cin, H, W)
+    xd, td = torch.from_numpy(x).cuda(), torch.from_numpy(t.reshape(-1, 3).astype(np.float32)).cuda()
+    args = (xd.data_ptr(), td.data_ptr(), B, H, W)
+    y0 = net.forward(xd.data_ptr(), B, H, W).clone()
+    loss0 = net.loss_grad(*args)
+    p0, backward = net.get_params(), net._backward
+
+    def failing(b):
+        backward(b)
+        assert M.lib.maf_nn_flag_timeout(net._stream()) == 0
+
+    net._backward = failing
+    for call in (lambda: net.loss_grad(*args), lambda: net.train_step(*args, 1e-3)):
+        with pytest.raises(M.MafError) as e:
+            call()
+        assert e.value.code == 5
+    net._backward = backward
+    assert np.array_equal(net.get_params(), p0) and net.step_count == 0
+    assert net.loss_grad(*args) == loss0
+
+    pool = M.lib.maf_nn_pool
+    try:  # a convolution of an inference fails
+        M.lib.maf_nn_pool = lambda *a: M.lib.maf_nn_flag_timeout(net._stream()) or pool(*a)
+        y = net.forward(xd.data_ptr(), B, H, W)
+    finally:
+        M.lib.maf_nn_pool = pool
+    assert torch.isnan(y).all()
+    with pytest.raises(M.MafError):
+        net.forward(xd.data_ptr(), B, H, W)
+    assert torch.equal(net.forward(xd.data_ptr(), B, H, W), y0)
+    net.check()
+    a = torch.ones((8, 8), dtype=torch.bfloat16, device="cuda")
+    c = torch.zeros((8, 8), dtype=torch.float32, device="cuda")
+    gemm = lambda: M.lib.maf_bf16_gemm(a.data_ptr(), 8, a.data_ptr(), 8, c.data_ptr(), 8, 8, 8, 8, net._stream())
+    assert gemm() == 0 and M.lib.maf_nn_flag_timeout(net._stream()) == 0 and gemm() == 5 and gemm() == 0
