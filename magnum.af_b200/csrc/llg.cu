@@ -162,10 +162,11 @@ struct KUnion {
 };
 
 // vmax <- max(vmax, |err / sc|), NaN-propagating.  The FP64 division is skipped where the
-// quotient, rounded, cannot exceed vmax (the finalize kernels are bound on FP64 division
-// and square root as much as on HBM); a NaN fails the comparison and is divided.
+// quotient is certainly below vmax (the finalize kernels are bound on FP64 division and
+// square root as much as on HBM).  The comparison is strict, so that 0 / 0 (atol = 0, a cell
+// without m) and inf / inf are divided and give NaN, as a NaN does, whose comparison fails.
 __device__ __forceinline__ void err_max(double err, double sc, double& vmax) {
-    if (!(fabs(err) <= vmax * sc * (1.0 - 1e-12))) vmax = nanmax(vmax, fabs(err / sc));
+    if (!(fabs(err) < vmax * sc * (1.0 - 1e-12))) vmax = nanmax(vmax, fabs(err / sc));
 }
 
 __device__ __forceinline__ double fin_one(double sumbk, double e, int form, double mi, double atol, double rtol,

@@ -77,3 +77,31 @@ def test_ensemble_chains_on_both_sides_of_their_bound(members, prec):
     for (_, sb), (it, ss) in zip(*made):
         it.steps(ss, 5)
         assert np.array_equal(np.asarray(sb.m), np.asarray(ss.m))
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32_field"])
+@pytest.mark.parametrize("shape", [(9, 7, 1), (10, 7, 1), (300, 301, 1), (301, 301, 1)])
+def test_error_norm_is_nan_where_a_quotient_is(shape, prec):
+    """The norm's quotients err / (atol + rtol |m|) in meshes of odd and even cell counts (two
+    kernels): 0 / 0 in empty cells with atol = 0, and a NaN in one cell, wherever it lies."""
+    gm, _ = mesh_pair(*shape, 3e-9, 3e-9, 3e-9)
+    terms = _terms()[0]
+    m0 = random_m(shape, 5)
+    s = M.State(gm, 8e5, m0, precision=prec)
+    for atol in (1e-6, 0.0):
+        assert np.isfinite(M.LLGIntegrator(0.1, terms, "RKF45", atol=atol).rk_attempt(s, "RKF45", 2e-14)[1])
+    holes = m0.copy()
+    holes[::3, 1::2] = 0.0
+    s = M.State(gm, 8e5, holes, precision=prec)
+    llg = M.LLGIntegrator(0.1, terms, "RKF45", atol=0.0)
+    assert np.isnan(llg.rk_attempt(s, "RKF45", 2e-14)[1])
+    with pytest.raises(M.MafError) as e:
+        llg.step(s)
+    assert e.value.code == 4
+    last = m0.copy()
+    for cell in ((0, 0, 0), (shape[0] - 1, shape[1] - 1, 0), (shape[0] // 2, shape[1] // 2, 0)):
+        zeeman = np.zeros(shape + (3,))
+        zeeman[cell] = np.nan
+        s = M.State(gm, 8e5, last, precision=prec)
+        err = M.LLGIntegrator(0.1, terms + [M.ExternalField(zeeman)], "RKF45").rk_attempt(s, "RKF45", 2e-14)[1]
+        assert np.isnan(err)
