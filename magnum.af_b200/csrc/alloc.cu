@@ -8,8 +8,12 @@
 // The pool belongs to this library (the device's default pool and its settings are left
 // alone) and is used on one internal stream: an allocation is synchronised before it is
 // handed out, and a buffer goes back only after the device has finished all work that may
-// use it (as cudaFree waits), so the buffers may be used on any stream and from any thread.
+// use it, so the buffers may be used on any stream and from any thread.  That wait is a
+// cudaFree of a small block (which waits for all streams of the device, 5 us with the next
+// block at hand), not cudaDeviceSynchronize: a thread may free while another one captures a
+// graph in thread-local mode, where the latter is not allowed and spoils the capture.
 #include <mutex>
+#include <vector>
 
 #include "engine.hpp"
 
@@ -20,17 +24,21 @@ namespace {
 constexpr size_t kPoolMax = 128u << 20;
 constexpr unsigned long long kPoolKeep = 256ull << 20;
 constexpr int kMaxOrdinals = 64;
+constexpr size_t kSmall = 64;
 
 struct DevicePool {
     cudaMemPool_t pool = nullptr;
     cudaStream_t stream = nullptr;
+    void* anchor = nullptr;        // keeps the driver's block of small allocations (340 us to make, 280 to unmake)
     bool failed = false;
+    std::mutex mu;
+    std::vector<void*> pending;    // buffers whose device could not be waited for yet
 };
 
 // The device's pool, made on first use; null when there is none (the caller uses cudaMalloc).
 DevicePool* device_pool() {
     static std::mutex mu;
-    static DevicePool pools[kMaxOrdinals];
+    static DevicePool* pools = new DevicePool[kMaxOrdinals];  // (outlives the buffers of static objects)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxOrdinals) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
@@ -41,7 +49,8 @@ DevicePool* device_pool() {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = dev;
         unsigned long long keep = kPoolKeep;
-        p.failed = cudaMemPoolCreate(&p.pool, &props) != cudaSuccess ||
+        p.failed = cudaMalloc(&p.anchor, kSmall) != cudaSuccess ||
+                   cudaMemPoolCreate(&p.pool, &props) != cudaSuccess ||
                    cudaMemPoolSetAttribute(p.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess ||
                    cudaStreamCreateWithFlags(&p.stream, cudaStreamNonBlocking) != cudaSuccess;
         if (p.failed) cudaGetLastError();
@@ -49,21 +58,60 @@ DevicePool* device_pool() {
     return p.failed ? nullptr : &p;
 }
 
+// Waits for all work of the device as cudaFree does; false where cudaFree is not allowed (a
+// thread that is capturing itself).
+bool wait_device() {
+    void* w = nullptr;
+    if (cudaMalloc(&w, kSmall) == cudaSuccess && cudaFree(w) == cudaSuccess) return true;
+    cudaGetLastError();
+    return false;
+}
+
+// Gives ptr (may be null) and the pending buffers back to the pool, or keeps them pending.
+void give_back(DevicePool& p, void* ptr) {
+    std::vector<void*> list;
+    {
+        std::lock_guard<std::mutex> lock(p.mu);
+        list.swap(p.pending);
+    }
+    if (ptr) list.push_back(ptr);
+    if (list.empty()) return;
+    if (wait_device()) {
+        for (void* q : list)
+            if (cudaFreeAsync(q, p.stream) != cudaSuccess) {
+                cudaGetLastError();
+                cudaFree(q);  // not the pool's
+            }
+        return;
+    }
+    std::lock_guard<std::mutex> lock(p.mu);
+    p.pending.insert(p.pending.end(), list.begin(), list.end());
+}
+
 }  // namespace
 
 void* dev_alloc(size_t n) {
     void* ptr = nullptr;
-    if (n <= kPoolMax) {
-        if (DevicePool* p = device_pool()) {
-            if (cudaMallocFromPoolAsync(&ptr, n, p->pool, p->stream) == cudaSuccess &&
-                cudaStreamSynchronize(p->stream) == cudaSuccess)
-                return ptr;
-            // no memory for the pool to grow, or a context that was reset under it
-            cudaGetLastError();
-            ptr = nullptr;
+    DevicePool* p = device_pool();
+    if (p && n <= kPoolMax) {
+        if (cudaMallocFromPoolAsync(&ptr, n, p->pool, p->stream) == cudaSuccess) {
+            if (cudaStreamSynchronize(p->stream) == cudaSuccess) return ptr;
+            cudaFreeAsync(ptr, p->stream);
         }
+        // no memory for the pool to grow, or a context that was reset under it
+        cudaGetLastError();
+        ptr = nullptr;
     }
-    MAF_CUDA(cudaMalloc(&ptr, n));
+    cudaError_t e = cudaMalloc(&ptr, n);
+    if (e == cudaErrorMemoryAllocation && p) {  // what the pool keeps may be enough
+        cudaGetLastError();
+        give_back(*p, nullptr);
+        cudaStreamSynchronize(p->stream);
+        cudaMemPoolTrimTo(p->pool, 0);
+        e = cudaMalloc(&ptr, n);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    MAF_CUDA(e);
     return ptr;
 }
 
@@ -80,16 +128,10 @@ void dev_free(void* ptr, size_t n) {
         return;
     }
     if (at.device != dev) cudaSetDevice(at.device);
-    // (a device that cannot be synchronised, as inside a capture, keeps the buffer)
-    if (cudaDeviceSynchronize() == cudaSuccess) {
-        DevicePool* p = device_pool();
-        if (!p || cudaFreeAsync(ptr, p->stream) != cudaSuccess) {
-            cudaGetLastError();
-            cudaFree(ptr);  // not the pool's
-        }
-    } else {
-        cudaGetLastError();
-    }
+    if (DevicePool* p = device_pool())
+        give_back(*p, ptr);
+    else
+        cudaFree(ptr);
     if (at.device != dev) cudaSetDevice(dev);
 }
 
