@@ -513,16 +513,9 @@ template <typename R> void FusedBatch::Chain::build(cudaStream_t st) {
     MAF_CUDA(cudaEventCreateWithFlags(&fork_ev, cudaEventDisableTiming));
     n_el3 = (int)we.size();
     n_cell = (int)wn.size();
-    // (only raised: another chain's launches may need the larger one)
-    auto smem_attr = [](auto k, size_t bytes) {
-        cudaFuncAttributes a;
-        MAF_CUDA(cudaFuncGetAttributes(&a, k));
-        if (bytes > 32 * 1024 && (int)bytes > a.maxDynamicSharedSizeBytes)
-            MAF_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    };
-    smem_attr(kb_xfwd<R>, s_xfwd);
-    smem_attr(kb_conv<R>, s_conv);
-    smem_attr(kb_xinv<R>, s_xinv);
+    raise_smem((const void*)kb_xfwd<R>, s_xfwd);
+    raise_smem((const void*)kb_conv<R>, s_conv);
+    raise_smem((const void*)kb_xinv<R>, s_xinv);
     MAF_CUDA(cudaStreamSynchronize(st));
 }
 

@@ -22,6 +22,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <mutex>
 
 #include "engine.hpp"
 #include "epilogue.cuh"
@@ -377,10 +378,17 @@ __global__ void k_d2f(const double* __restrict__ a, float* __restrict__ b, int64
 // ---------------------------------------------------------------------------
 // launch helpers
 // ---------------------------------------------------------------------------
-template <typename K> static void set_smem(K kernel, size_t bytes) {
+void raise_smem(const void* kernel, size_t bytes) {
     // opt in above 32 KB: the 48 KB default also has to hold the static shared memory
-    if (bytes > 32 * 1024) MAF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    if (bytes <= 32 * 1024) return;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    cudaFuncAttributes a;
+    MAF_CUDA(cudaFuncGetAttributes(&a, kernel));
+    if ((size_t)a.maxDynamicSharedSizeBytes < bytes)
+        MAF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
+template <typename K> static void set_smem(K kernel, size_t bytes) { raise_smem((const void*)kernel, bytes); }
 
 
 template <typename R>

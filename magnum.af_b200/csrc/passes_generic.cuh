@@ -24,6 +24,11 @@ inline int pick_nb(int L, int target, int ncols, int nbmax) {
     return nb < nc ? nb : nc;
 }
 
+// Opts a kernel in to `bytes` of dynamic shared memory (fields.cu).  Only ever raised: the
+// attribute belongs to the process, and another thread may be about to launch the same kernel
+// for a longer transform.
+void raise_smem(const void* kernel, size_t bytes);
+
 template <typename R> inline int tile_target() { return sizeof(R) == 4 ? 8192 : 4096; }
 
 // x-forward: rows of n_in reals (times Ms) zero-padded to Px = 2*Lc, real FFT by

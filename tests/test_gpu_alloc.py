@@ -1,5 +1,6 @@
 """The library's device memory: buffers given back while another thread captures a
-graph, the surplus of the pool, and its memory for a large buffer when the device is full."""
+graph, the surplus of the pool, its memory for a large buffer when the device is full,
+and objects made, used and dropped by several threads at once."""
 import threading
 
 import numpy as np
@@ -64,3 +65,32 @@ def test_pool_gives_its_memory_to_a_large_buffer():
         del fill
         torch.cuda.empty_cache()
     _stepped((64, 64, 1))
+
+
+def test_threads_make_use_and_drop_objects():
+    shapes = [(64, 48, 1), (33, 20, 3), (100, 25, 1), (300, 100, 2)]  # tensors on kernels of 1 to 64 KB
+
+    def run(shape, seed):
+        st = M.State(M.Mesh(*shape, 3e-9, 3e-9, 3e-9), 8e5, random_m(shape, seed))
+        llg = M.LLGIntegrator(0.1, [M.DemagField(st.mesh), M.ExchangeField(1.3e-11)], "RKF45", hmax=1e-14)
+        llg.steps(st, 5)
+        return np.asarray(st.m).copy()
+
+    want = {(i, k): run(s, k) for i, s in enumerate(shapes) for k in range(3)}
+    bad = []
+
+    def worker(i):
+        for rep in range(4):
+            for k in range(3):
+                try:
+                    if not np.array_equal(run(shapes[i], k), want[i, k]):
+                        bad.append((i, k, rep))
+                except M.MafError as e:
+                    bad.append((i, k, rep, str(e)))
+
+    threads = [threading.Thread(target=worker, args=(i,)) for i in range(len(shapes)) for _ in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
