@@ -25,20 +25,27 @@ def _stepped(shape, seed=1, stream=None):
 
 
 def test_buffers_dropped_while_another_thread_captures():
-    made = [_stepped((512, 512, 2)) for _ in range(6)]  # 100 MB of pool memory each
     x = torch.ones(1000, device="cuda")
+    graphs, s = [], torch.cuda.Stream()
+
+    def capture(meanwhile):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
+            y = x + 1
+            t = threading.Thread(target=meanwhile)
+            t.start()
+            t.join()
+            y = 2 * y
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.all(y == 4)
+        graphs.append((g, y))
+
+    capture(lambda: None)  # what the first capture of a process allocates is not counted
+    made = [_stepped((512, 512, 2)) for _ in range(6)]  # 100 MB of pool memory each
     torch.cuda.synchronize()
     free0 = torch.cuda.mem_get_info()[0]
-    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
-    with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
-        y = x + 1
-        t = threading.Thread(target=made.clear)
-        t.start()
-        t.join()
-        y = 2 * y
-    g.replay()
-    torch.cuda.synchronize()
-    assert torch.all(y == 4)
+    capture(made.clear)
     _stepped((8, 8, 1))  # an object made and dropped afterwards gives back what was pending
     torch.cuda.synchronize()
     # 6 x 126 MB came back but for the 256 MB that the pool keeps (and torch's graph memory)
