@@ -3,7 +3,9 @@
 // 200x120x10 cells, 2.5 of them kernels) and of a new state's first step.  Allocations of
 // up to kPoolMax bytes therefore come from a memory pool of the device that keeps up to
 // kPoolKeep unused bytes for the next object and gives the rest back to the driver at the
-// next synchronisation; larger ones are cudaMalloc's.
+// next synchronisation; larger ones are cudaMalloc's, and so are the buffers whose address
+// the application gets (DevBuf::alloc_own): pool memory has neither the IPC handles nor the
+// peer access of cudaMalloc memory.
 //
 // The pool belongs to this library (the device's default pool and its settings are left
 // alone) and is used on one internal stream: an allocation is synchronised before it is
@@ -77,11 +79,7 @@ void give_back(DevicePool& p, void* ptr) {
     if (ptr) list.push_back(ptr);
     if (list.empty()) return;
     if (wait_device()) {
-        for (void* q : list)
-            if (cudaFreeAsync(q, p.stream) != cudaSuccess) {
-                cudaGetLastError();
-                cudaFree(q);  // not the pool's
-            }
+        for (void* q : list) cudaFreeAsync(q, p.stream);
         return;
     }
     std::lock_guard<std::mutex> lock(p.mu);
@@ -90,12 +88,16 @@ void give_back(DevicePool& p, void* ptr) {
 
 }  // namespace
 
-void* dev_alloc(size_t n) {
+void* dev_alloc(size_t n, bool own, bool* pooled) {
     void* ptr = nullptr;
     DevicePool* p = device_pool();
-    if (p && n <= kPoolMax) {
+    *pooled = false;
+    if (p && !own && n <= kPoolMax) {
         if (cudaMallocFromPoolAsync(&ptr, n, p->pool, p->stream) == cudaSuccess) {
-            if (cudaStreamSynchronize(p->stream) == cudaSuccess) return ptr;
+            if (cudaStreamSynchronize(p->stream) == cudaSuccess) {
+                *pooled = true;
+                return ptr;
+            }
             cudaFreeAsync(ptr, p->stream);
         }
         // no memory for the pool to grow, or a context that was reset under it
@@ -115,8 +117,8 @@ void* dev_alloc(size_t n) {
     return ptr;
 }
 
-void dev_free(void* ptr, size_t n) {
-    if (n > kPoolMax) {
+void dev_free(void* ptr, bool pooled) {
+    if (!pooled) {
         cudaFree(ptr);
         return;
     }
@@ -128,10 +130,7 @@ void dev_free(void* ptr, size_t n) {
         return;
     }
     if (at.device != dev) cudaSetDevice(at.device);
-    if (DevicePool* p = device_pool())
-        give_back(*p, ptr);
-    else
-        cudaFree(ptr);
+    if (DevicePool* p = device_pool()) give_back(*p, ptr);
     if (at.device != dev) cudaSetDevice(dev);
 }
 

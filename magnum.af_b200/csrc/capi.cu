@@ -335,7 +335,7 @@ double rk_attempt(maf_llg_s* l, maf_state_s* st, const Scheme& sch, double dt, i
     double* const mstage64 = kbuf + np * sch.stages;
     float* const mstage32 = f32 ? reinterpret_cast<float*>(mstage64 + np) : nullptr;
     float* const mother32 = f32 ? mstage32 + np : nullptr;
-    l->mcand.ensure(sizeof(double) * n3);
+    l->mcand.ensure_own(sizeof(double) * n3);
     ensure_finalize_scratch(l->partials, s.stream);
     l->err.ensure();
     auto terms = raw_terms(l->terms);
@@ -455,8 +455,9 @@ double llg_energy(maf_llg_s* l, maf_state_s* st) {
     return e;
 }
 
-void upload(DevBuf& b, const double* host, size_t n, cudaStream_t st) {
-    b.alloc(sizeof(double) * n);
+void upload(DevBuf& b, const double* host, size_t n, cudaStream_t st, bool own = false) {
+    if (own) b.alloc_own(sizeof(double) * n);
+    else b.alloc(sizeof(double) * n);
     MAF_CUDA(cudaMemcpyAsync(b.p, host, sizeof(double) * n, cudaMemcpyHostToDevice, st));
     MAF_CUDA(cudaStreamSynchronize(st));
 }
@@ -538,7 +539,7 @@ void stoch_buffers(maf_stoch_s* h, maf_state_s* st) {
     for (int i = 0; i < stages; ++i) h->k[i].ensure(sizeof(double) * n3);
     h->mstage64.ensure(sizeof(double) * n3);
     if (st->s.precision == PREC_FP32_FIELD) h->mstage32.ensure(sizeof(float) * n3);
-    h->mcand.ensure(sizeof(double) * n3);
+    h->mcand.ensure_own(sizeof(double) * n3);
     ensure_finalize_scratch(h->partials, st->s.stream);
     h->errbuf.ensure(sizeof(double) * 4);
 }
@@ -1086,7 +1087,7 @@ int maf_state_create(maf_state* out, int nx, int ny, int nz, double dx, double d
         MAF_CUDA(cudaStreamCreateWithFlags(&s.stream, cudaStreamNonBlocking));
         s.own_stream = true;
         const int64_t N = s.md.N();
-        upload(s.m64, m_host, 3 * N, s.stream);
+        upload(s.m64, m_host, 3 * N, s.stream, true);
         // normalize (state.cpp:92) and count zero-norm cells
         h->scratch.ensure(sizeof(unsigned long long) * 2);
         MAF_CUDA(cudaMemsetAsync(h->scratch.p, 0, sizeof(unsigned long long), s.stream));
@@ -2309,7 +2310,7 @@ std::unique_ptr<maf_state_s> make_image(const maf_state_s& tmpl, cudaStream_t st
     s.stream = st;
     s.own_stream = false;
     const int64_t N = s.md.N();
-    s.m64.alloc(sizeof(double) * 3 * N);
+    s.m64.alloc_own(sizeof(double) * 3 * N);
     if (t.has_Ms_field) {
         s.Msf64.alloc(sizeof(double) * N);
         MAF_CUDA(cudaMemcpyAsync(s.Msf64.p, t.Msf64.p, sizeof(double) * N, cudaMemcpyDeviceToDevice, st));

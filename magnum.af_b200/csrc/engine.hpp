@@ -14,32 +14,38 @@ namespace mafb {
 
 enum Precision : int { PREC_FP64 = 0, PREC_FP32_FIELD = 1 };
 
-// Device memory (alloc.cu): dev_alloc throws, dev_free(p, the size asked for) waits for
-// the device's work, as cudaFree does.
-void* dev_alloc(size_t n);
-void dev_free(void* p, size_t n);
+// Device memory (alloc.cu): dev_alloc throws and says whether the memory is the pool's (never
+// when `own`); dev_free waits for the device's work, as cudaFree does.
+void* dev_alloc(size_t n, bool own, bool* pooled);
+void dev_free(void* p, bool pooled);
 
-// Owning device allocation.
+// Owning device allocation.  alloc_own / ensure_own: for a buffer whose address the
+// application may get (a state's m and the candidates that are swapped with it), an
+// allocation of its own (cudaMalloc), so that IPC handles and peer access work on it.
 struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
+    bool pooled = false;
     DevBuf() = default;
     explicit DevBuf(size_t n) { alloc(n); }
     DevBuf(const DevBuf&) = delete;
     DevBuf& operator=(const DevBuf&) = delete;
-    DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes) { o.p = nullptr; o.bytes = 0; }
+    DevBuf(DevBuf&& o) noexcept : p(o.p), bytes(o.bytes), pooled(o.pooled) { o.p = nullptr; o.bytes = 0; }
     DevBuf& operator=(DevBuf&& o) noexcept {
-        if (this != &o) { release(); p = o.p; bytes = o.bytes; o.p = nullptr; o.bytes = 0; }
+        if (this != &o) { release(); p = o.p; bytes = o.bytes; pooled = o.pooled; o.p = nullptr; o.bytes = 0; }
         return *this;
     }
     ~DevBuf() { release(); }
-    void alloc(size_t n) {
+    void alloc(size_t n) { get(n, false); }
+    void alloc_own(size_t n) { get(n, true); }
+    void ensure(size_t n) { if (bytes < n) alloc(n); }
+    void ensure_own(size_t n) { if (bytes < n) alloc_own(n); }
+    void release() { if (p) dev_free(p, pooled); p = nullptr; bytes = 0; }
+    void get(size_t n, bool own) {
         release();
-        if (n) p = dev_alloc(n);
+        if (n) p = dev_alloc(n, own, &pooled);
         bytes = n;
     }
-    void ensure(size_t n) { if (bytes < n) alloc(n); }
-    void release() { if (p) dev_free(p, bytes); p = nullptr; bytes = 0; }
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 

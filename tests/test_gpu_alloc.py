@@ -1,6 +1,7 @@
 """The library's device memory: buffers given back while another thread captures a
 graph, the surplus of the pool, its memory for a large buffer when the device is full,
-and objects made, used and dropped by several threads at once."""
+objects made, used and dropped by several threads at once, and the handle of a state's m."""
+import ctypes as C
 import threading
 
 import numpy as np
@@ -101,3 +102,18 @@ def test_threads_make_use_and_drop_objects():
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("shape", [(8, 6, 1), (300, 200, 3)])
+def test_device_m_has_an_ipc_handle(shape):
+    """State.device_m points to an allocation of its own (cudaMalloc), before and after steps."""
+    rt = C.CDLL("libcudart.so.12")  # torch's; the context is shared
+    st = M.State(M.Mesh(*shape, 3e-9, 3e-9, 3e-9), 8e5, random_m(shape, 2))
+    terms = [M.ExchangeField(1.3e-11)]
+    llg = M.LLGIntegrator(0.1, terms, "RKF45", hmax=1e-14)
+    it = M.Stochastic_LLG(0.1, 300.0, 1e-14, st, terms, "Heun", seed=1)
+    for use in (lambda: None, lambda: llg.step(st), lambda: it.step(st), lambda: llg.steps(st, 2)):
+        use()
+        st.mean_m()  # waits for the state's stream
+        handle = (C.c_char * 64)()
+        assert rt.cudaIpcGetMemHandle(handle, C.c_void_p(st.device_m())) == 0
