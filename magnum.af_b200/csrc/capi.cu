@@ -1,5 +1,6 @@
 // C ABI of the magnum.af B200 library (declared in include/maf_b200.h).
 #include <algorithm>
+#include <bitset>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -212,21 +213,72 @@ struct maf_state_s {
     }
 };
 
-// A pinned host double that kernels write directly: read after the stream's
-// synchronisation, without a copy of its own (a copy to pageable memory was another
-// 8-10 us per step).
+// Pinned host doubles that kernels write directly: read after the stream's synchronisation,
+// without a copy of their own (a copy to pageable memory was another 8-10 us per step).
+// cudaHostAlloc takes 1.4-2.7 ms and cudaFreeHost 0.4 ms, several times the first step of a
+// small state (100x25 cells: 3.0 ms with a word of its own, 0.4 with these), so the words of
+// all integrators come from pages of kWords; a page that no word is taken from is
+// freed unless it is the last one.
+class HostWords {
+  public:
+    static HostWords& get() {
+        static HostWords* w = new HostWords;  // (outlives the integrators of static objects)
+        return *w;
+    }
+    double* take() {
+        std::lock_guard<std::mutex> lock(mu_);
+        for (Page& g : pages_)
+            if (!g.used.all())
+                for (int i = 0; i < kWords; ++i)
+                    if (!g.used[i]) {
+                        g.used[i] = true;
+                        return g.p + i;
+                    }
+        void* p = nullptr;
+        MAF_CUDA(cudaHostAlloc(&p, sizeof(double) * kWords, cudaHostAllocMapped | cudaHostAllocPortable));
+        pages_.push_back(Page{static_cast<double*>(p), {}});
+        pages_.back().used[0] = true;
+        return pages_.back().p;
+    }
+    void give(double* w) {
+        std::lock_guard<std::mutex> lock(mu_);
+        auto g = page(w);
+        g->used[w - g->p] = false;
+        if (g->used.none() && pages_.size() > 1) {
+            cudaFreeHost(g->p);
+            pages_.erase(g);
+        }
+    }
+    double* device(double* w) {
+        std::lock_guard<std::mutex> lock(mu_);
+        auto g = page(w);
+        void* d = nullptr;
+        MAF_CUDA(cudaHostGetDevicePointer(&d, g->p, 0));
+        return static_cast<double*>(d) + (w - g->p);
+    }
+
+  private:
+    static constexpr int kWords = 512;  // 4 KB
+    struct Page {
+        double* p;
+        std::bitset<kWords> used;
+    };
+    std::vector<Page>::iterator page(double* w) {
+        return std::find_if(pages_.begin(), pages_.end(), [&](const Page& g) { return w >= g.p && w < g.p + kWords; });
+    }
+    std::mutex mu_;
+    std::vector<Page> pages_;
+};
+
+// One of them.
 struct HostWord {
     double* p = nullptr;
     HostWord() = default;
     HostWord(const HostWord&) = delete;
     HostWord& operator=(const HostWord&) = delete;
-    ~HostWord() { if (p) cudaFreeHost(p); }
-    void ensure() { if (!p) MAF_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&p), sizeof(double), cudaHostAllocMapped | cudaHostAllocPortable)); }
-    double* device() const {
-        void* d = nullptr;
-        MAF_CUDA(cudaHostGetDevicePointer(&d, p, 0));
-        return static_cast<double*>(d);
-    }
+    ~HostWord() { if (p) HostWords::get().give(p); }
+    void ensure() { if (!p) p = HostWords::get().take(); }
+    double* device() const { return HostWords::get().device(p); }
 };
 
 struct maf_term_s {
@@ -244,7 +296,7 @@ struct maf_llg_s {
     Controller ctrl;
     double h = 1.01e-15;
     bool dissipation_only = false;
-    // the k's and one stage buffer in one allocation (rk_work: each allocation above 2 MB costs
+    // the k's and one stage buffer in one allocation (each allocation above 2 MB costs
     // 0.5-1 ms of a first step); the stages' m goes to that stage buffer and mcand in turn (an
     // epilogue reads one and writes the other), its FP32 copy to two buffers likewise; mcand
     // then takes the candidate and is swapped with the state's m

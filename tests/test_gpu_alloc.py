@@ -117,3 +117,28 @@ def test_device_m_has_an_ipc_handle(shape):
         st.mean_m()  # waits for the state's stream
         handle = (C.c_char * 64)()
         assert rt.cudaIpcGetMemHandle(handle, C.c_void_p(st.device_m())) == 0
+
+
+def test_many_integrators_keep_their_own_error_norm():
+    """More integrators at once than one page of pinned words holds (512), some dropped and
+    made anew in between: each reads its own norm."""
+    st = M.State(M.Mesh(6, 5, 1, 3e-9, 3e-9, 3e-9), 8e5, random_m((6, 5, 1), 3))
+    term = M.ExchangeField(1.3e-11)
+
+    def make(i):
+        return M.LLGIntegrator(0.1, [term], "RKF45", atol=1e-6 * (i + 1))
+
+    def norm(llg):
+        return llg.rk_attempt(st, "RKF45", 2e-14)[1]
+
+    want = [norm(make(i)) for i in range(1100)]  # one after the other
+    assert len(set(want)) == len(want)
+    made = [make(i) for i in range(1100)]
+    assert [norm(llg) for llg in made] == want
+    for i in list(range(0, 1100, 3)) + list(range(512, 1024)):
+        made[i] = None
+    for i in range(1100):
+        if made[i] is None:
+            made[i] = make(i)
+            assert norm(made[i]) == want[i]
+    assert [norm(llg) for llg in made] == want
