@@ -218,6 +218,10 @@ int maf_term_demag_set_tune(maf_term t, const int choices[3]);
  * maf_stoch_batch_set_fused use) instead of the compile-time ones; on = 0 restores the default.  Both
  * compute the same field up to rounding (no counterpart in the reference). */
 int maf_term_demag_set_generic(maf_term t, int on);
+/* The transform lengths (x, y, z) that a DemagField of nx x ny x nz cells runs with by default: twice the mesh
+ * (1 along z for a single layer), or longer where a padded length has compile-time kernels and pays (no counterpart in
+ * the reference).  Needs no device. */
+int maf_demag_lengths(int nx, int ny, int nz, int lengths[3]);
 /* maf_llg_heff_device with a CUDA event after every pass kernel: synchronises and
  * returns each pass's duration in ms (the instrumentation LLGIntegrator::time_heff,
  * llg_integrator.cpp:11-16, and the per-term timers of field_term.hpp:49-86 provide,

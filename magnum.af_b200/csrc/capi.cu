@@ -1989,6 +1989,13 @@ int maf_term_demag_set_tune(maf_term t, const int choices[3]) {
     });
 }
 
+int maf_demag_lengths(int nx, int ny, int nz, int lengths[3]) {
+    return guarded([&] {
+        check(lengths && nx > 0 && ny > 0 && nz > 0, "maf_demag_lengths: bad argument");
+        demag_lengths(nx, ny, nz, lengths);
+    });
+}
+
 int maf_term_demag_set_generic(maf_term t, int on) {
     return guarded([&] {
         check(t && t->t->kind == TK_DEMAG && t->t->demag && !t->t->demag_pbc(),

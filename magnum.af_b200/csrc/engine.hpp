@@ -168,6 +168,10 @@ struct TuneChoice {
     int generic = 0;    // 1: the run-time-plan kernels for every pass (as the batched passes run)
 };
 
+// Transform lengths (x, y, z) that a mesh's field is evaluated with: twice the mesh, or padded
+// (fields.cu has the rule).
+void demag_lengths(int nx, int ny, int nz, int out[3]);
+
 // Transform lengths, buffers and tensor that an evaluation runs with.
 template <typename R> struct DemagPlan {
     int Px = 0, Py = 0, Pz = 0, nxh = 0, pitch = 0;
@@ -234,9 +238,8 @@ class Demag {
     MeshDims md_;
     bool pbc_ = false;
     int pitch_;  // complex row pitch of the half spectrum (>= nxh)
-    // Zero padding to any length of at least 2n - 1 gives the same linear convolution, so
-    // a mesh whose doubled sizes have no compile-time kernels is padded to the next lengths
-    // that have them; the tensor at those lengths is made from Nred64_ on first use.
+    // The lengths of demag_lengths; where they differ from twice the mesh, the tensor at them is
+    // made from Nred64_ on first use.
     bool padded_ = false;
     int pad_x_ = 0, pad_y_ = 0, pad_z_ = 0;
     DevBuf Nred64_, Nred32_, Npad64_, Npad32_;

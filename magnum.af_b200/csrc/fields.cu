@@ -457,6 +457,42 @@ static int ct_length(const int* list, int n) {
     return 0;
 }
 
+// Zero padding to any length of at least 2n - 1 gives the same linear convolution, so an axis
+// whose doubled size has no compile-time kernel is padded to the next length that has one.  All
+// axes are padded or, when one has no such length, none.  On 3-D meshes the y and z passes run
+// over the padded x spectrum, so there x keeps its own length (on the run-time-plan kernel)
+// where padding it costs the other passes more than it saves: when its spectrum grows by more
+// than 1.6, or by more than 1.25 beside a y transform of 4096 points (whose CTAs take one or
+// two columns, part of a sector per row); unless the padded spectrum has up to 2^16 values,
+// where launches dominate.  Field times in us on B200, FP64 / FP32, x at its own length and
+// padded (y and z padded in both), with x's growth:
+//      1 x 1024 x 64  8.5     72 / 63     341 / 192
+//      8 x 512 x 64   1.89   148 / 102    166 / 94
+//      9 x 300 x 20   1.70    58 / 43      69 / 55
+//     10 x 500 x 30   1.55    96 / 68      87 / 67
+//    520 x 520 x 18   1.48  3318 / 1659  3260 / 1488
+//   1040 x 600 x 9    1.48  3082 / 1727  2571 / 1168
+//   1040 x 1040 x 9   1.48  8400 / 4507  12099 / 5370   (4096)
+//   1100 x 1100 x 2   1.40  2184 / 1122  2389 / 1009    (4096)
+//    600 x 1040 x 9   1.28  4437 / 2370  5639 / 2490    (4096)
+//   1300 x 1300 x 4   1.18  5559 / 2880  4825 / 2017    (4096)
+//      6 x 60 x 6     2.43    29 / 27      21 / 20      (35 k values)
+//      1 x 256 x 4    8.5     23 / 21      35 / 28      (70 k values)
+// y and z padded (x as above) against their own lengths: 520 x 520 x 9 3034 / 1830 -> 1287 /
+// 607, 1040 x 1040 x 18 28650 / 14206 -> 20081 / 10563, 1024 x 1 x 16 31 / 25 -> 33 / 26.
+// 2-D meshes, both padded against both own: 1040 x 1000 864 / 546 -> 316 / 169, 1 x 1000 71 /
+// 60 -> 32 / 21.
+void demag_lengths(int nx, int ny, int nz, int out[3]) {
+    const int own[3] = {2 * nx, 2 * ny, nz == 1 ? 1 : 2 * nz};
+    const int pad[3] = {2 * ct_length(kCtX, nx), ct_length(nz == 1 ? kCtY2 : kCtY3, 2 * ny - 1),
+                        nz == 1 ? 1 : ct_length(kCtZ, 2 * nz - 1)};
+    const bool padded = pad[0] && pad[1] && pad[2];
+    for (int a = 0; a < 3; ++a) out[a] = padded ? pad[a] : own[a];
+    if (!padded || nz == 1) return;
+    const int64_t nxh = pad[0] / 2 + 1;
+    if (nxh * pad[1] * pad[2] > (1 << 16) && nxh > (pad[1] == 4096 ? 1.25 : 1.6) * (nx + 1)) out[0] = own[0];
+}
+
 unsigned long long Demag::next_id() {
     static std::atomic<unsigned long long> n{0};
     return ++n;
@@ -476,10 +512,12 @@ Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, boo
     }
     // complex pitch: multiple of 4 so that tiles of 4 complex values start on 32 B
     pitch_ = (nxh() + 3) / 4 * 4;
-    pad_x_ = 2 * ct_length(kCtX, md.nx);
-    pad_y_ = md.nz == 1 ? ct_length(kCtY2, 2 * md.ny - 1) : ct_length(kCtY3, 2 * md.ny - 1);
-    pad_z_ = md.nz == 1 ? 1 : ct_length(kCtZ, 2 * md.nz - 1);
-    padded_ = pad_x_ && pad_y_ && pad_z_ && (pad_x_ != Px() || pad_y_ != Py() || pad_z_ != Pz());
+    int len[3];
+    demag_lengths(md.nx, md.ny, md.nz, len);
+    pad_x_ = len[0];
+    pad_y_ = len[1];
+    pad_z_ = len[2];
+    padded_ = pad_x_ != Px() || pad_y_ != Py() || pad_z_ != Pz();
     // validate all FFT lengths early
     make_fft_plan(Px() / 2, nullptr);
     make_fft_plan(Py(), nullptr);
@@ -757,8 +795,8 @@ template <typename R> void Demag::forward_conv(const R* m, const MsInfo& ms, cud
             } else {
                 set_smem(k_conv<R, false>, smem);
                 k_conv<R, false><<<grid, threads, smem, st>>>(s2, Nr, fp, ip, nz, (int64_t)Py_ * pitch,
-                                                              (int64_t)nz * Py_ * pitch, pitch, nxh_, nb, 1, ny,
-                                                              nz, nxh_, pop);
+                                                              (int64_t)nz * Py_ * pitch, pitch, nxh_, nb, 1, Py_ / 2,
+                                                              pl.Pz / 2, nxh_, pop);
             }
             MAF_LAUNCH_CHECK();
         }
@@ -805,8 +843,8 @@ template <typename R>
 void Demag::inverse_x_epilogue(const R* m, const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep,
                                cudaStream_t st, int* nblocks_out, PassMarks* marks) {
     const bool f64 = sizeof(R) == 8;
-    const int Lc = Px() / 2;
     const DemagPlan<R> pl = plan<R>(st);
+    const int Lc = pl.Px / 2;
     if (!pbc_ && !tune.generic) {
         const R scale = (R)(1.0 / ((double)pl.Px * pl.Py * pl.Pz));
         if (ct_xinv<R>(pl.s1, pl.pitch, pl.Px, tw_, md_.geom(), scale, m, ms, tl, ep, tune, st, nblocks_out)) {
@@ -827,8 +865,8 @@ void Demag::inverse_x_epilogue(const R* m, const MsInfo& ms, const TermList& tl,
     const size_t smem = sizeof(cplx_t<R>) * (size_t)3 * nbr * spad_len(Lc);
     const int64_t blocks = ceil_div(rows_pc, nbr);
     if (nblocks_out) *nblocks_out = (int)blocks;
-    const R scale = (R)(1.0 / ((double)Px() * Py() * Pz()));
-    const cplx_t<R>* tP = static_cast<const cplx_t<R>*>(tw_.get(Px(), f64));
+    const R scale = (R)(1.0 / ((double)pl.Px * pl.Py * pl.Pz));
+    const cplx_t<R>* tP = static_cast<const cplx_t<R>*>(tw_.get(pl.Px, f64));
     const Geom g = md_.geom();
     switch (ep.kind) {
         case EPI_H:

@@ -166,6 +166,7 @@ _SIGS = {
     "maf_nn_adam": (_I, [_P, _P, _P, _P, C.c_longlong, C.c_float, _I, _P]),
     "maf_stoch_batch_is_fused": (_I, [_P, C.POINTER(_I)]),
     "maf_term_demag_set_generic": (_I, [_P, _I]),
+    "maf_demag_lengths": (_I, [_I, _I, _I, C.POINTER(_I)]),
     "maf_string_create": (_I, [C.POINTER(_P), _P, C.POINTER(_P), _I, _I, _D, _P]),
     "maf_string_destroy": (_I, [_P]),
     "maf_string_step": (_I, [_P]),
@@ -532,6 +533,13 @@ class DemagField(FieldTerm):
     def tune_ex(self, choices):
         ch = (_I * 5)(*[int(c) for c in choices])
         _ck(lib.maf_term_demag_set_tune_ex(self._h, ch))
+
+    @staticmethod
+    def lengths(nx: int, ny: int, nz: int):
+        """The transform lengths (x, y, z) that a mesh of this size runs with by default."""
+        v = (_I * 3)()
+        _ck(lib.maf_demag_lengths(int(nx), int(ny), int(nz), v))
+        return tuple(v)
 
     def get_N(self, symmetric=False) -> np.ndarray:
         """Real-space Newell tensor [Px, Py, Pz, 6] (the reference's setup_N layout);

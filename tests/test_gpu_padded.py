@@ -53,6 +53,16 @@ def test_padded_field_vs_oracle_and_own_lengths(shape):
         assert rel_l2(got[False][2], got[True][2]) < tol
 
 
+# 3-D meshes where x keeps its own length beside padded y and z (DemagField.lengths): a spectrum
+# that would grow by more than 1.6, and by more than 1.25 beside 4096 points along y; one axis
+# padded, two, rows of odd length
+@pytest.mark.parametrize("shape", [(9, 130, 20), (3, 64, 33), (1, 200, 16), (6, 300, 12), (20, 1040, 2)])
+def test_own_x_length_beside_padded_axes(shape):
+    lengths = M.DemagField.lengths(*shape)
+    assert lengths[0] == 2 * shape[0] and lengths != tuple(2 * n for n in shape)
+    test_padded_field_vs_oracle_and_own_lengths(shape)
+
+
 @pytest.mark.parametrize("shape", [(100, 25, 1), (33, 20, 3), (50, 18, 10)])
 def test_padded_ms_field_and_parameter_fields(shape):
     gm = M.Mesh(*shape, 3e-9, 3e-9, 3e-9)
