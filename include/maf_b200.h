@@ -287,11 +287,12 @@ int maf_stoch_batch_create(maf_stoch_batch* out, const maf_stoch* integrators, c
 int maf_stoch_batch_destroy(maf_stoch_batch b);
 int maf_stoch_batch_steps(maf_stoch_batch b, int nsteps);
 /* Batched passes (no counterpart in the reference): with on = 1 the next capture records every pass of
- * a step as ONE launch for all members -- each CTA takes a (member, tile) pair from a device work table
- * and runs that tile of the member's run-time-plan kernel -- instead of one launch per member and pass.
+ * a step as one launch for all members of the same transform lengths -- each CTA takes a (member, tile) pair
+ * from a device work table and runs that tile of the member's pass kernel -- instead of one launch per member and
+ * pass.
  * Members must be 2-D meshes with one non-periodic DemagField, scalar parameters, one scheme, dt and
  * precision; a batch that does not qualify keeps the per-member graph.  A member's trajectory equals
- * the one its own integrator computes with maf_term_demag_set_generic(demag, 1), bit for bit.
+ * the one its own integrator computes, bit for bit.
  * maf_stoch_batch_is_fused reports whether the current graph runs the batched passes. */
 int maf_stoch_batch_set_fused(maf_stoch_batch b, int on);
 int maf_stoch_batch_is_fused(maf_stoch_batch b, int* active);
@@ -365,8 +366,8 @@ int maf_string_image(maf_string h, int i, maf_state* image);
  * array arguments are DEVICE pointers, NCHW: x [B][cin][H][W], y and target
  * [B][3][H][W].  Parameters: per layer W[cout][cin][3][3] then b[cout]. */
 typedef struct maf_cnn_s* maf_cnn;
-/* BF16 GEMM on the tensor cores (tcgen05.mma, FP32 accumulation in tensor memory), the contraction of
- * the warm-start network's convolutions (no counterpart in the reference): C[M][N] (FP32, row stride ldc)
+/* BF16 GEMM on the tensor cores (tcgen05.mma, FP32 accumulation in tensor memory; no counterpart in the
+ * reference): C[M][N] (FP32, row stride ldc)
  * = A[M][K] . B[N][K]^T with A, B BF16 device arrays whose K elements are contiguous (row strides lda,
  * ldb and K multiples of 8, rows 16-byte aligned).  Queued on stream (NULL: the legacy default stream);
  * returns after the stream finished it.  MAF_ERR_TIMEOUT if a bounded tensor-core wait gave up. */
@@ -384,38 +385,15 @@ int maf_nn_flag_timeout(void* stream);
  * queued on stream st (NULL: the legacy default stream) and returns without synchronising. */
 /* x [B][C][H][W] FP32 -> act [P][Cp] BF16 and m [P][3] FP32 (channels 0..2) */
 int maf_nn_input(const float* x, int B, int C, int H, int W, int Cp, void* act_bf16, float* m, void* st);
-/* 3x3 im2col (zero padding): col [P][9 Cp] (tap t = 3 (dy + 1) + (dx + 1)), or colT [9 Cp][P] */
-int maf_nn_im2col(const void* act, int B, int H, int W, int Cp, void* col, int transposed, void* st);
-/* maf_bf16_gemm without the synchronisation, and with the K range split over `splits` partial slabs
- * work [splits][M][N] summed in split order into C [M][N] */
-int maf_nn_gemm(const void* A, int lda, const void* B, int ldb, float* C, int ldc, int M, int N, int K, void* st);
-int maf_nn_gemm_splitk(const void* A, int lda, const void* B, int ldb, float* C, int M, int N, int K, int splits,
-                       float* work, void* st);
-/* out [P][C] = relu?(y + bias) (FP32) and, when outb, its BF16 copy [P][Cp] */
-int maf_nn_bias_act(const float* y, int ldy, const float* bias, long long P, int C, int relu, float* out,
-                    void* outb, int Cp, void* st);
 /* 2x2 average pooling [B][H][W][C] -> [B][H/2][W/2][C] (FP32 and BF16 [.][Cp]) and its backward
  * (din (+)= dout / 4 at the four children) */
 int maf_nn_pool(const float* in, int B, int H, int W, int C, float* out, void* outb, int Cp, void* st);
 int maf_nn_pool_bwd(const float* dout, int B, int H, int W, int C, float* din, int accumulate, void* st);
 /* out [B][H][W][Cp] BF16 = nearest-2x-upsampled a [B][H/2][W/2][Ca] | s [B][H][W][Cs]; backward:
- * da = sum of the four children of the first Ca channels of dcat [P][Cp], ds += the next Cs */
+ * da = sum of the four children of the first Ca channels of dcat [P][Cp], ds = the next Cs */
 int maf_nn_up_cat(const float* a, int Ca, const float* s, int Cs, int B, int H, int W, void* out, int Cp, void* st);
-int maf_nn_up_cat_bwd(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
-                      void* st);
-/* dY = dA * relu'(A) (FP32 [P][C], and BF16 [P][Cp]) */
-int maf_nn_relu_bwd(const float* dA, const float* A, long long P, int C, int relu, float* dY, void* dYb, int Cp,
-                    void* st);
-/* BF16 [R][C] -> [C][R] */
-int maf_nn_transpose(const void* in, long long R, int C, void* out, void* st);
-/* adjoint of im2col: dX [P][C] (+)= sum over taps of dcol [P][9 Cp] (first C channels) */
-int maf_nn_col2im(const float* dcol, int B, int H, int W, int Cp, int C, float* dX, int accumulate, void* st);
-/* db [C] = sum over pixels of dY [P][C] (fixed order) */
-int maf_nn_colsum(const float* dY, long long P, int C, float* db, void* st);
-/* FP32 weights W [Cout][9][Cin] -> BF16 Wb [Cout][9 Cp] and WtB [9 Cp][CoutP] (zero padded); the
- * weight gradient [Cout][9][Cin] from a GEMM result [Cout][9 Cp] */
-int maf_nn_wcast(const float* W32, int Cout, int Cin, int Cp, int CoutP, void* Wb, void* WtB, void* st);
-int maf_nn_wgrad(const float* g, int Cout, int Cin, int Cp, float* dW, void* st);
+int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
+                          void* st);
 /* 3x3 convolution as an implicit GEMM on the tensor cores (zero padding, no im2col):
  * out [P][ldo] (FP32, channels 0 .. N-1) = relu?(bias + taps of act [P][Cp] . w [N][9 Cp]^T) and, when
  * outb, its BF16 copy [P][ldb]; bias may be NULL.  The data gradient is the same call on dY with the
@@ -433,9 +411,6 @@ int maf_nn_wcast_conv(const float* W32, int Cout, int Cin, int Cp, int CoutP, vo
 int maf_nn_relu_bias_bwd(const float* dA, const float* A, long long P, int C, int relu, void* dYb, int Cp, float* db,
                          double* part, void* st);
 int maf_nn_relu_bias_bwd_parts(int* n);
-/* maf_nn_up_cat_bwd with ds = instead of ds += */
-int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
-                          void* st);
 /* y = normalize(m + d) [P][3]; with a target t: per-pixel |y - t|^2, its mean in *loss (device) and
  * dL/dd [P][3] in gd.  While the timeout flag (maf_nn_check) is up, y is NaN. */
 int maf_nn_head(const float* m, const float* d, int ldd, const float* t, long long P, float* y, float* gd,

@@ -212,7 +212,6 @@ class Demag {
     void download_real_tensor(double* host, bool symmetric, cudaStream_t st);  // [6][Pz][Py][Px]
     size_t tensor_elems() const { return (size_t)ncomp() * (md_.nz == 1 ? 1 : md_.nz + 1) * (md_.ny + 1) * nxh(); }
     int pitch() const { return pitch_; }
-    template <typename R> int edens_blocks() const;
     // the plan of an evaluation at the current kernel choices; its tensor and buffers are made on first use.
     // The spectra grow when a plan needs longer rows: whoever keeps their addresses (a captured
     // graph) compares them, and id(), with the plan's before every use.

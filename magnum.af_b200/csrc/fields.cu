@@ -837,8 +837,6 @@ template <typename R> void Demag::forward_conv(const R* m, const MsInfo& ms, cud
     }
 }
 
-template <typename R> int Demag::edens_blocks() const { return 0; }
-
 template <typename R>
 void Demag::inverse_x_epilogue(const R* m, const MsInfo& ms, const TermList& tl, const EpilogueArgs& ep,
                                cudaStream_t st, int* nblocks_out, PassMarks* marks) {

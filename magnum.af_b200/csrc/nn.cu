@@ -1,11 +1,10 @@
-// Layer kernels of the warm-start U-net (magnumaf/warmstart.py): pixel-major
-// (NHWC) activations, 3x3 convolutions as im2col + the tensor-core BF16 GEMM of
-// umma.cu with FP32 accumulation, bias/ReLU epilogues, 2x2 average pooling,
-// nearest 2x upsampling with skip concatenation, their backward passes and
-// Adam.  A pixel p = (b, y, x) is row p = (b H + y) W + x; a layer's channel
-// count C is padded to Cp (a multiple of 8) in the BF16 tensors that feed a
-// GEMM, the padding is zero.  Every reduction runs in a fixed order, so
-// training is deterministic.
+// Layer kernels of the warm-start U-net (magnumaf/unet.py) beside the convolutions of
+// conv.cu: the BF16 input, 2x2 average pooling, nearest 2x upsampling with skip
+// concatenation, their backward passes, the normalising head with its loss gradient, and
+// Adam.  Activations are pixel-major (NHWC): pixel p = (b, y, x) is row p = (b H + y) W + x;
+// a layer's channel count C is padded to Cp (a multiple of 8) in the BF16 tensors that feed a
+// convolution, the padding is zero.  Every reduction runs in a fixed order, so training is
+// deterministic.
 #include <cuda_bf16.h>
 
 #include <initializer_list>
@@ -14,11 +13,6 @@
 #include "capi_internal.hpp"
 #include "engine.hpp"
 #include "tc_error.hpp"
-
-namespace mafb {
-void umma_gemm(const void* A, int lda, const void* B, int ldb, float* C, int ldc, int M, int N, int K,
-               cudaStream_t st, bool check, int splits);
-}
 
 using namespace mafb;
 
@@ -43,58 +37,6 @@ __global__ void k_in(const float* __restrict__ x, int B, int C, int H, int W, in
         const float v = c < C ? x[(b * C + c) * HW + r] : 0.f;
         act[i] = __float2bfloat16_rn(v);
         if (c < 3) m[p * 3 + c] = v;
-    }
-}
-
-// im2col: col[p][t Cp + c] = act[pixel (y + t/3 - 1, x + t%3 - 1)][c] (zero outside);
-// transposed: colT[t Cp + c][p].  Eight channels (16 bytes) per item.
-__global__ void k_im2col(const bf16* __restrict__ act, int B, int H, int W, int Cp, bf16* __restrict__ col,
-                         int transposed) {
-    const int64_t HW = (int64_t)H * W, P = B * HW;
-    const int c8 = Cp / 8;
-    GRID_STRIDE(i, P * 9 * c8) {
-        int64_t p;
-        int t, cc;
-        if (transposed) {  // consecutive items: consecutive pixels of one (t, channel group)
-            p = i % P;
-            const int64_t q = i / P;
-            t = (int)(q / c8);
-            cc = (int)(q - (int64_t)t * c8);
-        } else {
-            p = i / (9 * c8);
-            const int q = (int)(i - p * 9 * c8);
-            t = q / c8;
-            cc = q - t * c8;
-        }
-        const int64_t b = p / HW, r = p - b * HW;
-        const int y = (int)(r / W) + t / 3 - 1, x = (int)(r % W) + t % 3 - 1;
-        uint4 v = make_uint4(0, 0, 0, 0);
-        if (y >= 0 && y < H && x >= 0 && x < W)
-            v = *reinterpret_cast<const uint4*>(act + ((b * H + y) * W + x) * Cp + cc * 8);
-        if (transposed) {
-            const bf16* e = reinterpret_cast<const bf16*>(&v);
-            const int64_t k0 = (int64_t)t * Cp + cc * 8;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) col[(k0 + j) * P + p] = e[j];
-        } else {
-            *reinterpret_cast<uint4*>(col + p * 9 * Cp + (int64_t)t * Cp + cc * 8) = v;
-        }
-    }
-}
-
-// out = relu?(y + bias) in FP32 [P][C] and BF16 [P][Cp] (zero padded)
-__global__ void k_bias_act(const float* __restrict__ y, int ldy, const float* __restrict__ bias, int64_t P, int C,
-                           int relu, float* __restrict__ out, bf16* __restrict__ outb, int Cp) {
-    GRID_STRIDE(i, P * Cp) {
-        const int64_t p = i / Cp;
-        const int c = (int)(i - p * Cp);
-        float v = 0.f;
-        if (c < C) {
-            v = y[p * ldy + c] + bias[c];
-            if (relu) v = fmaxf(v, 0.f);
-            out[p * C + c] = v;
-        }
-        if (outb) outb[i] = __float2bfloat16_rn(v);
     }
 }
 
@@ -205,11 +147,10 @@ __global__ void __launch_bounds__(kT) k_up_cat(const float* __restrict__ a, int 
     }
 }
 
-// backward of k_up_cat: da [B][H/2][W/2][Ca] = sum of the four children; ds [B][H][W][Cs]
-// (+)= the skip part
+// backward of k_up_cat: da [B][H/2][W/2][Ca] = sum of the four children; ds [B][H][W][Cs] = the skip part
 template <int V>
 __global__ void __launch_bounds__(kT) k_up_cat_bwd(const float* __restrict__ dcat, int Cp, int Ca, int Cs, int rows, int W,
-                                                   float* __restrict__ da, float* __restrict__ ds, int accumulate) {
+                                                   float* __restrict__ da, float* __restrict__ ds) {
     const int w = W / 2, av = Ca / V, sv = Cs / V;
     ROW_LOOP(row, rows) {  // coarse row: fine rows 2 row and 2 row + 1
         const float* d0 = dcat + (int64_t)2 * row * W * Cp;
@@ -227,110 +168,10 @@ __global__ void __launch_bounds__(kT) k_up_cat_bwd(const float* __restrict__ dca
         }
         for (int i = threadIdx.x; i < 2 * W * sv; i += kT) {
             const int x = i / sv, c = (i - x * sv) * V;  // x over both fine rows
-            float v[V], e[V];
-            float* o = ds + ((int64_t)2 * row * W + x) * Cs + c;
+            float v[V];
             ldv<V>(d0 + (int64_t)x * Cp + Ca + c, v);
-            if (accumulate) {
-                ldv<V>(o, e);
-#pragma unroll
-                for (int k = 0; k < V; ++k) v[k] = e[k] + v[k];
-            }
-            stv<V>(o, v);
+            stv<V>(ds + ((int64_t)2 * row * W + x) * Cs + c, v);
         }
-    }
-}
-
-// dY = dA * relu'(A) (A the layer's output) in FP32 [P][C] and BF16 [P][Cp] (zero padded)
-__global__ void k_relu_bwd(const float* __restrict__ dA, const float* __restrict__ A, int64_t P, int C, int relu,
-                           float* __restrict__ dY, bf16* __restrict__ dYb, int Cp) {
-    GRID_STRIDE(i, P * Cp) {
-        const int64_t p = i / Cp;
-        const int c = (int)(i - p * Cp);
-        float v = 0.f;
-        if (c < C) {
-            v = dA[p * C + c];
-            if (relu && !(A[p * C + c] > 0.f)) v = 0.f;
-            dY[p * C + c] = v;
-        }
-        dYb[i] = __float2bfloat16_rn(v);
-    }
-}
-
-// out [C][R] = in [R][C] (BF16)
-__global__ void k_transpose(const bf16* __restrict__ in, int64_t R, int C, bf16* __restrict__ out) {
-    __shared__ bf16 tile[32][33];
-    const int64_t r0 = (int64_t)blockIdx.x * 32;
-    const int c0 = blockIdx.y * 32;
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int64_t r = r0 + k;
-        const int c = c0 + threadIdx.x;
-        tile[k][threadIdx.x] = (r < R && c < C) ? in[r * C + c] : __float2bfloat16_rn(0.f);
-    }
-    __syncthreads();
-    for (int k = threadIdx.y; k < 32; k += 8) {
-        const int c = c0 + k;
-        const int64_t r = r0 + threadIdx.x;
-        if (c < C && r < R) out[(int64_t)c * R + r] = tile[threadIdx.x][k];
-    }
-}
-
-// col2im: dX[p][c] (+)= sum_t dcol[p'][t Cp + c] over the outputs p' whose tap t read pixel p
-__global__ void k_col2im(const float* __restrict__ dcol, int B, int H, int W, int Cp, int C, float* __restrict__ dX,
-                         int accumulate) {
-    const int64_t HW = (int64_t)H * W;
-    GRID_STRIDE(i, B * HW * C) {
-        const int64_t p = i / C;
-        const int c = (int)(i - p * C);
-        const int64_t b = p / HW, r = p - b * HW;
-        const int y = (int)(r / W), x = (int)(r % W);
-        float s = 0.f;
-#pragma unroll
-        for (int t = 0; t < 9; ++t) {
-            const int yo = y - (t / 3 - 1), xo = x - (t % 3 - 1);  // output pixel whose tap t is (y, x)
-            if (yo >= 0 && yo < H && xo >= 0 && xo < W) s += dcol[((b * H + yo) * W + xo) * 9 * Cp + t * Cp + c];
-        }
-        dX[i] = accumulate ? dX[i] + s : s;
-    }
-}
-
-// db[c] = sum_p dY[p][c] (one block per channel, fixed order)
-__global__ void k_colsum(const float* __restrict__ dY, int64_t P, int C, float* __restrict__ db) {
-    const int c = blockIdx.x;
-    double s = 0.0;
-    for (int64_t p = threadIdx.x; p < P; p += blockDim.x) s += dY[p * C + c];
-    __shared__ double red[kT / 32];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < kT / 32; ++k) t += red[k];
-        db[c] = (float)t;
-    }
-}
-
-// weights: W32 [Cout][9][Cin] FP32 (master) -> Wb [Cout][9 Cp] BF16 and the
-// transposed WtB [9 Cp][CoutP] BF16 (zero padded) of the data gradient
-__global__ void k_wcast(const float* __restrict__ W32, int Cout, int Cin, int Cp, int CoutP, bf16* __restrict__ Wb,
-                        bf16* __restrict__ WtB) {
-    GRID_STRIDE(i, (int64_t)CoutP * 9 * Cp) {
-        const int co = (int)(i / (9 * Cp));
-        const int k = (int)(i - (int64_t)co * 9 * Cp);
-        const int t = k / Cp, c = k - t * Cp;
-        const float v = (co < Cout && c < Cin) ? W32[((int64_t)co * 9 + t) * Cin + c] : 0.f;
-        const bf16 b = __float2bfloat16_rn(v);
-        if (co < Cout) Wb[i] = b;
-        WtB[(int64_t)k * CoutP + co] = b;
-    }
-}
-
-// dW32 [Cout][9][Cin] from the GEMM result g [Cout][9 Cp]
-__global__ void k_wgrad(const float* __restrict__ g, int Cout, int Cin, int Cp, float* __restrict__ dW) {
-    GRID_STRIDE(i, (int64_t)Cout * 9 * Cin) {
-        const int co = (int)(i / (9 * Cin));
-        const int k = (int)(i - (int64_t)co * 9 * Cin);
-        const int t = k / Cin, c = k - t * Cin;
-        dW[i] = g[(int64_t)co * 9 * Cp + t * Cp + c];
     }
 }
 
@@ -394,14 +235,6 @@ __global__ void __launch_bounds__(kMeanT) k_mean(const float* __restrict__ v, in
     }
 }
 
-__global__ void k_sum_slabs(const float* __restrict__ work, int ns, int64_t n, float* __restrict__ out) {
-    GRID_STRIDE(i, n) {
-        float s = 0.f;
-        for (int k = 0; k < ns; ++k) s += work[(int64_t)k * n + i];
-        out[i] = s;
-    }
-}
-
 __global__ void k_adam_nn(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
                           float* __restrict__ m2, int64_t n, float lr, float c1, float c2) {
     GRID_STRIDE(i, n) {
@@ -426,41 +259,6 @@ int maf_nn_input(const float* x, int B, int C, int H, int W, int Cp, void* act_b
         if (Cp % 8 || Cp < C || C < 3) throw Error(1, "maf_nn_input: Cp must be a multiple of 8 >= C >= 3");
         const int64_t n = (int64_t)B * H * W * Cp;
         k_in<<<grid_for(n), kT, 0, S(st)>>>(x, B, C, H, W, Cp, static_cast<bf16*>(act_bf16), m);
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_im2col(const void* act, int B, int H, int W, int Cp, void* col, int transposed, void* st) {
-    return run([&] {
-        if (Cp % 8) throw Error(1, "maf_nn_im2col: Cp must be a multiple of 8");
-        const int64_t n = (int64_t)B * H * W * 9 * (Cp / 8);
-        k_im2col<<<grid_for(n), kT, 0, S(st)>>>(static_cast<const bf16*>(act), B, H, W, Cp, static_cast<bf16*>(col),
-                                                transposed);
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_gemm(const void* A, int lda, const void* B, int ldb, float* C, int ldc, int M, int N, int K, void* st) {
-    return run([&] { umma_gemm(A, lda, B, ldb, C, ldc, M, N, K, S(st), false, 1); });
-}
-
-// GEMM with the K range split over `splits` chunks (partial slabs in work
-// [splits][M][N]), summed into C [M][N] in split order
-int maf_nn_gemm_splitk(const void* A, int lda, const void* B, int ldb, float* C, int M, int N, int K, int splits,
-                       float* work, void* st) {
-    return run([&] {
-        umma_gemm(A, lda, B, ldb, work, N, M, N, K, S(st), false, splits);
-        const int kchunk = (int)ceil_div(ceil_div(K, splits), 64) * 64;
-        const int ns = (int)ceil_div(K, kchunk);
-        k_sum_slabs<<<grid_for((int64_t)M * N), kT, 0, S(st)>>>(work, ns, (int64_t)M * N, C);
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_bias_act(const float* y, int ldy, const float* bias, long long P, int C, int relu, float* out,
-                    void* outb, int Cp, void* st) {
-    return run([&] {
-        k_bias_act<<<grid_for(P * Cp), kT, 0, S(st)>>>(y, ldy, bias, P, C, relu, out, static_cast<bf16*>(outb), Cp);
         MAF_LAUNCH_CHECK();
     });
 }
@@ -506,70 +304,14 @@ int maf_nn_up_cat(const float* a, int Ca, const float* s, int Cs, int B, int H, 
     });
 }
 
-static int up_cat_bwd(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
-                      int accumulate, void* st) {
+int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
+                          void* st) {
     return run([&] {
         const int rows = B * (H / 2);
         if (by8({Cp, Ca, Cs}, {dcat, da, ds}))
-            k_up_cat_bwd<8><<<row_blocks(rows), kT, 0, S(st)>>>(dcat, Cp, Ca, Cs, rows, W, da, ds, accumulate);
+            k_up_cat_bwd<8><<<row_blocks(rows), kT, 0, S(st)>>>(dcat, Cp, Ca, Cs, rows, W, da, ds);
         else
-            k_up_cat_bwd<1><<<row_blocks(rows), kT, 0, S(st)>>>(dcat, Cp, Ca, Cs, rows, W, da, ds, accumulate);
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_up_cat_bwd(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
-                      void* st) {
-    return up_cat_bwd(dcat, Cp, Ca, Cs, B, H, W, da, ds, 1, st);
-}
-
-int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int H, int W, float* da, float* ds,
-                          void* st) {
-    return up_cat_bwd(dcat, Cp, Ca, Cs, B, H, W, da, ds, 0, st);
-}
-
-int maf_nn_relu_bwd(const float* dA, const float* A, long long P, int C, int relu, float* dY, void* dYb, int Cp,
-                    void* st) {
-    return run([&] {
-        k_relu_bwd<<<grid_for(P * Cp), kT, 0, S(st)>>>(dA, A, P, C, relu, dY, static_cast<bf16*>(dYb), Cp);
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_transpose(const void* in, long long R, int C, void* out, void* st) {
-    return run([&] {
-        dim3 grid((unsigned)ceil_div(R, 32), (unsigned)ceil_div(C, 32));
-        k_transpose<<<grid, dim3(32, 8), 0, S(st)>>>(static_cast<const bf16*>(in), R, C, static_cast<bf16*>(out));
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_col2im(const float* dcol, int B, int H, int W, int Cp, int C, float* dX, int accumulate, void* st) {
-    return run([&] {
-        k_col2im<<<grid_for((int64_t)B * H * W * C), kT, 0, S(st)>>>(dcol, B, H, W, Cp, C, dX, accumulate);
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_colsum(const float* dY, long long P, int C, float* db, void* st) {
-    return run([&] {
-        k_colsum<<<C, kT, 0, S(st)>>>(dY, P, C, db);
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_wcast(const float* W32, int Cout, int Cin, int Cp, int CoutP, void* Wb, void* WtB, void* st) {
-    return run([&] {
-        if (Cp % 8 || CoutP % 8 || CoutP < Cout || Cp < Cin) throw Error(1, "maf_nn_wcast: bad padding");
-        k_wcast<<<grid_for((int64_t)CoutP * 9 * Cp), kT, 0, S(st)>>>(W32, Cout, Cin, Cp, CoutP, static_cast<bf16*>(Wb),
-                                                                    static_cast<bf16*>(WtB));
-        MAF_LAUNCH_CHECK();
-    });
-}
-
-int maf_nn_wgrad(const float* g, int Cout, int Cin, int Cp, float* dW, void* st) {
-    return run([&] {
-        k_wgrad<<<grid_for((int64_t)Cout * 9 * Cin), kT, 0, S(st)>>>(g, Cout, Cin, Cp, dW);
+            k_up_cat_bwd<1><<<row_blocks(rows), kT, 0, S(st)>>>(dcat, Cp, Ca, Cs, rows, W, da, ds);
         MAF_LAUNCH_CHECK();
     });
 }

@@ -140,20 +140,9 @@ _SIGS = {
     "maf_bf16_gemm": (_I, [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P]),
     # layer kernels of the warm-start U-net (magnumaf.unet)
     "maf_nn_input": (_I, [_P, _I, _I, _I, _I, _I, _P, _P, _P]),
-    "maf_nn_im2col": (_I, [_P, _I, _I, _I, _I, _P, _I, _P]),
-    "maf_nn_gemm": (_I, [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P]),
-    "maf_nn_gemm_splitk": (_I, [_P, _I, _P, _I, _P, _I, _I, _I, _I, _P, _P]),
-    "maf_nn_bias_act": (_I, [_P, _I, _P, C.c_longlong, _I, _I, _P, _P, _I, _P]),
     "maf_nn_pool": (_I, [_P, _I, _I, _I, _I, _P, _P, _I, _P]),
     "maf_nn_pool_bwd": (_I, [_P, _I, _I, _I, _I, _P, _I, _P]),
     "maf_nn_up_cat": (_I, [_P, _I, _P, _I, _I, _I, _I, _P, _I, _P]),
-    "maf_nn_up_cat_bwd": (_I, [_P, _I, _I, _I, _I, _I, _I, _P, _P, _P]),
-    "maf_nn_relu_bwd": (_I, [_P, _P, C.c_longlong, _I, _I, _P, _P, _I, _P]),
-    "maf_nn_transpose": (_I, [_P, C.c_longlong, _I, _P, _P]),
-    "maf_nn_col2im": (_I, [_P, _I, _I, _I, _I, _I, _P, _I, _P]),
-    "maf_nn_colsum": (_I, [_P, C.c_longlong, _I, _P, _P]),
-    "maf_nn_wcast": (_I, [_P, _I, _I, _I, _I, _P, _P, _P]),
-    "maf_nn_wgrad": (_I, [_P, _I, _I, _I, _P, _P]),
     "maf_nn_check": (_I, [_P, _I]),
     "maf_nn_flag_timeout": (_I, [_P]),
     "maf_nn_conv": (_I, [_P, _I, _I, _I, _I, _P, _I, _P, _I, _P, _I, _P, _I, _P]),
@@ -974,10 +963,9 @@ class StochasticBatch:
     pairs of steps of every member replay one captured CUDA graph with each member
     on its own stream.  Bit-identical to stepping the members one by one.
 
-    fused=True: every pass of a step is one launch for all members (a device
-    work table of (member, tile) pairs over the run-time-plan kernels) when every
-    member is a 2-D mesh with one DemagField and scalar parameters; bit-identical
-    to the members stepped one by one with DemagField.generic = True."""
+    fused=True: every pass of a step is one launch for all members of the same
+    transform lengths (a device work table of (member, tile) pairs) when every
+    member is a 2-D mesh with one DemagField and scalar parameters."""
 
     def __init__(self, members, fused=False):
         self._members = list(members)
