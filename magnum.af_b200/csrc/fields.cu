@@ -34,6 +34,14 @@ namespace mafb {
 // ---------------------------------------------------------------------------
 // twiddles and plans
 // ---------------------------------------------------------------------------
+// A copy that is complete on return.  cudaMemcpy from pageable memory returns when a small
+// buffer has been staged, before the device holds it, and orders the legacy stream only, which
+// the library's non-blocking streams do not wait for: a pass could read a new table too early.
+static void copy_now(void* dst, const void* src, size_t n, cudaMemcpyKind kind) {
+    MAF_CUDA(cudaMemcpyAsync(dst, src, n, kind, cudaStreamPerThread));
+    MAF_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
+}
+
 const void* Twiddles::get(int L, bool fp64) {
     auto key = std::make_pair(L, fp64 ? 1 : 0);
     auto it = tables_.find(key);
@@ -61,12 +69,12 @@ const void* Twiddles::get(int L, bool fp64) {
         std::vector<double2> h(L);
         for (int k = 0; k < L; ++k) h[k] = make_double2((double)c[k], (double)s[k]);
         buf.alloc(sizeof(double2) * L);
-        MAF_CUDA(cudaMemcpy(buf.p, h.data(), sizeof(double2) * L, cudaMemcpyHostToDevice));
+        copy_now(buf.p, h.data(), sizeof(double2) * L, cudaMemcpyHostToDevice);
     } else {
         std::vector<float2> h(L);
         for (int k = 0; k < L; ++k) h[k] = make_float2((float)c[k], (float)s[k]);
         buf.alloc(sizeof(float2) * L);
-        MAF_CUDA(cudaMemcpy(buf.p, h.data(), sizeof(float2) * L, cudaMemcpyHostToDevice));
+        copy_now(buf.p, h.data(), sizeof(float2) * L, cudaMemcpyHostToDevice);
     }
     const void* p = buf.p;
     tables_.emplace(key, std::move(buf));
@@ -83,7 +91,7 @@ const void* Twiddles::get_ct(int L, bool fp64, const int* radix, int nstages) {
     const void* base = get(L, fp64);
     const size_t esz = fp64 ? sizeof(double2) : sizeof(float2);
     std::vector<unsigned char> tab((size_t)L * esz);
-    MAF_CUDA(cudaMemcpy(tab.data(), base, (size_t)L * esz, cudaMemcpyDeviceToHost));
+    copy_now(tab.data(), base, (size_t)L * esz, cudaMemcpyDeviceToHost);
     std::vector<unsigned char> out(tab);
     int NS = 1;
     for (int st = 0; st < nstages; ++st) {
@@ -99,7 +107,7 @@ const void* Twiddles::get_ct(int L, bool fp64, const int* radix, int nstages) {
         NS *= RAD;
     }
     DevBuf buf(out.size());
-    MAF_CUDA(cudaMemcpy(buf.p, out.data(), out.size(), cudaMemcpyHostToDevice));
+    copy_now(buf.p, out.data(), out.size(), cudaMemcpyHostToDevice);
     const void* p = buf.p;
     tables_.emplace(key, std::move(buf));
     return p;

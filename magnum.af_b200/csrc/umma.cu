@@ -190,7 +190,8 @@ DeviceFlag& device_flag() {
     if (!f.host) {
         void *d = nullptr, *h = nullptr, *hd = nullptr;
         MAF_CUDA(cudaMalloc(&d, sizeof(int)));
-        MAF_CUDA(cudaMemset(d, 0, sizeof(int)));
+        MAF_CUDA(cudaMemsetAsync(d, 0, sizeof(int), cudaStreamPerThread));
+        MAF_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
         MAF_CUDA(cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped));
         MAF_CUDA(cudaHostGetDevicePointer(&hd, h, 0));
         *static_cast<int*>(h) = 0;

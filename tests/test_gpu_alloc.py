@@ -88,7 +88,7 @@ def test_threads_make_use_and_drop_objects():
     bad = []
 
     def worker(i):
-        for rep in range(4):
+        for rep in range(30):
             for k in range(3):
                 try:
                     if not np.array_equal(run(shapes[i], k), want[i, k]):
