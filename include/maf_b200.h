@@ -48,6 +48,9 @@ const char* maf_last_error(void);
 int maf_version(int* major, int* minor);
 /* Number of visible CUDA devices (0 without a GPU). */
 int maf_device_count(int* n);
+/* Gives the device memory that the library keeps unused for its next objects (at most 512 MB per device: 256 MB in
+ * its memory pool and 256 MB in former m buffers of states) back to the driver. */
+int maf_memory_trim(void);
 
 /* ---------------------------------------------------------------- State ---
  * Replaces magnumaf::State(Mesh, double Ms, af::array m) and

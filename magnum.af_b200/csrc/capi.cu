@@ -1989,6 +1989,13 @@ int maf_term_demag_set_tune(maf_term t, const int choices[3]) {
     });
 }
 
+int maf_memory_trim(void) {
+    return guarded([&] {
+        require_device();
+        dev_trim();
+    });
+}
+
 int maf_demag_lengths(int nx, int ny, int nz, int lengths[3]) {
     return guarded([&] {
         check(lengths && nx > 0 && ny > 0 && nz > 0, "maf_demag_lengths: bad argument");

@@ -15,9 +15,11 @@ namespace mafb {
 enum Precision : int { PREC_FP64 = 0, PREC_FP32_FIELD = 1 };
 
 // Device memory (alloc.cu): dev_alloc throws and says whether the memory is the pool's (never
-// when `own`); dev_free waits for the device's work, as cudaFree does.
+// when `own`); dev_free (n: the size asked for) waits for the device's work, as cudaFree does,
+// unless nothing uses the buffer any more (idle); dev_trim gives unused memory back to the driver.
 void* dev_alloc(size_t n, bool own, bool* pooled);
-void dev_free(void* p, bool pooled);
+void dev_free(void* p, size_t n, bool pooled, bool idle);
+void dev_trim();
 
 // Owning device allocation.  alloc_own / ensure_own: for a buffer whose address the
 // application may get (a state's m and the candidates that are swapped with it), an
@@ -40,7 +42,7 @@ struct DevBuf {
     void alloc_own(size_t n) { get(n, true); }
     void ensure(size_t n) { if (bytes < n) alloc(n); }
     void ensure_own(size_t n) { if (bytes < n) alloc_own(n); }
-    void release() { if (p) dev_free(p, pooled); p = nullptr; bytes = 0; }
+    void release(bool idle = false) { if (p) dev_free(p, bytes, pooled, idle); p = nullptr; bytes = 0; }
     void get(size_t n, bool own) {
         release();
         if (n) p = dev_alloc(n, own, &pooled);

@@ -622,6 +622,7 @@ void Demag::build_tensor(cudaStream_t st) {
         transform_octants(t, Kx, Ky, Kz, comps + ci, nb, Px(), Py(), Pz(), t, 1.0, work.as<char>(), st);
     }
     MAF_CUDA(cudaStreamSynchronize(st));
+    work.release(true);
 }
 
 // The tensor at the padded lengths (FP64 or FP32), from the one at twice the mesh
@@ -656,6 +657,7 @@ void Demag::build_padded_tensor(double* out64, float* out32, cudaStream_t st) {
         }
     }
     MAF_CUDA(cudaStreamSynchronize(st));
+    scratch.release(true);
 }
 
 void Demag::download_tensor(double* host, cudaStream_t st) const {

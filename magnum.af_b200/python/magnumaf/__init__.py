@@ -155,6 +155,7 @@ _SIGS = {
     "maf_nn_adam": (_I, [_P, _P, _P, _P, C.c_longlong, C.c_float, _I, _P]),
     "maf_stoch_batch_is_fused": (_I, [_P, C.POINTER(_I)]),
     "maf_term_demag_set_generic": (_I, [_P, _I]),
+    "maf_memory_trim": (_I, []),
     "maf_demag_lengths": (_I, [_I, _I, _I, C.POINTER(_I)]),
     "maf_string_create": (_I, [C.POINTER(_P), _P, C.POINTER(_P), _I, _I, _D, _P]),
     "maf_string_destroy": (_I, [_P]),
@@ -230,6 +231,11 @@ class Mesh:
     @property
     def n(self):
         return self.nx * self.ny * self.nz
+
+
+def trim_memory() -> None:
+    """Gives the device memory that the library keeps unused for its next objects back to the driver."""
+    _ck(lib.maf_memory_trim())
 
 
 def device_count() -> int:

@@ -109,7 +109,7 @@ class UNet:
         """Raises (MAF_ERR_TIMEOUT) when a convolution's bounded wait gave up since the last check; wait: once
         the current stream's work has finished.  forward() returns before that, with y NaN in such a case;
         loss_grad and train_step check themselves, and every call first reports an earlier one's."""
-        _ck(lib.maf_nn_check(self._stream(), int(wait)))
+        _ck(lib.maf_nn_check(self._stream() if wait else None, int(wait)))
 
     def _cast_weights(self):
         """BF16 copies of every layer's weights: [cout][9 cp] (forward) and [cin][9 coutp] (data gradient)."""

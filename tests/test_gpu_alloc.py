@@ -48,9 +48,9 @@ def test_buffers_dropped_while_another_thread_captures():
     free0 = torch.cuda.mem_get_info()[0]
     capture(made.clear)
     _stepped((8, 8, 1))  # an object made and dropped afterwards gives back what was pending
-    torch.cuda.synchronize()
-    # 6 x 126 MB came back but for the 256 MB that the pool keeps (and torch's graph memory)
-    assert torch.cuda.mem_get_info()[0] - free0 >= (6 * 126 - 256 - 64) * MB
+    M.trim_memory()
+    # all of the 6 x 126 MB came back (but for torch's graph memory)
+    assert torch.cuda.mem_get_info()[0] - free0 >= (6 * 126 - 64) * MB
 
 
 def test_pool_gives_its_memory_to_a_large_buffer():
@@ -142,3 +142,27 @@ def test_many_integrators_keep_their_own_error_norm():
             made[i] = make(i)
             assert norm(made[i]) == want[i]
     assert [norm(llg) for llg in made] == want
+
+
+def test_unused_buffers_are_kept_within_bounds_and_given_back():
+    """States dropped and made again reuse their m buffers; what is kept unused stays below 512
+    MB, trim_memory gives it back, and a state made of a used buffer holds its own m."""
+    shape = (512, 512, 2)
+    _stepped(shape)
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    M.trim_memory()
+    free0 = torch.cuda.mem_get_info()[0]
+    made = [_stepped(shape, seed) for seed in range(14)]  # 96 MB of the pool and twice 12 of m each
+    assert free0 - torch.cuda.mem_get_info()[0] >= 14 * (96 + 2 * 12) * MB
+    made.clear()
+    big = [M.State(M.Mesh(512, 512, 16, 1e-9, 1e-9, 1e-9), 8e5, np.ones((512, 512, 16, 3)))
+           for _ in range(4)]  # 4 x 101 MB of m
+    big.clear()
+    assert free0 - torch.cuda.mem_get_info()[0] < 512 * MB + 32 * MB
+    m = random_m(shape, 77)
+    st = M.State(M.Mesh(*shape, 3e-9, 3e-9, 3e-9), 8e5, m)
+    np.testing.assert_allclose(np.asarray(st.m), m, rtol=0, atol=1e-15)
+    del st
+    M.trim_memory()
+    assert free0 - torch.cuda.mem_get_info()[0] < 16 * MB
