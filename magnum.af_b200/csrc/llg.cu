@@ -162,11 +162,11 @@ struct KUnion {
 };
 
 // vmax <- max(vmax, |err / sc|), NaN-propagating.  The FP64 division is skipped where the
-// quotient is certainly below vmax (the finalize kernels are bound on FP64 division and
-// square root as much as on HBM).  The comparison is strict, so that 0 / 0 (atol = 0, a cell
-// without m) and inf / inf are divided and give NaN, as a NaN does, whose comparison fails.
+// quotient is certainly below vmax or a zero (the finalize kernels are bound on FP64 division
+// and square root as much as on HBM).  The comparisons are strict, so that 0 / 0 (atol = 0, a
+// cell without m) and inf / inf are divided and give NaN, as a NaN does, which fails both.
 __device__ __forceinline__ void err_max(double err, double sc, double& vmax) {
-    if (!(fabs(err) < vmax * sc * (1.0 - 1e-12))) vmax = nanmax(vmax, fabs(err / sc));
+    if (!(fabs(err) < vmax * sc * (1.0 - 1e-12) || (err == 0.0 && sc > 0.0))) vmax = nanmax(vmax, fabs(err / sc));
 }
 
 __device__ __forceinline__ double fin_one(double sumbk, double e, int form, double mi, double atol, double rtol,
