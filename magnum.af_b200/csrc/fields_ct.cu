@@ -8,6 +8,7 @@
 // z convolution handles the rows ky and Py - ky in one CTA so that the stored
 // tensor quadrant is read from HBM once.
 #include <algorithm>
+#include <atomic>
 
 #include "ct_dispatch.hpp"
 #include "epilogue.cuh"
@@ -798,17 +799,17 @@ static void xfwd_L(const R* in, int n_in, int64_t rows, int64_t rows_pc, const R
             auto kp = rag ? k_xfwd_pipe<R, LC, NB, NT, true> : k_xfwd_pipe<R, LC, NB, NT, false>;
             const size_t smem_p = xfwd_pipe_smem<R, LC, NB>();
             ct_smem(kp, smem_p);
-            static int per_sm[2] = {0, 0}, sms = 0;  // exact and shorter rows, measured once per process
-            int& ps = per_sm[rag];
+            // CTAs per SM of the kernels for exact and for shorter rows, asked for once per process (by
+            // several threads at most, with the same answer)
+            static std::atomic<int> per_sm[2];
+            int ps = per_sm[rag].load(std::memory_order_relaxed);
             if (!ps) {
                 MAF_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ps, kp, NT, smem_p));
-                int dev = 0;
-                MAF_CUDA(cudaGetDevice(&dev));
-                MAF_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
                 if (ps < 1) ps = 1;
+                per_sm[rag].store(ps, std::memory_order_relaxed);
             }
             const int64_t ntiles = ceil_div(rows, NB);
-            const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)ps * sms);
+            const unsigned grid = (unsigned)std::min<int64_t>(ntiles, (int64_t)ps * sm_count());
             launch_chain(kp, dim3(grid), NT, smem_p, st, in, n_in, rows, ms, out, pitch,
                          static_cast<const cplx_t<R>*>(tw), static_cast<const cplx_t<R>*>(twP));
             return;
