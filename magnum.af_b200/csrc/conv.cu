@@ -166,7 +166,7 @@ struct ConvArgs {
     bf16* outb;         // [P][ldb] (zero beyond N) or null
     int H, W, Cp, N, ldo, ldb, relu;
     int64_t P;
-    TcError err;
+    TcFlag* err;
 };
 
 // out[p][n] = relu?(bias[n] + sum_{t, c} act[tap t of p][c] w[n][t Cp + c]): CTA =
@@ -290,7 +290,7 @@ struct WgradArgs {
     float* work;      // [splits][9 Cp][Np]
     int H, W, Cp, Np;
     int64_t P, chunk;  // pixels per split, a multiple of kBK
-    TcError err;
+    TcFlag* err;
 };
 
 // work[s][t Cp + c][n] = sum over the split's pixels of act[tap t of p][c] dy[p][n]:
@@ -505,7 +505,7 @@ int maf_nn_conv(const void* act, int B, int H, int W, int Cp, const void* w, int
             throw Error(1, "maf_nn_conv: 16-byte aligned buffers expected");
         ConvArgs a{static_cast<const __nv_bfloat16*>(act), static_cast<const __nv_bfloat16*>(w), bias, out,
                    static_cast<__nv_bfloat16*>(outb), H, W, Cp, N, ldo, ldb, relu, (int64_t)B * H * W,
-                   tc_error()};
+                   tc_flag()};
         cudaStream_t s = static_cast<cudaStream_t>(st);
         // the widest tile that the channels fill, so that a pixel's taps are gathered once;
         // narrower when the tiles would leave SMs idle (a single film's deeper levels)
@@ -529,7 +529,7 @@ int maf_nn_conv_wgrad(const void* act, int B, int H, int W, int Cp, int Cin, con
             throw Error(1, "maf_nn_conv_wgrad: 16-byte aligned buffers expected");
         cudaStream_t s = static_cast<cudaStream_t>(st);
         WgradArgs a{static_cast<const __nv_bfloat16*>(act), static_cast<const __nv_bfloat16*>(dy), work, H, W, Cp,
-                    CoutP, (int64_t)B * H * W, 0, tc_error()};
+                    CoutP, (int64_t)B * H * W, 0, tc_flag()};
         const int bn = CoutP <= 32 ? 32 : CoutP <= 64 ? 64 : 128;
         // about four CTAs per SM, at least four K blocks each
         const int64_t tiles = ceil_div(9 * Cp, kBM) * ceil_div(CoutP, bn);

@@ -319,7 +319,7 @@ int maf_nn_up_cat_bwd_set(const float* dcat, int Cp, int Ca, int Cs, int B, int 
 int maf_nn_head(const float* m, const float* d, int ldd, const float* tgt, long long P, float* y, float* gd,
                 float* cell_loss, float* loss, void* st) {
     return run([&] {
-        k_head<<<grid_for(P), kT, 0, S(st)>>>(m, d, ldd, tgt, P, y, gd, cell_loss, tc_error().dev);
+        k_head<<<grid_for(P), kT, 0, S(st)>>>(m, d, ldd, tgt, P, y, gd, cell_loss, &tc_flag()->up);
         MAF_LAUNCH_CHECK();
         if (tgt && loss) {
             k_mean<<<1, kMeanT, 0, S(st)>>>(cell_loss, P, loss);

@@ -69,7 +69,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase) {
 template <int BN>
 __global__ void __launch_bounds__(128) k_umma_gemm(const __nv_bfloat16* __restrict__ A, int lda,
                                                    const __nv_bfloat16* __restrict__ B, int ldb, float* __restrict__ C,
-                                                   int ldc, int M, int N, int K, TcError err) {
+                                                   int ldc, int M, int N, int K, TcFlag* err) {
     static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "tile width");
     constexpr uint32_t A_KC = (kBM / 8) * 128;  // bytes between the K chunks of the A tile (LBO)
     constexpr uint32_t B_KC = (BN / 8) * 128;   // of the B tile
@@ -172,11 +172,11 @@ __global__ void __launch_bounds__(128) k_umma_gemm(const __nv_bfloat16* __restri
 }
 
 // the flag as a wait that gave up raises it (maf_nn_flag_timeout)
-__global__ void k_tc_raise(TcError e) { tc_raise(e); }
+__global__ void k_tc_raise(TcFlag* f) { tc_raise(f); }
 
 constexpr int kMaxOrdinals = 64;
 struct DeviceFlag {
-    TcError e;
+    TcFlag* dev = nullptr;
     std::atomic<volatile int*> host{nullptr};  // host address of the host word
 };
 DeviceFlag flags[kMaxOrdinals];
@@ -197,13 +197,14 @@ DeviceFlag& device_flag() {
     DeviceFlag& f = flags[dev];
     if (!f.host) {
         void *d = nullptr, *h = nullptr, *hd = nullptr;
-        MAF_CUDA(cudaMalloc(&d, sizeof(int)));
-        MAF_CUDA(cudaMemsetAsync(d, 0, sizeof(int), cudaStreamPerThread));
-        MAF_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
+        MAF_CUDA(cudaMalloc(&d, sizeof(TcFlag)));
         MAF_CUDA(cudaHostAlloc(&h, sizeof(int), cudaHostAllocMapped));
         MAF_CUDA(cudaHostGetDevicePointer(&hd, h, 0));
         *static_cast<int*>(h) = 0;
-        f.e = TcError{static_cast<int*>(d), static_cast<int*>(hd)};
+        const TcFlag t{0, static_cast<int*>(hd)};
+        MAF_CUDA(cudaMemcpyAsync(d, &t, sizeof(t), cudaMemcpyHostToDevice, cudaStreamPerThread));
+        MAF_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
+        f.dev = static_cast<TcFlag*>(d);
         f.host = static_cast<volatile int*>(h);
     }
     return f;
@@ -211,7 +212,7 @@ DeviceFlag& device_flag() {
 
 }  // namespace
 
-TcError tc_error() { return device_flag().e; }
+TcFlag* tc_flag() { return device_flag().dev; }
 
 void tc_check(cudaStream_t st, bool wait) {
     DeviceFlag& f = device_flag();
@@ -219,7 +220,7 @@ void tc_check(cudaStream_t st, bool wait) {
     volatile int* h = f.host;
     if (!*h) return;
     *h = 0;
-    MAF_CUDA(cudaMemsetAsync(f.e.dev, 0, sizeof(int), st));
+    MAF_CUDA(cudaMemsetAsync(&f.dev->up, 0, sizeof(int), st));
     throw Error(5, "a tensor-core kernel's wait timed out: its outputs are not valid");
 }
 
@@ -229,7 +230,7 @@ static void umma_gemm(const void* A, int lda, const void* B, int ldb, float* C, 
     if (M <= 0 || N <= 0 || K <= 0) return;
     if (K % 8 || lda % 8 || ldb % 8 || lda < K || ldb < K || ldc < N || ((uintptr_t)A | (uintptr_t)B) % 16)
         throw Error(1, "bf16 gemm: K and the row strides must be multiples of 8 elements, rows 16-byte aligned");
-    const TcError err = tc_error();
+    TcFlag* err = tc_flag();
     const auto* a = static_cast<const __nv_bfloat16*>(A);
     const auto* b = static_cast<const __nv_bfloat16*>(B);
     const unsigned gx = (unsigned)ceil_div(M, kBM);
@@ -260,7 +261,7 @@ extern "C" int maf_nn_check(void* stream, int wait) {
 
 extern "C" int maf_nn_flag_timeout(void* stream) {
     return mafb::capi_run([&] {
-        mafb::k_tc_raise<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(mafb::tc_error());
+        mafb::k_tc_raise<<<1, 1, 0, static_cast<cudaStream_t>(stream)>>>(mafb::tc_flag());
         MAF_LAUNCH_CHECK();
     });
 }
