@@ -220,7 +220,9 @@ void tc_check(cudaStream_t st, bool wait) {
     volatile int* h = f.host;
     if (!*h) return;
     *h = 0;
-    MAF_CUDA(cudaMemsetAsync(&f.dev->up, 0, sizeof(int), st));
+    // (complete before the caller's next launch, on whatever stream)
+    MAF_CUDA(cudaMemsetAsync(&f.dev->up, 0, sizeof(int), cudaStreamPerThread));
+    MAF_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
     throw Error(5, "a tensor-core kernel's wait timed out: its outputs are not valid");
 }
 

@@ -63,6 +63,21 @@ def test_own_x_length_beside_padded_axes(shape):
     test_padded_field_vs_oracle_and_own_lengths(shape)
 
 
+def test_attempt_with_own_x_length():
+    """A whole Runge-Kutta attempt of that form (the stage's epilogue writes the next stage's m)."""
+    shape = (9, 130, 20)
+    gm, om = M.Mesh(*shape, 3e-9, 2e-9, 4e-9), O.Mesh(*shape, 3e-9, 2e-9, 4e-9)
+    m = random_m(shape, 41)
+    d = M.DemagField(gm)
+    os_ = O.State(om, MS, m)
+    sumbk, _ = O.LLGIntegrator(0.1, [O.DemagField(om, N_real=d.get_N(symmetric=True)), O.ExchangeField(1.3e-11)],
+                               "DP45").attempt(os_, 2e-14)
+    llg = M.LLGIntegrator(0.1, [d, M.ExchangeField(1.3e-11)], "DP45")
+    for prec, tol in (("fp64", 1e-12), ("fp32_field", 1e-6)):
+        got, _ = llg.rk_attempt(M.State(gm, MS, m, precision=prec), "DP45", 2e-14)
+        assert rel_max(got, os_.m + sumbk) < tol
+
+
 @pytest.mark.parametrize("shape", [(100, 25, 1), (33, 20, 3), (50, 18, 10)])
 def test_padded_ms_field_and_parameter_fields(shape):
     gm = M.Mesh(*shape, 3e-9, 3e-9, 3e-9)
