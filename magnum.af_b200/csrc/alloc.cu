@@ -195,4 +195,22 @@ void dev_free(void* ptr, size_t n, bool pooled, bool idle) {
     if (at.device != dev) cudaSetDevice(dev);
 }
 
+void release_all(const std::vector<DevBuf*>& bufs) {
+    const DevBuf* any = nullptr;
+    for (const DevBuf* b : bufs)
+        if (b->p) any = b;
+    if (!any) return;
+    int dev = 0;
+    cudaPointerAttributes at = {};
+    cudaGetDevice(&dev);
+    if (cudaPointerGetAttributes(&at, any->p) != cudaSuccess) {
+        cudaGetLastError();
+        at.device = dev;
+    }
+    if (at.device != dev) cudaSetDevice(at.device);
+    const bool idle = wait_device();
+    if (at.device != dev) cudaSetDevice(dev);
+    for (DevBuf* b : bufs) b->release(idle);
+}
+
 }  // namespace mafb

@@ -51,6 +51,9 @@ struct DevBuf {
     template <typename T> T* as() const { return static_cast<T*>(p); }
 };
 
+// Releases the buffers of one object (of one device) after a single wait for the device's work.
+void release_all(const std::vector<DevBuf*>& bufs);
+
 struct MeshDims {
     int nx = 0, ny = 0, nz = 0;
     double dx = 0, dy = 0, dz = 0;
@@ -69,6 +72,7 @@ class Twiddles {
     // sequence (fft_ct.cuh: entry (jm, r - 1) of the stage with NS, RAD is
     // W_L^(r jm L / (NS RAD))), for the compile-time transforms of length L
     const void* get_ct(int L, bool fp64, const int* radix, int nstages);
+    void append_buffers(std::vector<DevBuf*>& v) { for (auto& t : tables_) v.push_back(&t.second); }
   private:
     std::map<std::pair<int, int>, DevBuf> tables_;
 };
@@ -195,6 +199,9 @@ class Demag {
     // tensor; the z (or, for nz == 1, y) pass applies the discrete Poisson
     // operator instead of the tensor product.
     Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host = nullptr, bool pbc = false);
+    ~Demag();
+    Demag(const Demag&) = delete;
+    Demag& operator=(const Demag&) = delete;
     const MeshDims& mesh() const { return md_; }
     bool pbc() const { return pbc_; }
     int Px() const { return pbc_ ? md_.nx : 2 * md_.nx; }

@@ -539,6 +539,12 @@ Demag::Demag(const MeshDims& md, cudaStream_t st, const double* tensor_host, boo
     }
 }
 
+Demag::~Demag() {
+    std::vector<DevBuf*> v = {&Nred64_, &Nred32_, &Npad64_, &Npad32_, &S1_64_, &S2_64_, &S1_32_, &S2_32_};
+    tw_.append_buffers(v);
+    release_all(v);
+}
+
 // Real spectra (times scale) on the quadrant [Lz/2+1][Ly/2+1][Lx/2+1] (Lz = 1: one
 // plane) of the periodic functions of lengths (Lx, Ly, Lz) that the octants `oct`
 // [o2][o1][o0] of nc tensor components complete by parity (oct and quad: one component
