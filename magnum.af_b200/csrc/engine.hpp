@@ -74,7 +74,11 @@ class Twiddles {
     const void* get_ct(int L, bool fp64, const int* radix, int nstages);
     void append_buffers(std::vector<DevBuf*>& v) { for (auto& t : tables_) v.push_back(&t.second); }
   private:
+    // the table of get() on the host: double2 or float2 [L]
+    const std::vector<unsigned char>& host(int L, bool fp64);
+    const void* upload(std::pair<int, int> key, const std::vector<unsigned char>& tab);
     std::map<std::pair<int, int>, DevBuf> tables_;
+    std::map<std::pair<int, int>, std::vector<unsigned char>> host_;
 };
 
 FFTPlan make_fft_plan(int L, const void* tw);  // throws MAF_ERR_UNSUPPORTED for primes > 13

@@ -34,22 +34,13 @@ namespace mafb {
 // ---------------------------------------------------------------------------
 // twiddles and plans
 // ---------------------------------------------------------------------------
-// A copy that is complete on return.  cudaMemcpy from pageable memory returns when a small
-// buffer has been staged, before the device holds it, and orders the legacy stream only, which
-// the library's non-blocking streams do not wait for: a pass could read a new table too early.
-static void copy_now(void* dst, const void* src, size_t n, cudaMemcpyKind kind) {
-    MAF_CUDA(cudaMemcpyAsync(dst, src, n, kind, cudaStreamPerThread));
-    MAF_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
-}
-
-const void* Twiddles::get(int L, bool fp64) {
-    auto key = std::make_pair(L, fp64 ? 1 : 0);
-    auto it = tables_.find(key);
-    if (it != tables_.end()) return it->second.p;
+const std::vector<unsigned char>& Twiddles::host(int L, bool fp64) {
+    std::vector<unsigned char>& tab = host_[std::make_pair(L, fp64 ? 1 : 0)];
+    if (!tab.empty()) return tab;
     // W_L^k = exp(-2 pi i k / L) in long double, reduced to the first octant
     // so that the table is symmetric to the last bit.
-    std::vector<long double> c(L), s(L);
     const long double pi = 3.141592653589793238462643383279502884L;
+    std::vector<unsigned char> t((fp64 ? sizeof(double2) : sizeof(float2)) * (size_t)L);
     for (int k = 0; k < L; ++k) {
         // angle = 2 pi k / L; use k/L in [0,1)
         long double a = 2.0L * pi * (long double)k / (long double)L;
@@ -61,24 +52,28 @@ const void* Twiddles::get(int L, bool fp64) {
         else if (k4 == 2 * (int64_t)L) { cv = -1; sv = 0; }
         else if (k4 == 3 * (int64_t)L) { cv = 0; sv = -1; }
         else { cv = cosl(a); sv = sinl(a); }
-        c[k] = cv;
-        s[k] = -sv;  // exp(-i a)
+        sv = -sv;  // exp(-i a)
+        if (fp64) reinterpret_cast<double2*>(t.data())[k] = make_double2((double)cv, (double)sv);
+        else reinterpret_cast<float2*>(t.data())[k] = make_float2((float)cv, (float)sv);
     }
-    DevBuf buf;
-    if (fp64) {
-        std::vector<double2> h(L);
-        for (int k = 0; k < L; ++k) h[k] = make_double2((double)c[k], (double)s[k]);
-        buf.alloc(sizeof(double2) * L);
-        copy_now(buf.p, h.data(), sizeof(double2) * L, cudaMemcpyHostToDevice);
-    } else {
-        std::vector<float2> h(L);
-        for (int k = 0; k < L; ++k) h[k] = make_float2((float)c[k], (float)s[k]);
-        buf.alloc(sizeof(float2) * L);
-        copy_now(buf.p, h.data(), sizeof(float2) * L, cudaMemcpyHostToDevice);
-    }
-    const void* p = buf.p;
-    tables_.emplace(key, std::move(buf));
-    return p;
+    tab = std::move(t);
+    return tab;
+}
+
+// The upload is complete on return.  cudaMemcpy from pageable memory returns when a small
+// buffer has been staged, before the device holds it, and orders the legacy stream only, which
+// the library's non-blocking streams do not wait for: a pass could read a new table too early.
+const void* Twiddles::upload(std::pair<int, int> key, const std::vector<unsigned char>& tab) {
+    DevBuf buf(tab.size());
+    MAF_CUDA(cudaMemcpyAsync(buf.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, cudaStreamPerThread));
+    MAF_CUDA(cudaStreamSynchronize(cudaStreamPerThread));
+    return tables_.emplace(key, std::move(buf)).first->second.p;
+}
+
+const void* Twiddles::get(int L, bool fp64) {
+    auto key = std::make_pair(L, fp64 ? 1 : 0);
+    auto it = tables_.find(key);
+    return it != tables_.end() ? it->second.p : upload(key, host(L, fp64));
 }
 
 const void* Twiddles::get_ct(int L, bool fp64, const int* radix, int nstages) {
@@ -88,10 +83,8 @@ const void* Twiddles::get_ct(int L, bool fp64, const int* radix, int nstages) {
     auto key = std::make_pair(L, 2 + (fp64 ? 1 : 0) + 2 * code);
     auto it = tables_.find(key);
     if (it != tables_.end()) return it->second.p;
-    const void* base = get(L, fp64);
     const size_t esz = fp64 ? sizeof(double2) : sizeof(float2);
-    std::vector<unsigned char> tab((size_t)L * esz);
-    copy_now(tab.data(), base, (size_t)L * esz, cudaMemcpyDeviceToHost);
+    const std::vector<unsigned char>& tab = host(L, fp64);
     std::vector<unsigned char> out(tab);
     int NS = 1;
     for (int st = 0; st < nstages; ++st) {
@@ -106,11 +99,7 @@ const void* Twiddles::get_ct(int L, bool fp64, const int* radix, int nstages) {
         }
         NS *= RAD;
     }
-    DevBuf buf(out.size());
-    copy_now(buf.p, out.data(), out.size(), cudaMemcpyHostToDevice);
-    const void* p = buf.p;
-    tables_.emplace(key, std::move(buf));
-    return p;
+    return upload(key, out);
 }
 
 FFTPlan make_fft_plan(int L, const void* tw) {
