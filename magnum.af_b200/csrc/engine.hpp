@@ -234,7 +234,7 @@ class Demag {
     Twiddles& twiddle_tables() { return tw_; }
 
   private:
-    template <typename R> const R* tensor() ;
+    template <typename R> const R* tensor(cudaStream_t st);
     template <typename R> cplx_t<R>* S1(int pitch);
     template <typename R> cplx_t<R>* S2(int Py, int pitch);
     void build_tensor(cudaStream_t st);

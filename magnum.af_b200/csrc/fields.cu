@@ -679,15 +679,16 @@ void Demag::download_real_tensor(double* host, bool symmetric, cudaStream_t st) 
     MAF_CUDA(cudaStreamSynchronize(st));
 }
 
-template <> const double* Demag::tensor<double>() { return Nred64_.as<double>(); }
-template <> const float* Demag::tensor<float>() {
+template <> const double* Demag::tensor<double>(cudaStream_t) { return Nred64_.as<double>(); }
+template <> const float* Demag::tensor<float>(cudaStream_t st) {
     if (!Nred32_.p) {
         const int64_t n = (int64_t)tensor_elems();
-        Nred32_.alloc(sizeof(float) * n);
-        k_d2f<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16), 256>>>(Nred64_.as<double>(),
-                                                                                   Nred32_.as<float>(), n);
+        DevBuf t(sizeof(float) * n);
+        k_d2f<<<(unsigned)std::min<int64_t>(ceil_div(n, 256), (int64_t)sm_count() * 16), 256, 0, st>>>(
+            Nred64_.as<double>(), t.as<float>(), n);
         MAF_LAUNCH_CHECK();
-        MAF_CUDA(cudaDeviceSynchronize());
+        MAF_CUDA(cudaStreamSynchronize(st));  // other streams may use it next
+        Nred32_ = std::move(t);
     }
     return Nred32_.as<float>();
 }
@@ -748,7 +749,7 @@ template <typename R> DemagPlan<R> Demag::plan(cudaStream_t st) {
     p.s1 = S1<R>(pitch_);
     p.s2 = md_.nz > 1 ? S2<R>(Py(), pitch_) : nullptr;
     // the periodic form has no tensor and runs the run-time plans only
-    p.tensor = pbc_ ? nullptr : tensor<R>();
+    p.tensor = pbc_ ? nullptr : tensor<R>(st);
     return p;
 }
 

@@ -25,32 +25,52 @@ def _stepped(shape, seed=1, stream=None):
     return llg, st
 
 
-def test_buffers_dropped_while_another_thread_captures():
+def _capture_while(meanwhile):
+    """A graph captured in thread-local mode while another thread runs `meanwhile`, and replayed."""
     x = torch.ones(1000, device="cuda")
-    graphs, s = [], torch.cuda.Stream()
+    g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    raised = []
 
-    def capture(meanwhile):
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
-            y = x + 1
-            t = threading.Thread(target=meanwhile)
-            t.start()
-            t.join()
-            y = 2 * y
-        g.replay()
-        torch.cuda.synchronize()
-        assert torch.all(y == 4)
-        graphs.append((g, y))
+    def run():
+        try:
+            meanwhile()
+        except M.MafError as e:
+            raised.append(e)
 
-    capture(lambda: None)  # what the first capture of a process allocates is not counted
+    with torch.cuda.graph(g, stream=s, capture_error_mode="thread_local"):
+        y = x + 1
+        t = threading.Thread(target=run)
+        t.start()
+        t.join()
+        y = 2 * y
+    assert not raised
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.all(y == 4)
+    return g, y
+
+
+def test_buffers_dropped_while_another_thread_captures():
+    graphs = [_capture_while(lambda: None)]  # what the first capture of a process allocates is not counted
     made = [_stepped((512, 512, 2)) for _ in range(6)]  # 100 MB of pool memory each
     torch.cuda.synchronize()
     free0 = torch.cuda.mem_get_info()[0]
-    capture(made.clear)
+    graphs.append(_capture_while(made.clear))
     _stepped((8, 8, 1))  # an object made and dropped afterwards gives back what was pending
     M.trim_memory()
     # all of the 6 x 126 MB came back (but for torch's graph memory)
     assert torch.cuda.mem_get_info()[0] - free0 >= (6 * 126 - 64) * MB
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32_field"])
+@pytest.mark.parametrize("shape", [(64, 64, 1), (100, 25, 1)])
+def test_first_evaluation_while_another_thread_captures(shape, prec):
+    """A new mesh's tensor, tables and FP32 copies are made without waiting for the whole device."""
+    mesh, m = M.Mesh(*shape, 3e-9, 3e-9, 3e-9), random_m(shape, 4)
+    want = M.DemagField(mesh).H_in_Apm(M.State(mesh, 8e5, m, precision=prec))
+    got = []
+    _capture_while(lambda: got.append(M.DemagField(mesh).H_in_Apm(M.State(mesh, 8e5, m, precision=prec))))
+    assert np.array_equal(got[0], want)
 
 
 def test_pool_gives_its_memory_to_a_large_buffer():
